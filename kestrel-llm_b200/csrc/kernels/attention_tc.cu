@@ -123,7 +123,18 @@ enum {
 };
 #define AT_RESCALE_STEP 8.0f            // log2 units by which a row's maximum may outgrow its reference
 
-template <bool MAPS>
+// What the softmax threads do to the scores is a fact of the instance: with all kinds in one kernel the plain softmax carried
+// every option's registers and code, spilled (172 bytes stored, 236 loaded a thread) and took 109 us where it now takes
+// 63 (2,048 tokens, 32 / 8 heads; 242 -> 50 for 16 / 4 heads with the extra term).
+enum {
+    AT_PLAIN = 0,               // softmax of the scaled scores; the extra term in its denominator only closes the row
+    AT_CAP = 1,                 // capped scores
+    AT_CAP_DIST_SIGMOID = 2,    // capped scores with a distance term, sigmoid weights
+    AT_REL = 3,                 // a table of distance terms
+    AT_ANY = 4                  // any other combination, decided at run time
+};
+
+template <bool MAPS, int KIND>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                     const AttnParams p, int cache_pages, int rows_per_tile) {
@@ -334,10 +345,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         const uint32_t lane_base = ((uint32_t)(32 * (warp & 3))) << 16;
         const uint32_t s_addr = tmem + lane_base + x * 128, o_addr = tmem + lane_base + 256 + x * 128;
         float m_ref = -INFINITY, l_run = 0.f;       // the reference the output is accumulated against, and the row's sum
-        const bool sigmoid = p.scored && p.opts.weighting == KESTREL_WEIGH_SIGMOID, sink = p.scored && p.opts.weighting == KESTREL_WEIGH_SOFTMAX_SINK;
-        const ScoreOpts no_opts = {0.f, nullptr, nullptr, nullptr, 0};
-        const HeadScore hs(p.scored ? p.opts : no_opts, kvh * G + (tile_row + (row_ok ? r : 0)) % G);
-        const float eff_scale = p.scored ? 1.f : p.scale_log2;   // transformed scores are in base-2 units already
+        const bool sigmoid = KIND == AT_CAP_DIST_SIGMOID || (KIND == AT_ANY && p.opts.weighting == KESTREL_WEIGH_SIGMOID);
+        const bool sink = KIND != AT_REL && KIND != AT_CAP_DIST_SIGMOID && p.opts.weighting == KESTREL_WEIGH_SOFTMAX_SINK;
+        const HeadScore hs(p.opts, kvh * G + (tile_row + (row_ok ? r : 0)) % G);
+        const float eff_scale = KIND == AT_PLAIN ? p.scale_log2 : 1.f;   // transformed scores are in base-2 units already
         bool ok = true;             // after a wait gave up the loop runs on without waiting, so that the warps still meet
 
         for (int t = 0; t < n_tiles_x; ++t) {
@@ -351,19 +362,19 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
 #pragma unroll
                 for (int c = 0; c < 128; c += 32) at_ld32(s_addr + c, sr + c);
                 at_ld_wait();
-                if (p.scored) {
+                if (KIND != AT_PLAIN) {
                     // the layer's options on the raw scores, before the mask (a key that may not be seen is overwritten
-                    // below, whatever its transformed score); the two layer kinds in use as loops of their own
+                    // below, whatever its transformed score)
                     const int d0 = my_pos - kbase;
-                    if (hs.cap > 0.f && !hs.dist && !sigmoid) {
+                    if (KIND == AT_CAP) {
 #pragma unroll
                         for (int j = 0; j < 128; ++j) sr[j] = __float_as_uint(hs.fast_as<true, false, false>(__uint_as_float(sr[j]) * p.scale, 0));
-                    } else if (hs.cap > 0.f && hs.dist && sigmoid) {
+                    } else if (KIND == AT_CAP_DIST_SIGMOID) {
 #pragma unroll
                         for (int j = 0; j < 128; ++j) sr[j] = __float_as_uint(hs.fast_as<true, true, true>(__uint_as_float(sr[j]) * p.scale, max(d0 - j, 0)));
-                    } else if (hs.rel && hs.cap == 0.f && !hs.dist && !sigmoid && !sink) {
-                        // a table of distance terms alone: one term for the whole tile where all of its keys lie beyond the table's
-                        // last distance, a look-up per score otherwise
+                    } else if (KIND == AT_REL) {
+                        // one term for the whole tile where all of its keys lie beyond the table's last distance, a look-up per
+                        // score otherwise
                         constexpr float LOG2E = 1.4426950408889634f;
                         const float s2 = p.scale * LOG2E;
                         if (d0 - 127 >= hs.rel_far) {
@@ -584,6 +595,20 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     }
 }
 
+template <bool MAPS, int KIND>
+static int at_launch(dim3 grid, cudaStream_t stream, const CUtensorMap &map_k, const CUtensorMap &map_v, const AttnParams &p, int cache_pages,
+                     int rows_per_tile) {
+    const size_t smem = 12 * AT_PANEL + 8 * B_COUNT + 16 + 1024;
+    static bool attr_set = false;
+    if (!attr_set) {
+        cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel<MAPS, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return kestrel_fail(-3, "attention_tc: cannot raise the shared-memory limit: %s", cudaGetErrorString(e));
+        attr_set = true;
+    }
+    kestrel_launch(attention_tc_kernel<MAPS, KIND>, grid, dim3(AT_THREADS), smem, stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    return 0;
+}
+
 // Whether the kernel takes this head size and page size.
 KESTREL_API int kestrel_attention_tc_supported(int hd, int page_size) {
     return hd == AT_HD && page_size > 0 && page_size % 8 == 0 && (AT_BN % page_size == 0 || page_size % AT_BN == 0);
@@ -661,14 +686,14 @@ KESTREL_API int kestrel_attention_tc_biased(const void *q, const void *k_cache, 
     p.scale = scale;
     p.opts = {softcap, r1, r2, head_bias, weighting, sink, rel, rel_bucket, rel_far, nq};
     p.scored = scored ? 1 : 0;
-    size_t smem = 12 * AT_PANEL + 8 * B_COUNT + 16 + 1024;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return kestrel_fail(-3, "attention_tc: cannot raise the shared-memory limit: %s", cudaGetErrorString(e));
-        attr_set = true;
-    }
-    kestrel_launch(attention_tc_kernel<false>, dim3((unsigned)((long long)tiles * nkv), 1, slices), dim3(AT_THREADS), smem, stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    const bool capped = softcap > 0.f, dist = r1 != nullptr, sigmoid = weighting == KESTREL_WEIGH_SIGMOID;
+    const dim3 grid((unsigned)((long long)tiles * nkv), 1, slices);
+    if (!capped && !dist && !rel && !sigmoid) rc = at_launch<false, AT_PLAIN>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    else if (capped && !dist && !rel && !sigmoid) rc = at_launch<false, AT_CAP>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    else if (capped && dist && !rel && sigmoid) rc = at_launch<false, AT_CAP_DIST_SIGMOID>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    else if (rel && !capped && !dist && weighting == KESTREL_WEIGH_SOFTMAX) rc = at_launch<false, AT_REL>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    else rc = at_launch<false, AT_ANY>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    if (rc) return rc;
     rc = kestrel_check_launch("attention_tc");
     if (rc || slices == 1) return rc;
     return kestrel_attention_merge(part_o, part_ml, out, tile_seq, tile_row0, tiles, rows_per_tile, cu_seqlens, slices, hd, nq, nkv,
@@ -708,14 +733,8 @@ KESTREL_API int kestrel_attention_tc_maps(const void *q, const void *k_cache, co
     p.scale_log2 = scale * 1.4426950408889634f;
     p.scale = scale;
     p.maps = {lq1, lk1, lq2, lk2, dim, diff, eps};
-    const size_t smem = 12 * AT_PANEL + 8 * B_COUNT + 16 + 1024;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return kestrel_fail(-3, "attention_tc_maps: cannot raise the shared-memory limit: %s", cudaGetErrorString(e));
-        attr_set = true;
-    }
-    kestrel_launch(attention_tc_kernel<true>, dim3((unsigned)((long long)tiles * nkv), 1, slices), dim3(AT_THREADS), smem, stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    rc = at_launch<true, AT_PLAIN>(dim3((unsigned)((long long)tiles * nkv), 1, slices), stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    if (rc) return rc;
     rc = kestrel_check_launch("attention_tc_maps");
     if (rc || slices == 1) return rc;
     return kestrel_differential_merge(part_o, part_ml, slices, AT_HD, lq1, lk1, lq2, lk2, dim, diff, eps, out, T, nq, vd, stream);
