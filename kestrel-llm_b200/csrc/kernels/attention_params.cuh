@@ -28,6 +28,9 @@ struct AttnParams {
     int partial_only;               // attention_decode.cu: the unnormalised outputs go to part_o / part_ml even from one slice
     float cap_in, cap_out;          // attention_decode.cu: a bound on the scores, in base-2 units (cap_out 0: none)
     int slices_from_window;         // attention_decode.cu: slices count from the first key tile the window touches
+    // a window that keeps a request's first tokens, and a factor per (token, head) on the outputs (or null); attention_tc.cu's kept form only
+    int keep_first;
+    const float *gate;
     // two maps a head over the same values (differential attention); read by attention_tc.cu only
     DifferentialOpts maps;
 };

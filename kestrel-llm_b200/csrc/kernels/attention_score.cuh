@@ -60,11 +60,15 @@ struct HeadScore {
     // anyway): tanh(x) = 1 - 2 / (1 + e^2x) from one ex2 and one rcp - an absolute error of a few 2^-23,
     // so of cap * 1e-6 in the score, also where x is small - and the logarithm from lg2.
     __device__ __forceinline__ float fast(float s, int distance) const {
-        if (cap > 0.f) s = fmaf(-2.0f * cap, score_rcp(1.0f + score_exp2(s * (inv_cap * 2.8853900817779268f))), cap);
-        if (dist) s -= r1 * __logf(fmaf(r2, (float)distance, 1.0f));
+        if (cap > 0.f) s = fast_cap(s);
+        if (dist) s = fast_dist(s, distance);
         if (rel) s += rel_of(distance);
         return s + bias;
     }
+    __device__ __forceinline__ float fast_cap(float s) const {
+        return fmaf(-2.0f * cap, score_rcp(1.0f + score_exp2(s * (inv_cap * 2.8853900817779268f))), cap);
+    }
+    __device__ __forceinline__ float fast_dist(float s, int distance) const { return s - r1 * __logf(fmaf(r2, (float)distance, 1.0f)); }
     // The same with the layer's options as compile-time facts, for loops over many scores: nothing of an option that
     // is off is issued.  Returns the score in base-2 units (times log2 e) unless SIGMOID, which returns the weight.
     template <bool CAP, bool DIST, bool SIGMOID>

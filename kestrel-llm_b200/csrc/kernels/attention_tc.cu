@@ -123,15 +123,16 @@ enum {
 };
 #define AT_RESCALE_STEP 8.0f            // log2 units by which a row's maximum may outgrow its reference
 
-// What the softmax threads do to the scores is a fact of the instance: with all kinds in one kernel the plain softmax carried
-// every option's registers and code, spilled (172 bytes stored, 236 loaded a thread) and took 109 us where it now takes
-// 63 (2,048 tokens, 32 / 8 heads; 242 -> 50 for 16 / 4 heads with the extra term).
+// What the softmax threads do to the scores is a fact of the instance: with all kinds in one kernel the plain softmax carried every
+// option's registers and took 109 us where it now takes 63 (2,048 tokens, 32 / 8 heads), and a kind without a loop of its own went
+// through branches around every score: 242 us for 16 / 4 heads with the extra term, now 50.
 enum {
     AT_PLAIN = 0,               // softmax of the scaled scores; the extra term in its denominator only closes the row
     AT_CAP = 1,                 // capped scores
     AT_CAP_DIST_SIGMOID = 2,    // capped scores with a distance term, sigmoid weights
     AT_REL = 3,                 // a table of distance terms
-    AT_ANY = 4                  // any other combination, decided at run time
+    AT_ANY = 4,                 // any other combination, decided at run time
+    AT_KEPT = 5                 // AT_PLAIN over a window that keeps a request's first tokens, the heads' outputs gated
 };
 
 template <bool MAPS, int KIND>
@@ -189,12 +190,16 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     const int k_hi = min(pos_begin + last_tok + 1, (slice + 1) * slice_len);
     const int k_first = max(p.window > 0 ? max(0, pos_begin + first_tok - p.window + 1) : 0, slice * slice_len);
     const int k_lo = (k_first / AT_BN) * AT_BN;
-    const int n_tiles = k_hi > k_lo ? (k_hi - k_lo + AT_BN - 1) / AT_BN : 0;
+    // kept first tokens [0, keep): their key tiles come in front of the window's, those the window begins in are its own
+    const int keep = KIND == AT_KEPT ? p.keep_first : 0;
+    const int n_kept = KIND == AT_KEPT ? min((keep + AT_BN - 1) / AT_BN, k_lo / AT_BN) : 0;
+    const int n_tiles = n_kept + (k_hi > k_lo ? (k_hi - k_lo + AT_BN - 1) / AT_BN : 0);
+    auto key_base = [&](int t) { return KIND == AT_KEPT && t < n_kept ? t * AT_BN : k_lo + (t - n_kept) * AT_BN; };
     // row tile A ends earlier: it skips the key tiles beyond its last row
     const int rows_a = min(rows_here, AT_BM);
     const bool has_b = MAPS || rows_here > AT_BM;
     const int k_hi_a = MAPS ? k_hi : min(pos_begin + (row0 + rows_a - 1) / G + 1, (slice + 1) * slice_len);
-    const int n_tiles_a = MAPS ? n_tiles : has_b ? (k_hi_a > k_lo ? (k_hi_a - k_lo + AT_BN - 1) / AT_BN : 0) : n_tiles;
+    const int n_tiles_a = MAPS ? n_tiles : has_b ? n_kept + (k_hi_a > k_lo ? (k_hi_a - k_lo + AT_BN - 1) / AT_BN : 0) : n_tiles;
 
     if (warp == 8 || warp == 10) {
         // ------------------------------------------------------------------ loaders
@@ -211,7 +216,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
             const uint32_t par = (uint32_t)(t >> 1) & 1u;
             int row = 0;
             if (lane < boxes) {
-                int s0 = k_lo + t * AT_BN + lane * box_rows;
+                int s0 = key_base(t) + lane * box_rows;
                 int idx = s0 / p.page_size;
                 int page = idx < p.table_width ? table[idx] : 0;
                 if (page < 0 || page >= cache_pages) page = 0;      // a released or absent page: its keys are masked, its values zeroed
@@ -348,12 +353,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         const bool sigmoid = KIND == AT_CAP_DIST_SIGMOID || (KIND == AT_ANY && p.opts.weighting == KESTREL_WEIGH_SIGMOID);
         const bool sink = KIND != AT_REL && KIND != AT_CAP_DIST_SIGMOID && p.opts.weighting == KESTREL_WEIGH_SOFTMAX_SINK;
         const HeadScore hs(p.opts, kvh * G + (tile_row + (row_ok ? r : 0)) % G);
-        const float eff_scale = KIND == AT_PLAIN ? p.scale_log2 : 1.f;   // transformed scores are in base-2 units already
+        constexpr bool RAW = KIND == AT_PLAIN || KIND == AT_KEPT;        // no options on the scores
+        const float eff_scale = RAW ? p.scale_log2 : 1.f;                // transformed scores are in base-2 units already
         bool ok = true;             // after a wait gave up the loop runs on without waiting, so that the warps still meet
 
         for (int t = 0; t < n_tiles_x; ++t) {
             const int b = t & 1;
-            const int kbase = k_lo + t * AT_BN;
+            const int kbase = key_base(t);
             // S_X(t) is done - and with it, in the issuer's order, O_X += P_X(t-1) V(t-1)
             if (ok && !mbar_wait(bar(B_S_FULL + x), (uint32_t)t & 1u)) { atomicExch(&g_at_error, 7); ok = false; }
             tc_fence_after();
@@ -362,7 +368,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
 #pragma unroll
                 for (int c = 0; c < 128; c += 32) at_ld32(s_addr + c, sr + c);
                 at_ld_wait();
-                if (KIND != AT_PLAIN) {
+                if (!RAW) {
                     // the layer's options on the raw scores, before the mask (a key that may not be seen is overwritten
                     // below, whatever its transformed score)
                     const int d0 = my_pos - kbase;
@@ -386,14 +392,33 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                             for (int j = 0; j < 128; ++j) sr[j] = __float_as_uint(fmaf(__uint_as_float(sr[j]), s2, hs.rel_of(max(d0 - j, 0)) * LOG2E));
                         }
                     } else {
+                        // the options one after the other over all scores (hs.fast with its branches around every score cost 22,000
+                        // cycles a tile)
 #pragma unroll
-                        for (int j = 0; j < 128; ++j) {
-                            const float z = hs.fast(__uint_as_float(sr[j]) * p.scale, max(d0 - j, 0));
-                            sr[j] = __float_as_uint(sigmoid ? sigmoid_fast(z) : z * 1.4426950408889634f);
+                        for (int j = 0; j < 128; ++j) sr[j] = __float_as_uint(__uint_as_float(sr[j]) * p.scale);
+                        if (hs.cap > 0.f) {
+#pragma unroll
+                            for (int j = 0; j < 128; ++j) sr[j] = __float_as_uint(hs.fast_cap(__uint_as_float(sr[j])));
+                        }
+                        if (hs.dist) {
+#pragma unroll
+                            for (int j = 0; j < 128; ++j) sr[j] = __float_as_uint(hs.fast_dist(__uint_as_float(sr[j]), max(d0 - j, 0)));
+                        }
+                        if (hs.rel) {
+#pragma unroll
+                            for (int j = 0; j < 128; ++j) sr[j] = __float_as_uint(__uint_as_float(sr[j]) + hs.rel_of(max(d0 - j, 0)));
+                        }
+                        if (sigmoid) {
+#pragma unroll
+                            for (int j = 0; j < 128; ++j) sr[j] = __float_as_uint(sigmoid_fast(__uint_as_float(sr[j]) + hs.bias));
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 128; ++j) sr[j] = __float_as_uint(__uint_as_float(sr[j]) * 1.4426950408889634f);
                         }
                     }
                 }
-                const bool whole = kbase >= k_first && kbase + AT_BN <= k_hi_x && kbase + AT_BN - 1 <= my_pos && kbase >= my_lo;
+                const bool whole = (kbase >= k_first && kbase + AT_BN <= k_hi_x && kbase + AT_BN - 1 <= my_pos && kbase >= my_lo) ||
+                                   (KIND == AT_KEPT && kbase + AT_BN <= keep && kbase + AT_BN - 1 <= my_pos);
                 if (!__all_sync(0xffffffffu, whole)) {
                     // keys this row may not see count as minus infinity: no maximum, a weight of zero (sigmoid weights: zero itself)
                     const uint32_t hidden = sigmoid ? 0u : 0xff800000u;
@@ -401,6 +426,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                     for (int j = 0; j < 128; ++j) {
                         int key = kbase + j;
                         bool vis = key <= my_pos && key >= my_lo && key < k_hi_x && key >= k_first;
+                        if (KIND == AT_KEPT) vis |= key < keep && key <= my_pos;
                         if (!vis) sr[j] = hidden;
                     }
                 }
@@ -478,14 +504,14 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                 }
             p_written:;
             }
-            if (kbase < k_first || kbase + AT_BN > k_hi) {
+            if ((kbase < k_first && min(kbase + AT_BN, k_first) > keep) || kbase + AT_BN > k_hi) {
                 // V rows of keys outside the CTA's range become zero before this row tile's product
                 // reads them (both row tiles write the same zeros: either may be the only one at a tile)
                 if (ok && !mbar_wait(bar(B_V_FULL + b), (uint32_t)(t >> 1) & 1u)) { atomicExch(&g_at_error, 8); ok = false; }
-                const int lo_rows = max(0, k_first - kbase), hi_row = min(AT_BN, k_hi - kbase);
+                const int lo_rows = max(0, k_first - kbase), hi_row = min(AT_BN, k_hi - kbase), kept_rows = keep - kbase;
                 for (int idx = r; idx < AT_BN * 16; idx += 128) {
                     int row = idx >> 4, c = idx & 15;
-                    if (row < lo_rows || row >= hi_row)
+                    if ((row < lo_rows && row >= kept_rows) || row >= hi_row)
                         *reinterpret_cast<uint4 *>(v_ptr + b * TILE_BYTES + (c >> 3) * AT_PANEL + row * 128 + (c & 7) * 16) = make_uint4(0, 0, 0, 0);
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // zeroed V rows -> tensor-core reads
@@ -546,6 +572,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
             if (MAPS) qrow = qrow * 2 + x;
             float inv = p.slices > 1 ? 1.f : 1.0f / l_run;
             if (sigmoid) inv = 1.f;
+            if (KIND == AT_KEPT && write && p.gate) inv *= p.gate[qrow];
             if (sink) inv = 1.0f / (l_run + at_exp2(hs.sink * 1.4426950408889634f - m_ref));     // one more term exp(sink), against the same reference
 #pragma unroll
             for (int c = 0; c < 128; c += 32) {
@@ -609,6 +636,31 @@ static int at_launch(dim3 grid, cudaStream_t stream, const CUtensorMap &map_k, c
     return 0;
 }
 
+// The checks that the entry points share, the tensor maps, and the parameters of a launch over one slice of keys
+static int at_fill(AttnParams *p, CUtensorMap *map_k, CUtensorMap *map_v, const void *q, const void *k_cache, const void *v_cache, void *out,
+                   const int *tile_seq, const int *tile_row0, int tiles, int rows_per_tile, const int *cu_seqlens, const int *kv_lens,
+                   const int *block_table, int table_width, int table_stride, int page_size, int cache_pages, int nq, int nkv, int hd, int window,
+                   float scale) {
+    KESTREL_REQUIRE(hd == AT_HD, "attention_tc: head size %d; this kernel is built for %d", hd, AT_HD);
+    KESTREL_REQUIRE(rows_per_tile >= 1 && rows_per_tile <= 2 * AT_BM, "attention_tc: tiles of %d rows; a CTA takes up to %d", rows_per_tile, 2 * AT_BM);
+    KESTREL_REQUIRE(nq > 0 && nkv > 0 && nq % nkv == 0, "attention_tc: %d query heads over %d kv heads", nq, nkv);
+    KESTREL_REQUIRE((long long)tiles * nkv < (1ll << 31), "attention_tc: grid too large");
+    KESTREL_REQUIRE(kestrel_attention_tc_supported(hd, page_size), "attention_tc: pages of %d keys; the page size must be a multiple of 8 that divides 128 or is a multiple of it", page_size);
+    KESTREL_REQUIRE(cache_pages > 0 && (long long)cache_pages * nkv * page_size < (1ll << 31), "attention_tc: a cache of %d pages is beyond the 32-bit row coordinate", cache_pages);
+    const long long cache_rows = (long long)cache_pages * nkv * page_size;
+    int rc = kestrel_tensor_map_bf16(map_k, k_cache, cache_rows, AT_HD, AT_HD, page_size < AT_BN ? page_size : AT_BN);
+    if (rc == 0) rc = kestrel_tensor_map_bf16(map_v, v_cache, cache_rows, AT_HD, AT_HD, page_size < AT_BN ? page_size : AT_BN);
+    if (rc) return rc;
+    *p = AttnParams();
+    p->q = (const __nv_bfloat16 *)q; p->k_cache = (const __nv_bfloat16 *)k_cache; p->v_cache = (const __nv_bfloat16 *)v_cache;
+    p->out = (__nv_bfloat16 *)out; p->tile_seq = tile_seq; p->tile_row0 = tile_row0;
+    p->cu_seqlens = cu_seqlens; p->kv_lens = kv_lens; p->block_table = block_table; p->table_width = table_width; p->table_stride = table_stride;
+    p->page_size = page_size; p->nq = nq; p->nkv = nkv; p->hd = hd; p->window = window; p->slices = 1; p->slice_len = 1 << 30;
+    p->scale_log2 = scale * 1.4426950408889634f;
+    p->scale = scale;
+    return 0;
+}
+
 // Whether the kernel takes this head size and page size.
 KESTREL_API int kestrel_attention_tc_supported(int hd, int page_size) {
     return hd == AT_HD && page_size > 0 && page_size % 8 == 0 && (AT_BN % page_size == 0 || page_size % AT_BN == 0);
@@ -662,28 +714,15 @@ KESTREL_API int kestrel_attention_tc_biased(const void *q, const void *k_cache, 
     KESTREL_REQUIRE(weighting >= 0 && weighting <= 2 && softcap >= 0.f && (r1 == nullptr) == (r2 == nullptr), "attention_tc: bad score options");
     KESTREL_REQUIRE(!scored || slices == 1 || (weighting != KESTREL_WEIGH_SIGMOID && (weighting != KESTREL_WEIGH_SOFTMAX_SINK || sink)),
                     "attention_tc: sigmoid weights, and an extra term without its numbers, go with one slice of keys, not %d", slices);
-    KESTREL_REQUIRE(hd == AT_HD, "attention_tc: head size %d; this kernel is built for %d", hd, AT_HD);
-    KESTREL_REQUIRE(rows_per_tile >= 1 && rows_per_tile <= 2 * AT_BM, "attention_tc: tiles of %d rows; a CTA takes up to %d", rows_per_tile, 2 * AT_BM);
-    KESTREL_REQUIRE(nq > 0 && nkv > 0 && nq % nkv == 0, "attention_tc: %d query heads over %d kv heads", nq, nkv);
     KESTREL_REQUIRE(slices >= 1 && slice_len > 0 && slice_len % AT_BN == 0, "attention_tc: slice length %d must be a positive multiple of %d", slice_len, AT_BN);
     KESTREL_REQUIRE(slices == 1 || (part_o && part_ml), "attention_tc: %d slices without scratch", slices);
-    KESTREL_REQUIRE((long long)tiles * nkv < (1ll << 31) && slices <= 65535, "attention_tc: grid too large");
-    KESTREL_REQUIRE(kestrel_attention_tc_supported(hd, page_size), "attention_tc: pages of %d keys; the page size must be a multiple of 8 that divides 128 or is a multiple of it", page_size);
-    KESTREL_REQUIRE(cache_pages > 0 && (long long)cache_pages * nkv * page_size < (1ll << 31), "attention_tc: a cache of %d pages is beyond the 32-bit row coordinate", cache_pages);
+    KESTREL_REQUIRE(slices <= 65535, "attention_tc: grid too large");
+    AttnParams p;
     CUtensorMap map_k, map_v;
-    const long long cache_rows = (long long)cache_pages * nkv * page_size;
-    int rc = kestrel_tensor_map_bf16(&map_k, k_cache, cache_rows, AT_HD, AT_HD, page_size < AT_BN ? page_size : AT_BN);
+    int rc = at_fill(&p, &map_k, &map_v, q, k_cache, v_cache, out, tile_seq, tile_row0, tiles, rows_per_tile, cu_seqlens, kv_lens, block_table,
+                     table_width, table_stride, page_size, cache_pages, nq, nkv, hd, window, scale);
     if (rc) return rc;
-    rc = kestrel_tensor_map_bf16(&map_v, v_cache, cache_rows, AT_HD, AT_HD, page_size < AT_BN ? page_size : AT_BN);
-    if (rc) return rc;
-    AttnParams p = {};
-    p.q = (const __nv_bfloat16 *)q; p.k_cache = (const __nv_bfloat16 *)k_cache; p.v_cache = (const __nv_bfloat16 *)v_cache;
-    p.out = (__nv_bfloat16 *)out; p.part_o = part_o; p.part_ml = part_ml; p.tile_seq = tile_seq; p.tile_row0 = tile_row0;
-    p.cu_seqlens = cu_seqlens; p.kv_lens = kv_lens; p.block_table = block_table; p.table_width = table_width; p.table_stride = table_stride;
-    p.page_size = page_size; p.nq = nq; p.nkv = nkv; p.hd = hd; p.window = window; p.slices = slices; p.slice_len = slice_len;
-    p.max_kv_ptr = max_kv_ptr;
-    p.scale_log2 = scale * 1.4426950408889634f;
-    p.scale = scale;
+    p.part_o = part_o; p.part_ml = part_ml; p.slices = slices; p.slice_len = slice_len; p.max_kv_ptr = max_kv_ptr;
     p.opts = {softcap, r1, r2, head_bias, weighting, sink, rel, rel_bucket, rel_far, nq};
     p.scored = scored ? 1 : 0;
     const bool capped = softcap > 0.f, dist = r1 != nullptr, sigmoid = weighting == KESTREL_WEIGH_SIGMOID;
@@ -698,6 +737,25 @@ KESTREL_API int kestrel_attention_tc_biased(const void *q, const void *k_cache, 
     if (rc || slices == 1) return rc;
     return kestrel_attention_merge(part_o, part_ml, out, tile_seq, tile_row0, tiles, rows_per_tile, cu_seqlens, slices, hd, nq, nkv,
                                    scored && weighting == KESTREL_WEIGH_SOFTMAX_SINK ? sink : nullptr, stream);
+}
+
+// Softmax attention over a window that keeps a request's first `keep_first` tokens visible, each head's output times gate[token, head]
+// (float32 [T, nq], or null), in one slice of keys.  A window is needed for kept tokens; window 0 sees everything.
+KESTREL_API int kestrel_attention_tc_kept(const void *q, const void *k_cache, const void *v_cache, void *out, const int *tile_seq,
+                                          const int *tile_row0, int tiles, int rows_per_tile, const int *cu_seqlens, const int *kv_lens,
+                                          const int *block_table, int table_width, int table_stride, int page_size, int cache_pages, int T, int nq,
+                                          int nkv, int hd, int window, int keep_first, const float *gate, float scale, cudaStream_t stream) {
+    if (T == 0 || tiles == 0) return 0;
+    KESTREL_REQUIRE(window >= 0 && keep_first >= 0, "attention_tc_kept: window %d, %d kept tokens", window, keep_first);
+    AttnParams p;
+    CUtensorMap map_k, map_v;
+    int rc = at_fill(&p, &map_k, &map_v, q, k_cache, v_cache, out, tile_seq, tile_row0, tiles, rows_per_tile, cu_seqlens, kv_lens, block_table,
+                     table_width, table_stride, page_size, cache_pages, nq, nkv, hd, window, scale);
+    if (rc) return rc;
+    p.keep_first = window > 0 ? keep_first : 0;
+    p.gate = gate;
+    rc = at_launch<false, AT_KEPT>(dim3((unsigned)((long long)tiles * nkv)), stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    return rc ? rc : kestrel_check_launch("attention_tc_kept");
 }
 
 // Differential attention on the same kernel: q [T, nq, 2, 64] (the two maps' queries of a head), K pages of rows [k_1 | k_2] of 2 * 64

@@ -627,8 +627,9 @@ def attention_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
                  tile_seq: torch.Tensor, tile_row0: torch.Tensor, cu_seqlens: torch.Tensor, kv_lens: torch.Tensor,
                  block_table: torch.Tensor, page_size: int, nq: int, nkv: int, hd: int, window: int, scale: float,
                  slices: int = 1, slice_len: int = 1 << 30, max_kv_dev: Optional[torch.Tensor] = None,
-                 rows_per_tile: int = 128, score: Optional["ScoreOptions"] = None) -> None:
-    """tcgen05 attention of the listed tiles, head size 128 (with a layer's `ScoreOptions`; sigmoid weights in one slice): tiles of ``rows_per_tile`` rows, up
+                 rows_per_tile: int = 128, score: Optional["ScoreOptions"] = None, keep_first: int = 0, gate: Optional[torch.Tensor] = None) -> None:
+    """tcgen05 attention of the listed tiles, head size 128 (with a layer's `ScoreOptions`; sigmoid weights in one slice; or, plain softmax
+    in one slice, with ``keep_first`` tokens that stay visible to a windowed layer and a ``gate`` float32 [T, nq] on the heads' outputs): tiles of ``rows_per_tile`` rows, up
     to 256 (prompt portions; 16 for decode tokens); the key range may be cut into
     ``slices`` slices of ``slice_len`` keys (a multiple of 128) that are merged in ascending
     order; ``slices * slice_len`` must reach the longest request.  The cache tensors are
@@ -646,6 +647,18 @@ def attention_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
         raise KernelError("attention_tc: shapes differ")
     if tuple(k_cache.shape[1:]) != (nkv, page_size, hd) or v_cache.shape != k_cache.shape:
         raise KernelError(f"attention_tc: cache of shape {tuple(k_cache.shape)}, expected [pages, {nkv}, {page_size}, {hd}]")
+    if gate is not None or keep_first:
+        if slices != 1 or score is not None:
+            raise KernelError("attention_tc: kept tokens and a gate go with one slice of keys and plain softmax weights")
+        if gate is not None:
+            _need(gate, "attention_tc.gate", torch.float32, 2)
+            if tuple(gate.shape) != (T, nq):
+                raise KernelError(f"attention_tc: gate of shape {tuple(gate.shape)}, expected [{T}, {nq}]")
+        _check(library().kestrel_attention_tc_kept(
+            q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), tile_seq.data_ptr(), tile_row0.data_ptr(), tiles,
+            int(rows_per_tile), cu_seqlens.data_ptr(), kv_lens.data_ptr(), block_table.data_ptr(), block_table.shape[1], block_table.stride(0),
+            int(page_size), int(k_cache.shape[0]), T, nq, nkv, hd, int(window), int(keep_first), _p(gate), float(scale), _stream()))
+        return
     part_o = part_ml = None
     if slices > 1:
         part_o = torch.empty((T * nq, slices, hd), dtype=torch.float32, device=q.device)

@@ -37,9 +37,10 @@ projection of its own).
 
 Kernels: float32 and head sizes that are no multiples of 8 run on the plain kernel; bfloat16 on the
 ``mma.sync`` kernel of `ops.attention_window` (single-token steps share their keys out over CTAs),
-except steps with prompt portions of head size 128 without gate and kept tokens, which take the
-tcgen05 kernel (`ops.attention_tc`) with the same options; without a window it cuts a long key range
-into slices (softmax weights only) so that the request's last tile does not set the kernel's time.
+except steps with prompt portions of head size 128, which take the tcgen05 kernel (`ops.attention_tc`)
+with the same options (a gate per head and kept tokens beside plain softmax weights: 2,048 tokens of 16 / 4
+heads, window 1,024, 177 us on the ``mma.sync`` kernel, 45 on this one); without a window it cuts a long
+key range into slices (softmax weights only) so that the request's last tile does not set the kernel's time.
 """
 from __future__ import annotations
 
@@ -229,7 +230,8 @@ class GatedWindowAttention(Mixer):
         a = torch.empty((T, self.heads * self.v_head_dim), dtype=self.dtype, device=x.device)
         G = self.heads // self.kv_heads
         if self.dtype == torch.bfloat16 and not self.force_plain and self.tcgen05 and self.head_dim == self.v_head_dim == 128 and \
-                gate is None and self.keep_first == 0 and not batch.captured and batch.max_count * G > self.TC_MIN_ROWS and \
+                (gate is None and self.keep_first == 0 or not self._scored) and not batch.captured and \
+                batch.max_count * G > self.TC_MIN_ROWS and \
                 ops.attention_tc_supported(128, cache.page_size):
             # prompt portions of head size 128: the tcgen05 kernel, rows in tiles of 256 per request
             tile_seq, tile_row0 = ops.row_tiles(batch, G, 256)
@@ -239,14 +241,14 @@ class GatedWindowAttention(Mixer):
             # instead of 171 us: the slices' float32 outputs and their merge cost more than the even load gains).
             slices, slice_len = 1, 1 << 30
             fill = self.TC_SLICE_FILL // max(1, int(tile_seq.shape[0]) * self.kv_heads)
-            if self.window == 0 and self.score.weighting != "sigmoid" and fill >= 2 and batch.max_kv_len > 2 * self.TC_SLICE and \
+            if self.window == 0 and gate is None and self.score.weighting != "sigmoid" and fill >= 2 and batch.max_kv_len > 2 * self.TC_SLICE and \
                     (self.score.weighting != "softmax_sink" or self.score.sink is not None):
                 per = -(-batch.max_kv_len // min(32, fill))          # keys a slice if the chip is to be filled, in whole key tiles
                 slice_len = max(self.TC_SLICE, (per + 127) // 128 * 128)
                 slices = -(-batch.max_kv_len // slice_len)
             ops.attention_tc(q, cache.k, cache.v, a, tile_seq, tile_row0, batch.cu_seqlens, batch.kv_lens, table, cache.page_size, self.heads,
                              self.kv_heads, 128, self.window, self.scale, slices=slices,
-                             slice_len=slice_len, rows_per_tile=256, score=score)
+                             slice_len=slice_len, rows_per_tile=256, score=score, keep_first=self.keep_first, gate=gate)
         elif self.dtype == torch.bfloat16 and not self.force_plain and self.decode and self._capped_only and gate is None and \
                 self.head_dim == self.v_head_dim and self.keep_first == 0 and \
                 ops.attention_decode_capped(q, cache.k, cache.v, batch, table, cache.page_size, a, self.heads, self.kv_heads, self.head_dim, self.window,

@@ -147,6 +147,38 @@ def test_attention_on_tensor_cores_against_the_plain_kernel(H, G, d, dv, size, k
     assert np.abs(fast - slow).max() <= 2e-2 * np.abs(want).max()
 
 
+@pytest.mark.parametrize("H,G,size,keep,page,n,cuts", [
+    (4, 1, 100, 4, 16, 600, [600]),                      # the kept tokens' key tile apart from the window's
+    (4, 1, 100, 4, 16, 600, [17, 300, 283]),             # tiles that begin inside a tile of keys, one row tile and two
+    (2, 2, 300, 129, 32, 700, [700]),                    # kept tokens over two key tiles, the second of one key
+    (16, 1, 40, 256, 128, 500, [100, 400]),              # kept tokens to a tile's edge, window inside one tile
+    (3, 1, 128, 1, 8, 420, [420]), (8, 2, 1000, 5, 16, 300, [65, 235]),     # window of a tile; window longer than the request
+    (4, 2, None, 0, 16, 390, [390]), (4, 1, 60, 0, 64, 300, [150, 150])])   # a gate alone, without and with a window
+def test_attention_with_kept_tokens_on_tcgen05_against_the_plain_kernel(H, G, size, keep, page, n, cuts):
+    """bfloat16, heads of 128: portions on the tcgen05 kernel, against the plain statement and the plain kernel.  Both kernels
+    round P or their output to bfloat16 (2^-9 of a value): they agree to the same 2e-2 of the largest as the pair above."""
+    from kestrel_llm_b200.csrc import ops
+    from kestrel_llm_b200.parts import GatedWindowAttention
+    calls, real = [], ops.attention_tc
+
+    def seen(*a, **kw):
+        calls.append(kw.get("keep_first"))
+        return real(*a, **kw)
+    ops.attention_tc = seen
+    try:
+        fast, want, _ = _attention_case("bfloat16", H, G, 128, 128, 0.12, size, keep, page, n, cuts, seed=n)
+    finally:
+        ops.attention_tc = real
+    assert len(calls) == sum(1 for c in cuts if c * (H // G) > GatedWindowAttention.TC_MIN_ROWS)
+    _close(fast, want, "bfloat16", "tcgen05 attention with kept tokens and a gate")
+    GatedWindowAttention.force_plain = True
+    try:
+        slow, _, _ = _attention_case("bfloat16", H, G, 128, 128, 0.12, size, keep, page, n, cuts, seed=n)
+    finally:
+        GatedWindowAttention.force_plain = False
+    assert np.abs(fast - slow).max() <= 2e-2 * np.abs(want).max()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_attention_over_another_layers_pages(dtype):
     """A mixer without key and value projections attends over the pages another wrote, with its own mask and scale."""
