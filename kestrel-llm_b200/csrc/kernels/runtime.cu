@@ -56,6 +56,7 @@ KESTREL_API int kestrel_kernel_errors(void) {
     int bits = 0;
     if (kestrel_gemm_tc_error() != 0) bits |= 1;
     if (kestrel_attention_tc_error() != 0) bits |= 2;
+    if (kestrel_attention_rows_tc_error() != 0) bits |= 2;
     if (kestrel_attention_decode_error() != 0) bits |= 4;
     return bits;
 }

@@ -675,6 +675,52 @@ def attention_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
         launches += 1          # the merge kernel
 
 
+def attention_rows_tc_supported(hd: int, vd: int, page_size: int) -> bool:
+    """Whether the tcgen05 kernel over cache rows that are key and value takes these sizes."""
+    return bool(library().kestrel_attention_rows_tc_supported(int(hd), int(vd), int(page_size)))
+
+
+def attention_rows_tc(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, batch, block_table: torch.Tensor, page_size: int, nq: int, nkv: int,
+                      hd: int, vd: int, window: int, scale: float, gate: Optional[torch.Tensor] = None) -> None:
+    """tcgen05 attention of a step's prompt portions over cache rows [pages, nkv, page size, hd] that are key (whole) and value (their first
+    ``vd`` numbers), heads' outputs times ``gate`` (float32 [T, nq]) if given.  Few tiles far into a context without a window cut the
+    key range into slices, merged in ascending order (the gate is then a kernel of its own)."""
+    _need(q, "attention_rows_tc.q", torch.bfloat16, 2)
+    _need(out, "attention_rows_tc.out", torch.bfloat16, 2)
+    _need(cache, "attention_rows_tc.cache", torch.bfloat16, 4)
+    _need(block_table, "attention_rows_tc.block_table", torch.int32, 2)
+    T = q.shape[0]
+    if q.shape[1] != nq * hd or out.shape != (T, nq * vd) or T != batch.num_tokens or tuple(cache.shape[1:]) != (nkv, page_size, hd):
+        raise KernelError("attention_rows_tc: shapes differ")
+    if gate is not None:
+        _need(gate, "attention_rows_tc.gate", torch.float32, 2)
+        if tuple(gate.shape) != (T, nq):
+            raise KernelError(f"attention_rows_tc: gate of shape {tuple(gate.shape)}, expected [{T}, {nq}]")
+    tile_seq, tile_row0 = row_tiles(batch, nq // nkv, 128)
+    tiles = tile_seq.shape[0]
+    # A CTA walks its keys at some 1.5 us per 64.  Half of the SMs idle or more, and keys enough for two slices of 512: as many
+    # slices as fill the SMs once.
+    slices, slice_len = 1, (1 << 30) // 128 * 128
+    fill = library().kestrel_attention_tc_slots() // max(1, tiles * nkv)
+    if window == 0 and fill >= 2 and batch.max_kv_len > 1024:
+        per = -(-int(batch.max_kv_len) // min(32, fill))
+        slice_len = max(512, (per + 127) // 128 * 128)
+        slices = -(-int(batch.max_kv_len) // slice_len)
+    part_o = part_ml = None
+    if slices > 1:
+        part_o = torch.empty((T * nq, slices, vd), dtype=torch.float32, device=q.device)
+        part_ml = torch.empty((T * nq, slices, 2), dtype=torch.float32, device=q.device)
+    _check(library().kestrel_attention_rows_tc(
+        q.data_ptr(), cache.data_ptr(), out.data_ptr(), _p(part_o), _p(part_ml), tile_seq.data_ptr(), tile_row0.data_ptr(), tiles, 128,
+        batch.cu_seqlens.data_ptr(), batch.kv_lens.data_ptr(), block_table.data_ptr(), block_table.shape[1], block_table.stride(0), int(page_size),
+        int(cache.shape[0]), T, nq, nkv, hd, vd, int(window), slices, slice_len, _p(gate) if slices == 1 else None, float(scale), _stream()))
+    if slices > 1:
+        global launches
+        launches += 1          # the merge kernel
+        if gate is not None:
+            head_scale(out, gate, nq)
+
+
 def attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, out: torch.Tensor,
                      tile_seq: torch.Tensor, tile_row0: torch.Tensor, cu_seqlens: torch.Tensor, kv_lens: torch.Tensor,
                      block_table: torch.Tensor, page_size: int, nq: int, nkv: int, hd: int, window: int, scale: float,
@@ -737,6 +783,7 @@ def raise_on_kernel_error() -> None:
     lib = library()
     bad = [(name, code) for name, code in (("gemm_tcgen05", lib.kestrel_gemm_tc_error()),
                                            ("attention_tc", lib.kestrel_attention_tc_error()),
+                                           ("attention_rows_tc", lib.kestrel_attention_rows_tc_error()),
                                            ("attention_decode", lib.kestrel_attention_decode_error()),
                                            ("moe_tcgen05", lib.kestrel_moe_tc_error())) if code]
     if bad:

@@ -46,6 +46,8 @@ from .linear import Linear
 
 class LatentAttention(Mixer):
     force_plain = False        # tests: bfloat16 through the plain attention kernel too
+    tcgen05 = True             # tests: off, portions stay on the mma.sync kernel
+    TC_MIN_ROWS = 64           # a step whose longest portion has more rows (tokens x heads) takes the tcgen05 kernel
     expand_prompts = True      # tests: off, starting portions too run over the cached latents
     EXPAND_MIN_TOKENS = 64     # a step whose longest portion has more tokens may take the expanded form
     graph_safe = True          # forward launches kernels over device tensors of the batch only (the expanded form reads the
@@ -117,7 +119,12 @@ class LatentAttention(Mixer):
             q_lat = ops.head_gemm(q, self.up_k_w, H, w_kn=True)                # [T, H kv_rank]: Uk_n^T q_n
         # keys are whole cache rows, values their first kv_rank numbers: the V plane is the K plane with rows of D numbers
         a = torch.empty((T, H * R), dtype=self.dtype, device=x.device)
-        if self.dtype == torch.bfloat16 and not self.force_plain and ops.attention_window_supported(D, R, H, 1):
+        if self.dtype == torch.bfloat16 and not self.force_plain and self.tcgen05 and not batch.captured and \
+                batch.max_count * H > self.TC_MIN_ROWS and ops.attention_rows_tc_supported(D, R, cache.page_size):
+            # portions: the cache rows fetched once as key and value, tcgen05 (1,024 tokens of 16 heads behind 2,000, rows of 256:
+            # 389 us on the mma.sync kernel, 77 on this one)
+            ops.attention_rows_tc(q_lat, cache.k, a, batch, table, cache.page_size, H, 1, D, R, self.window, self.scale, gate)
+        elif self.dtype == torch.bfloat16 and not self.force_plain and ops.attention_window_supported(D, R, H, 1):
             ops.attention_window(q_lat, cache.k, cache.k, batch, table, cache.page_size, a, H, 1, D, R, self.window, 0, gate, self.scale,
                                  v_ld=D)
         else:

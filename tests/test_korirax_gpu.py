@@ -165,6 +165,38 @@ SPIKE_LAYERS = {"attention": K.attn(4, 2, 16, 24, 0.5, 40, 10, (0.7, 16)),
                 "rglru": K.rglru(64, 4, 3)}
 
 
+@pytest.mark.parametrize("layer,page,cuts", [
+    (K.latent(4, 32, 64, 32, 64, 192, 0.1, 64, 10000.0), 16, [200, 63, 150]),     # rows of 256, values of 192: four whole panels
+    (K.latent(3, 16, 8, 24, 40, 64, 0.2, 8, 100.0), 8, [65, 64, 22]),              # rows of 72: the last panel holds one chunk
+    (K.latent(2, 16, 16, 8, 24, 24, 0.3, 16, 100.0), 64, [130]),                   # rows of 40, values of 24: half a step of the second product
+    (K.latent(20, 16, 8, 16, 24, 248, 0.1, 8, 100.0), 128, [33, 100]),             # values of 248: all columns of the second product
+    (K.latent(1, 64, 64, 16, 48, 128, 0.15, 64, 10000.0), 32, [1300, 129, 200])])  # few tiles far into a context: slices of keys
+def test_latent_portions_on_tcgen05_against_the_other_kernel(layer, page, cuts):
+    """bfloat16 portions over the cache rows, tcgen05 against the plain statement and against the mma.sync kernel.  Both round P, the
+    mixed latents and every product's operands to bfloat16: the limit is the one of the other kernels' tests."""
+    from kestrel_llm_b200.csrc import ops
+    from kestrel_llm_b200.parts import LatentAttention
+    n = sum(cuts)
+    calls, real = [], ops.attention_rows_tc
+
+    def seen(*a, **kw):
+        calls.append(1)
+        return real(*a, **kw)
+    ops.attention_rows_tc = seen
+    try:
+        fast, want, _ = _mixer_case(layer, "bfloat16", page, n, cuts, seed=page, width=64)
+    finally:
+        ops.attention_rows_tc = real
+    assert len(calls) == sum(1 for c in cuts if c * layer["mixer"]["heads"] > LatentAttention.TC_MIN_ROWS)
+    _close(fast, want, "bfloat16", "tcgen05 attention over cache rows")
+    LatentAttention.tcgen05 = False
+    try:
+        slow, _, _ = _mixer_case(layer, "bfloat16", page, n, cuts, seed=page, width=64)
+    finally:
+        LatentAttention.tcgen05 = True
+    assert np.abs(fast - slow).max() <= 2e-2 * np.abs(want).max()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("decode", [False, True])
 @pytest.mark.parametrize("where", ["far", "page_end", "page_start", "first_token", "previous_token"])
