@@ -1,0 +1,588 @@
+// The sequential recurrences of linear_recurrence.cu and delta_rule.cu for portions of many tokens, in blocks of 16: the same sums in
+// another order, all of them float32.
+//
+// A token's step, S <- diag(w_t) S + a_t (b_t^T S) + k_t v_t^T, is a chain of two reductions over the key channels, some 600 cycles
+// however many threads share it.  Over a block of 16 tokens the state S_0 at its start is all that has to be read in order:
+// with P(s, t) the product of the decays of tokens s + 1 .. t (per channel, at most 1, so nothing overflows whatever the decays),
+//
+//     h_t = b_t^T S_(t-1) = (b_t P(0, t - 1))^T S_0 + sum_(s<t) [b_t P(s, t - 1) a_s] h_s + [b_t P(s, t - 1) k_s] v_s
+//     o_t = r_t^T S_t     = (r_t P(0, t))^T S_0     + sum_(s<=t) [r_t P(s, t) a_s] h_s    + [r_t P(s, t) k_s] v_s
+//     S_16                = P(0, 16) S_0            + sum_s (P(s, 16) a_s) h_s            + (P(s, 16) k_s) v_s
+//
+// The brackets are numbers per pair of tokens and head.  `blocks_prepare` makes them for all blocks at once, with the decayed vectors,
+// and solves the triangular system: h = X (b^T S_0) + XK v with X = (I - A)^-1, and what o takes from b^T S_0 and v.  `blocks_scan` then
+// walks a request's blocks: a CTA takes 16 value columns of a head, transposed, its four warps a quarter of the channels each, S^T in the
+// accumulators of m16n8k8 products: the accumulators are the next product's operand A as they stand (the sum over channels may run in any
+// order, so the unit's k index takes the channels in the order in which the accumulators hold them).  Per block: S^T times the decayed b and r
+// (the warps' parts meet in shared memory), the 16 x 16 matrices, S^T update; two barriers.  A prepared block (38 KB at 128 channels) comes
+// by one bulk copy into a ring, values by cp.async four blocks ahead.
+//
+// Every product is float32: operands as two terms of 11 bits, three products (rb_split, rb_mma3).  From float64 the read-outs are as far as the
+// sequential scan's within the tests' limit.  With plain multiply-adds the same blocks are bound by the shared-memory reads of
+// operands that 16 columns cannot reuse: 3,300 cycles a block against 1,500 here (DELTA).
+//
+// Three forms: GATE (no correction), REMOVAL (a, b given) and DELTA (a gated delta rule: with u = beta (v - (diag(w) S)^T k),
+// S <- diag(w) S + k u^T, so that b = w k and the writes u = X beta (v - b^T S_0) take the place of v).
+//
+// Measured, 16 heads, prepare + scan against the sequential scan: DELTA (128 channels, requests of 592 and 1,185 tokens) 53 + 132 us against
+// 523; GATE (64 channels, 2,048 tokens) 23 + 101 against 291; REMOVAL (128 channels, 700 tokens in three requests, 350 the longest) 34 + 69
+// against 205.  What is left of a block is the chain of its three products and their barriers.
+#include "common.cuh"
+#include "tcgen05.cuh"
+#include <math.h>
+
+#define RB_B 16                 // tokens of a block
+#define RB_LD 24                // floats of a row of a 16 x 16 matrix: pairs of four rows fall on all 32 banks
+#define RB_MAT (RB_B * RB_LD)
+#define RB_COLS 16              // value columns of a CTA
+#define RB_VLD 20               // floats of a token's row of them
+#define RB_STAGES 8             // most stages of the ring of prepared blocks
+
+enum { RB_GATE = 0, RB_REMOVAL = 1, RB_DELTA = 2 };
+
+__device__ int g_rb_error = 0;
+
+// a prepared block of a head: [b decayed | r decayed | k to the block's end | a to the block's end | P(0, 16) | matrices]
+template <int D, int FORM> struct RbLayout {
+    static constexpr int ROW_LD = D + 8, END_LD = D + 4;        // rows read as pairs along the channels, and as pairs of rows
+    static constexpr int BD = 0;
+    static constexpr int RD = FORM == RB_GATE ? 0 : RB_B * ROW_LD;
+    static constexpr int KW = RD + RB_B * ROW_LD;
+    static constexpr int AW = KW + RB_B * END_LD;
+    static constexpr int DT = FORM == RB_REMOVAL ? AW + RB_B * END_LD : AW;
+    static constexpr int M = DT + D;            // GATE: Qk; DELTA: X beta, Qk X beta; REMOVAL: X, X K, Qa X, Qa X K + Qk
+    static constexpr int FLOATS = M + (FORM == RB_GATE ? 1 : FORM == RB_DELTA ? 2 : 4) * RB_MAT;
+};
+
+struct RbParams {
+    const float *r, *w, *k, *a, *b, *beta;      // r, k [T, G d] (DELTA) or [T, H d]; w, a, b [T, H d]; beta [T, H]
+    const float *v;                             // [T, ldv], head h's columns at h * dv
+    size_t ldv;
+    float *state;
+    size_t state_stride;
+    const int *cu_seqlens, *slots;
+    float *out;                                 // [T, H dv]
+    float *blocks;                              // scratch: block (cu_seqlens[seq] / 16 + seq + i) of a request, head by head
+    int H, G, d, dv;
+};
+
+// One exchange of a sum of N values over the lanes: a lane keeps the half of the values that its bit of MASK names and adds the other
+// lane's share of them.  Five of them, from 32 values, leave lane l with the sum of value l.
+template <int N, int MASK> __device__ __forceinline__ void rb_exchange(float *x, int lane) {
+    const bool up = (lane & MASK) != 0;
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+        const float keep = up ? x[i + N / 2] : x[i], give = up ? x[i] : x[i + N / 2];
+        x[i] = keep + __shfl_xor_sync(0xffffffffu, give, MASK);
+    }
+}
+
+template <int D, int FORM>
+__global__ void __launch_bounds__(128)
+blocks_prepare_kernel(const RbParams p) {
+    using L = RbLayout<D, FORM>;
+    constexpr int V = D / 32;                   // channels of a lane
+    pdl_launch_dependents();
+    pdl_wait();
+    const int blk = blockIdx.x, h = blockIdx.y, seq = blockIdx.z;
+    const int t0 = p.cu_seqlens[seq] + blk * RB_B, t1 = p.cu_seqlens[seq + 1];
+    if (t0 >= t1) return;
+    extern __shared__ __align__(16) float rb_sm[];
+    // [w | r | k | b | a] of the block's tokens, zero (w: one) beyond the head's channels and the request's tokens
+    float *sw = rb_sm, *sr = sw + RB_B * D, *sk = sr + RB_B * D, *sb = sk + RB_B * D, *sa = sb + (FORM == RB_GATE ? 0 : RB_B * D);
+    float *mat = sa + (FORM == RB_REMOVAL ? RB_B * D : 0);                     // A, K, Qa, Qk and two more, rows of RB_LD
+    float *mA = mat, *mK = mA + RB_MAT, *mQa = mK + RB_MAT, *mQk = mQa + RB_MAT, *mX = mQk + RB_MAT, *mY = mX + RB_MAT;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int kh = FORM == RB_DELTA ? h / (p.H / p.G) : h, KH = FORM == RB_DELTA ? p.G : p.H;
+    __shared__ float sbeta[RB_B];
+    if (FORM == RB_DELTA && tid < RB_B) sbeta[tid] = t0 + tid < t1 ? p.beta[(size_t)(t0 + tid) * p.H + h] : 0.f;
+    const bool vec = p.d % 4 == 0 && (((uintptr_t)p.r | (uintptr_t)p.w | (uintptr_t)p.k | (uintptr_t)p.a | (uintptr_t)p.b) & 15) == 0;
+    if (vec) {                                  // all of a thread's loads in flight together
+        constexpr int N = RB_B * D / 512;
+        float4 w4[N], r4[N], k4[N], a4[FORM == RB_REMOVAL ? N : 1], b4[FORM == RB_REMOVAL ? N : 1];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int idx = (tid + 128 * i) * 4, t = idx / D, c = idx % D;
+            const bool in = t0 + t < t1 && c < p.d;
+            const size_t oh = in ? ((size_t)(t0 + t) * p.H + h) * p.d + c : 0, ok = in ? ((size_t)(t0 + t) * KH + kh) * p.d + c : 0;
+            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            w4[i] = in ? *reinterpret_cast<const float4 *>(p.w + oh) : make_float4(1.f, 1.f, 1.f, 1.f);
+            r4[i] = in ? *reinterpret_cast<const float4 *>(p.r + ok) : zero;
+            k4[i] = in ? *reinterpret_cast<const float4 *>(p.k + ok) : zero;
+            if (FORM == RB_REMOVAL) {
+                a4[i] = in ? *reinterpret_cast<const float4 *>(p.a + oh) : zero;
+                b4[i] = in ? *reinterpret_cast<const float4 *>(p.b + oh) : zero;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int idx = (tid + 128 * i) * 4;
+            *reinterpret_cast<float4 *>(sw + idx) = w4[i];
+            *reinterpret_cast<float4 *>(sr + idx) = r4[i];
+            *reinterpret_cast<float4 *>(sk + idx) = k4[i];
+            if (FORM == RB_REMOVAL) {
+                *reinterpret_cast<float4 *>(sb + idx) = b4[i];
+                *reinterpret_cast<float4 *>(sa + idx) = a4[i];
+            }
+            if (FORM == RB_DELTA)
+                *reinterpret_cast<float4 *>(sb + idx) = make_float4(w4[i].x * k4[i].x, w4[i].y * k4[i].y, w4[i].z * k4[i].z, w4[i].w * k4[i].w);
+        }
+    } else {
+#pragma unroll 4
+        for (int idx = tid; idx < RB_B * D; idx += 128) {
+            const int t = idx / D, c = idx % D;
+            const bool in = t0 + t < t1 && c < p.d;
+            const size_t oh = ((size_t)(t0 + t) * p.H + h) * p.d + c, ok = ((size_t)(t0 + t) * KH + kh) * p.d + c;
+            const float w = in ? p.w[oh] : 1.f, k = in ? p.k[ok] : 0.f;
+            sw[idx] = w;
+            sr[idx] = in ? p.r[ok] : 0.f;
+            sk[idx] = k;
+            if (FORM == RB_REMOVAL) {
+                sb[idx] = in ? p.b[oh] : 0.f;
+                sa[idx] = in ? p.a[oh] : 0.f;
+            }
+            if (FORM == RB_DELTA) sb[idx] = w * k;
+        }
+    }
+    for (int idx = tid; idx < 6 * RB_MAT; idx += 128) mat[idx] = 0.f;
+    __syncthreads();
+
+    float *blkp = p.blocks + ((size_t)(p.cu_seqlens[seq] / RB_B + seq + blk) * p.H + h) * L::FLOATS;
+    // vectors decayed from the block's start and to its end, a channel a thread
+    for (int c = tid; c < D; c += 128) {
+        float run = 1.f;
+#pragma unroll
+        for (int t = 0; t < RB_B; ++t) {
+            if (FORM != RB_GATE) blkp[L::BD + t * L::ROW_LD + c] = sb[t * D + c] * run;
+            run *= sw[t * D + c];
+            blkp[L::RD + t * L::ROW_LD + c] = sr[t * D + c] * run;
+        }
+        blkp[L::DT + c] = run;
+        run = 1.f;
+#pragma unroll
+        for (int t = RB_B - 1; t >= 0; --t) {
+            blkp[L::KW + t * L::END_LD + c] = sk[t * D + c] * run;
+            if (FORM == RB_REMOVAL) blkp[L::AW + t * L::END_LD + c] = sa[t * D + c] * run;
+            run *= sw[t * D + c];
+        }
+    }
+    // the pairs: a warp takes four tokens s, evenly long walks t = s .. 15 among them; eight t's sums go through the lanes together
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+        const int s = i == 0 ? warp : i == 1 ? 7 - warp : i == 2 ? 8 + warp : 15 - warp;
+        float xk[V], xa[V];
+#pragma unroll
+        for (int j = 0; j < V; ++j) {           // neighbouring channels: they come in one load
+            xk[j] = sk[s * D + lane * V + j];
+            xa[j] = FORM == RB_REMOVAL ? sa[s * D + lane * V + j] : 0.f;
+        }
+#pragma unroll 1
+        for (int half = s >> 3; half < 2; ++half) {
+            float x[32];                        // [t][A, K, Qa, Qk]
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int t = half * 8 + u;
+                float fA = 0.f, fK = 0.f, fQa = 0.f, fQk = 0.f;
+                if (t >= s) {
+#pragma unroll
+                    for (int j = 0; j < V; ++j) {
+                        const int o = t * D + lane * V + j;
+                        if (t > s) {
+                            if (FORM != RB_GATE) {
+                                const float bb = sb[o];
+                                fK = fmaf(bb, xk[j], fK);
+                                if (FORM == RB_REMOVAL) fA = fmaf(bb, xa[j], fA);
+                            }
+                            xk[j] *= sw[o];
+                            if (FORM == RB_REMOVAL) xa[j] *= sw[o];
+                        }
+                        const float rr = sr[o];
+                        fQk = fmaf(rr, xk[j], fQk);
+                        if (FORM == RB_REMOVAL) fQa = fmaf(rr, xa[j], fQa);
+                    }
+                }
+                x[4 * u] = fA;
+                x[4 * u + 1] = fK;
+                x[4 * u + 2] = fQa;
+                x[4 * u + 3] = fQk;
+            }
+            rb_exchange<32, 16>(x, lane);
+            rb_exchange<16, 8>(x, lane);
+            rb_exchange<8, 4>(x, lane);
+            rb_exchange<4, 2>(x, lane);
+            rb_exchange<2, 1>(x, lane);
+            // lane l holds value l: token half * 8 + l / 4, matrix l % 4
+            mat[(lane & 3) * RB_MAT + (half * 8 + (lane >> 2)) * RB_LD + s] = x[0];
+        }
+    }
+    __syncthreads();
+    if (FORM == RB_GATE) {
+        for (int idx = tid; idx < RB_MAT; idx += 128) blkp[L::M + idx] = mQk[idx];
+        return;
+    }
+    // X, a column a thread, by substitution: REMOVAL (I - A)^-1; DELTA (I + beta A)^-1 beta with A in mK
+    if (tid < RB_B) {
+        float x[RB_B];
+#pragma unroll
+        for (int t = 0; t < RB_B; ++t) {
+            const float beta = FORM == RB_DELTA ? sbeta[t] : 0.f;
+            float sum = 0.f;
+#pragma unroll
+            for (int s = 0; s < t; ++s) sum = fmaf((FORM == RB_DELTA ? mK : mA)[t * RB_LD + s], x[s], sum);
+            const float one = t == tid ? 1.f : 0.f;
+            x[t] = FORM == RB_DELTA ? beta * (one - sum) : one + sum;
+            mX[t * RB_LD + tid] = x[t];
+        }
+    }
+    __syncthreads();
+    for (int idx = tid; idx < RB_B * RB_B; idx += 128) {
+        const int t = idx / RB_B, j = idx % RB_B;
+        if (FORM == RB_DELTA) {
+            float m = 0.f;
+#pragma unroll
+            for (int s = 0; s < RB_B; ++s) m = fmaf(mQk[t * RB_LD + s], mX[s * RB_LD + j], m);
+            blkp[L::M + t * RB_LD + j] = mX[t * RB_LD + j];
+            blkp[L::M + RB_MAT + t * RB_LD + j] = m;
+        } else {
+            float xk = 0.f, m1 = 0.f;
+#pragma unroll
+            for (int s = 0; s < RB_B; ++s) {
+                xk = fmaf(mX[t * RB_LD + s], mK[s * RB_LD + j], xk);
+                m1 = fmaf(mQa[t * RB_LD + s], mX[s * RB_LD + j], m1);
+            }
+            mY[t * RB_LD + j] = xk;
+            blkp[L::M + t * RB_LD + j] = mX[t * RB_LD + j];
+            blkp[L::M + RB_MAT + t * RB_LD + j] = xk;
+            blkp[L::M + 2 * RB_MAT + t * RB_LD + j] = m1;
+        }
+    }
+    if (FORM == RB_REMOVAL) {
+        __syncthreads();
+        for (int idx = tid; idx < RB_B * RB_B; idx += 128) {
+            const int t = idx / RB_B, j = idx % RB_B;
+            float m2 = mQk[t * RB_LD + j];
+#pragma unroll
+            for (int s = 0; s < RB_B; ++s) m2 = fmaf(mQa[t * RB_LD + s], mY[s * RB_LD + j], m2);
+            blkp[L::M + 3 * RB_MAT + t * RB_LD + j] = m2;
+        }
+    }
+}
+
+// One step of 8 along the sum, m16n8k8 with float32 results; operands are float32 numbers whose low 13 bits the unit ignores
+__device__ __forceinline__ void rb_mma(float *c, const uint32_t *a, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// x as two terms of 11 bits, both rounded to the nearest: the first leaves 2^-12 of x (exactly what the subtraction gives), the second
+// 2^-24.  (Cut off instead of rounded the two terms leave 2^-21 and the products of the second ones, which are dropped, 2^-20: read-outs
+// were 5e-7 of the largest off where the scan is 8e-8 off.)  The unit ignores the low 13 bits of the second.
+__device__ __forceinline__ void rb_split(float x, uint32_t &hi, uint32_t &lo) {
+    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+    lo = __float_as_uint(x - __uint_as_float(hi)) + 0x1000u;
+}
+struct RbA { uint32_t hi[4], lo[4]; };
+// Operand A from a row-major pair of numbers per row: (row l / 4: x0 at 2 (l % 4), x1 behind it; row l / 4 + 8: x2, x3).  The unit's k index
+// l % 4 is taken for the even, l % 4 + 4 for the odd of the two; operand B pairs its numbers the same way.
+__device__ __forceinline__ void rb_a(RbA &a, float x0, float x1, float x2, float x3) {
+    rb_split(x0, a.hi[0], a.lo[0]);
+    rb_split(x2, a.hi[1], a.lo[1]);
+    rb_split(x1, a.hi[2], a.lo[2]);
+    rb_split(x3, a.hi[3], a.lo[3]);
+}
+// c += a * b in three products of the terms (the fourth is 2^-24 of the first); the small ones in a sum of their own, for shorter chains
+__device__ __forceinline__ void rb_mma3(float *c, float *small, const RbA &a, float y0, float y1) {
+    uint32_t h0, l0, h1, l1;
+    rb_split(y0, h0, l0);
+    rb_split(y1, h1, l1);
+    rb_mma(small, a.lo, h0, h1);
+    rb_mma(c, a.hi, h0, h1);
+    rb_mma(small, a.hi, l0, l1);
+}
+
+template <int D, int FORM>
+__global__ void __launch_bounds__(128)
+blocks_scan_kernel(const RbParams p, int stages) {
+    using L = RbLayout<D, FORM>;
+    constexpr int ROWS = FORM == RB_GATE ? RB_B : 2 * RB_B;      // rows that meet the state: b and r
+    constexpr int NT = ROWS / 8;                                 // tiles of eight of them
+    constexpr int CT = D / 32;                                   // tiles of eight channels of a warp
+    constexpr int STAGE = L::FLOATS, RED_LD = ROWS + 8;
+    pdl_launch_dependents();
+    extern __shared__ float4 rb_smem4[];
+    float *ring = reinterpret_cast<float *>(rb_smem4);
+    __shared__ __align__(8) unsigned long long bar_words[RB_STAGES];
+    // values of a block [token][column], four blocks in flight: loaded for the next block alone they set the pace (2,400 cycles a block)
+    __shared__ __align__(16) float red_s[FORM == RB_GATE ? 2 : 1][4][RB_COLS][RED_LD], vals[4][RB_B][RB_VLD], corr[RB_COLS][RB_LD];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int lr = lane >> 2, lc = (lane & 3) * 2;               // a fragment's row (and row + 8) and its pair of columns
+    const int h = blockIdx.y, seq = blockIdx.z, col0 = blockIdx.x * RB_COLS;
+    const int ch0 = warp * (D / 4);
+    const uint32_t bar0 = smem_u32(&bar_words[0]);
+    if (tid == 0) {
+        for (int b = 0; b < stages; ++b) mbar_init(bar0 + 8 * b, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    pdl_wait();
+    const int t0 = p.cu_seqlens[seq], t1 = p.cu_seqlens[seq + 1];
+    const int n_blocks = (t1 - t0 + RB_B - 1) / RB_B;
+    const float *src = p.blocks + ((size_t)(t0 / RB_B + seq) * p.H + h) * STAGE;
+    auto fetch = [&](int i) {           // one thread: block i into stage i % stages
+        const uint32_t bar = bar0 + 8u * (uint32_t)(i % stages);
+        mbar_expect_tx(bar, STAGE * 4);
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(smem_u32(ring + (i % stages) * STAGE)), "l"(src + (size_t)i * p.H * STAGE), "r"(STAGE * 4), "r"(bar)
+                     : "memory");
+    };
+    if (tid == 0)
+        for (int i = 0; i < min(stages, n_blocks); ++i) fetch(i);
+    float *Sg = p.state + (size_t)p.slots[seq] * p.state_stride + (size_t)h * p.d * p.dv;     // [d][dv]
+    // S^T of the warp's channels: S[ct] = columns lr, lr + 8 of the CTA by channels lc, lc + 1 of the tile
+    float S[CT][4];
+#pragma unroll
+    for (int ct = 0; ct < CT; ++ct)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int c = ch0 + ct * 8 + lc + (e & 1), j = col0 + lr + (e >> 1) * 8;
+            S[ct][e] = (c < p.d && j < p.dv) ? Sg[(size_t)c * p.dv + j] : 0.f;
+        }
+    // thread moves columns vj, vj + 1 of token vt; zeros beyond the request and the head
+    const int vt = tid >> 3, vj = (tid & 7) * 2;
+    auto load_v = [&](int i) {
+        const int t = t0 + i * RB_B + vt;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const bool in = i < n_blocks && t < t1 && col0 + vj + e < p.dv;
+            const float *from = in ? p.v + (size_t)t * p.ldv + (size_t)h * p.dv + col0 + vj + e : p.v;
+            const int bytes = in ? 4 : 0;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(&vals[i & 3][vt][vj + e])), "l"(from), "r"(bytes) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load_v(0);
+    load_v(1);
+    load_v(2);
+    bool ok = true;
+    for (int i = 0; i < n_blocks; ++i) {
+        const int stage = i % stages;
+        const float *st = ring + stage * STAGE;
+        float(*red)[RB_COLS][RED_LD] = red_s[FORM == RB_GATE ? i & 1 : 0];       // GATE has one barrier a block: two buffers in turn
+        asm volatile("cp.async.wait_group 2;" ::: "memory");       // this block's values; the barrier below shows them to all
+        if (ok && !mbar_wait(bar0 + 8u * stage, (uint32_t)(i / stages) & 1u)) { atomicExch(&g_rb_error, 1); ok = false; }
+        {   // what the warp's channels of the state give to the block's rows
+            float acc[NT][4], small[NT][4];
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[n][e] = small[n][e] = 0.f;
+#pragma unroll
+            for (int ct = 0; ct < CT; ++ct) {
+                RbA a;
+                rb_a(a, S[ct][0], S[ct][1], S[ct][2], S[ct][3]);
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {                   // rows: BD, then RD (GATE: RD)
+                    const float2 b = *reinterpret_cast<const float2 *>(st + (n * 8 + lr) * L::ROW_LD + ch0 + ct * 8 + lc);
+                    rb_mma3(acc[n], small[n], a, b.x, b.y);
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    *reinterpret_cast<float2 *>(&red[warp][lr + 8 * e][n * 8 + lc]) = make_float2(acc[n][2 * e] + small[n][2 * e], acc[n][2 * e + 1] + small[n][2 * e + 1]);
+        }
+        __syncthreads();                        // and every warp is done with the block before
+        if (tid == 0 && i > 0 && i - 1 + stages < n_blocks) fetch(i - 1 + stages);
+        load_v(i + 3);
+        const float(*vr)[RB_VLD] = vals[i & 3];
+        // sum over the warps' channels of rows 8 n + lc, + 1 for columns lr, lr + 8
+        auto total = [&](int n, float *x) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    const float2 y = *reinterpret_cast<const float2 *>(&red[w][lr + 8 * e][n * 8 + lc]);
+                    s.x += y.x;
+                    s.y += y.y;
+                }
+                x[2 * e] = s.x;
+                x[2 * e + 1] = s.y;
+            }
+        };
+        // columns by tokens: warps 0, 1 the corrections (DELTA: the writes) of tokens 0-7, 8-15, warps 2, 3 the read-outs
+        const bool reads = warp >= 2;
+        const int half = warp & 1;
+        if (reads || FORM != RB_GATE) {
+            float acc[4] = {0.f, 0.f, 0.f, 0.f}, small[4] = {0.f, 0.f, 0.f, 0.f};
+            const float *m0 = st + L::M, *m1 = m0 + RB_MAT;
+            const int row = (half * 8 + lr) * RB_LD + lc;
+            if (reads) total((FORM == RB_GATE ? 0 : 2) + half, acc);
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) {
+                const float *u0 = &vr[ks * 8 + lc][lr], *u1 = &vr[ks * 8 + lc + 1][lr];
+                RbA av;
+                if (FORM == RB_DELTA) {         // v - b^T S_0 takes the values' place
+                    float x[4];
+                    total(ks, x);
+                    rb_a(av, u0[0] - x[0], u1[0] - x[1], u0[8] - x[2], u1[8] - x[3]);
+                } else {
+                    rb_a(av, u0[0], u1[0], u0[8], u1[8]);
+                }
+                const float *mv = FORM == RB_GATE ? m0 : FORM == RB_DELTA ? (reads ? m1 : m0) : (reads ? m0 + 3 * RB_MAT : m1);
+                float2 b = *reinterpret_cast<const float2 *>(mv + row + ks * 8);
+                rb_mma3(acc, small, av, b.x, b.y);
+                if (FORM == RB_REMOVAL) {
+                    float x[4];
+                    RbA ah;
+                    total(ks, x);
+                    rb_a(ah, x[0], x[1], x[2], x[3]);
+                    b = *reinterpret_cast<const float2 *>((reads ? m0 + 2 * RB_MAT : m0) + row + ks * 8);
+                    rb_mma3(acc, small, ah, b.x, b.y);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[e] += small[e];
+            if (reads) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int t = t0 + i * RB_B + half * 8 + lc + (e & 1), j = col0 + lr + (e >> 1) * 8;
+                    if (t < t1 && j < p.dv) p.out[((size_t)t * p.H + h) * p.dv + j] = acc[e];
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) *reinterpret_cast<float2 *>(&corr[lr + 8 * e][half * 8 + lc]) = make_float2(acc[2 * e], acc[2 * e + 1]);
+            }
+        }
+        if (FORM != RB_GATE) __syncthreads();
+        // the state at the block's end
+        float small[CT][4];
+#pragma unroll
+        for (int ct = 0; ct < CT; ++ct) {
+            const float2 d2 = *reinterpret_cast<const float2 *>(st + L::DT + ch0 + ct * 8 + lc);
+            S[ct][0] *= d2.x;
+            S[ct][1] *= d2.y;
+            S[ct][2] *= d2.x;
+            S[ct][3] *= d2.y;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) small[ct][e] = 0.f;
+        }
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+            auto write = [&](const RbA &a, const float *rows) {
+#pragma unroll
+                for (int ct = 0; ct < CT; ++ct) {
+                    const float *b = rows + (ks * 8 + lc) * L::END_LD + ch0 + ct * 8 + lr;
+                    rb_mma3(S[ct], small[ct], a, b[0], b[L::END_LD]);
+                }
+            };
+            RbA a;
+            if (FORM != RB_DELTA) {
+                const float *u0 = &vr[ks * 8 + lc][lr], *u1 = &vr[ks * 8 + lc + 1][lr];
+                rb_a(a, u0[0], u1[0], u0[8], u1[8]);
+                write(a, st + L::KW);
+            }
+            if (FORM != RB_GATE) {
+                const float2 x0 = *reinterpret_cast<const float2 *>(&corr[lr][ks * 8 + lc]), x1 = *reinterpret_cast<const float2 *>(&corr[lr + 8][ks * 8 + lc]);
+                rb_a(a, x0.x, x0.y, x1.x, x1.y);
+                write(a, st + (FORM == RB_DELTA ? L::KW : L::AW));
+            }
+        }
+#pragma unroll
+        for (int ct = 0; ct < CT; ++ct)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) S[ct][e] += small[ct][e];
+    }
+#pragma unroll
+    for (int ct = 0; ct < CT; ++ct)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int c = ch0 + ct * 8 + lc + (e & 1), j = col0 + lr + (e >> 1) * 8;
+            if (c < p.d && j < p.dv) Sg[(size_t)c * p.dv + j] = S[ct][e];
+        }
+}
+
+static int rb_padded(int d) { return d <= 32 ? 32 : d <= 64 ? 64 : 128; }
+static long long rb_floats(int D, int form) {
+    const int rows = form == RB_GATE ? 1 : 2, ends = form == RB_REMOVAL ? 2 : 1, mats = form == RB_GATE ? 1 : form == RB_DELTA ? 2 : 4;
+    return (long long)RB_B * (rows * (D + 8) + ends * (D + 4)) + D + (long long)mats * RB_MAT;
+}
+
+template <int D, int FORM>
+static int rb_launch(const RbParams &p, int nseq, int max_count, cudaStream_t stream) {
+    static_assert(RbLayout<D, FORM>::FLOATS % 4 == 0, "bulk copies move 16 bytes");
+    const size_t prep = (size_t)((FORM == RB_GATE ? 3 : FORM == RB_DELTA ? 4 : 5) * RB_B * D + 6 * RB_MAT) * sizeof(float);
+    constexpr size_t stage = (size_t)RbLayout<D, FORM>::FLOATS * sizeof(float), fixed = 18 * 1024;    // beside the ring: under 18 KB of static memory
+    static bool attr_set = false;
+    if (!attr_set) {
+        if (cudaFuncSetAttribute(blocks_prepare_kernel<D, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep) != cudaSuccess ||
+            cudaFuncSetAttribute(blocks_scan_kernel<D, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(KESTREL_SMEM_MAX_DYNAMIC - fixed)) != cudaSuccess)
+            return kestrel_fail(-3, "recurrence_blocks: cannot set the shared memory size");
+        attr_set = true;
+    }
+    kestrel_launch(blocks_prepare_kernel<D, FORM>, dim3((max_count + RB_B - 1) / RB_B, p.H, nseq), dim3(128), prep, stream, p);
+    static_assert(RbLayout<D, FORM>::FLOATS * 8 + 18 * 1024 <= KESTREL_SMEM_MAX_DYNAMIC, "two stages fit an SM");
+    const dim3 grid((p.dv + RB_COLS - 1) / RB_COLS, p.H, nseq);
+    // as many stages as the CTAs that share an SM leave room for, two at least
+    const size_t room = kestrel_spread_smem((long)grid.x * grid.y * grid.z, 2 * stage + fixed) - fixed;
+    const int stages = (int)(room / stage) < RB_STAGES ? (int)(room / stage) : RB_STAGES;
+    kestrel_launch(blocks_scan_kernel<D, FORM>, grid, dim3(128), room, stream, p, stages);
+    return kestrel_check_launch("recurrence_blocks");
+}
+
+template <int FORM>
+static int rb_run(const RbParams &p, int nseq, int max_count, cudaStream_t stream) {
+    switch (rb_padded(p.d)) {
+        case 32: return rb_launch<32, FORM>(p, nseq, max_count, stream);
+        case 64: return rb_launch<64, FORM>(p, nseq, max_count, stream);
+        default: return rb_launch<128, FORM>(p, nseq, max_count, stream);
+    }
+}
+
+static int rb_check(const RbParams &p, int T, int nseq, int max_count, long long floats, int form) {
+    KESTREL_REQUIRE(T > 0 && nseq > 0 && max_count > 0 && p.H > 0 && p.G > 0 && p.H % p.G == 0 && p.d > 0 && p.dv > 0, "recurrence_blocks: bad sizes");
+    KESTREL_REQUIRE(p.d <= 128, "recurrence_blocks: %d key channels; the kernel holds up to 128", p.d);
+    KESTREL_REQUIRE(p.H <= 65535 && nseq <= 65535, "recurrence_blocks: grid too large");
+    KESTREL_REQUIRE(floats >= ((long long)T / RB_B + nseq) * p.H * rb_floats(rb_padded(p.d), form), "recurrence_blocks: scratch of %lld floats is too small", floats);
+    KESTREL_REQUIRE(((uintptr_t)p.blocks & 15) == 0, "recurrence_blocks: the scratch must start on a 16-byte boundary");
+    return 0;
+}
+
+// floats of scratch for a step of T tokens of nseq requests; form 0: no correction, 1: with a and b, 2: the gated delta rule
+KESTREL_API long long kestrel_recurrence_blocks_floats(int T, int nseq, int H, int d, int form) {
+    if (T <= 0 || nseq <= 0 || H <= 0 || d <= 0 || d > 128 || form < 0 || form > 2) return -1;
+    return ((long long)T / RB_B + nseq) * H * rb_floats(rb_padded(d), form);
+}
+
+// kestrel_recurrence_scan for portions of many tokens (max_count: the most tokens of one request); a and b null: no correction
+KESTREL_API int kestrel_recurrence_blocks(const float *r, const float *w, const float *k, const float *v, const float *a, const float *b,
+                                          float *state, long long state_stride, long long state_off, const int *cu_seqlens, const int *slots,
+                                          float *out, float *scratch, long long scratch_floats, int T, int nseq, int max_count, int H, int d, int dv,
+                                          cudaStream_t stream) {
+    if (T == 0 || nseq == 0) return 0;
+    KESTREL_REQUIRE((a == nullptr) == (b == nullptr), "recurrence_blocks: a and b come together");
+    const RbParams p = {r, w, k, a, b, nullptr, v, (size_t)H * dv, state + state_off, (size_t)state_stride, cu_seqlens, slots, out, scratch, H, H, d, dv};
+    const int rc = rb_check(p, T, nseq, max_count, scratch_floats, a ? RB_REMOVAL : RB_GATE);
+    if (rc) return rc;
+    return a ? rb_run<RB_REMOVAL>(p, nseq, max_count, stream) : rb_run<RB_GATE>(p, nseq, max_count, stream);
+}
+
+// kestrel_delta_scan for portions of many tokens
+KESTREL_API int kestrel_delta_blocks(const float *qn, const float *kn, const float *decay, const float *v, long long ldv, const float *beta,
+                                     float *state, long long state_stride, const int *cu_seqlens, const int *slots, float *out, float *scratch,
+                                     long long scratch_floats, int T, int nseq, int max_count, int H, int G, int d, int dv, cudaStream_t stream) {
+    if (T == 0 || nseq == 0) return 0;
+    const RbParams p = {qn, decay, kn, nullptr, nullptr, beta, v, (size_t)ldv, state, (size_t)state_stride, cu_seqlens, slots, out, scratch, H, G, d, dv};
+    const int rc = rb_check(p, T, nseq, max_count, scratch_floats, RB_DELTA);
+    if (rc) return rc;
+    return rb_run<RB_DELTA>(p, nseq, max_count, stream);
+}
+
+// Error word of the bounded waits (0: none, 1: a block's copy).  Synchronises the device and clears the word.
+KESTREL_API int kestrel_recurrence_blocks_error(void) {
+    int v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_rb_error, sizeof(int)) != cudaSuccess) return -1;
+    if (v) cudaMemcpyToSymbol(g_rb_error, &zero, sizeof(int));
+    return v;
+}

@@ -50,13 +50,14 @@ KESTREL_API int kestrel_sm_count(void) {
 }
 
 // Error words of all kernels with bounded waits in one call: bit 0 the tensor-core product,
-// bit 1 the prompt-portion attention, bit 2 the decode attention.  Synchronises the device and
-// clears the words.
+// bit 1 the prompt-portion attention, bit 2 the decode attention, bit 3 the recurrences in blocks.
+// Synchronises the device and clears the words.
 KESTREL_API int kestrel_kernel_errors(void) {
     int bits = 0;
     if (kestrel_gemm_tc_error() != 0) bits |= 1;
     if (kestrel_attention_tc_error() != 0) bits |= 2;
     if (kestrel_attention_rows_tc_error() != 0) bits |= 2;
+    if (kestrel_recurrence_blocks_error() != 0) bits |= 8;
     if (kestrel_attention_decode_error() != 0) bits |= 4;
     return bits;
 }

@@ -784,6 +784,7 @@ def raise_on_kernel_error() -> None:
     bad = [(name, code) for name, code in (("gemm_tcgen05", lib.kestrel_gemm_tc_error()),
                                            ("attention_tc", lib.kestrel_attention_tc_error()),
                                            ("attention_rows_tc", lib.kestrel_attention_rows_tc_error()),
+                                           ("recurrence_blocks", lib.kestrel_recurrence_blocks_error()),
                                            ("attention_decode", lib.kestrel_attention_decode_error()),
                                            ("moe_tcgen05", lib.kestrel_moe_tc_error())) if code]
     if bad:
@@ -1730,6 +1731,69 @@ def recurrence_scan(r: torch.Tensor, w: torch.Tensor, k: torch.Tensor, v: torch.
                                              int(state_off), batch.cu_seqlens.data_ptr(), batch.slots.data_ptr(), out.data_ptr(), batch.num_seqs,
                                              H, d, dv, _stream()))
     return out
+
+
+BLOCK_TOKENS = 32       # a step whose longest portion has as many tokens takes the recurrences in blocks
+
+
+def recurrence_in_blocks(batch, dtype: torch.dtype, d: int) -> bool:
+    """Whether a step runs its recurrences in blocks of 16 tokens.  Not in float32, whose logits are the same bits however a request was
+    cut, and not in a recorded step."""
+    return dtype == torch.bfloat16 and not batch.captured and batch.max_count >= BLOCK_TOKENS and d <= 128
+
+
+def _block_scratch(T: int, batch, H: int, d: int, form: int, device) -> torch.Tensor:
+    n = library().kestrel_recurrence_blocks_floats(T, batch.num_seqs, H, d, form)
+    if n < 0:
+        raise KernelError(f"recurrence_blocks: no blocks for {T} tokens, {H} heads of {d}")
+    return torch.empty(n, dtype=torch.float32, device=device)
+
+
+def recurrence_blocks(r: torch.Tensor, w: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: Optional[torch.Tensor], b: Optional[torch.Tensor],
+                      state: torch.Tensor, state_off: int, batch, H: int, d: int, dv: int) -> torch.Tensor:
+    """`recurrence_scan` in blocks of 16 tokens (two launches): other order of sums, all of them float32."""
+    _need(state, "recurrence_blocks.state", torch.float32, 2)
+    T = r.shape[0]
+    for t, name, n in ((r, "r", H * d), (w, "w", H * d), (k, "k", H * d), (v, "v", H * dv), (a, "a", H * d), (b, "b", H * d)):
+        if t is not None:
+            _need(t, f"recurrence_blocks.{name}", torch.float32, 2)
+            if t.shape != (T, n):
+                raise KernelError(f"recurrence_blocks.{name}: shape {tuple(t.shape)}, expected ({T}, {n})")
+    if state_off < 0 or state_off + H * d * dv > state.shape[1]:
+        raise KernelError("recurrence_blocks: the state does not fit the slot")
+    if T != batch.num_tokens:
+        raise KernelError(f"recurrence_blocks: {T} rows for a step of {batch.num_tokens} tokens")
+    out = torch.empty((T, H * dv), dtype=torch.float32, device=r.device)
+    scratch = _block_scratch(T, batch, H, d, 0 if a is None else 1, r.device)
+    _check(library().kestrel_recurrence_blocks(r.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), _p(a), _p(b), state.data_ptr(),
+                                               state.stride(0), int(state_off), batch.cu_seqlens.data_ptr(), batch.slots.data_ptr(),
+                                               out.data_ptr(), scratch.data_ptr(), scratch.numel(), T, batch.num_seqs, batch.max_count, H, d, dv,
+                                               _stream()))
+    global launches
+    launches += 1
+    return out
+
+
+def delta_blocks(qn: torch.Tensor, kn: torch.Tensor, decay: torch.Tensor, act: torch.Tensor, col_v: int, beta: torch.Tensor,
+                 state: torch.Tensor, batch, out: torch.Tensor, H: int, G: int, d: int, dv: int) -> None:
+    """`delta_scan` in blocks of 16 tokens (two launches): other order of sums, all of them float32."""
+    _need(out, "delta_blocks.out", torch.float32, 2)
+    _need(state, "delta_blocks.state", torch.float32, 2)
+    _need(act, "delta_blocks.act", torch.float32, 2)
+    T = out.shape[0]
+    for t, name, n in ((qn, "qn", G * d), (kn, "kn", G * d), (decay, "decay", H * d), (beta, "beta", H), (out, "out", H * dv)):
+        _need(t, f"delta_blocks.{name}", torch.float32, 2)
+        if t.shape != (T, n):
+            raise KernelError(f"delta_blocks.{name}: shape {tuple(t.shape)}, expected ({T}, {n})")
+    if T != batch.num_tokens or act.shape[0] != T or col_v + H * dv > act.shape[1] or H * d * dv > state.shape[1]:
+        raise KernelError("delta_blocks: the values do not fit the heads, or the state not the slot")
+    scratch = _block_scratch(T, batch, H, d, 2, out.device)
+    _check(library().kestrel_delta_blocks(qn.data_ptr(), kn.data_ptr(), decay.data_ptr(), act.data_ptr() + 4 * int(col_v), act.shape[1],
+                                          beta.data_ptr(), state.data_ptr(), state.stride(0), batch.cu_seqlens.data_ptr(),
+                                          batch.slots.data_ptr(), out.data_ptr(), scratch.data_ptr(), scratch.numel(), T, batch.num_seqs,
+                                          batch.max_count, H, G, d, dv, _stream()))
+    global launches
+    launches += 1
 
 
 def recurrence_scan_bonus(r: torch.Tensor, w: torch.Tensor, k: torch.Tensor, v: torch.Tensor, u: torch.Tensor, state: torch.Tensor,

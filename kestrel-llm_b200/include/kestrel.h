@@ -227,6 +227,14 @@ KESTREL_API int kestrel_attn_prepare_tempered(const float *partial, int S, long 
 /* the same for heads of `maps` queries and keys of size hd over one value, laid out [head][map]: columns [q: nq maps hd | k: nkv maps hd | v: nkv vd | gate: nq], K pages [page][kv head][slot][maps hd], q_out [T, nq maps, hd] or, with q_pad, [T, nq maps, maps hd] with zeros outside a row's own map */
 KESTREL_API int kestrel_attn_prepare_maps(const float *partial, int S, long long slice_stride, int ld, const float *bias, const float *q_norm_w, const float *k_norm_w, int qk_norm, int v_norm, float norm_eps, const float *inv_freq, int rot, int rot_mode, float rot_scale, float q_temp_coef, int q_temp_every, const int *positions, const int *seq_of_token, const int *block_table, int table_stride, int page_size, void *k_cache, void *v_cache, void *q_out, float *gate_out, int dtype, int T, int nq, int nkv, int hd, int vd, int has_kv, int maps, int q_pad, kestrel_stream_t stream);
 
+/* ---- the recurrences of kestrel_recurrence_scan and kestrel_delta_scan in blocks of 16 tokens (recurrence_blocks.cu): portions of many tokens, key channels up to 128; max_count: the most tokens of one request ---- */
+/* floats of scratch; form 0: no correction term, 1: with a and b, 2: the gated delta rule */
+KESTREL_API long long kestrel_recurrence_blocks_floats(int T, int nseq, int H, int d, int form);
+KESTREL_API int kestrel_recurrence_blocks(const float *r, const float *w, const float *k, const float *v, const float *a, const float *b, float *state, long long state_stride, long long state_off, const int *cu_seqlens, const int *slots, float *out, float *scratch, long long scratch_floats, int T, int nseq, int max_count, int H, int d, int dv, kestrel_stream_t stream);
+/* v: [T, ldv], head h's values at column h * dv */
+KESTREL_API int kestrel_delta_blocks(const float *qn, const float *kn, const float *decay, const float *v, long long ldv, const float *beta, float *state, long long state_stride, const int *cu_seqlens, const int *slots, float *out, float *scratch, long long scratch_floats, int T, int nseq, int max_count, int H, int G, int d, int dv, kestrel_stream_t stream);
+KESTREL_API int kestrel_recurrence_blocks_error(void);
+
 /* ---- attention over cached latents (attention_latent.cu) ---- */
 /* product columns [q latent: q_rank | kv latent: kv_rank | gate: n_gate]: both latents RMS-normed with their weights; the query latent to q_out [T, q_rank], the kv latent into the token's slot of latent_cache [pages, 1, page_size, kv_rank], sigmoid of the gate columns to gate_out [T, n_gate]; kv_out (may be NULL) receives the kv latents as rows [T, kv_rank] too */
 KESTREL_API int kestrel_latent_prepare(const float *partial, int S, long long slice_stride, int ld, const float *q_norm_w, const float *kv_norm_w, float norm_eps, const int *positions, const int *seq_of_token, const int *block_table, int table_stride, int page_size, void *latent_cache, void *q_out, float *gate_out, void *kv_out, int dtype, int T, int q_rank, int kv_rank, int n_gate, kestrel_stream_t stream);

@@ -31,7 +31,9 @@ from .linear import Linear
 
 
 class ChannelDeltaMixer(Mixer):
-    graph_safe = True          # forward launches kernels over device tensors of the batch only
+    graph_safe = True          # forward launches kernels over device tensors of the batch only (the form in blocks reads the host's
+                               # copy of the step, and is never taken while a step is recorded)
+    blocks = True              # tests: off, portions of many tokens stay on the sequential scan
 
     def __init__(self, width: int, heads: int, kv_heads: int, key_dim: int, value_dim: int, taps: int, decay_rank: int,
                  gate_rank: int, norm_eps: float, dtype: torch.dtype, device, prefix: str):
@@ -87,7 +89,8 @@ class ChannelDeltaMixer(Mixer):
         beta = torch.empty((T, H), dtype=f32, device=dev)
         ops.delta_gates(act, fused, self.col_beta, a, self.A_log, self.dt_bias, qn, kn, decay, beta, H, G, d)
         o = torch.empty((T, H * dv), dtype=f32, device=dev)
-        ops.delta_scan(qn, kn, decay, act, self.col_v, beta, cache.state, batch, o, H, G, d, dv)
+        scan = ops.delta_blocks if self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d) else ops.delta_scan
+        scan(qn, kn, decay, act, self.col_v, beta, cache.state, batch, o, H, G, d, dv)
         y = torch.empty((T, H * dv), dtype=self.dtype, device=dev)
         ops.delta_out(o, self.norm_w, self.eps, g, y, H, dv)
         return self.out.forward(y)

@@ -4,7 +4,8 @@ request's state slot (float32, zero at admission).  Both run on one scan,
     S_t = diag(w_t) S_{t-1} + a_t (b_t^T S_{t-1}) + k_t v_t^T,      o_t = S_t^T r_t        (`ops.recurrence_scan`)
 
 with everything that enters it in float32; what differs is how a layer makes w, a, b, k, v, r
-from its input h.
+from its input h.  In bfloat16, portions of many tokens take the scan in blocks of 16 tokens
+(`ops.recurrence_blocks`), float32 sums in another order.
 
 `ForgetGateRecurrence` (the HGRN2 form of linear attention): H heads, d key and dv value channels,
 
@@ -36,7 +37,8 @@ from .linear import Linear
 
 
 class ForgetGateRecurrence(Mixer):
-    graph_safe = True          # forward launches kernels over device tensors of the batch only
+    graph_safe = True          # forward launches kernels over device tensors of the batch only (never the blocks while a step is recorded)
+    blocks = True              # tests: off, portions of many tokens stay on the sequential scan
 
     def __init__(self, width: int, heads: int, key_dim: int, value_dim: int, norm_eps: float, dtype: torch.dtype, device, prefix: str,
                  names=("q", "f", "v", "o", "lower", "norm")):
@@ -68,7 +70,8 @@ class ForgetGateRecurrence(Mixer):
         H, d, dv = self.H, self.d, self.dv
         fused = self.in_proj.forward(x)
         r, w, k, v = ops.forget_gates(fused, self.col_q, self.col_f, self.col_v, self.f_bias, self.lower, H * d, H * dv)
-        o = ops.recurrence_scan(r, w, k, v, None, None, cache.state, 0, batch, H, d, dv)
+        scan = ops.recurrence_blocks if self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d) else ops.recurrence_scan
+        o = scan(r, w, k, v, None, None, cache.state, 0, batch, H, d, dv)
         y = torch.empty((x.shape[0], H * dv), dtype=self.dtype, device=x.device)
         ops.head_norm_gate(o, self.norm_w, self.eps, None, 0, y, H, dv)
         return self.out.forward(y)
@@ -76,6 +79,7 @@ class ForgetGateRecurrence(Mixer):
 
 class RemovalDeltaMixer(Mixer):
     graph_safe = True
+    blocks = True              # tests: off, portions of many tokens stay on the sequential scan
 
     def __init__(self, width: int, heads: int, dim: int, decay_rank: int, decay_rate: float, norm_eps: float, dtype: torch.dtype, device,
                  prefix: str):
@@ -113,7 +117,8 @@ class RemovalDeltaMixer(Mixer):
         wz = self.w2.forward(ops.partial_columns_act(fused, self.col_w1, self.rank, self.dtype, "tanh"))
         r, w, k, v, a, b = ops.removal_gates(fused, self.col_r, self.col_k, self.col_v, self.col_a, self.a_bias, wz, self.w0, self.decay_rate,
                                              H, d)
-        o = ops.recurrence_scan(r, w, k, v, a, b, cache.state, 0, batch, H, d, d)
+        scan = ops.recurrence_blocks if self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d) else ops.recurrence_scan
+        o = scan(r, w, k, v, a, b, cache.state, 0, batch, H, d, d)
         y = torch.empty((x.shape[0], H * d), dtype=self.dtype, device=x.device)
         ops.head_norm_gate(o, self.norm_w, self.eps, fused, self.col_g, y, H, d)
         return self.out.forward(y)

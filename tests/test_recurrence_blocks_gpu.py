@@ -1,0 +1,111 @@
+"""The recurrences in blocks of 16 tokens against a float64 evaluation and against the sequential scans they stand in for."""
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+COUNTS = [(1,), (15, 16), (17, 1, 40), (33, 160), (16, 48, 31, 2)]      # edges of a block, one token, many blocks, requests side by side
+
+
+def _step(counts, seed):
+    import torch
+    cu = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    slots = np.random.default_rng(seed).permutation(len(counts) + 1)[:len(counts)].astype(np.int32)
+    return SimpleNamespace(num_tokens=int(cu[-1]), num_seqs=len(counts), max_count=max(counts), captured=False,
+                           cu_seqlens=torch.from_numpy(cu).cuda(), slots=torch.from_numpy(slots).cuda()), cu, slots
+
+
+def _decays(rng, shape):
+    """Mostly a memory of some tens of tokens; some channels forget at once, one in fifty to the smallest numbers there are."""
+    w = np.exp(-rng.exponential(0.05, shape))
+    w = np.where(rng.random(shape) < 0.1, rng.random(shape) * 0.1, w)
+    return np.where(rng.random(shape) < 0.02, 1e-38, w)
+
+
+def _check(name, blocks, scan, want):
+    """Both kernels sum in float32.  A block's solved system and its decayed operands take up to a few sums of 16 more than the sequential
+    form: the distance from float64 is allowed to be three times the scan's and 2^-21 of the largest number, whichever is more."""
+    scale = np.abs(want).max()
+    err, ref = np.abs(blocks - want).max() / scale, np.abs(scan - want).max() / scale
+    assert np.isfinite(blocks).all() and err <= max(3.0 * ref, 2.0 ** -21), f"{name}: {err:.2e} of the largest, the scan {ref:.2e}"
+
+
+@pytest.mark.parametrize("counts", COUNTS)
+@pytest.mark.parametrize("H,d,dv", [(3, 64, 128), (2, 128, 128), (2, 100, 24), (1, 20, 17), (4, 32, 16), (1, 7, 1)])
+@pytest.mark.parametrize("correction", [False, True])
+def test_recurrence_in_blocks(counts, H, d, dv, correction):
+    import torch
+    from kestrel_llm_b200.csrc import ops
+    rng = np.random.default_rng(d + len(counts))
+    batch, cu, slots = _step(counts, d)
+    T = batch.num_tokens
+    r, k, v = rng.standard_normal((T, H, d)), rng.standard_normal((T, H, d)), rng.standard_normal((T, H, dv))
+    w = _decays(rng, (T, H, d))
+    u = k / np.sqrt((k * k).sum(-1, keepdims=True) + 1e-6)
+    a, b = (-rng.random((T, H, d)) * u, u) if correction else (None, None)
+    off = 8
+    state0 = rng.standard_normal((len(counts) + 1, off + H * d * dv + 4))
+
+    def f32(x):
+        return None if x is None else torch.from_numpy(np.ascontiguousarray(x.reshape(x.shape[0], -1), dtype=np.float32)).cuda()
+    args = [f32(x) for x in (r, w, k, v, a, b)]
+    r, w, k, v, a, b = (None if x is None else t.cpu().numpy().astype(np.float64).reshape(x.shape) for x, t in zip((r, w, k, v, a, b), args))
+    got = {}
+    for name, fn in (("blocks", ops.recurrence_blocks), ("scan", ops.recurrence_scan)):
+        state = f32(state0)
+        out = fn(*args, state, off, batch, H, d, dv)
+        got[name] = out.cpu().numpy().astype(np.float64), state.cpu().numpy().astype(np.float64)
+    ops.raise_on_kernel_error()
+    want_o, want_s = np.zeros((T, H, dv)), f32(state0).cpu().numpy().astype(np.float64)
+    for i, slot in enumerate(slots):
+        S = want_s[slot, off:off + H * d * dv].reshape(H, d, dv).copy()
+        for t in range(cu[i], cu[i + 1]):
+            new = w[t][:, :, None] * S + k[t][:, :, None] * v[t][:, None, :]
+            if correction:
+                new += a[t][:, :, None] * np.einsum("hd,hdv->hv", b[t], S)[:, None, :]
+            S = new
+            want_o[t] = np.einsum("hdv,hd->hv", S, r[t])
+        want_s[slot, off:off + H * d * dv] = S.reshape(-1)
+    _check("read-outs", got["blocks"][0], got["scan"][0], want_o.reshape(T, -1))
+    _check("states", got["blocks"][1], got["scan"][1], want_s)
+
+
+@pytest.mark.parametrize("counts", COUNTS)
+@pytest.mark.parametrize("H,G,d,dv", [(4, 2, 128, 128), (2, 2, 64, 40), (3, 1, 24, 20), (2, 1, 128, 8)])
+def test_delta_rule_in_blocks(counts, H, G, d, dv):
+    import torch
+    from kestrel_llm_b200.csrc import ops
+    rng = np.random.default_rng(d + dv)
+    batch, cu, slots = _step(counts, dv)
+    T = batch.num_tokens
+
+    def unit(x):
+        return x / np.sqrt((x * x).sum(-1, keepdims=True) + 1e-6)
+
+    def f32(x):
+        return torch.from_numpy(np.ascontiguousarray(x.reshape(x.shape[0], -1), dtype=np.float32)).cuda()
+    q, k = f32(unit(rng.standard_normal((T, G, d))) * d ** -0.5), f32(unit(rng.standard_normal((T, G, d))))
+    decay, beta = f32(_decays(rng, (T, H, d))), f32(rng.random((T, H)))
+    act = f32(rng.standard_normal((T, 5 + H * dv)))                    # the values stand behind other columns
+    state0 = f32(rng.standard_normal((len(counts) + 1, H * d * dv + 12)))
+    got = {}
+    for name, fn in (("blocks", ops.delta_blocks), ("scan", ops.delta_scan)):
+        state, out = state0.clone(), torch.empty((T, H * dv), dtype=torch.float32, device="cuda")
+        fn(q, k, decay, act, 5, beta, state, batch, out, H, G, d, dv)
+        got[name] = out.cpu().numpy().astype(np.float64), state.cpu().numpy().astype(np.float64)
+    ops.raise_on_kernel_error()
+    q, k, w, bt, vals, want_s = (x.cpu().numpy().astype(np.float64) for x in (q, k, decay, beta, act, state0))
+    q, k = (np.repeat(x.reshape(T, G, d), H // G, axis=1) for x in (q, k))
+    w, v, want_o = w.reshape(T, H, d), vals[:, 5:].reshape(T, H, dv), np.zeros((T, H, dv))
+    for i, slot in enumerate(slots):
+        S = want_s[slot, :H * d * dv].reshape(H, d, dv).copy()
+        for t in range(cu[i], cu[i + 1]):
+            S = w[t][:, :, None] * S
+            u = bt[t][:, None] * (v[t] - np.einsum("hdv,hd->hv", S, k[t]))
+            S = S + k[t][:, :, None] * u[:, None, :]
+            want_o[t] = np.einsum("hdv,hd->hv", S, q[t])
+        want_s[slot, :H * d * dv] = S.reshape(-1)
+    _check("read-outs", got["blocks"][0], got["scan"][0], want_o.reshape(T, -1))
+    _check("states", got["blocks"][1], got["scan"][1], want_s)
