@@ -1733,13 +1733,16 @@ def recurrence_scan(r: torch.Tensor, w: torch.Tensor, k: torch.Tensor, v: torch.
     return out
 
 
-BLOCK_TOKENS = 32       # a step whose longest portion has as many tokens takes the recurrences in blocks
+BLOCK_TOKENS, BLOCK_TOKENS_ALL = 112, 256       # in blocks: as many tokens of one request, or a quarter of them where the step has as many in all
 
 
 def recurrence_in_blocks(batch, dtype: torch.dtype, d: int) -> bool:
     """Whether a step runs its recurrences in blocks of 16 tokens.  Not in float32, whose logits are the same bits however a request was
-    cut, and not in a recorded step."""
-    return dtype == torch.bfloat16 and not batch.captured and batch.max_count >= BLOCK_TOKENS and d <= 128
+    cut, and not in a recorded step.  One request's scan of few tokens ends before two launches do (16 heads, scan against blocks: 64
+    tokens 10 / 12 us without a correction, 21 / 26 with one, 23 / 27 the delta rule; 128 tokens 19 / 21, 41 / 32, 45 / 32); several
+    requests' scans share the SMs and lose earlier (eight of 32 tokens: 20 / 16, 56 / 42, 43 / 38)."""
+    enough = batch.max_count >= BLOCK_TOKENS or (4 * batch.max_count >= BLOCK_TOKENS and batch.num_tokens >= BLOCK_TOKENS_ALL)
+    return dtype == torch.bfloat16 and not batch.captured and enough and d <= 128
 
 
 def _block_scratch(T: int, batch, H: int, d: int, form: int, device) -> torch.Tensor:
