@@ -4,8 +4,10 @@
 // the true 32-bit path, the fallback of the bfloat16 path for sizes the tensor-core kernel
 // refuses, and the twin that the tensor-core kernel is tested against.  Any T, N, K.
 //
-// Tile 64x64, 256 threads, 4x4 outputs per thread, K in steps of 16 through shared memory.
+// float32 operands whose rows 16-byte copies can fetch go to the kernel of gemm_f32.cuh, the same bits; this one
+// takes the others: tile 64x64, 256 threads, 4x4 outputs per thread, K in steps of 16 through shared memory.
 #include "common.cuh"
+#include "gemm_f32.cuh"
 
 #define PG_BM 64
 #define PG_BN 64
@@ -75,6 +77,20 @@ KESTREL_API int kestrel_gemm_plain(const void *x, const void *w, float *out, int
                                    cudaStream_t stream) {
     if (T == 0) return 0;
     KESTREL_REQUIRE(T > 0 && N > 0 && K > 0, "gemm_plain: bad sizes T=%d N=%d K=%d", T, N, K);
+    if (dtype == KESTREL_F32 && K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
+        // The largest tile of which there are two a SM; beyond that what few tokens waste of a tile counts (a tile of 64 rows for 16 tokens
+        // of N = 32,000 takes 225 us, one of 16 rows 113).  Measured, N = 2,048, K = 6,144 | N = 12,288, K = 2,048 in us, beside the one tile
+        // of 64 x 64 in steps of 16 this replaces: T = 1 30 | 28 (619 | 407), T = 8 40 | 31 (618 | 411), T = 100 167 | 171 (593 | 472),
+        // T = 411 306 | 545 (1,188 | 1,195), T = 2,048 1,158 | 2,266 (2,477 | 4,578).
+        const float *xf = (const float *)x, *wf = (const float *)w;
+        const long long want = 2ll * kestrel_sms();
+        auto tiles = [&](int bm, int bn) { return (long long)((T + bm - 1) / bm) * ((N + bn - 1) / bn); };
+        if (T > 32 && tiles(64, 64) >= want) return gf_launch<64, 64, 8, 4, 32, 3>(xf, wf, out, T, N, K, ldx, ldw, ldo, stream);
+        if (T > 16 && tiles(32, 32) >= want) return gf_launch<32, 32, 4, 4, 32, 4>(xf, wf, out, T, N, K, ldx, ldw, ldo, stream);
+        if (T > 8) return gf_launch<16, 32, 4, 2, 64, 6>(xf, wf, out, T, N, K, ldx, ldw, ldo, stream);
+        if (T > 4 && tiles(8, 32) >= want) return gf_launch<8, 32, 2, 2, 64, 6>(xf, wf, out, T, N, K, ldx, ldw, ldo, stream);
+        return gf_launch<4, 16, 1, 1, 128, 6>(xf, wf, out, T, N, K, ldx, ldw, ldo, stream);
+    }
     dim3 grid((N + PG_BN - 1) / PG_BN, (T + PG_BM - 1) / PG_BM);
     KESTREL_REQUIRE(grid.y <= 65535, "gemm_plain: T=%d needs more than 65535 row tiles", T);
     if (dtype == KESTREL_F32)

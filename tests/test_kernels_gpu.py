@@ -38,6 +38,21 @@ def test_gemm_plain(dtype, T, N, K):
     np.testing.assert_allclose(out.cpu().numpy(), ref, rtol=0, atol=2e-6 * math.sqrt(K) * np.abs(ref).max() + 1e-7)
 
 
+@pytest.mark.parametrize("T", [1, 4, 5, 8, 9, 16, 17, 33, 64, 65, 130, 411])
+@pytest.mark.parametrize("N,K", [(16, 4), (17, 68), (300, 132), (2048, 200), (12300, 64)])
+def test_gemm_plain_has_the_same_bits_on_every_tile(T, N, K):
+    """float32 in tiles of five sizes, against the kernel that takes weights 16-byte copies cannot fetch: both sum in ascending k."""
+    import torch
+    from kestrel_llm_b200.csrc import ops
+    x, w = torch.randn(T, K, device=DEV), torch.randn(N, K, device=DEV)
+    odd = torch.empty(N * K + 1, device=DEV)[1:].view(N, K)
+    odd.copy_(w)
+    fast, plain = (torch.full((T, N), float("nan"), device=DEV) for _ in range(2))
+    ops.gemm_plain(x, w, fast)
+    ops.gemm_plain(x, odd, plain)
+    assert torch.equal(fast, plain)
+
+
 def test_gemm_plain_is_the_same_for_any_batch():
     ops = _ops()
     x, _ = _rand((70, 333), torch.float32, 3)
