@@ -160,6 +160,166 @@ attention_plain_kernel(const T *__restrict__ q, const T *__restrict__ k_cache, c
     }
 }
 
+// The same attention for float32 layers that see every earlier token and have no options: up to eight rows - (token, head) pairs of one kv
+// head and request - a block, the warps' streams of keys and every sum of a row as above, so that a row's bits still depend on its position
+// alone, whatever rows share its block.  One row a block read every key again for each row and spent five shuffles, ten
+// additions and five exponentials in all lanes on a key of a row; here a warp reads four keys for all rows, the 32 dot products of four
+// keys and eight rows take 31 exchanges together (the same tree over the lanes), a lane makes the exponential of one of them, and
+// the weights go through shared memory: 411 tokens of 16 / 4 heads 604 -> 72 us, bound by the issue of what is left.
+#define PR_ROWS 8
+
+template <int N, int MASK> __device__ __forceinline__ void pr_exchange(float *x, int lane) {
+    const bool up = (lane & MASK) != 0;
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+        const float keep = up ? x[i + N / 2] : x[i], give = up ? x[i] : x[i + N / 2];
+        x[i] = keep + __shfl_xor_sync(0xffffffffu, give, MASK);
+    }
+}
+
+// C: channels of a lane; chunk: heads of a kv head's group that a block takes, tokens: tokens of its rows
+template <int C>
+__global__ void __launch_bounds__(PA_WARPS * 32)
+attention_plain_rows_kernel(const float *__restrict__ q, const float *__restrict__ k_cache, const float *__restrict__ v_cache,
+                            const int *__restrict__ positions, const int *__restrict__ seq_of_token, const int *__restrict__ block_table,
+                            int table_stride, int page_size, float *__restrict__ out, int T, int nq, int nkv, int hd, int vd, int v_ld,
+                            const float *__restrict__ gate, float scale, int chunk, int tokens) {
+    __shared__ float sm_m[PA_WARPS][PR_ROWS], sm_l[PA_WARPS][PR_ROWS], sm_acc[PA_WARPS][PR_ROWS][C * 32];
+    __shared__ __align__(16) float sm_p[PA_WARPS][PR_ROWS][4], sm_c[PA_WARPS][PR_ROWS];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int G = nq / nkv, chunks = (G + chunk - 1) / chunk;
+    const int kvh = blockIdx.y / chunks, h0 = kvh * G + (blockIdx.y % chunks) * chunk;
+    const int heads = min(chunk, (kvh + 1) * G - h0);
+    const int tile = (int)gridDim.x - 1 - (int)blockIdx.x;                  // late tokens see the most keys: they go first
+    const int t_end = min(T, (tile + 1) * tokens);
+    for (int ta = tile * tokens; ta < t_end;) {
+        // the tile's tokens of one request
+        const int seq = seq_of_token[ta];
+        int tb = ta + 1;
+        while (tb < t_end && seq_of_token[tb] == seq) ++tb;
+        const int rows = (tb - ta) * heads;
+        const int *table = block_table + (size_t)seq * table_stride;
+        float qv[PR_ROWS][C], acc[PR_ROWS][C];
+#pragma unroll
+        for (int r = 0; r < PR_ROWS; ++r)
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const int i = lane + 32 * c;
+                qv[r][c] = r < rows && i < hd ? q[((size_t)(ta + r / heads) * nq + h0 + r % heads) * hd + i] : 0.f;
+                acc[r][c] = 0.f;
+            }
+        // this lane's row among the softmax lanes (row lane / 4, key lane % 4 of a group), and the keys it sees
+        const int my_row = lane >> 2, my_key = lane & 3;
+        const int my_keys = my_row < rows ? positions[ta + my_row / heads] + 1 : 0;
+        int n_keys = my_keys;
+#pragma unroll
+        for (int o = 16; o >= 4; o >>= 1) n_keys = max(n_keys, __shfl_xor_sync(0xffffffffu, n_keys, o));
+        float m = -INFINITY, l = 0.f;
+        float kk[PA_KEYS][C], vv[PA_KEYS][C];
+        auto load = [&](int base) {
+#pragma unroll
+            for (int u = 0; u < PA_KEYS; ++u) {
+                const int s = base + u;
+                const bool in = s < n_keys;
+                const size_t row = in ? ((size_t)table[s / page_size] * nkv + kvh) * page_size + s % page_size : 0;
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    const int i = lane + 32 * c;
+                    kk[u][c] = in && i < hd ? k_cache[row * hd + i] : 0.f;
+                    vv[u][c] = in && i < vd ? v_cache[row * v_ld + i] : 0.f;
+                }
+            }
+        };
+        for (int base = warp * PA_KEYS; base < n_keys; base += PA_WARPS * PA_KEYS) {
+            load(base);
+            float x[4 * PR_ROWS];
+#pragma unroll
+            for (int r = 0; r < PR_ROWS; ++r)
+#pragma unroll
+                for (int u = 0; u < PA_KEYS; ++u) {
+                    float dot = 0.f;
+#pragma unroll
+                    for (int c = 0; c < C; ++c) dot = fmaf(qv[r][c], kk[u][c], dot);
+                    x[r * 4 + u] = dot;
+                }
+            pr_exchange<32, 16>(x, lane);
+            pr_exchange<16, 8>(x, lane);
+            pr_exchange<8, 4>(x, lane);
+            pr_exchange<4, 2>(x, lane);
+            pr_exchange<2, 1>(x, lane);
+            const bool seen = base + my_key < my_keys;
+            const uint32_t visible = __ballot_sync(0xffffffffu, seen);        // bit 4 r + u: row r sees key u of the group
+            const float sc = seen ? x[0] * scale : -INFINITY;
+            float mn = fmaxf(sc, __shfl_xor_sync(0xffffffffu, sc, 1));
+            mn = fmaxf(m, fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 2)));
+            const bool any = base < my_keys;              // a row that sees none of the group's keys stays as it is
+            const float corr = any ? expf(m - mn) : 1.f;
+            const float p = seen ? expf(sc - mn) : 0.f;
+            if (any) m = mn;
+            __syncwarp();
+            sm_p[warp][my_row][my_key] = p;
+            if (my_key == 0) sm_c[warp][my_row] = corr;
+            __syncwarp();
+            const float4 mine = *reinterpret_cast<const float4 *>(sm_p[warp][my_row]);
+            l = __fmul_rn(l, corr);
+            l = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(l, mine.x), mine.y), mine.z), mine.w);
+#pragma unroll
+            for (int r = 0; r < PR_ROWS; ++r) {
+                const float4 pr = *reinterpret_cast<const float4 *>(sm_p[warp][r]);
+                const float cr = sm_c[warp][r];
+                const float w[4] = {pr.x, pr.y, pr.z, pr.w};
+#pragma unroll
+                for (int c = 0; c < C; ++c) acc[r][c] = __fmul_rn(acc[r][c], cr);
+                // a key that the row does not see adds nothing, whatever its value (0 x inf would not be 0)
+#pragma unroll
+                for (int u = 0; u < PA_KEYS; ++u)
+#pragma unroll
+                    for (int c = 0; c < C; ++c) acc[r][c] = (visible >> (4 * r + u)) & 1u ? fmaf(w[u], vv[u][c], acc[r][c]) : acc[r][c];
+            }
+        }
+        // merge the warps' states in warp order: a warp closes two rows
+        if (my_key == 0) {
+            sm_m[warp][my_row] = m;
+            sm_l[warp][my_row] = l;
+        }
+#pragma unroll
+        for (int r = 0; r < PR_ROWS; ++r)
+#pragma unroll
+            for (int c = 0; c < C; ++c) sm_acc[warp][r][lane + 32 * c] = acc[r][c];
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < PR_ROWS / PA_WARPS; ++e) {
+            const int r = warp * (PR_ROWS / PA_WARPS) + e;
+            if (r >= rows) continue;
+            float M = -INFINITY, L = 0.f, o[C];
+#pragma unroll
+            for (int w = 0; w < PA_WARPS; ++w) M = fmaxf(M, sm_m[w][r]);
+#pragma unroll
+            for (int c = 0; c < C; ++c) o[c] = 0.f;
+#pragma unroll
+            for (int w = 0; w < PA_WARPS; ++w) {
+                if (sm_m[w][r] == -INFINITY) continue;              // a warp that saw no key
+                const float f = expf(sm_m[w][r] - M);
+                L = fmaf(sm_l[w][r], f, L);
+#pragma unroll
+                for (int c = 0; c < C; ++c) o[c] = fmaf(sm_acc[w][r][lane + 32 * c], f, o[c]);
+            }
+            const size_t at = (size_t)(ta + r / heads) * nq + h0 + r % heads;
+            float inv = 1.0f / L;
+            if (gate) inv *= gate[at];
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const int i = lane + 32 * c;
+                if (i < vd) out[at * vd + i] = o[c] * inv;
+            }
+        }
+        ta = tb;
+        if (ta < t_end) __syncthreads();
+    }
+}
+
 KESTREL_API int kestrel_attention_plain_scored(const void *q, const void *k_cache, const void *v_cache,
                                                const int *positions, const int *seq_of_token,
                                                const int *block_table, int table_stride, int page_size,
@@ -204,6 +364,22 @@ KESTREL_API int kestrel_attention_plain_to(const void *q, const void *k_cache, c
     KESTREL_REQUIRE(hd <= 32 * PA_MAX_PER_LANE && vd <= 32 * PA_MAX_PER_LANE, "attention_plain: head size %d / %d exceeds %d", hd, vd, 32 * PA_MAX_PER_LANE);
     KESTREL_REQUIRE(nq <= 65535, "attention_plain: %d query heads exceed the grid", nq);
     dim3 grid(T, nq);
+    // Whether a layer takes the kernel of eight rows depends on the layer alone, not on the step: a row has the same bits in every step.
+    if (dtype == KESTREL_F32 && window == 0 && softcap == 0.f && !r1 && !rel && weighting == KESTREL_WEIGH_SOFTMAX && hd <= 128 && vd <= 128 && nq % nkv == 0) {
+        const int G = nq / nkv, chunk = G < PR_ROWS ? G : PR_ROWS, chunks = (G + chunk - 1) / chunk;
+        // several tokens a block where there are blocks enough, tokens of one request mostly then
+        int tokens = PR_ROWS / chunk;
+        while (tokens > 1 && (long long)((T + tokens - 1) / tokens) * nkv * chunks < 2 * kestrel_sms()) --tokens;
+        const dim3 rows_grid((T + tokens - 1) / tokens, nkv * chunks);
+        KESTREL_REQUIRE(rows_grid.y <= 65535, "attention_plain: %d query heads exceed the grid", nq);
+        if (hd <= 64 && vd <= 64)
+            kestrel_launch(attention_plain_rows_kernel<2>, rows_grid, dim3(PA_WARPS * 32), 0, stream, (const float *)q, (const float *)k_cache, (const float *)v_cache, positions,
+                           seq_of_token, block_table, table_stride, page_size, (float *)out, T, nq, nkv, hd, vd, v_ld > 0 ? v_ld : vd, gate, scale, chunk, tokens);
+        else
+            kestrel_launch(attention_plain_rows_kernel<4>, rows_grid, dim3(PA_WARPS * 32), 0, stream, (const float *)q, (const float *)k_cache, (const float *)v_cache, positions,
+                           seq_of_token, block_table, table_stride, page_size, (float *)out, T, nq, nkv, hd, vd, v_ld > 0 ? v_ld : vd, gate, scale, chunk, tokens);
+        return kestrel_check_launch("attention_plain");
+    }
     if (dtype == KESTREL_F32)
         kestrel_launch(attention_plain_kernel<float, float>, dim3(grid), dim3(PA_WARPS * 32), 0, stream, (const float *)q, (const float *)k_cache, (const float *)v_cache, positions, seq_of_token,
             block_table, table_stride, page_size, (float *)out, nq, nkv, hd, vd, v_ld > 0 ? v_ld : vd, window, keep_first, gate, scale, opts);

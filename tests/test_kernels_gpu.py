@@ -371,6 +371,37 @@ def _paged(dense_k, dense_v, page_size, num_pages, seed):
     return kc, vc, pages.astype(np.int32)
 
 
+@pytest.mark.parametrize("nq,nkv,hd", [(4, 4, 64), (6, 2, 128), (10, 2, 40), (8, 1, 96), (12, 1, 128), (16, 4, 128)])
+@pytest.mark.parametrize("cuts", [((0, 1), (30, 1), (16, 1)), ((0, 37), (5, 1), (11, 70)), ((3, 2), (0, 3), (15, 17), (40, 1))])
+def test_float32_attention_of_eight_rows_a_block(nq, nkv, hd, cuts):
+    """Layers that see every earlier token, against a window as long as the request (the kernel of one row a block): the same sums, so
+    they agree to the last bits (2^-20: the sums of four streams and exp of both), and a row has the same bits alone and beside others,
+    also where a token behind it holds a value that is not finite."""
+    import torch
+    from kestrel_llm_b200.csrc import ops
+    torch.manual_seed(nq)
+    page, width = 16, 8
+    n = len(cuts)
+    k, v = (torch.randn(n * width, nkv, page, hd, device=DEV) for _ in range(2))
+    table = torch.randperm(n * width, dtype=torch.int32).view(n, width).to(DEV)
+    pos = torch.cat([torch.arange(a, a + c) for a, c in cuts]).to(torch.int32).to(DEV)
+    seq = torch.cat([torch.full((c,), i) for i, (_, c) in enumerate(cuts)]).to(torch.int32).to(DEV)
+    q = torch.randn(pos.shape[0], nq * hd, device=DEV)
+
+    def run(q, pos, seq, window, v):
+        out = torch.full_like(q, float("nan"))
+        ops.attention_plain(q, k, v, pos, seq, table, page, out, nq, nkv, hd, window, hd ** -0.5)
+        return out
+    whole, twin = run(q, pos, seq, 0, v), run(q, pos, seq, 1 << 20, v)
+    assert (whole - twin).abs().max() <= 2.0 ** -20 * twin.abs().max()
+    for t in (0, 1, pos.shape[0] // 2, pos.shape[0] - 1):
+        assert torch.equal(run(q[t:t + 1].contiguous(), pos[t:t + 1].contiguous(), seq[t:t + 1].contiguous(), 0, v)[0], whole[t])
+    late = v.clone()
+    a, c = cuts[-1]
+    late[table[n - 1, (a + c - 1) // page].item(), :, (a + c - 1) % page] = float("inf")
+    assert torch.equal(run(q, pos, seq, 0, late)[:-1], whole[:-1])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("nq,nkv,hd,window,page", [(6, 2, 32, 0, 16), (5, 5, 48, 40, 16), (8, 1, 128, 0, 4),
                                                    (3, 3, 80, 7, 16), (4, 2, 16, 0, 1), (2, 1, 256, 100, 32)])
