@@ -24,11 +24,13 @@
 // Three forms: GATE (no correction), REMOVAL (a, b given) and DELTA (a gated delta rule: with u = beta (v - (diag(w) S)^T k),
 // S <- diag(w) S + k u^T, so that b = w k and the writes u = X beta (v - b^T S_0) take the place of v).
 //
-// Measured, 16 heads, prepare + scan against the sequential scan: DELTA (128 channels, requests of 592 and 1,185 tokens) 53 + 132 us against
-// 523; GATE (64 channels, 2,048 tokens) 23 + 101 against 291; REMOVAL (128 channels, 700 tokens in three requests, 350 the longest) 34 + 69
-// against 205.  What is left of a block is the chain of its three products and their barriers.
+// Measured, 16 heads, gates and blocks prepared + scan against gates kernel + sequential scan: DELTA (128 channels, requests of 592 and 1,185
+// tokens) 67 + 131 us against 37 + 523; GATE (64 channels, 2,048 tokens) 22 + 101 against 27 + 291; REMOVAL (128 channels, 700 tokens in
+// three requests, 350 the longest) 50 + 63 against 55 + 205.  (With the gates still a kernel of its own: 36 + 53 + 132, 27 + 23 + 101 and
+// 56 + 34 + 69.)  The scan's blocks are the chain of three products and their barriers; the preparation is bound by its instructions.
 #include "common.cuh"
 #include "tcgen05.cuh"
+#include <initializer_list>
 #include <math.h>
 
 #define RB_B 16                 // tokens of a block
@@ -66,6 +68,27 @@ struct RbParams {
     int H, G, d, dv;
 };
 
+// Where the vectors come from when `blocks_prepare` makes them itself, as the gates kernels do, instead of reading what those left:
+// GATE and REMOVAL from the columns of a product x (r or q, k, v, f or rate logits), DELTA from x = the convolved q | k | v and, for beta,
+// the product y; z: the decay's product (REMOVAL, DELTA).  Sums over slices in ascending order; all rows and columns in whole vectors of four.
+struct RbSource {
+    const float *x, *y, *z;
+    int Sx, Sy, Sz, ldx, ldy, ldz, col_r, col_k, col_v, col_a;      // col_a: rate logits (REMOVAL), f (GATE), beta logits in y (DELTA)
+    size_t x_stride, y_stride, z_stride;
+    const float *bias, *bias2;                  // GATE: f_bias, lower; REMOVAL: a_bias, w_bias; DELTA: dt_bias, A_log
+    float rate;
+    float *v_out;                               // [T, H dv]: the values' slices summed, or null where they are one slice and read from there
+};
+__device__ __forceinline__ float4 rb_sum4(const float *p, int S, size_t stride) {
+    float4 v = *reinterpret_cast<const float4 *>(p);
+    for (int s = 1; s < S; ++s) {
+        const float4 x = *reinterpret_cast<const float4 *>(p + (size_t)s * stride);
+        v.x += x.x, v.y += x.y, v.z += x.z, v.w += x.w;
+    }
+    return v;
+}
+__device__ __forceinline__ float rb_sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
+
 // One exchange of a sum of N values over the lanes: a lane keeps the half of the values that its bit of MASK names and adds the other
 // lane's share of them.  Five of them, from 32 values, leave lane l with the sum of value l.
 template <int N, int MASK> __device__ __forceinline__ void rb_exchange(float *x, int lane) {
@@ -77,9 +100,9 @@ template <int N, int MASK> __device__ __forceinline__ void rb_exchange(float *x,
     }
 }
 
-template <int D, int FORM>
+template <int D, int FORM, bool MADE>
 __global__ void __launch_bounds__(128)
-blocks_prepare_kernel(const RbParams p) {
+blocks_prepare_kernel(const RbParams p, const RbSource src) {
     using L = RbLayout<D, FORM>;
     constexpr int V = D / 32;                   // channels of a lane
     pdl_launch_dependents();
@@ -94,9 +117,100 @@ blocks_prepare_kernel(const RbParams p) {
     float *mA = mat, *mK = mA + RB_MAT, *mQa = mK + RB_MAT, *mQk = mQa + RB_MAT, *mX = mQk + RB_MAT, *mY = mX + RB_MAT;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kh = FORM == RB_DELTA ? h / (p.H / p.G) : h, KH = FORM == RB_DELTA ? p.G : p.H;
-    __shared__ float sbeta[RB_B];
-    if (FORM == RB_DELTA && tid < RB_B) sbeta[tid] = t0 + tid < t1 ? p.beta[(size_t)(t0 + tid) * p.H + h] : 0.f;
-    const bool vec = p.d % 4 == 0 && (((uintptr_t)p.r | (uintptr_t)p.w | (uintptr_t)p.k | (uintptr_t)p.a | (uintptr_t)p.b) & 15) == 0;
+    __shared__ float sbeta[RB_B], sinv[2][RB_B];
+    if (FORM == RB_DELTA && !MADE && tid < RB_B) sbeta[tid] = t0 + tid < t1 ? p.beta[(size_t)(t0 + tid) * p.H + h] : 0.f;
+    const bool vec = MADE || (p.d % 4 == 0 && (((uintptr_t)p.r | (uintptr_t)p.w | (uintptr_t)p.k | (uintptr_t)p.a | (uintptr_t)p.b) & 15) == 0);
+    if (MADE) {
+        constexpr int N = RB_B * D / 512;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 rs[N], ks[N], as[N], zs[N];       // all of a thread's loads in flight together, then the gates
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int idx = (tid + 128 * i) * 4, t = idx / D, c = idx % D;
+            rs[i] = ks[i] = as[i] = zs[i] = zero;
+            if (t0 + t < t1 && c < p.d) {
+                const float *row = src.x + (size_t)(t0 + t) * src.ldx;
+                rs[i] = rb_sum4(row + src.col_r + kh * p.d + c, src.Sx, src.x_stride);
+                if (FORM != RB_GATE) ks[i] = rb_sum4(row + src.col_k + kh * p.d + c, src.Sx, src.x_stride);
+                if (FORM != RB_DELTA) as[i] = rb_sum4(row + src.col_a + h * p.d + c, src.Sx, src.x_stride);
+                if (FORM != RB_GATE) zs[i] = rb_sum4(src.z + (size_t)(t0 + t) * src.ldz + h * p.d + c, src.Sz, src.z_stride);
+            }
+        }
+        const float A = FORM == RB_DELTA ? expf(src.bias2[h]) : 0.f;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int idx = (tid + 128 * i) * 4, t = idx / D, c = idx % D;
+            float4 r4 = rs[i], k4 = ks[i], a4 = as[i], w4 = make_float4(1.f, 1.f, 1.f, 1.f);
+            if (t0 + t < t1 && c < p.d) {
+                float *r = &r4.x, *k = &k4.x, *a = &a4.x, *w = &w4.x;
+                const float *z = &zs[i].x;
+                const int hc = h * p.d + c;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    if (FORM == RB_GATE) {
+                        const float lo = src.bias2 ? src.bias2[hc + e] : 0.f;
+                        w[e] = lo + (1.0f - lo) * rb_sigmoid(a[e] + (src.bias ? src.bias[hc + e] : 0.f));
+                        r[e] *= rb_sigmoid(r[e]);
+                        k[e] = 1.0f - w[e];
+                    } else if (FORM == RB_REMOVAL) {
+                        a[e] = rb_sigmoid(a[e] + (src.bias ? src.bias[hc + e] : 0.f));
+                        w[e] = expf(-src.rate * rb_sigmoid(z[e] + (src.bias2 ? src.bias2[hc + e] : 0.f)));
+                    } else {
+                        const float x = z[e] + src.bias[hc + e];
+                        w[e] = expf(-A * (x > 20.f ? x : log1pf(expf(x))));
+                    }
+                }
+            }
+            *reinterpret_cast<float4 *>(sw + idx) = w4;
+            *reinterpret_cast<float4 *>(sr + idx) = r4;
+            *reinterpret_cast<float4 *>(sk + idx) = k4;
+            if (FORM == RB_REMOVAL) *reinterpret_cast<float4 *>(sa + idx) = a4;
+        }
+        if (FORM == RB_DELTA && tid < RB_B) {
+            float z = 0.f;
+            if (t0 + tid < t1) z = sum_slices(src.y, src.Sy, src.y_stride, (size_t)(t0 + tid) * src.ldy + src.col_a + h);
+            sbeta[tid] = t0 + tid < t1 ? rb_sigmoid(z) : 0.f;
+        }
+        if (FORM != RB_DELTA && src.v_out)
+            for (int idx = tid; idx < RB_B * p.dv; idx += 128) {
+                const int t = t0 + idx / p.dv, c = h * p.dv + idx % p.dv;
+                if (t < t1) src.v_out[(size_t)t * p.H * p.dv + c] = sum_slices(src.x, src.Sx, src.x_stride, (size_t)t * src.ldx + src.col_v + c);
+            }
+        if (FORM != RB_GATE) {                  // unit keys (DELTA: and queries): a warp a token's head, four tokens a warp
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < RB_B / 4; ++i) {
+                const int t = warp * (RB_B / 4) + i;
+                float sk2 = 0.f, sr2 = 0.f;
+#pragma unroll
+                for (int j = 0; j < V; ++j) {
+                    const float k = sk[t * D + lane * V + j], r = sr[t * D + lane * V + j];
+                    sk2 = fmaf(k, k, sk2);
+                    sr2 = fmaf(r, r, sr2);
+                }
+                sk2 = warp_sum(sk2);
+                if (FORM == RB_DELTA) sr2 = warp_sum(sr2);
+                if (lane == 0) {
+                    sinv[0][t] = 1.0f / sqrtf(sk2 + 1e-6f);
+                    sinv[1][t] = (1.0f / sqrtf(sr2 + 1e-6f)) * (1.0f / sqrtf((float)p.d));
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < RB_B * D / 128; ++i) {
+                const int idx = tid + 128 * i, t = idx / D;
+                const float u = sk[idx] * sinv[0][t];
+                if (FORM == RB_REMOVAL) {
+                    sb[idx] = u;
+                    sa[idx] = -(sa[idx] * u);
+                } else {
+                    sk[idx] = u;
+                    sr[idx] *= sinv[1][t];
+                    sb[idx] = sw[idx] * u;
+                }
+            }
+        }
+    } else
     if (vec) {                                  // all of a thread's loads in flight together
         constexpr int N = RB_B * D / 512;
         float4 w4[N], r4[N], k4[N], a4[FORM == RB_REMOVAL ? N : 1], b4[FORM == RB_REMOVAL ? N : 1];
@@ -166,7 +280,8 @@ blocks_prepare_kernel(const RbParams p) {
             run *= sw[t * D + c];
         }
     }
-    // the pairs: a warp takes four tokens s, evenly long walks t = s .. 15 among them; eight t's sums go through the lanes together
+    // the pairs: a warp takes four tokens s, evenly long walks t = s .. 15 among them; the sums of TG t's go through the lanes together
+    constexpr int TG = FORM == RB_REMOVAL ? 8 : RB_B;
 #pragma unroll 1
     for (int i = 0; i < 4; ++i) {
         const int s = i == 0 ? warp : i == 1 ? 7 - warp : i == 2 ? 8 + warp : 15 - warp;
@@ -177,11 +292,11 @@ blocks_prepare_kernel(const RbParams p) {
             xa[j] = FORM == RB_REMOVAL ? sa[s * D + lane * V + j] : 0.f;
         }
 #pragma unroll 1
-        for (int half = s >> 3; half < 2; ++half) {
-            float x[32];                        // [t][A, K, Qa, Qk]
+        for (int part = s / TG; part < RB_B / TG; ++part) {
+            float x[32];                        // [t][the form's matrices]
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int t = half * 8 + u;
+            for (int u = 0; u < TG; ++u) {
+                const int t = part * TG + u;
                 float fA = 0.f, fK = 0.f, fQa = 0.f, fQk = 0.f;
                 if (t >= s) {
 #pragma unroll
@@ -201,18 +316,27 @@ blocks_prepare_kernel(const RbParams p) {
                         if (FORM == RB_REMOVAL) fQa = fmaf(rr, xa[j], fQa);
                     }
                 }
-                x[4 * u] = fA;
-                x[4 * u + 1] = fK;
-                x[4 * u + 2] = fQa;
-                x[4 * u + 3] = fQk;
+                if (FORM == RB_REMOVAL) x[4 * u] = fA, x[4 * u + 1] = fK, x[4 * u + 2] = fQa, x[4 * u + 3] = fQk;
+                else if (FORM == RB_DELTA) x[2 * u] = fK, x[2 * u + 1] = fQk;
+                else x[u] = fQk;
             }
-            rb_exchange<32, 16>(x, lane);
-            rb_exchange<16, 8>(x, lane);
-            rb_exchange<8, 4>(x, lane);
-            rb_exchange<4, 2>(x, lane);
-            rb_exchange<2, 1>(x, lane);
-            // lane l holds value l: token half * 8 + l / 4, matrix l % 4
-            mat[(lane & 3) * RB_MAT + (half * 8 + (lane >> 2)) * RB_LD + s] = x[0];
+            // lane l ends with value l (GATE: l / 2)
+            if (FORM == RB_GATE) {
+                rb_exchange<16, 16>(x, lane);
+                rb_exchange<8, 8>(x, lane);
+                rb_exchange<4, 4>(x, lane);
+                rb_exchange<2, 2>(x, lane);
+                x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
+                mQk[(lane >> 1) * RB_LD + s] = x[0];
+            } else {
+                rb_exchange<32, 16>(x, lane);
+                rb_exchange<16, 8>(x, lane);
+                rb_exchange<8, 4>(x, lane);
+                rb_exchange<4, 2>(x, lane);
+                rb_exchange<2, 1>(x, lane);
+                if (FORM == RB_REMOVAL) mat[(lane & 3) * RB_MAT + (part * TG + (lane >> 2)) * RB_LD + s] = x[0];
+                else (lane & 1 ? mQk : mK)[(lane >> 1) * RB_LD + s] = x[0];
+            }
         }
     }
     __syncthreads();
@@ -510,18 +634,21 @@ static long long rb_floats(int D, int form) {
 }
 
 template <int D, int FORM>
-static int rb_launch(const RbParams &p, int nseq, int max_count, cudaStream_t stream) {
+static int rb_launch(const RbParams &p, const RbSource *src, int nseq, int max_count, cudaStream_t stream) {
     static_assert(RbLayout<D, FORM>::FLOATS % 4 == 0, "bulk copies move 16 bytes");
     const size_t prep = (size_t)((FORM == RB_GATE ? 3 : FORM == RB_DELTA ? 4 : 5) * RB_B * D + 6 * RB_MAT) * sizeof(float);
     constexpr size_t stage = (size_t)RbLayout<D, FORM>::FLOATS * sizeof(float), fixed = 18 * 1024;    // beside the ring: under 18 KB of static memory
     static bool attr_set = false;
     if (!attr_set) {
-        if (cudaFuncSetAttribute(blocks_prepare_kernel<D, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep) != cudaSuccess ||
+        if (cudaFuncSetAttribute(blocks_prepare_kernel<D, FORM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep) != cudaSuccess ||
+            cudaFuncSetAttribute(blocks_prepare_kernel<D, FORM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep) != cudaSuccess ||
             cudaFuncSetAttribute(blocks_scan_kernel<D, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(KESTREL_SMEM_MAX_DYNAMIC - fixed)) != cudaSuccess)
             return kestrel_fail(-3, "recurrence_blocks: cannot set the shared memory size");
         attr_set = true;
     }
-    kestrel_launch(blocks_prepare_kernel<D, FORM>, dim3((max_count + RB_B - 1) / RB_B, p.H, nseq), dim3(128), prep, stream, p);
+    const dim3 blocks((max_count + RB_B - 1) / RB_B, p.H, nseq);
+    if (src) kestrel_launch(blocks_prepare_kernel<D, FORM, true>, blocks, dim3(128), prep, stream, p, *src);
+    else kestrel_launch(blocks_prepare_kernel<D, FORM, false>, blocks, dim3(128), prep, stream, p, RbSource());
     static_assert(RbLayout<D, FORM>::FLOATS * 8 + 18 * 1024 <= KESTREL_SMEM_MAX_DYNAMIC, "two stages fit an SM");
     const dim3 grid((p.dv + RB_COLS - 1) / RB_COLS, p.H, nseq);
     // as many stages as the CTAs that share an SM leave room for, two at least
@@ -532,11 +659,11 @@ static int rb_launch(const RbParams &p, int nseq, int max_count, cudaStream_t st
 }
 
 template <int FORM>
-static int rb_run(const RbParams &p, int nseq, int max_count, cudaStream_t stream) {
+static int rb_run(const RbParams &p, int nseq, int max_count, cudaStream_t stream, const RbSource *src = nullptr) {
     switch (rb_padded(p.d)) {
-        case 32: return rb_launch<32, FORM>(p, nseq, max_count, stream);
-        case 64: return rb_launch<64, FORM>(p, nseq, max_count, stream);
-        default: return rb_launch<128, FORM>(p, nseq, max_count, stream);
+        case 32: return rb_launch<32, FORM>(p, src, nseq, max_count, stream);
+        case 64: return rb_launch<64, FORM>(p, src, nseq, max_count, stream);
+        default: return rb_launch<128, FORM>(p, src, nseq, max_count, stream);
     }
 }
 
@@ -577,6 +704,63 @@ KESTREL_API int kestrel_delta_blocks(const float *qn, const float *kn, const flo
     const int rc = rb_check(p, T, nseq, max_count, scratch_floats, RB_DELTA);
     if (rc) return rc;
     return rb_run<RB_DELTA>(p, nseq, max_count, stream);
+}
+
+// Whether vectors of four fetch everything that a kernel with gates reads
+static bool rb_whole(int d, std::initializer_list<long long> sizes, std::initializer_list<const void *> ptrs) {
+    bool ok = d % 4 == 0;
+    for (const long long x : sizes) ok = ok && x % 4 == 0;
+    for (const void *p : ptrs) ok = ok && ((uintptr_t)p & 15) == 0;
+    return ok;
+}
+
+// The whole recurrence of a mixer in blocks, its gates included: forget_gates / removal_gates (wz not null) and recurrence_scan.  x: the product,
+// S slices; vsum: scratch [T, H dv] for the values of a product of several slices (may be null for one).  Returns 1 if vectors of four do not fit.
+KESTREL_API int kestrel_gated_blocks(const float *x, int S, long long slice_stride, int ld, int col_r, int col_k, int col_v, int col_a,
+                                     const float *bias, const float *bias2, const float *wz, int Sw, long long w_stride, float rate, float *vsum,
+                                     float *state, long long state_stride, const int *cu_seqlens, const int *slots, float *out, float *scratch,
+                                     long long scratch_floats, int T, int nseq, int max_count, int H, int d, int dv, cudaStream_t stream) {
+    if (T == 0 || nseq == 0) return 0;
+    KESTREL_REQUIRE(S > 0 && (!wz || Sw > 0) && (S == 1 || vsum), "gated_blocks: bad slices");
+    if (!rb_whole(d, {slice_stride, ld, col_r, col_k, col_a, w_stride}, {x, wz})) return 1;
+    RbSource src = {};
+    src.x = x; src.Sx = S; src.x_stride = (size_t)slice_stride; src.ldx = ld;
+    src.z = wz; src.Sz = Sw; src.z_stride = (size_t)w_stride; src.ldz = H * d;
+    src.col_r = col_r; src.col_k = col_k; src.col_v = col_v; src.col_a = col_a;
+    src.bias = bias; src.bias2 = bias2; src.rate = rate;
+    src.v_out = S > 1 ? vsum : nullptr;
+    RbParams p = {};
+    p.v = S > 1 ? vsum : x + col_v;
+    p.ldv = S > 1 ? (size_t)H * dv : (size_t)ld;
+    p.state = state; p.state_stride = (size_t)state_stride; p.cu_seqlens = cu_seqlens; p.slots = slots; p.out = out; p.blocks = scratch;
+    p.H = H; p.G = H; p.d = d; p.dv = dv;
+    const int rc = rb_check(p, T, nseq, max_count, scratch_floats, wz ? RB_REMOVAL : RB_GATE);
+    if (rc) return rc;
+    return wz ? rb_run<RB_REMOVAL>(p, nseq, max_count, stream, &src) : rb_run<RB_GATE>(p, nseq, max_count, stream, &src);
+}
+
+// delta_gates (a decay per head and channel) and delta_scan in blocks.  act [T, C] = q | k | v after the convolution; beta logits at col_beta of
+// the product y, decay logits the product a [T, H d].  Returns 1 if vectors of four do not fit.
+KESTREL_API int kestrel_gated_delta_blocks(const float *act, int C, int col_v, const float *y, int Sy, long long y_stride, int ldy, int col_beta,
+                                           const float *a, int Sa, long long a_stride, const float *A_log, const float *dt_bias, float *state,
+                                           long long state_stride, const int *cu_seqlens, const int *slots, float *out, float *scratch,
+                                           long long scratch_floats, int T, int nseq, int max_count, int H, int G, int d, int dv, cudaStream_t stream) {
+    if (T == 0 || nseq == 0) return 0;
+    KESTREL_REQUIRE(Sy > 0 && Sa > 0, "gated_delta_blocks: bad slices");
+    if (!rb_whole(d, {C, a_stride}, {act, a})) return 1;
+    RbSource src = {};
+    src.x = act; src.Sx = 1; src.ldx = C; src.col_r = 0; src.col_k = G * d;
+    src.y = y; src.Sy = Sy; src.y_stride = (size_t)y_stride; src.ldy = ldy; src.col_a = col_beta;
+    src.z = a; src.Sz = Sa; src.z_stride = (size_t)a_stride; src.ldz = H * d;
+    src.bias = dt_bias; src.bias2 = A_log;
+    RbParams p = {};
+    p.v = act + col_v;
+    p.ldv = (size_t)C;
+    p.state = state; p.state_stride = (size_t)state_stride; p.cu_seqlens = cu_seqlens; p.slots = slots; p.out = out; p.blocks = scratch;
+    p.H = H; p.G = G; p.d = d; p.dv = dv;
+    const int rc = rb_check(p, T, nseq, max_count, scratch_floats, RB_DELTA);
+    if (rc) return rc;
+    return rb_run<RB_DELTA>(p, nseq, max_count, stream, &src);
 }
 
 // Error word of the bounded waits (0: none, 1: a block's copy).  Synchronises the device and clears the word.

@@ -1799,6 +1799,59 @@ def delta_blocks(qn: torch.Tensor, kn: torch.Tensor, decay: torch.Tensor, act: t
     launches += 1
 
 
+def gated_blocks(fused: Partials, col_r: int, col_k: int, col_v: int, col_a: int, bias: Optional[torch.Tensor], bias2: Optional[torch.Tensor],
+                 wz: Optional[Partials], rate: float, state: torch.Tensor, batch, H: int, d: int, dv: int) -> Optional[torch.Tensor]:
+    """`forget_gates` (``wz`` None: ``col_a`` the forget logits, ``bias`` and ``bias2`` their bias and the lower bound) or `removal_gates`
+    (``bias`` the rates', ``bias2`` the decays') and `recurrence_blocks` in two launches; None if the sizes are no vectors of four."""
+    T, dev = fused.tokens, fused.data.device
+    _need(state, "gated_blocks.state", torch.float32, 2)
+    if fused.bias is not None or (wz is not None and (wz.bias is not None or wz.tokens != T or wz.width != H * d)):
+        raise KernelError("gated_blocks: shapes differ, or a bias is pending")
+    if T != batch.num_tokens or max(col_r + H * d, col_v + H * dv, col_a + H * d, (col_k + H * d) if wz is not None else 0) > fused.width or \
+            H * d * dv > state.shape[1]:
+        raise KernelError("gated_blocks: the product does not fit the heads, or the state not the slot")
+    for t, n in ((bias, H * d), (bias2, H * d)):
+        if t is not None and t.numel() != n:
+            raise KernelError("gated_blocks: a bias does not fit the heads")
+    out = torch.empty((T, H * dv), dtype=torch.float32, device=dev)
+    vsum = torch.empty((T, H * dv), dtype=torch.float32, device=dev) if fused.slices > 1 else None
+    scratch = _block_scratch(T, batch, H, d, 0 if wz is None else 1, dev)
+    rc = library().kestrel_gated_blocks(fused.data.data_ptr(), fused.slices, fused.slice_stride, fused.width, int(col_r), int(col_k), int(col_v),
+                                        int(col_a), _p(bias), _p(bias2), _p(wz.data) if wz is not None else None, wz.slices if wz is not None else 0,
+                                        wz.slice_stride if wz is not None else 0, float(rate), _p(vsum), state.data_ptr(), state.stride(0),
+                                        batch.cu_seqlens.data_ptr(), batch.slots.data_ptr(), out.data_ptr(), scratch.data_ptr(), scratch.numel(), T,
+                                        batch.num_seqs, batch.max_count, H, d, dv, _stream())
+    return _blocks_done(rc, out)
+
+
+def _blocks_done(rc: int, out: torch.Tensor) -> Optional[torch.Tensor]:
+    if rc == 1:
+        return None
+    _check(rc)
+    global launches
+    launches += 1
+    return out
+
+
+def gated_delta_blocks(act: torch.Tensor, col_v: int, x: Partials, col_beta: int, a: Partials, A_log: torch.Tensor, dt_bias: torch.Tensor,
+                       state: torch.Tensor, batch, out: torch.Tensor, H: int, G: int, d: int, dv: int) -> bool:
+    """`delta_gates` (a decay per head and channel) and `delta_blocks` in two launches; False if the sizes are no vectors of four."""
+    T = act.shape[0]
+    _need(act, "gated_delta_blocks.act", torch.float32, 2)
+    _need(state, "gated_delta_blocks.state", torch.float32, 2)
+    _need(out, "gated_delta_blocks.out", torch.float32, 2)
+    if T != batch.num_tokens or a.tokens != T or x.tokens != T or a.width != H * d or out.shape != (T, H * dv) or x.width < col_beta + H or \
+            act.shape[1] < max(2 * G * d, col_v + H * dv) or A_log.numel() != H or dt_bias.numel() != H * d or H * d * dv > state.shape[1]:
+        raise KernelError("gated_delta_blocks: shapes differ")
+    scratch = _block_scratch(T, batch, H, d, 2, out.device)
+    rc = library().kestrel_gated_delta_blocks(act.data_ptr(), act.shape[1], int(col_v), x.data.data_ptr(), x.slices, x.slice_stride, x.width,
+                                              int(col_beta), a.data.data_ptr(), a.slices, a.slice_stride, A_log.data_ptr(), dt_bias.data_ptr(),
+                                              state.data_ptr(), state.stride(0), batch.cu_seqlens.data_ptr(), batch.slots.data_ptr(),
+                                              out.data_ptr(), scratch.data_ptr(), scratch.numel(), T, batch.num_seqs, batch.max_count, H, G, d, dv,
+                                              _stream())
+    return _blocks_done(rc, out) is not None
+
+
 def recurrence_scan_bonus(r: torch.Tensor, w: torch.Tensor, k: torch.Tensor, v: torch.Tensor, u: torch.Tensor, state: torch.Tensor,
                           state_off: int, batch, H: int, d: int, dv: int) -> torch.Tensor:
     """o = (S + diag(u) k v^T)^T r of the OLD state, then S <- diag(w) S + k v^T, per head; otherwise as `recurrence_scan`."""

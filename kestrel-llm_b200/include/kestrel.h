@@ -233,6 +233,10 @@ KESTREL_API long long kestrel_recurrence_blocks_floats(int T, int nseq, int H, i
 KESTREL_API int kestrel_recurrence_blocks(const float *r, const float *w, const float *k, const float *v, const float *a, const float *b, float *state, long long state_stride, long long state_off, const int *cu_seqlens, const int *slots, float *out, float *scratch, long long scratch_floats, int T, int nseq, int max_count, int H, int d, int dv, kestrel_stream_t stream);
 /* v: [T, ldv], head h's values at column h * dv */
 KESTREL_API int kestrel_delta_blocks(const float *qn, const float *kn, const float *decay, const float *v, long long ldv, const float *beta, float *state, long long state_stride, const int *cu_seqlens, const int *slots, float *out, float *scratch, long long scratch_floats, int T, int nseq, int max_count, int H, int G, int d, int dv, kestrel_stream_t stream);
+/* forget_gates (wz NULL; bias f_bias, bias2 lower, col_a the f column) or removal_gates (bias a_bias, bias2 w_bias) and the recurrence in blocks, two launches; vsum: scratch [T, H dv] where S > 1; returns 1 without a launch if vectors of four floats do not fit the sizes */
+KESTREL_API int kestrel_gated_blocks(const float *x, int S, long long slice_stride, int ld, int col_r, int col_k, int col_v, int col_a, const float *bias, const float *bias2, const float *wz, int Sw, long long w_stride, float rate, float *vsum, float *state, long long state_stride, const int *cu_seqlens, const int *slots, float *out, float *scratch, long long scratch_floats, int T, int nseq, int max_count, int H, int d, int dv, kestrel_stream_t stream);
+/* delta_gates with a decay per head and channel (a [T, H d]) and delta_scan the same way */
+KESTREL_API int kestrel_gated_delta_blocks(const float *act, int C, int col_v, const float *y, int Sy, long long y_stride, int ldy, int col_beta, const float *a, int Sa, long long a_stride, const float *A_log, const float *dt_bias, float *state, long long state_stride, const int *cu_seqlens, const int *slots, float *out, float *scratch, long long scratch_floats, int T, int nseq, int max_count, int H, int G, int d, int dv, kestrel_stream_t stream);
 KESTREL_API int kestrel_recurrence_blocks_error(void);
 
 /* ---- attention over cached latents (attention_latent.cu) ---- */

@@ -83,14 +83,17 @@ class ChannelDeltaMixer(Mixer):
         ops.short_conv(fused, self.conv_w, None, cache.state, self.tail_off, batch, act)
         a = self.a2.forward(ops.partial_columns(fused, self.col_a1, self.ra, self.dtype))
         g = self.g2.forward(ops.partial_columns(fused, self.col_g1, self.rg, self.dtype))
-        qn = torch.empty((T, G * d), dtype=f32, device=dev)
-        kn = torch.empty((T, G * d), dtype=f32, device=dev)
-        decay = torch.empty((T, H * d), dtype=f32, device=dev)
-        beta = torch.empty((T, H), dtype=f32, device=dev)
-        ops.delta_gates(act, fused, self.col_beta, a, self.A_log, self.dt_bias, qn, kn, decay, beta, H, G, d)
         o = torch.empty((T, H * dv), dtype=f32, device=dev)
-        scan = ops.delta_blocks if self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d) else ops.delta_scan
-        scan(qn, kn, decay, act, self.col_v, beta, cache.state, batch, o, H, G, d, dv)
+        in_blocks = self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d)
+        if not (in_blocks and ops.gated_delta_blocks(act, self.col_v, fused, self.col_beta, a, self.A_log, self.dt_bias, cache.state, batch, o,
+                                                     H, G, d, dv)):
+            qn = torch.empty((T, G * d), dtype=f32, device=dev)
+            kn = torch.empty((T, G * d), dtype=f32, device=dev)
+            decay = torch.empty((T, H * d), dtype=f32, device=dev)
+            beta = torch.empty((T, H), dtype=f32, device=dev)
+            ops.delta_gates(act, fused, self.col_beta, a, self.A_log, self.dt_bias, qn, kn, decay, beta, H, G, d)
+            scan = ops.delta_blocks if in_blocks else ops.delta_scan
+            scan(qn, kn, decay, act, self.col_v, beta, cache.state, batch, o, H, G, d, dv)
         y = torch.empty((T, H * dv), dtype=self.dtype, device=dev)
         ops.delta_out(o, self.norm_w, self.eps, g, y, H, dv)
         return self.out.forward(y)

@@ -69,9 +69,13 @@ class ForgetGateRecurrence(Mixer):
     def forward(self, x: torch.Tensor, batch, cache) -> ops.Partials:
         H, d, dv = self.H, self.d, self.dv
         fused = self.in_proj.forward(x)
-        r, w, k, v = ops.forget_gates(fused, self.col_q, self.col_f, self.col_v, self.f_bias, self.lower, H * d, H * dv)
-        scan = ops.recurrence_blocks if self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d) else ops.recurrence_scan
-        o = scan(r, w, k, v, None, None, cache.state, 0, batch, H, d, dv)
+        o, in_blocks = None, self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d)
+        if in_blocks:
+            o = ops.gated_blocks(fused, self.col_q, 0, self.col_v, self.col_f, self.f_bias, self.lower, None, 0.0, cache.state, batch, H, d, dv)
+        if o is None:
+            r, w, k, v = ops.forget_gates(fused, self.col_q, self.col_f, self.col_v, self.f_bias, self.lower, H * d, H * dv)
+            scan = ops.recurrence_blocks if in_blocks else ops.recurrence_scan
+            o = scan(r, w, k, v, None, None, cache.state, 0, batch, H, d, dv)
         y = torch.empty((x.shape[0], H * dv), dtype=self.dtype, device=x.device)
         ops.head_norm_gate(o, self.norm_w, self.eps, None, 0, y, H, dv)
         return self.out.forward(y)
@@ -115,10 +119,15 @@ class RemovalDeltaMixer(Mixer):
         H, d = self.H, self.d
         fused = self.in_proj.forward(x)
         wz = self.w2.forward(ops.partial_columns_act(fused, self.col_w1, self.rank, self.dtype, "tanh"))
-        r, w, k, v, a, b = ops.removal_gates(fused, self.col_r, self.col_k, self.col_v, self.col_a, self.a_bias, wz, self.w0, self.decay_rate,
-                                             H, d)
-        scan = ops.recurrence_blocks if self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d) else ops.recurrence_scan
-        o = scan(r, w, k, v, a, b, cache.state, 0, batch, H, d, d)
+        o, in_blocks = None, self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d)
+        if in_blocks:
+            o = ops.gated_blocks(fused, self.col_r, self.col_k, self.col_v, self.col_a, self.a_bias, self.w0, wz, self.decay_rate, cache.state,
+                                 batch, H, d, d)
+        if o is None:
+            r, w, k, v, a, b = ops.removal_gates(fused, self.col_r, self.col_k, self.col_v, self.col_a, self.a_bias, wz, self.w0,
+                                                 self.decay_rate, H, d)
+            scan = ops.recurrence_blocks if in_blocks else ops.recurrence_scan
+            o = scan(r, w, k, v, a, b, cache.state, 0, batch, H, d, d)
         y = torch.empty((x.shape[0], H * d), dtype=self.dtype, device=x.device)
         ops.head_norm_gate(o, self.norm_w, self.eps, fused, self.col_g, y, H, d)
         return self.out.forward(y)

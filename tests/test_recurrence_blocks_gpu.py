@@ -109,3 +109,79 @@ def test_delta_rule_in_blocks(counts, H, G, d, dv):
         want_s[slot, :H * d * dv] = S.reshape(-1)
     _check("read-outs", got["blocks"][0], got["scan"][0], want_o.reshape(T, -1))
     _check("states", got["blocks"][1], got["scan"][1], want_s)
+
+
+def _evaluate(r, w, k, v, a, b, state, cu, slots):
+    """Read-outs and states in float64 from float32 operands [T, H, .]."""
+    out, state = np.zeros(v.shape), state.copy()
+    H, d, dv = r.shape[1], r.shape[2], v.shape[2]
+    for i, slot in enumerate(slots):
+        S = state[slot, :H * d * dv].reshape(H, d, dv).copy()
+        for t in range(cu[i], cu[i + 1]):
+            new = w[t][:, :, None] * S + k[t][:, :, None] * v[t][:, None, :]
+            if a is not None:
+                new += a[t][:, :, None] * np.einsum("hd,hdv->hv", b[t], S)[:, None, :]
+            S = new
+            out[t] = np.einsum("hdv,hd->hv", S, r[t])
+        state[slot, :H * d * dv] = S.reshape(-1)
+    return out.reshape(out.shape[0], -1), state
+
+
+def _product(rng, S, T, N):
+    import torch
+    from kestrel_llm_b200.csrc import ops
+    return ops.Partials(torch.from_numpy(rng.standard_normal((S, T, N)).astype(np.float32) / S ** 0.5).cuda())
+
+
+@pytest.mark.parametrize("counts", COUNTS[1:])
+@pytest.mark.parametrize("H,d,dv", [(3, 64, 128), (2, 128, 128), (2, 100, 17), (1, 20, 24), (4, 32, 16)])
+@pytest.mark.parametrize("S", [1, 3])
+@pytest.mark.parametrize("form", ["gate", "removal", "delta"])
+def test_blocks_with_their_gates(counts, H, d, dv, S, form):
+    """The gates made where the blocks are prepared against the gates kernels and the scan, from one slice of the product and from three;
+    some decays and rates at the ends of their ranges."""
+    import torch
+    from kestrel_llm_b200.csrc import ops
+    rng = np.random.default_rng(d + S)
+    batch, cu, slots = _step(counts, d)
+    T, n, nv = batch.num_tokens, H * d, H * dv
+
+    def vec(m, scale=1.0, shift=0.0):
+        x = rng.standard_normal(m) * scale + shift
+        return torch.from_numpy(np.where(rng.random(m) < 0.05, -60.0, x).astype(np.float32)).cuda()
+    state0 = torch.from_numpy(rng.standard_normal((len(counts) + 1, H * d * dv)).astype(np.float32)).cuda()
+    sa, sb = state0.clone(), state0.clone()
+    f64 = lambda x, m: x.cpu().numpy().astype(np.float64).reshape(T, H, m)       # noqa: E731
+    if form == "gate":
+        x, bias, lower = _product(rng, S, T, 2 * n + nv + 4 + -nv % 4), vec(n, 1.0, 2.0), torch.rand(n, device="cuda") * 0.5
+        r, w, k, v = ops.forget_gates(x, 0, n, 2 * n, bias, lower, n, nv)
+        scan = ops.recurrence_scan(r, w, k, v, None, None, sa, 0, batch, H, d, dv)
+        got = ops.gated_blocks(x, 0, 0, 2 * n, n, bias, lower, None, 0.0, sb, batch, H, d, dv)
+        want, ws = _evaluate(f64(r, d), f64(w, d), f64(k, d), f64(v, dv), None, None, state0.cpu().numpy().astype(np.float64), cu, slots)
+    elif form == "removal":
+        if dv != d:
+            pytest.skip("the generalised delta rule has values of its keys' size")
+        x, wz, ab, w0 = _product(rng, S, T, 5 * n + 8), _product(rng, S, T, n), vec(n), vec(n, 1.0, -1.0)
+        r, w, k, v, a, b = ops.removal_gates(x, 0, n, 2 * n, 3 * n, ab, wz, w0, 0.6, H, d)
+        scan = ops.recurrence_scan(r, w, k, v, a, b, sa, 0, batch, H, d, dv)
+        got = ops.gated_blocks(x, 0, n, 2 * n, 3 * n, ab, w0, wz, 0.6, sb, batch, H, d, dv)
+        want, ws = _evaluate(*(f64(y, d) for y in (r, w, k, v, a, b)), state0.cpu().numpy().astype(np.float64), cu, slots)
+    else:
+        G = 2 if H % 2 == 0 else 1
+        C = 2 * G * d + nv + (-(2 * G * d + nv) % 4)
+        act = _product(rng, 1, T, C).data[0]
+        x, az, A, dt = _product(rng, S, T, H + 5), _product(rng, S, T, n), vec(H, 1.0, -0.5).clamp_(-3, 3), vec(n, 1.0, -1.0)
+        dt[::17] = 30.0
+        q, k, w = (torch.empty((T, m), device="cuda") for m in (G * d, G * d, n))
+        beta, scan, got = (torch.empty((T, m), device="cuda") for m in (H, nv, nv))
+        ops.delta_gates(act, x, 3, az, A, dt, q, k, w, beta, H, G, d)
+        ops.delta_scan(q, k, w, act, 2 * G * d, beta, sa, batch, scan, H, G, d, dv)
+        assert ops.gated_delta_blocks(act, 2 * G * d, x, 3, az, A, dt, sb, batch, got, H, G, d, dv)
+        rep = lambda y: np.repeat(y.cpu().numpy().astype(np.float64).reshape(T, G, d), H // G, axis=1)       # noqa: E731
+        w, k, bt = f64(w, d), rep(k), beta.cpu().numpy().astype(np.float64)[:, :, None]
+        v = f64(act[:, 2 * G * d:2 * G * d + nv].contiguous(), dv)
+        want, ws = _evaluate(rep(q), w, k, bt * v, -bt * k, w * k, state0.cpu().numpy().astype(np.float64), cu, slots)
+    ops.raise_on_kernel_error()
+    assert got is not None
+    _check("read-outs", got.cpu().numpy().astype(np.float64), scan.cpu().numpy().astype(np.float64), want)
+    _check("states", sb.cpu().numpy().astype(np.float64), sa.cpu().numpy().astype(np.float64), ws)
