@@ -273,13 +273,12 @@ KESTREL_API int kestrel_attention(void *planner, long long step_serial, const in
     const int gs = nq / nkv;
     const bool use_tc = kestrel_attention_tc_supported(hd, page_size) != 0;
     // The tcgen05 kernel takes two row tiles of 128 a CTA, so that the tensor cores work on one
-    // while the other is in its softmax.  Few rows leave SMs idle, one CTA per SM.  Where the keys
-    // are many the key range is cut into slices instead, as many as fill the SMs once, of at least
-    // 512 keys each, merged through scratch (a warp a row; measured alone, 4,096 keys of context:
-    // 512 tokens 86.7 -> 61.1 us with 2 slices, 256 tokens 81.6 -> 36.2 with 4, 64 tokens 78.7 ->
-    // 24.6 with 8; more CTAs than SMs lose again).  Where the keys are too few to cut, one row
-    // tile a CTA and twice the CTAs is the faster form (512 tokens from position 0: 20.2 -> 15.7 us;
-    // behind 1,024 keys 36.8 -> 31.2).
+    // while the other is in its softmax.  Few rows leave SMs idle, one CTA per SM.  While tiles of 128
+    // fit the SMs at once, a CTA takes one of them and its key tiles go to the two streams in turn:
+    // twice the CTAs, half of the chain each (500 tokens behind 750 keys 44 us with tiles of 256, 29
+    // with tiles of 128; 512 behind 4,000 84 and 49).  Where the keys are many the key range is cut
+    // into slices too, as many as fill the SMs once, of at least 512 keys each, merged through scratch
+    // (a warp a row; more CTAs than SMs lose again).
     int rows_large = use_tc ? 256 : kestrel_attention_mma_rows_per_tile(hd);
     int tc_slices = 1;
     const bool use_decode = kestrel_attention_decode_supported(hd, page_size) && gs <= 16;
@@ -297,21 +296,22 @@ KESTREL_API int kestrel_attention(void *planner, long long step_serial, const in
         if (tiles16 * nkv > kestrel_attention_decode_slots(hd)) small_rows = 16;
     }
     if (use_tc) {
-        // the portions of this step that go to this kernel: their rows, their tiles of 256, their longest context
+        // the portions of this step that go to this kernel: their tiles, their longest context
         const int *cu_h = batch_host + layout[KB_O_CU_SEQLENS], *kv_h = batch_host + layout[KB_O_KV_LENS];
-        long long rows = 0, tiles256 = 0;
+        long long tiles256 = 0, tiles128 = 0;
         int kv = 0;
         for (int i = 0; i < n; ++i) {
             const long long r = (long long)(cu_h[i + 1] - cu_h[i]) * gs;
             if (small_request(r, kv_h[i], small_rows)) continue;
-            rows += r;
             tiles256 += (r + 255) / 256;
+            tiles128 += (r + 127) / 128;
             kv = std::max(kv, kv_h[i]);
         }
         const int sms = kestrel_attention_tc_slots();
-        const int cand = window > 0 ? 1 : (int)std::min<long long>(std::min<long long>(sms / std::max<long long>(1, tiles256 * nkv), kv / 512), 16);
+        if (tiles128 * nkv <= sms) rows_large = 128;
+        const long long ctas = std::max<long long>(1, (rows_large == 128 ? tiles128 : tiles256) * nkv);
+        const int cand = window > 0 ? 1 : (int)std::min<long long>(std::min<long long>(sms / ctas, kv / 512), 16);
         if (cand >= 2 && (cand > 2 || kv >= 2048)) tc_slices = cand;
-        else if (rows * nkv <= 128ll * sms) rows_large = 128;
     }
     const Plan *plan = nullptr;
     int rc = plan_for(*pl, step_serial, batch_host, batch_dev, layout, gs, rows_large, small_rows, captured != 0, stream, &plan);

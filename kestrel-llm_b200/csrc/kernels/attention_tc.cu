@@ -135,7 +135,11 @@ enum {
     AT_KEPT = 5                 // AT_PLAIN over a window that keeps a request's first tokens, the heads' outputs gated
 };
 
-template <bool MAPS, int KIND>
+// HALVES: a CTA with one row tile (up to 128 rows).  Its key tiles then go to the two streams in turn - A takes the even ones, B the odd
+// ones, both over the same queries, stage t % 2 of the rings belonging to one stream - and the rows' two states, which lie in the same TMEM
+// lanes, are merged at the end, 64 columns a stream.  With one stream a tile's chain - scores, softmax, P, values - had nothing beside it:
+// 500 tokens of 32 / 8 heads behind 750 keys 40 -> 29 us, 512 behind 4,000 76 -> 49, 1,024 of 16 / 4 heads behind 3,000 71 -> 45.
+template <bool MAPS, int KIND, bool HALVES>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                     const AttnParams p, int cache_pages, int rows_per_tile) {
@@ -197,9 +201,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     auto key_base = [&](int t) { return KIND == AT_KEPT && t < n_kept ? t * AT_BN : k_lo + (t - n_kept) * AT_BN; };
     // row tile A ends earlier: it skips the key tiles beyond its last row
     const int rows_a = min(rows_here, AT_BM);
-    const bool has_b = MAPS || rows_here > AT_BM;
-    const int k_hi_a = MAPS ? k_hi : min(pos_begin + (row0 + rows_a - 1) / G + 1, (slice + 1) * slice_len);
-    const int n_tiles_a = MAPS ? n_tiles : has_b ? n_kept + (k_hi_a > k_lo ? (k_hi_a - k_lo + AT_BN - 1) / AT_BN : 0) : n_tiles;
+    const bool has_b = MAPS || HALVES || rows_here > AT_BM;
+    const int k_hi_a = MAPS || HALVES ? k_hi : min(pos_begin + (row0 + rows_a - 1) / G + 1, (slice + 1) * slice_len);
+    const int n_tiles_a = HALVES ? (n_tiles + 1) / 2 : MAPS ? n_tiles : has_b ? n_kept + (k_hi_a > k_lo ? (k_hi_a - k_lo + AT_BN - 1) / AT_BN : 0) : n_tiles;
 
     if (warp == 8 || warp == 10) {
         // ------------------------------------------------------------------ loaders
@@ -245,20 +249,20 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                     if (MAPS)           // map x: its own queries, panel x of the key tile
                         tc_mma(tmem + x * 128, smem_desc(q_s + x * TILE_BYTES + off), smem_desc(k_s + b * TILE_BYTES + x * AT_PANEL + off), IDESC_S, ks > 0 ? 1u : 0u);
                     else
-                        tc_mma(tmem + x * 128, smem_desc(q_s + x * TILE_BYTES + off), smem_desc(k_s + b * TILE_BYTES + off), IDESC_S, ks > 0 ? 1u : 0u);
+                        tc_mma(tmem + x * 128, smem_desc(q_s + (HALVES ? 0 : x * TILE_BYTES) + off), smem_desc(k_s + b * TILE_BYTES + off), IDESC_S, ks > 0 ? 1u : 0u);
                 }
                 tc_commit(bar(B_S_FULL + x));
             };
             // O_X (+)= P_X(t) V(t): P is read from the first 64 columns of S_X
             auto issue_pv = [&](int x, int t) {
                 const int b = t & 1;
-                if (!mbar_wait(bar(B_P_FULL + x), (uint32_t)t & 1u)) { atomicExch(&g_at_error, 2); return false; }
+                if (!mbar_wait(bar(B_P_FULL + x), (uint32_t)(HALVES ? t >> 1 : t) & 1u)) { atomicExch(&g_at_error, 2); return false; }
                 tc_fence_after();
 #pragma unroll
                 for (int ks = 0; ks < AT_BN / 16; ++ks) {
                     // A = P: keys 16 ks.. are columns 8 ks..; B = V: 16 keys down = 2 groups of 8 rows
                     uint64_t db = smem_desc_mn_major(v_s + b * TILE_BYTES + ks * 2048, AT_PANEL);
-                    tc_mma_ts(tmem + 256 + x * 128, tmem + x * 128 + ks * 8, db, IDESC_PV, (t > 0 || ks > 0) ? 1u : 0u);
+                    tc_mma_ts(tmem + 256 + x * 128, tmem + x * 128 + ks * 8, db, IDESC_PV, (t > (HALVES ? 1 : 0) || ks > 0) ? 1u : 0u);
                 }
                 tc_commit(bar(B_PV_DONE + x));
                 return true;
@@ -268,7 +272,26 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                 atomicExch(&g_at_error, 1);
                 return false;
             };
-            if (ok) ok = wait_k(0);
+            if (HALVES) {
+                // per stream: S(t) | PV(t), S(t + 2); tile t is stream t % 2's step t / 2, and so is its stage
+                for (int t = 0; t < min(2, n_tiles) && ok; ++t) {
+                    if (!(ok = wait_k(t))) break;
+                    issue_s(t, t);
+                    tc_commit(bar(B_K_EMPTY + t));
+                }
+                for (int t = 0; t < n_tiles && ok; ++t) {
+                    const int x = t & 1;
+                    if (!mbar_wait(bar(B_V_FULL + x), (uint32_t)(t >> 1) & 1u)) { atomicExch(&g_at_error, 6); ok = false; break; }
+                    if (!(ok = issue_pv(x, t))) break;
+                    tc_commit(bar(B_V_EMPTY + x));
+                    if (t + 2 < n_tiles) {
+                        if (!(ok = wait_k(t + 2))) break;
+                        issue_s(x, t + 2);
+                        tc_commit(bar(B_K_EMPTY + x));
+                    }
+                }
+                ok = false;                     // the loops below are the other forms'
+            } else if (ok) ok = wait_k(0);
             if (ok) {
                 if (n_tiles_a > 0) issue_s(0, 0);
                 if (has_b) issue_s(1, 0);
@@ -319,7 +342,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
             const int ld_c = tid & 15, ld_r0 = (tid >> 4) * 8;
             const uint32_t ld_panel = (uint32_t)(ld_c >> 3) * AT_PANEL;
 #pragma unroll
-            for (int xt = 0; xt < 2; ++xt) {
+            for (int xt = 0; xt < (HALVES ? 1 : 2); ++xt) {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     int rr = ld_r0 + j;
@@ -338,9 +361,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(B_Q_FULL));
         }
-        const int tile_row = MAPS ? row0 : row0 + x * AT_BM;             // the tile's first row among the request's
-        const int rows_x = x == 0 || MAPS ? rows_a : rows_here - AT_BM;  // rows of this row tile (<= 0: none)
-        const int n_tiles_x = x == 0 ? n_tiles_a : (has_b ? n_tiles : 0);
+        const int tile_row = MAPS || HALVES ? row0 : row0 + x * AT_BM;             // the tile's first row among the request's
+        const int rows_x = x == 0 || MAPS || HALVES ? rows_a : rows_here - AT_BM;  // rows of this row tile (<= 0: none)
+        const int n_tiles_x = x == 0 ? n_tiles_a : HALVES ? n_tiles / 2 : (has_b ? n_tiles : 0);
         const int k_hi_x = x == 0 ? k_hi_a : k_hi;
         const bool row_ok = r < rows_x;
         const int my_pos = row_ok ? pos_begin + (tile_row + r) / G : -1;
@@ -357,11 +380,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         const float eff_scale = RAW ? p.scale_log2 : 1.f;                // transformed scores are in base-2 units already
         bool ok = true;             // after a wait gave up the loop runs on without waiting, so that the warps still meet
 
-        for (int t = 0; t < n_tiles_x; ++t) {
-            const int b = t & 1;
+        for (int step = 0; step < n_tiles_x; ++step) {
+            const int t = HALVES ? 2 * step + x : step, b = t & 1;
             const int kbase = key_base(t);
             // S_X(t) is done - and with it, in the issuer's order, O_X += P_X(t-1) V(t-1)
-            if (ok && !mbar_wait(bar(B_S_FULL + x), (uint32_t)t & 1u)) { atomicExch(&g_at_error, 7); ok = false; }
+            if (ok && !mbar_wait(bar(B_S_FULL + x), (uint32_t)step & 1u)) { atomicExch(&g_at_error, 7); ok = false; }
             tc_fence_after();
             if (warp_has_rows) {
                 uint32_t sr[128];
@@ -565,6 +588,62 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                     *reinterpret_cast<uint4 *>(po + j) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
             }
+        } else if (HALVES) {
+            // both streams' last products, then the two states of a row as one
+            const int n_other = x == 0 ? n_tiles / 2 : n_tiles_a;
+            if (n_other > 0 && ok && !mbar_wait(bar(B_PV_DONE + (x ^ 1)), (uint32_t)(n_other - 1) & 1u)) { atomicExch(&g_at_error, 9); ok = false; }
+            tc_fence_after();
+            float m_a = -INFINITY, l_a = 0.f, m_b = -INFINITY, l_b = 0.f;
+            if (n_tiles > 0) {          // (a slice without keys: nothing has waited for all of Q, whose copies may still arrive)
+                float *xch = reinterpret_cast<float *>(aligned);             // Q's memory: every product that read it is done
+                xch[(x * 128 + r) * 2] = m_ref;
+                xch[(x * 128 + r) * 2 + 1] = l_run;
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                m_a = xch[2 * r], l_a = xch[2 * r + 1], m_b = xch[256 + 2 * r], l_b = xch[256 + 2 * r + 1];
+            }
+            const float m = fmaxf(m_a, m_b), f_a = m_a == -INFINITY ? 0.f : at_exp2(m_a - m), f_b = m_b == -INFINITY ? 0.f : at_exp2(m_b - m);
+            float l = l_a * f_a + l_b * f_b;
+            if (warp_has_rows) {
+                const bool write = row_ok && ok;
+                const int row = tile_row + r;
+                const size_t qrow = write ? (size_t)(tok_begin + row / G) * p.nq + kvh * G + row % G : 0;
+                float inv = p.slices > 1 ? 1.f : 1.0f / (sink ? l + at_exp2(hs.sink * 1.4426950408889634f - m) : l);
+                if (KIND == AT_KEPT && write && p.gate) inv *= p.gate[qrow];
+                const float i_a = f_a * inv, i_b = f_b * inv;
+#pragma unroll
+                for (int c = 0; c < 64; c += 32) {
+                    uint32_t oa[32], ob[32];
+                    at_ld32(tmem + lane_base + 256 + x * 64 + c, oa);             // warp-wide, whatever rows exist
+                    at_ld32(tmem + lane_base + 384 + x * 64 + c, ob);
+                    at_ld_wait();
+                    if (!write) continue;
+                    // a stream without a tile has left its columns as they were: not a number, perhaps
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        oa[j] = __float_as_uint((n_tiles > 0 ? __uint_as_float(oa[j]) * i_a : 0.f) + (n_tiles > 1 ? __uint_as_float(ob[j]) * i_b : 0.f));
+                    if (p.slices > 1) {
+                        float *po = p.part_o + (qrow * p.slices + slice) * AT_HD + x * 64 + c;
+#pragma unroll
+                        for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4 *>(po + j) = make_uint4(oa[j], oa[j + 1], oa[j + 2], oa[j + 3]);
+                    } else {
+                        __nv_bfloat16 *po = p.out + qrow * AT_HD + x * 64 + c;
+#pragma unroll
+                        for (int j = 0; j < 32; j += 8) {
+                            uint32_t w[4];
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(oa[j + 2 * k]), __uint_as_float(oa[j + 2 * k + 1]));
+                                w[k] = *reinterpret_cast<uint32_t *>(&b2);
+                            }
+                            *reinterpret_cast<uint4 *>(po + j) = make_uint4(w[0], w[1], w[2], w[3]);
+                        }
+                    }
+                }
+                if (write && p.slices > 1 && x == 0) {
+                    p.part_ml[(qrow * p.slices + slice) * 2] = m;
+                    p.part_ml[(qrow * p.slices + slice) * 2 + 1] = l;
+                }
+            }
         } else if (warp_has_rows) {
             const bool write = row_ok && ok;
             int row = tile_row + r;
@@ -622,17 +701,17 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     }
 }
 
-template <bool MAPS, int KIND>
+template <bool MAPS, int KIND, bool HALVES = false>
 static int at_launch(dim3 grid, cudaStream_t stream, const CUtensorMap &map_k, const CUtensorMap &map_v, const AttnParams &p, int cache_pages,
                      int rows_per_tile) {
     const size_t smem = 12 * AT_PANEL + 8 * B_COUNT + 16 + 1024;
     static bool attr_set = false;
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel<MAPS, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel<MAPS, KIND, HALVES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return kestrel_fail(-3, "attention_tc: cannot raise the shared-memory limit: %s", cudaGetErrorString(e));
         attr_set = true;
     }
-    kestrel_launch(attention_tc_kernel<MAPS, KIND>, grid, dim3(AT_THREADS), smem, stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    kestrel_launch(attention_tc_kernel<MAPS, KIND, HALVES>, grid, dim3(AT_THREADS), smem, stream, map_k, map_v, p, cache_pages, rows_per_tile);
     return 0;
 }
 
@@ -727,10 +806,17 @@ KESTREL_API int kestrel_attention_tc_biased(const void *q, const void *k_cache, 
     p.scored = scored ? 1 : 0;
     const bool capped = softcap > 0.f, dist = r1 != nullptr, sigmoid = weighting == KESTREL_WEIGH_SIGMOID;
     const dim3 grid((unsigned)((long long)tiles * nkv), 1, slices);
-    if (!capped && !dist && !rel && !sigmoid) rc = at_launch<false, AT_PLAIN>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
-    else if (capped && !dist && !rel && !sigmoid) rc = at_launch<false, AT_CAP>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    const bool halves = rows_per_tile <= AT_BM;         // one row tile: its key tiles by two streams (softmax weights: the states merge)
+    if (!capped && !dist && !rel && !sigmoid)
+        rc = halves ? at_launch<false, AT_PLAIN, true>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile)
+                    : at_launch<false, AT_PLAIN>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    else if (capped && !dist && !rel && !sigmoid)
+        rc = halves ? at_launch<false, AT_CAP, true>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile)
+                    : at_launch<false, AT_CAP>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
     else if (capped && dist && !rel && sigmoid) rc = at_launch<false, AT_CAP_DIST_SIGMOID>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
-    else if (rel && !capped && !dist && weighting == KESTREL_WEIGH_SOFTMAX) rc = at_launch<false, AT_REL>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    else if (rel && !capped && !dist && weighting == KESTREL_WEIGH_SOFTMAX)
+        rc = halves ? at_launch<false, AT_REL, true>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile)
+                    : at_launch<false, AT_REL>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
     else rc = at_launch<false, AT_ANY>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
     if (rc) return rc;
     rc = kestrel_check_launch("attention_tc");
@@ -754,7 +840,9 @@ KESTREL_API int kestrel_attention_tc_kept(const void *q, const void *k_cache, co
     if (rc) return rc;
     p.keep_first = window > 0 ? keep_first : 0;
     p.gate = gate;
-    rc = at_launch<false, AT_KEPT>(dim3((unsigned)((long long)tiles * nkv)), stream, map_k, map_v, p, cache_pages, rows_per_tile);
+    const dim3 grid((unsigned)((long long)tiles * nkv));
+    rc = rows_per_tile <= AT_BM ? at_launch<false, AT_KEPT, true>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile)
+                                 : at_launch<false, AT_KEPT>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);
     return rc ? rc : kestrel_check_launch("attention_tc_kept");
 }
 

@@ -1352,6 +1352,32 @@ def row_tiles(batch, rows_per_token: int, rows_per_tile: int = 256):
     return kept[key]
 
 
+def attention_tc_tiles(batch, group: int, nkv: int, window: int, keep_first: int = 0):
+    """`row_tiles` for `attention_tc` and the rows of a tile: 128 where such tiles fit the SMs at once (a CTA's two streams then share its key
+    tiles out), or come in up to two rounds of them and the longest walk of a tile of 256 - one request's last tokens - would set the time: at
+    half a step a key tile, spread over the SMs, plus three steps for a second round's start, at most three quarters of that walk
+    (2,048 tokens of 16 / 4 heads 44 -> 35 us; four portions of 500, whose walks are short, 24 -> 27 and stay).  256 otherwise."""
+    kept = batch.__dict__.setdefault("_tc_rows", {})
+    key = (group, nkv, window, keep_first)
+    if key not in kept:
+        sms = library().kestrel_attention_tc_slots()
+        n128 = sum(-(-n * group // 128) for n in batch.counts)
+        rows = 128 if n128 * nkv <= sms else 256
+        if rows == 256 and n128 * nkv <= 2 * sms:
+            walk, longest = 0, 0
+            for n, start in zip(batch.counts, batch.starts):
+                for r in range(0, n * group, 128):
+                    last = start + min(n * group - 1, r + 127) // group
+                    first = max(0, start + r // group - window + 1) if window else 0
+                    tiles = last // 128 - first // 128 + 1 + min(-(-keep_first // 128), first // 128)
+                    walk, longest = walk + tiles, max(longest, tiles)
+            if walk * nkv / (2.0 * sms) + 3.0 <= 0.75 * longest:
+                rows = 128
+        kept[key] = rows
+    tile_seq, tile_row0 = row_tiles(batch, group, kept[key])
+    return tile_seq, tile_row0, kept[key]
+
+
 # ---- differential attention: two maps a head over the same values --------------------------------
 
 def differential_combine(a: torch.Tensor, lq1: torch.Tensor, lk1: torch.Tensor, lq2: torch.Tensor, lk2: torch.Tensor, diff: float, eps: float,

@@ -233,8 +233,11 @@ class GatedWindowAttention(Mixer):
                 (gate is None and self.keep_first == 0 or not self._scored) and not batch.captured and \
                 batch.max_count * G > self.TC_MIN_ROWS and \
                 ops.attention_tc_supported(128, cache.page_size):
-            # prompt portions of head size 128: the tcgen05 kernel, rows in tiles of 256 per request
-            tile_seq, tile_row0 = ops.row_tiles(batch, G, 256)
+            # prompt portions of head size 128: the tcgen05 kernel, rows in tiles of 256 or (softmax weights) 128 per request
+            if self.score.weighting == "sigmoid":
+                (tile_seq, tile_row0), rows = ops.row_tiles(batch, G, 256), 256
+            else:
+                tile_seq, tile_row0, rows = ops.attention_tc_tiles(batch, G, self.kv_heads, self.window, self.keep_first)
             # Few tiles far into a long context (a later portion of a long prompt) leave most SMs idle: softmax weights
             # without a window then take the key range in slices, as many as fill the chip, merged in ascending order.
             # A whole prompt has tiles enough and stays in one slice (cut at 512 keys, 2,048 tokens of 16 heads took 188
@@ -248,7 +251,7 @@ class GatedWindowAttention(Mixer):
                 slices = -(-batch.max_kv_len // slice_len)
             ops.attention_tc(q, cache.k, cache.v, a, tile_seq, tile_row0, batch.cu_seqlens, batch.kv_lens, table, cache.page_size, self.heads,
                              self.kv_heads, 128, self.window, self.scale, slices=slices,
-                             slice_len=slice_len, rows_per_tile=256, score=score, keep_first=self.keep_first, gate=gate)
+                             slice_len=slice_len, rows_per_tile=rows, score=score, keep_first=self.keep_first, gate=gate)
         elif self.dtype == torch.bfloat16 and not self.force_plain and self.decode and self._capped_only and gate is None and \
                 self.head_dim == self.v_head_dim and self.keep_first == 0 and \
                 ops.attention_decode_capped(q, cache.k, cache.v, batch, table, cache.page_size, a, self.heads, self.kv_heads, self.head_dim, self.window,
