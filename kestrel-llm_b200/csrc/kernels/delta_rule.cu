@@ -17,6 +17,7 @@
 //   out_norm_gate o / sqrt(mean(o^2) + eps) * w * sigmoid(gate) per head, in the storage type
 #include "common.cuh"
 #include "recurrence_step.cuh"
+#include "head_norm.cuh"
 #include <math.h>
 
 // sum of a product's slices at (token, column)
@@ -240,6 +241,8 @@ KESTREL_API int kestrel_delta_out(const float *o, const float *w, float eps, con
     KESTREL_REQUIRE(T > 0 && H > 0 && dv > 0 && Sg > 0, "delta_out: bad sizes");
     if (dtype == KESTREL_F32)
         kestrel_launch(delta_out_kernel<float>, dim3(T), dim3(128), 0, stream, o, w, eps, g_part, Sg, (size_t)g_stride, (float *)out, H, dv);
+    else if (dtype == KESTREL_BF16 && kestrel_head_norm_vec(o, w, 0, eps, g_part, Sg, (size_t)g_stride, H * dv, 0, 0, (__nv_bfloat16 *)out, (long long)H * dv, 1.f, T, H, dv, stream))
+        return kestrel_check_launch("delta_out");
     else if (dtype == KESTREL_BF16)
         kestrel_launch(delta_out_kernel<__nv_bfloat16>, dim3(T), dim3(128), 0, stream, o, w, eps, g_part, Sg, (size_t)g_stride, (__nv_bfloat16 *)out, H, dv);
     else

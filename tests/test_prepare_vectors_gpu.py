@@ -39,3 +39,25 @@ def test_vector_form_against_the_general_kernel(nq, nkv, hd, T, S, rot, pairing,
     for a, c in zip(*got):
         if a.numel():
             assert (a - c).abs().le((2.0 ** -8 + 2.0 ** -21) * a.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("H,dv", [(16, 128), (5, 64), (3, 32), (1, 128), (9, 32)])
+@pytest.mark.parametrize("T,S", [(1, 2), (37, 1), (513, 3)])
+@pytest.mark.parametrize("gate,per_channel", [(True, True), (True, False), (False, False)])
+def test_head_norm_in_vectors(H, dv, T, S, gate, per_channel):
+    """bfloat16 results of the read-outs' norm and gate against the float32 ones: a rounding to eight bits, and the order of a sum of squares."""
+    import torch
+    from kestrel_llm_b200.csrc import ops
+    torch.manual_seed(T)
+    o = torch.randn(T, H * dv, device="cuda")
+    w = torch.rand(H * dv if per_channel else dv, device="cuda") + 0.5
+    g = ops.Partials(torch.randn(S, T, H * dv + 8, device="cuda")) if gate else None
+    exact, got = torch.empty(T, H * dv, device="cuda"), torch.empty(T, H * dv, dtype=torch.bfloat16, device="cuda")
+    for out in (exact, got):
+        ops.head_norm_gate(o, w, 1e-6, g, 4 if gate else 0, out, H, dv)
+    assert (exact - got.float()).abs().le((2.0 ** -8 + 2.0 ** -20) * exact.abs() + 1e-30).all()
+    if gate and not per_channel:
+        z = ops.Partials(g.data[:, :, 4:4 + H * dv].contiguous())
+        ops.delta_out(o, w, 1e-6, z, exact, H, dv)
+        ops.delta_out(o, w, 1e-6, z, got, H, dv)
+        assert (exact - got.float()).abs().le((2.0 ** -8 + 2.0 ** -20) * exact.abs() + 1e-30).all()
