@@ -400,10 +400,13 @@ __device__ __forceinline__ void rb_mma(float *c, const uint32_t *a, uint32_t b0,
 }
 // x as two terms of 11 bits, both rounded to the nearest: the first leaves 2^-12 of x (exactly what the subtraction gives), the second
 // 2^-24.  (Cut off instead of rounded the two terms leave 2^-21 and the products of the second ones, which are dropped, 2^-20: read-outs
-// were 5e-7 of the largest off where the scan is 8e-8 off.)  The unit ignores the low 13 bits of the second.
+// were 5e-7 of the largest off where the scan is 8e-8 off.)  The unit ignores the low 13 bits of the second.  What is not finite is its
+// own first term: rounded as a number, the sum would carry out of the exponent and a NaN of all ones become a zero.
 __device__ __forceinline__ void rb_split(float x, uint32_t &hi, uint32_t &lo) {
-    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-    lo = __float_as_uint(x - __uint_as_float(hi)) + 0x1000u;
+    const uint32_t u = __float_as_uint(x);
+    const bool number = (u & 0x7f800000u) != 0x7f800000u;
+    hi = number ? (u + 0x1000u) & 0xffffe000u : u;
+    lo = number ? __float_as_uint(x - __uint_as_float(hi)) + 0x1000u : 0u;
 }
 struct RbA { uint32_t hi[4], lo[4]; };
 // Operand A from a row-major pair of numbers per row: (row l / 4: x0 at 2 (l % 4), x1 behind it; row l / 4 + 8: x2, x3).  The unit's k index

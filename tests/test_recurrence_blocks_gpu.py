@@ -185,3 +185,48 @@ def test_blocks_with_their_gates(counts, H, d, dv, S, form):
     assert got is not None
     _check("read-outs", got.cpu().numpy().astype(np.float64), scan.cpu().numpy().astype(np.float64), want)
     _check("states", sb.cpu().numpy().astype(np.float64), sa.cpu().numpy().astype(np.float64), ws)
+
+
+def _poisoned(form, what, at, value):
+    """(read-outs, states) of the scan and of the blocks for two requests, with `value` in one number of an operand at token `at` of the first."""
+    import torch
+    from kestrel_llm_b200.csrc import ops
+    rng = np.random.default_rng(at)
+    counts, H, d, dv = (40, 17), 2, 64, 24
+    batch, cu, slots = _step(counts, 1)
+    T = batch.num_tokens
+
+    def unit(x):
+        return x / np.sqrt((x * x).sum(-1, keepdims=True) + 1e-6)
+    x = {"r": rng.standard_normal((T, H, d)), "k": unit(rng.standard_normal((T, H, d))), "v": rng.standard_normal((T, H, dv)),
+         "w": np.exp(-rng.random((T, H, d))), "state": rng.standard_normal((3, H, d, dv)), "beta": rng.random((T, H, 1))}
+    x["a"], x["b"] = -rng.random((T, H, d)) * x["k"], x["k"].copy()
+    x[what][(slots[0] if what == "state" else at, 1, 0 if what == "beta" else 3) + ((5,) if what == "state" else ())] = value
+    t = {n: torch.from_numpy(np.ascontiguousarray(y.reshape(y.shape[0], -1), dtype=np.float32)).cuda() for n, y in x.items()}
+    got = []
+    for blocks in (False, True):
+        state = t["state"].clone()
+        if form == "delta":
+            out = torch.empty((T, H * dv), device="cuda")
+            (ops.delta_blocks if blocks else ops.delta_scan)(t["r"], t["k"], t["w"], t["v"], 0, t["beta"], state, batch, out, H, H, d, dv)
+        else:
+            fn, pair = ops.recurrence_blocks if blocks else ops.recurrence_scan, (t["a"], t["b"]) if form == "removal" else (None, None)
+            out = fn(t["r"], t["w"], t["k"], t["v"], *pair, state, 0, batch, H, d, dv)
+        got.append((out.cpu().numpy(), state.cpu().numpy()))
+    ops.raise_on_kernel_error()
+    return got
+
+
+POISONED = [("gate", w) for w in "rkvw"] + [("removal", w) for w in "rkvwab"] + [("delta", w) for w in ("r", "k", "v", "w", "beta")] + \
+    [(f, "state") for f in ("gate", "removal", "delta")]
+
+
+@pytest.mark.parametrize("form,what", POISONED)
+@pytest.mark.parametrize("at", [0, 5, 15, 39])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+def test_what_is_not_finite_stays_so_in_blocks(form, what, at, value):
+    """NaN and infinities in every operand: where the scan's numbers are not finite, neither are the blocks'."""
+    scan, blocks = _poisoned(form, what, at, value)
+    assert not np.isfinite(scan[0]).all()
+    for name, a, b in zip(("read-outs", "states"), scan, blocks):
+        assert not np.isfinite(b[~np.isfinite(a)]).any(), name
