@@ -21,6 +21,9 @@
 // sequential scan's within the tests' limit.  With plain multiply-adds the same blocks are bound by the shared-memory reads of
 // operands that 16 columns cannot reuse: 3,300 cycles a block against 1,500 here (DELTA).
 //
+// What is not finite stays so, and reaches the tokens and channels that it reaches in the scan: a block whose read-outs or corrections are
+// not finite sums them again token by token (an infinity may come out as NaN, whose terms have both signs).
+//
 // Three forms: GATE (no correction), REMOVAL (a, b given) and DELTA (a gated delta rule: with u = beta (v - (diag(w) S)^T k),
 // S <- diag(w) S + k u^T, so that b = w k and the writes u = X beta (v - b^T S_0) take the place of v).
 //
@@ -359,21 +362,24 @@ blocks_prepare_kernel(const RbParams p, const RbSource src) {
         }
     }
     __syncthreads();
+    // (sums over the tokens up to t alone: a later token's numbers may not be finite, and 0 x inf would not be 0)
     for (int idx = tid; idx < RB_B * RB_B; idx += 128) {
         const int t = idx / RB_B, j = idx % RB_B;
         if (FORM == RB_DELTA) {
             float m = 0.f;
 #pragma unroll
-            for (int s = 0; s < RB_B; ++s) m = fmaf(mQk[t * RB_LD + s], mX[s * RB_LD + j], m);
+            for (int s = 0; s < RB_B; ++s)
+                if (s <= t) m = fmaf(mQk[t * RB_LD + s], mX[s * RB_LD + j], m);
             blkp[L::M + t * RB_LD + j] = mX[t * RB_LD + j];
             blkp[L::M + RB_MAT + t * RB_LD + j] = m;
         } else {
             float xk = 0.f, m1 = 0.f;
 #pragma unroll
-            for (int s = 0; s < RB_B; ++s) {
-                xk = fmaf(mX[t * RB_LD + s], mK[s * RB_LD + j], xk);
-                m1 = fmaf(mQa[t * RB_LD + s], mX[s * RB_LD + j], m1);
-            }
+            for (int s = 0; s < RB_B; ++s)
+                if (s <= t) {
+                    xk = fmaf(mX[t * RB_LD + s], mK[s * RB_LD + j], xk);
+                    m1 = fmaf(mQa[t * RB_LD + s], mX[s * RB_LD + j], m1);
+                }
             mY[t * RB_LD + j] = xk;
             blkp[L::M + t * RB_LD + j] = mX[t * RB_LD + j];
             blkp[L::M + RB_MAT + t * RB_LD + j] = xk;
@@ -386,7 +392,8 @@ blocks_prepare_kernel(const RbParams p, const RbSource src) {
             const int t = idx / RB_B, j = idx % RB_B;
             float m2 = mQk[t * RB_LD + j];
 #pragma unroll
-            for (int s = 0; s < RB_B; ++s) m2 = fmaf(mQa[t * RB_LD + s], mY[s * RB_LD + j], m2);
+            for (int s = 0; s < RB_B; ++s)
+                if (s <= t) m2 = fmaf(mQa[t * RB_LD + s], mY[s * RB_LD + j], m2);
             blkp[L::M + 3 * RB_MAT + t * RB_LD + j] = m2;
         }
     }
@@ -569,8 +576,34 @@ blocks_scan_kernel(const RbParams p, int stages) {
                     rb_mma3(acc, small, ah, b.x, b.y);
                 }
             }
+            bool number = true;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[e] += small[e];
+            for (int e = 0; e < 4; ++e) {
+                acc[e] += small[e];
+                number = number && fabsf(acc[e]) < INFINITY;
+            }
+            if (!__all_sync(0xffffffffu, number)) {
+                // The products above meet the zeros of the matrices with the numbers of later tokens, and 0 x inf is not 0: a token's
+                // result from itself and the tokens before it alone, as the scan has it.
+                auto total_of = [&](int n, int j) { return red[0][j][n] + red[1][j][n] + red[2][j][n] + red[3][j][n]; };
+#pragma unroll 1
+                for (int e = 0; e < 4; ++e) {
+                    const int t = half * 8 + lc + (e & 1), j = lr + (e >> 1) * 8;
+                    float x = reads ? total_of((FORM == RB_GATE ? 0 : RB_B) + t, j) : 0.f;
+#pragma unroll 1
+                    for (int s = 0; s <= t; ++s) {
+                        const float *m = m0 + t * RB_LD + s;        // matrix i at i * RB_MAT
+                        const float v = vr[s][j], h = FORM == RB_GATE ? 0.f : total_of(s, j);
+                        if (FORM == RB_GATE) x = fmaf(m[0], v, x);
+                        if (FORM == RB_DELTA) x = fmaf(m[reads ? RB_MAT : 0], v - h, x);
+                        if (FORM == RB_REMOVAL) {
+                            x = fmaf(m[reads ? 2 * RB_MAT : 0], h, x);
+                            if (reads || s < t) x = fmaf(m[(reads ? 3 : 1) * RB_MAT], v, x);
+                        }
+                    }
+                    acc[0] = e == 0 ? x : acc[0], acc[1] = e == 1 ? x : acc[1], acc[2] = e == 2 ? x : acc[2], acc[3] = e == 3 ? x : acc[3];
+                }
+            }
             if (reads) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
@@ -578,8 +611,11 @@ blocks_scan_kernel(const RbParams p, int stages) {
                     if (t < t1 && j < p.dv) p.out[((size_t)t * p.H + h) * p.dv + j] = acc[e];
                 }
             } else {
+                // (none of the tokens beyond the request's end: what is not finite before them reaches their rows too)
+                const int left = t1 - t0 - i * RB_B - half * 8 - lc;
 #pragma unroll
-                for (int e = 0; e < 2; ++e) *reinterpret_cast<float2 *>(&corr[lr + 8 * e][half * 8 + lc]) = make_float2(acc[2 * e], acc[2 * e + 1]);
+                for (int e = 0; e < 2; ++e)
+                    *reinterpret_cast<float2 *>(&corr[lr + 8 * e][half * 8 + lc]) = make_float2(left > 0 ? acc[2 * e] : 0.f, left > 1 ? acc[2 * e + 1] : 0.f);
             }
         }
         if (FORM != RB_GATE) __syncthreads();

@@ -230,3 +230,16 @@ def test_what_is_not_finite_stays_so_in_blocks(form, what, at, value):
     assert not np.isfinite(scan[0]).all()
     for name, a, b in zip(("read-outs", "states"), scan, blocks):
         assert not np.isfinite(b[~np.isfinite(a)]).any(), name
+
+
+@pytest.mark.parametrize("form,what", POISONED)
+@pytest.mark.parametrize("at", [0, 5, 15, 39])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_what_is_not_finite_reaches_later_tokens_alone(form, what, at, value):
+    """The blocks' numbers that are not finite are the scan's: tokens before the poisoned one in its block, other heads, channels and requests
+    keep theirs, within the bound of the tests above."""
+    scan, blocks = _poisoned(form, what, at, value)
+    for name, a, b in zip(("read-outs", "states"), scan, blocks):
+        assert (np.isfinite(a) == np.isfinite(b)).all(), name
+        a, b = a[np.isfinite(a)].astype(np.float64), b[np.isfinite(a)]
+        assert np.abs(a - b).max(initial=0) <= 2.0 ** -20 * np.abs(a).max(initial=1), name
