@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(AMG_THREADS)
 attention_merge_kernel(const float *__restrict__ part_o, const float *__restrict__ part_ml,
                        __nv_bfloat16 *__restrict__ out, const int *__restrict__ tile_seq,
                        const int *__restrict__ tile_row0, const int *__restrict__ cu_seqlens,
-                       int slices, int hd, int nq, int nkv, const float *__restrict__ sink) {
+                       int slices, int hd, int nq, int nkv, const float *__restrict__ sink, const float *__restrict__ gate) {
     pdl_launch_dependents();
     __shared__ float f_s[AMG_MAX_SLICES], lf_s[AMG_MAX_SLICES];
     __shared__ float red[AMG_THREADS / 32];
@@ -426,7 +426,7 @@ attention_merge_kernel(const float *__restrict__ part_o, const float *__restrict
         inv_l = L;
     }
     __syncthreads();
-    const float L = inv_l;
+    const float L = inv_l, g = gate ? gate[qrow] : 1.f;
     const float *po = part_o + qrow * slices * hd;
     for (int d = tid; d < hd; d += AMG_THREADS) {
         float acc = 0.f;
@@ -441,7 +441,7 @@ attention_merge_kernel(const float *__restrict__ part_o, const float *__restrict
         }
         for (; s < slices; ++s)
             if (f_s[s] != 0.f) acc += po[(size_t)s * hd + d] * f_s[s];
-        out[qrow * hd + d] = __float2bfloat16_rn(acc / L);
+        out[qrow * hd + d] = __float2bfloat16_rn(acc / L * g);
     }
 }
 
@@ -455,7 +455,8 @@ __global__ void __launch_bounds__(256)
 attention_merge_rows_kernel(const float *__restrict__ part_o, const float *__restrict__ part_ml,
                             __nv_bfloat16 *__restrict__ out, const int *__restrict__ tile_seq,
                             const int *__restrict__ tile_row0, const int *__restrict__ cu_seqlens,
-                            int slices, int hd, int nq, int nkv, int rows_per_tile, const float *__restrict__ sink) {
+                            int slices, int hd, int nq, int nkv, int rows_per_tile, const float *__restrict__ sink,
+                            const float *__restrict__ gate) {
     pdl_launch_dependents();
     const int tile = blockIdx.x, kvh = blockIdx.y, lane = threadIdx.x & 31;
     const int r = blockIdx.z * 8 + (threadIdx.x >> 5);
@@ -493,7 +494,8 @@ attention_merge_rows_kernel(const float *__restrict__ part_o, const float *__res
     }
     if (sink) L += exp2f(sink[qrow % nq] * 1.4426950408889634f - M);      // the softmax's extra term, once, as in the kernel above
     if (d < hd) {
-        __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x / L, acc.y / L), hi = __floats2bfloat162_rn(acc.z / L, acc.w / L);
+        const float g = gate ? gate[qrow] : 1.f;
+        __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x / L * g, acc.y / L * g), hi = __floats2bfloat162_rn(acc.z / L * g, acc.w / L * g);
         uint2 u2;
         u2.x = *reinterpret_cast<uint32_t *>(&lo);
         u2.y = *reinterpret_cast<uint32_t *>(&hi);
@@ -518,22 +520,28 @@ static int launch_attention(const AttnParams &p, int tiles, cudaStream_t stream)
     return kestrel_check_launch("attention_mma");
 }
 
-// merges the slices of the listed tiles (at most rows_per_tile rows each) into out; also used by
-// attention_decode.cu and attention_tc.cu
-KESTREL_API int kestrel_attention_merge(const float *part_o, const float *part_ml, void *out, const int *tile_seq,
-                                        const int *tile_row0, int tiles, int rows_per_tile, const int *cu_seqlens, int slices,
-                                        int hd, int nq, int nkv, const float *sink, cudaStream_t stream) {
+// merges the slices of the listed tiles (at most rows_per_tile rows each) into out, each head's output times gate[token, head]
+// (float32 [T, nq], or null) before its one rounding; also used by attention_decode.cu, attention_tc.cu and attention_rows_tc.cu
+int attention_merge_gated(const float *part_o, const float *part_ml, void *out, const int *tile_seq, const int *tile_row0, int tiles,
+                          int rows_per_tile, const int *cu_seqlens, int slices, int hd, int nq, int nkv, const float *sink, const float *gate,
+                          cudaStream_t stream) {
     KESTREL_REQUIRE(rows_per_tile >= 1 && rows_per_tile <= 65535, "attention_merge: tiles of %d rows", rows_per_tile);
     KESTREL_REQUIRE(slices >= 1 && slices <= AMG_MAX_SLICES, "attention_merge: %d slices; the kernel merges up to %d", slices, AMG_MAX_SLICES);
     KESTREL_REQUIRE(tiles <= 0x7fffffff && nkv <= 65535, "attention_merge: grid too large");
     if (rows_per_tile > 16 && slices <= AMW_MAX_SLICES && hd % 4 == 0 && hd <= 128 && (((uintptr_t)part_o | (uintptr_t)out) & 15) == 0) {
         kestrel_launch(attention_merge_rows_kernel, dim3(tiles, nkv, (rows_per_tile + 7) / 8), dim3(256), 0, stream, part_o, part_ml,
-                       (__nv_bfloat16 *)out, tile_seq, tile_row0, cu_seqlens, slices, hd, nq, nkv, rows_per_tile, sink);
+                       (__nv_bfloat16 *)out, tile_seq, tile_row0, cu_seqlens, slices, hd, nq, nkv, rows_per_tile, sink, gate);
         return kestrel_check_launch("attention_merge");
     }
     kestrel_launch(attention_merge_kernel, dim3(tiles, nkv, rows_per_tile), dim3(AMG_THREADS), 0, stream, part_o, part_ml, (__nv_bfloat16 *)out,
-                   tile_seq, tile_row0, cu_seqlens, slices, hd, nq, nkv, sink);
+                   tile_seq, tile_row0, cu_seqlens, slices, hd, nq, nkv, sink, gate);
     return kestrel_check_launch("attention_merge");
+}
+
+KESTREL_API int kestrel_attention_merge(const float *part_o, const float *part_ml, void *out, const int *tile_seq,
+                                        const int *tile_row0, int tiles, int rows_per_tile, const int *cu_seqlens, int slices,
+                                        int hd, int nq, int nkv, const float *sink, cudaStream_t stream) {
+    return attention_merge_gated(part_o, part_ml, out, tile_seq, tile_row0, tiles, rows_per_tile, cu_seqlens, slices, hd, nq, nkv, sink, nullptr, stream);
 }
 
 // rows (token, head) of a ROWS-mode tile for this head size

@@ -45,5 +45,8 @@ __device__ __forceinline__ int attn_slice_len(const AttnParams &p) {
     return len < 128 ? 128 : len;
 }
 
-// attention_mma.cu: merges the key-range slices of the listed tiles (at most 16 rows each) into out
-// (kestrel_attention_merge, declared in kestrel.h)
+// attention_mma.cu: merges the key-range slices of the listed tiles into out (kestrel_attention_merge, declared in kestrel.h), or with
+// a factor per (token, head) on the outputs
+int attention_merge_gated(const float *part_o, const float *part_ml, void *out, const int *tile_seq, const int *tile_row0, int tiles,
+                          int rows_per_tile, const int *cu_seqlens, int slices, int hd, int nq, int nkv, const float *sink, const float *gate,
+                          cudaStream_t stream);

@@ -345,7 +345,7 @@ KESTREL_API int kestrel_attention_rows_tc_supported(int hd, int vd, int page_siz
 
 // q [T, nq * hd], cache [pages, nkv, page_size, hd], out [T, nq * vd] = gate[token, head] (float32 [T, nq], or null) * softmax(q . row * scale) row[:vd]
 // over causal keys (the last `window` of them, 0: all).  Tiles of up to 128 rows, listed by tile_seq / tile_row0.  With slices > 1 every CTA takes
-// slice_len keys (a multiple of 128); scratch part_o [T * nq, slices, vd], part_ml [T * nq, slices, 2]; no gate then.
+// slice_len keys (a multiple of 128); scratch part_o [T * nq, slices, vd], part_ml [T * nq, slices, 2]; the gate is then the merge's.
 KESTREL_API int kestrel_attention_rows_tc(const void *q, const void *cache, void *out, float *part_o, float *part_ml, const int *tile_seq,
                                           const int *tile_row0, int tiles, int rows_per_tile, const int *cu_seqlens, const int *kv_lens,
                                           const int *block_table, int table_width, int table_stride, int page_size, int cache_pages, int T, int nq,
@@ -357,7 +357,7 @@ KESTREL_API int kestrel_attention_rows_tc(const void *q, const void *cache, void
     KESTREL_REQUIRE(nq > 0 && nkv > 0 && nq % nkv == 0, "attention_rows_tc: %d query heads over %d kv heads", nq, nkv);
     KESTREL_REQUIRE(window >= 0 && scale > 0.f, "attention_rows_tc: window %d, scale %g", window, (double)scale);
     KESTREL_REQUIRE(slices >= 1 && slices <= 1024 && slice_len > 0 && slice_len % 128 == 0, "attention_rows_tc: %d slices of %d keys", slices, slice_len);
-    KESTREL_REQUIRE(slices == 1 || (part_o && part_ml && !gate), "attention_rows_tc: slices need scratch and take no gate");
+    KESTREL_REQUIRE(slices == 1 || (part_o && part_ml), "attention_rows_tc: %d slices without scratch", slices);
     KESTREL_REQUIRE((long long)tiles * nkv < (1ll << 31), "attention_rows_tc: grid too large");
     KESTREL_REQUIRE(cache_pages > 0 && (long long)cache_pages * nkv * page_size < (1ll << 31), "attention_rows_tc: a cache of %d pages is beyond the 32-bit row coordinate", cache_pages);
     KESTREL_REQUIRE((((uintptr_t)q | (uintptr_t)cache | (uintptr_t)out | (uintptr_t)part_o) & 15) == 0, "attention_rows_tc: tensors must start on 16-byte boundaries");
@@ -370,7 +370,7 @@ KESTREL_API int kestrel_attention_rows_tc(const void *q, const void *cache, void
     p.cu_seqlens = cu_seqlens; p.kv_lens = kv_lens; p.block_table = block_table; p.table_width = table_width; p.table_stride = table_stride;
     p.page_size = page_size; p.nq = nq; p.nkv = nkv; p.hd = hd; p.window = window; p.slices = slices; p.slice_len = slice_len;
     p.scale_log2 = scale * 1.4426950408889634f;
-    p.gate = gate;
+    p.gate = slices > 1 ? nullptr : gate;
     ap.vd = vd;
     // as much for every size: a CTA has all of an SM's TMEM and shares the SM with no other kernel that takes some
     const size_t smem = (size_t)(AR_MAX_HD / 64) * (AR_Q_PANEL + AR_STAGES * AR_K_PANEL) + 8 * R_COUNT + 16 + 1024;
@@ -383,7 +383,7 @@ KESTREL_API int kestrel_attention_rows_tc(const void *q, const void *cache, void
     kestrel_launch(attention_rows_tc_kernel, dim3((unsigned)((long long)tiles * nkv), 1, slices), dim3(AR_THREADS), smem, stream, map_k, ap, cache_pages, rows_per_tile);
     rc = kestrel_check_launch("attention_rows_tc");
     if (rc || slices == 1) return rc;
-    return kestrel_attention_merge(part_o, part_ml, out, tile_seq, tile_row0, tiles, rows_per_tile, cu_seqlens, slices, vd, nq, nkv, nullptr, stream);
+    return attention_merge_gated(part_o, part_ml, out, tile_seq, tile_row0, tiles, rows_per_tile, cu_seqlens, slices, vd, nq, nkv, nullptr, gate, stream);
 }
 
 // Error word of the bounded waits (0: none; 1 loader, 2-4 issuer, 5-7 softmax).  Synchronises the device and clears the word.

@@ -684,7 +684,7 @@ def attention_rows_tc(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, b
                       hd: int, vd: int, window: int, scale: float, gate: Optional[torch.Tensor] = None) -> None:
     """tcgen05 attention of a step's prompt portions over cache rows [pages, nkv, page size, hd] that are key (whole) and value (their first
     ``vd`` numbers), heads' outputs times ``gate`` (float32 [T, nq]) if given.  Few tiles far into a context without a window cut the
-    key range into slices, merged in ascending order (the gate is then a kernel of its own)."""
+    key range into slices, merged in ascending order, gated there."""
     _need(q, "attention_rows_tc.q", torch.bfloat16, 2)
     _need(out, "attention_rows_tc.out", torch.bfloat16, 2)
     _need(cache, "attention_rows_tc.cache", torch.bfloat16, 4)
@@ -713,12 +713,10 @@ def attention_rows_tc(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, b
     _check(library().kestrel_attention_rows_tc(
         q.data_ptr(), cache.data_ptr(), out.data_ptr(), _p(part_o), _p(part_ml), tile_seq.data_ptr(), tile_row0.data_ptr(), tiles, 128,
         batch.cu_seqlens.data_ptr(), batch.kv_lens.data_ptr(), block_table.data_ptr(), block_table.shape[1], block_table.stride(0), int(page_size),
-        int(cache.shape[0]), T, nq, nkv, hd, vd, int(window), slices, slice_len, _p(gate) if slices == 1 else None, float(scale), _stream()))
+        int(cache.shape[0]), T, nq, nkv, hd, vd, int(window), slices, slice_len, _p(gate), float(scale), _stream()))
     if slices > 1:
         global launches
         launches += 1          # the merge kernel
-        if gate is not None:
-            head_scale(out, gate, nq)
 
 
 def attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, out: torch.Tensor,

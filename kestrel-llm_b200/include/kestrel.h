@@ -432,7 +432,7 @@ KESTREL_API int kestrel_attention_tc(const void *q, const void *k_cache, const v
 KESTREL_API int kestrel_attention_tc_supported(int hd, int page_size);
 KESTREL_API int kestrel_attention_tc_slots(void);
 KESTREL_API int kestrel_attention_tc_error(void);
-/* prompt portions over cache rows that are key (all hd numbers, up to 256) and value (the first vd): tiles of up to 128 rows; slices > 1: scratch part_o [T * nq, slices, vd], part_ml [T * nq, slices, 2], slice_len a multiple of 128, no gate */
+/* prompt portions over cache rows that are key (all hd numbers, up to 256) and value (the first vd): tiles of up to 128 rows; slices > 1: scratch part_o [T * nq, slices, vd], part_ml [T * nq, slices, 2], slice_len a multiple of 128 */
 KESTREL_API int kestrel_attention_rows_tc_supported(int hd, int vd, int page_size);
 KESTREL_API int kestrel_attention_rows_tc(const void *q, const void *cache, void *out, float *part_o, float *part_ml, const int *tile_seq, const int *tile_row0, int tiles, int rows_per_tile, const int *cu_seqlens, const int *kv_lens, const int *block_table, int table_width, int table_stride, int page_size, int cache_pages, int T, int nq, int nkv, int hd, int vd, int window, int slices, int slice_len, const float *gate, float scale, kestrel_stream_t stream);
 KESTREL_API int kestrel_attention_rows_tc_error(void);
