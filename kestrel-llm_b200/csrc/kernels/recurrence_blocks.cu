@@ -59,6 +59,16 @@ template <int D, int FORM> struct RbLayout {
     static constexpr int FLOATS = M + (FORM == RB_GATE ? 1 : FORM == RB_DELTA ? 2 : 4) * RB_MAT;
 };
 
+// What a CTA of the scan holds beside its ring (a GATE block corrects nothing, and alternates between two buffers of sums)
+template <int FORM> struct RbScan {
+    static constexpr int ROWS = FORM == RB_GATE ? RB_B : 2 * RB_B;      // rows that meet the state: b and r
+    static constexpr int RED_LD = ROWS + 8;
+    unsigned long long bars[RB_STAGES];
+    float red[FORM == RB_GATE ? 2 : 1][4][RB_COLS][RED_LD];
+    float vals[4][RB_B][RB_VLD];                // values [token][column] of four blocks in flight: loaded for the next block alone they set the pace (2,400 cycles a block)
+    float corr[FORM == RB_GATE ? 1 : RB_COLS][RB_LD];
+};
+
 struct RbParams {
     const float *r, *w, *k, *a, *b, *beta;      // r, k [T, G d] (DELTA) or [T, H d]; w, a, b [T, H d]; beta [T, H]
     const float *v;                             // [T, ldv], head h's columns at h * dv
@@ -438,21 +448,20 @@ template <int D, int FORM>
 __global__ void __launch_bounds__(128)
 blocks_scan_kernel(const RbParams p, int stages) {
     using L = RbLayout<D, FORM>;
-    constexpr int ROWS = FORM == RB_GATE ? RB_B : 2 * RB_B;      // rows that meet the state: b and r
-    constexpr int NT = ROWS / 8;                                 // tiles of eight of them
+    constexpr int NT = RbScan<FORM>::ROWS / 8;                   // tiles of eight rows that meet the state
     constexpr int CT = D / 32;                                   // tiles of eight channels of a warp
-    constexpr int STAGE = L::FLOATS, RED_LD = ROWS + 8;
+    constexpr int STAGE = L::FLOATS, RED_LD = RbScan<FORM>::RED_LD;
     pdl_launch_dependents();
     extern __shared__ float4 rb_smem4[];
     float *ring = reinterpret_cast<float *>(rb_smem4);
-    __shared__ __align__(8) unsigned long long bar_words[RB_STAGES];
-    // values of a block [token][column], four blocks in flight: loaded for the next block alone they set the pace (2,400 cycles a block)
-    __shared__ __align__(16) float red_s[FORM == RB_GATE ? 2 : 1][4][RB_COLS][RED_LD], vals[4][RB_B][RB_VLD], corr[RB_COLS][RB_LD];
+    __shared__ __align__(16) RbScan<FORM> sm;
+    auto &vals = sm.vals;
+    auto &corr = sm.corr;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int lr = lane >> 2, lc = (lane & 3) * 2;               // a fragment's row (and row + 8) and its pair of columns
     const int h = blockIdx.y, seq = blockIdx.z, col0 = blockIdx.x * RB_COLS;
     const int ch0 = warp * (D / 4);
-    const uint32_t bar0 = smem_u32(&bar_words[0]);
+    const uint32_t bar0 = smem_u32(&sm.bars[0]);
     if (tid == 0) {
         for (int b = 0; b < stages; ++b) mbar_init(bar0 + 8 * b, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -501,7 +510,7 @@ blocks_scan_kernel(const RbParams p, int stages) {
     for (int i = 0; i < n_blocks; ++i) {
         const int stage = i % stages;
         const float *st = ring + stage * STAGE;
-        float(*red)[RB_COLS][RED_LD] = red_s[FORM == RB_GATE ? i & 1 : 0];       // GATE has one barrier a block: two buffers in turn
+        float(*red)[RB_COLS][RED_LD] = sm.red[FORM == RB_GATE ? i & 1 : 0];       // GATE has one barrier a block: two buffers in turn
         asm volatile("cp.async.wait_group 2;" ::: "memory");       // this block's values; the barrier below shows them to all
         if (ok && !mbar_wait(bar0 + 8u * stage, (uint32_t)(i / stages) & 1u)) { atomicExch(&g_rb_error, 1); ok = false; }
         {   // what the warp's channels of the state give to the block's rows
@@ -676,7 +685,7 @@ template <int D, int FORM>
 static int rb_launch(const RbParams &p, const RbSource *src, int nseq, int max_count, cudaStream_t stream) {
     static_assert(RbLayout<D, FORM>::FLOATS % 4 == 0, "bulk copies move 16 bytes");
     const size_t prep = (size_t)((FORM == RB_GATE ? 3 : FORM == RB_DELTA ? 4 : 5) * RB_B * D + 6 * RB_MAT) * sizeof(float);
-    constexpr size_t stage = (size_t)RbLayout<D, FORM>::FLOATS * sizeof(float), fixed = 18 * 1024;    // beside the ring: under 18 KB of static memory
+    constexpr size_t stage = (size_t)RbLayout<D, FORM>::FLOATS * sizeof(float), fixed = (sizeof(RbScan<FORM>) + 1023) / 1024 * 1024;
     static bool attr_set = false;
     if (!attr_set) {
         if (cudaFuncSetAttribute(blocks_prepare_kernel<D, FORM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep) != cudaSuccess ||
@@ -688,7 +697,7 @@ static int rb_launch(const RbParams &p, const RbSource *src, int nseq, int max_c
     const dim3 blocks((max_count + RB_B - 1) / RB_B, p.H, nseq);
     if (src) kestrel_launch(blocks_prepare_kernel<D, FORM, true>, blocks, dim3(128), prep, stream, p, *src);
     else kestrel_launch(blocks_prepare_kernel<D, FORM, false>, blocks, dim3(128), prep, stream, p, RbSource());
-    static_assert(RbLayout<D, FORM>::FLOATS * 8 + 18 * 1024 <= KESTREL_SMEM_MAX_DYNAMIC, "two stages fit an SM");
+    static_assert(2 * stage + fixed <= KESTREL_SMEM_MAX_DYNAMIC, "two stages fit an SM");
     const dim3 grid((p.dv + RB_COLS - 1) / RB_COLS, p.H, nseq);
     // as many stages as the CTAs that share an SM leave room for, two at least
     const size_t room = kestrel_spread_smem((long)grid.x * grid.y * grid.z, 2 * stage + fixed) - fixed;
