@@ -387,15 +387,17 @@ __global__ void __launch_bounds__(AMG_THREADS)
 attention_merge_kernel(const float *__restrict__ part_o, const float *__restrict__ part_ml,
                        __nv_bfloat16 *__restrict__ out, const int *__restrict__ tile_seq,
                        const int *__restrict__ tile_row0, const int *__restrict__ cu_seqlens,
-                       int slices, int hd, int nq, int nkv, const float *__restrict__ sink, const float *__restrict__ gate) {
+                       int slices, int hd, int nq, int nkv, const float *__restrict__ sink, const float *__restrict__ gate, int nseq) {
     pdl_launch_dependents();
     __shared__ float f_s[AMG_MAX_SLICES], lf_s[AMG_MAX_SLICES];
     __shared__ float red[AMG_THREADS / 32];
     __shared__ float inv_l;
     const int tile = blockIdx.x, kvh = blockIdx.y, r = blockIdx.z;
     const int tid = threadIdx.x;
-    const int seq = tile_seq[tile], row0 = tile_row0[tile];
     const int G = nq / nkv;
+    int seq, row0;
+    if (tile_seq) seq = tile_seq[tile], row0 = tile_row0[tile];
+    else attn_find_tile(cu_seqlens, nseq, G, (int)gridDim.z, tile, seq, row0);
     const int tok_begin = cu_seqlens[seq];
     const int n_rows = (cu_seqlens[seq + 1] - tok_begin) * G;
     if (r >= min((int)gridDim.z, n_rows - row0)) return;
@@ -456,12 +458,14 @@ attention_merge_rows_kernel(const float *__restrict__ part_o, const float *__res
                             __nv_bfloat16 *__restrict__ out, const int *__restrict__ tile_seq,
                             const int *__restrict__ tile_row0, const int *__restrict__ cu_seqlens,
                             int slices, int hd, int nq, int nkv, int rows_per_tile, const float *__restrict__ sink,
-                            const float *__restrict__ gate) {
+                            const float *__restrict__ gate, int nseq) {
     pdl_launch_dependents();
     const int tile = blockIdx.x, kvh = blockIdx.y, lane = threadIdx.x & 31;
     const int r = blockIdx.z * 8 + (threadIdx.x >> 5);
-    const int seq = tile_seq[tile], row0 = tile_row0[tile];
     const int G = nq / nkv;
+    int seq, row0;
+    if (tile_seq) seq = tile_seq[tile], row0 = tile_row0[tile];
+    else attn_find_tile(cu_seqlens, nseq, G, rows_per_tile, tile, seq, row0);
     const int tok_begin = cu_seqlens[seq];
     const int n_rows = (cu_seqlens[seq + 1] - tok_begin) * G;
     if (r >= min(rows_per_tile, n_rows - row0)) return;
@@ -523,25 +527,25 @@ static int launch_attention(const AttnParams &p, int tiles, cudaStream_t stream)
 // merges the slices of the listed tiles (at most rows_per_tile rows each) into out, each head's output times gate[token, head]
 // (float32 [T, nq], or null) before its one rounding; also used by attention_decode.cu, attention_tc.cu and attention_rows_tc.cu
 int attention_merge_gated(const float *part_o, const float *part_ml, void *out, const int *tile_seq, const int *tile_row0, int tiles,
-                          int rows_per_tile, const int *cu_seqlens, int slices, int hd, int nq, int nkv, const float *sink, const float *gate,
+                          int rows_per_tile, const int *cu_seqlens, int nseq, int slices, int hd, int nq, int nkv, const float *sink, const float *gate,
                           cudaStream_t stream) {
     KESTREL_REQUIRE(rows_per_tile >= 1 && rows_per_tile <= 65535, "attention_merge: tiles of %d rows", rows_per_tile);
     KESTREL_REQUIRE(slices >= 1 && slices <= AMG_MAX_SLICES, "attention_merge: %d slices; the kernel merges up to %d", slices, AMG_MAX_SLICES);
     KESTREL_REQUIRE(tiles <= 0x7fffffff && nkv <= 65535, "attention_merge: grid too large");
     if (rows_per_tile > 16 && slices <= AMW_MAX_SLICES && hd % 4 == 0 && hd <= 128 && (((uintptr_t)part_o | (uintptr_t)out) & 15) == 0) {
         kestrel_launch(attention_merge_rows_kernel, dim3(tiles, nkv, (rows_per_tile + 7) / 8), dim3(256), 0, stream, part_o, part_ml,
-                       (__nv_bfloat16 *)out, tile_seq, tile_row0, cu_seqlens, slices, hd, nq, nkv, rows_per_tile, sink, gate);
+                       (__nv_bfloat16 *)out, tile_seq, tile_row0, cu_seqlens, slices, hd, nq, nkv, rows_per_tile, sink, gate, nseq);
         return kestrel_check_launch("attention_merge");
     }
     kestrel_launch(attention_merge_kernel, dim3(tiles, nkv, rows_per_tile), dim3(AMG_THREADS), 0, stream, part_o, part_ml, (__nv_bfloat16 *)out,
-                   tile_seq, tile_row0, cu_seqlens, slices, hd, nq, nkv, sink, gate);
+                   tile_seq, tile_row0, cu_seqlens, slices, hd, nq, nkv, sink, gate, nseq);
     return kestrel_check_launch("attention_merge");
 }
 
 KESTREL_API int kestrel_attention_merge(const float *part_o, const float *part_ml, void *out, const int *tile_seq,
                                         const int *tile_row0, int tiles, int rows_per_tile, const int *cu_seqlens, int slices,
                                         int hd, int nq, int nkv, const float *sink, cudaStream_t stream) {
-    return attention_merge_gated(part_o, part_ml, out, tile_seq, tile_row0, tiles, rows_per_tile, cu_seqlens, slices, hd, nq, nkv, sink, nullptr, stream);
+    return attention_merge_gated(part_o, part_ml, out, tile_seq, tile_row0, tiles, rows_per_tile, cu_seqlens, 0, slices, hd, nq, nkv, sink, nullptr, stream);
 }
 
 // rows (token, head) of a ROWS-mode tile for this head size

@@ -31,6 +31,7 @@ struct AttnParams {
     // a window that keeps a request's first tokens, and a factor per (token, head) on the outputs (or null); attention_tc.cu's kept form only
     int keep_first;
     const float *gate;
+    int nseq;                       // where tile_seq is null: the requests of cu_seqlens, in whose rows a CTA looks for its tile (attn_find_tile)
     // two maps a head over the same values (differential attention); read by attention_tc.cu only
     DifferentialOpts maps;
 };
@@ -45,8 +46,36 @@ __device__ __forceinline__ int attn_slice_len(const AttnParams &p) {
     return len < 128 ? 128 : len;
 }
 
+// (request, its first row) of a tile where no list was made for the step: every request's rows - `group` a token - cut into tiles of
+// rows_per_tile, request by request.  A list costs its making and a copy on the host, once a step and size: 20 us of a step that the host
+// paces, which a layer of few tokens does not win back; this is a scan over a warp per 32 requests.  All lanes of a warp take part.
+__device__ __forceinline__ void attn_find_tile(const int *cu_seqlens, int nseq, int group, int rows_per_tile, int tile, int &seq, int &row0) {
+    const int lane = threadIdx.x & 31;
+    int left = tile;
+    for (int base = 0; base < nseq; base += 32) {
+        const int i = base + lane;
+        const int n = i < nseq ? ((cu_seqlens[i + 1] - cu_seqlens[i]) * group + rows_per_tile - 1) / rows_per_tile : 0;
+        int end = n;                // tiles of the requests up to this lane's
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += x;
+        }
+        const uint32_t behind = __ballot_sync(0xffffffffu, left < end);
+        if (behind) {
+            const int at = __ffs(behind) - 1;
+            seq = base + at;
+            row0 = (left - __shfl_sync(0xffffffffu, end - n, at)) * rows_per_tile;
+            return;
+        }
+        left -= __shfl_sync(0xffffffffu, end, 31);
+    }
+    seq = nseq - 1;                 // no such tile: a tile that is there, whose rows another CTA writes too, with the same numbers
+    row0 = 0;
+}
+
 // attention_mma.cu: merges the key-range slices of the listed tiles into out (kestrel_attention_merge, declared in kestrel.h), or with
-// a factor per (token, head) on the outputs
+// a factor per (token, head) on the outputs; tile_seq null: the tiles of nseq requests, found from cu_seqlens
 int attention_merge_gated(const float *part_o, const float *part_ml, void *out, const int *tile_seq, const int *tile_row0, int tiles,
-                          int rows_per_tile, const int *cu_seqlens, int slices, int hd, int nq, int nkv, const float *sink, const float *gate,
+                          int rows_per_tile, const int *cu_seqlens, int nseq, int slices, int hd, int nq, int nkv, const float *sink, const float *gate,
                           cudaStream_t stream);

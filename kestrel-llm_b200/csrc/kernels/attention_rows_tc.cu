@@ -114,8 +114,10 @@ attention_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const ArPara
     pdl_wait();
 
     const int kvh = blockIdx.x % p.nkv, tile = (int)(gridDim.x / p.nkv) - 1 - (int)(blockIdx.x / p.nkv), slice = blockIdx.z;
-    const int seq = p.tile_seq[tile], row0 = p.tile_row0[tile];
     const int G = p.nq / p.nkv;
+    int seq, row0;
+    if (p.tile_seq) seq = p.tile_seq[tile], row0 = p.tile_row0[tile];
+    else attn_find_tile(p.cu_seqlens, p.nseq, G, rows_per_tile, tile, seq, row0);
     const int tok_begin = p.cu_seqlens[seq], n_tok = p.cu_seqlens[seq + 1] - tok_begin;
     const int pos_begin = p.kv_lens[seq] - n_tok;
     const int rows_here = min(rows_per_tile, n_tok * G - row0);
@@ -344,16 +346,18 @@ KESTREL_API int kestrel_attention_rows_tc_supported(int hd, int vd, int page_siz
 }
 
 // q [T, nq * hd], cache [pages, nkv, page_size, hd], out [T, nq * vd] = gate[token, head] (float32 [T, nq], or null) * softmax(q . row * scale) row[:vd]
-// over causal keys (the last `window` of them, 0: all).  Tiles of up to 128 rows, listed by tile_seq / tile_row0.  With slices > 1 every CTA takes
+// over causal keys (the last `window` of them, 0: all).  Tiles of up to 128 rows, listed by tile_seq / tile_row0, or
+// with null for both all of the nseq requests' tiles.  With slices > 1 every CTA takes
 // slice_len keys (a multiple of 128); scratch part_o [T * nq, slices, vd], part_ml [T * nq, slices, 2]; the gate is then the merge's.
 KESTREL_API int kestrel_attention_rows_tc(const void *q, const void *cache, void *out, float *part_o, float *part_ml, const int *tile_seq,
-                                          const int *tile_row0, int tiles, int rows_per_tile, const int *cu_seqlens, const int *kv_lens,
+                                          const int *tile_row0, int tiles, int rows_per_tile, const int *cu_seqlens, int nseq, const int *kv_lens,
                                           const int *block_table, int table_width, int table_stride, int page_size, int cache_pages, int T, int nq,
                                           int nkv, int hd, int vd, int window, int slices, int slice_len, const float *gate, float scale,
                                           cudaStream_t stream) {
     if (T == 0 || tiles == 0) return 0;
     KESTREL_REQUIRE(kestrel_attention_rows_tc_supported(hd, vd, page_size), "attention_rows_tc: rows of %d, values of %d, pages of %d", hd, vd, page_size);
     KESTREL_REQUIRE(rows_per_tile >= 1 && rows_per_tile <= AR_BM, "attention_rows_tc: tiles of %d rows; a CTA takes up to %d", rows_per_tile, AR_BM);
+    KESTREL_REQUIRE((tile_seq == nullptr) == (tile_row0 == nullptr) && (tile_seq || nseq > 0), "attention_rows_tc: no tiles, and %d requests to cut into some", nseq);
     KESTREL_REQUIRE(nq > 0 && nkv > 0 && nq % nkv == 0, "attention_rows_tc: %d query heads over %d kv heads", nq, nkv);
     KESTREL_REQUIRE(window >= 0 && scale > 0.f, "attention_rows_tc: window %d, scale %g", window, (double)scale);
     KESTREL_REQUIRE(slices >= 1 && slices <= 1024 && slice_len > 0 && slice_len % 128 == 0, "attention_rows_tc: %d slices of %d keys", slices, slice_len);
@@ -370,6 +374,7 @@ KESTREL_API int kestrel_attention_rows_tc(const void *q, const void *cache, void
     p.cu_seqlens = cu_seqlens; p.kv_lens = kv_lens; p.block_table = block_table; p.table_width = table_width; p.table_stride = table_stride;
     p.page_size = page_size; p.nq = nq; p.nkv = nkv; p.hd = hd; p.window = window; p.slices = slices; p.slice_len = slice_len;
     p.scale_log2 = scale * 1.4426950408889634f;
+    p.nseq = nseq;
     p.gate = slices > 1 ? nullptr : gate;
     ap.vd = vd;
     // as much for every size: a CTA has all of an SM's TMEM and shares the SM with no other kernel that takes some
@@ -383,7 +388,7 @@ KESTREL_API int kestrel_attention_rows_tc(const void *q, const void *cache, void
     kestrel_launch(attention_rows_tc_kernel, dim3((unsigned)((long long)tiles * nkv), 1, slices), dim3(AR_THREADS), smem, stream, map_k, ap, cache_pages, rows_per_tile);
     rc = kestrel_check_launch("attention_rows_tc");
     if (rc || slices == 1) return rc;
-    return attention_merge_gated(part_o, part_ml, out, tile_seq, tile_row0, tiles, rows_per_tile, cu_seqlens, slices, vd, nq, nkv, nullptr, gate, stream);
+    return attention_merge_gated(part_o, part_ml, out, tile_seq, tile_row0, tiles, rows_per_tile, cu_seqlens, nseq, slices, vd, nq, nkv, nullptr, gate, stream);
 }
 
 // Error word of the bounded waits (0: none; 1 loader, 2-4 issuer, 5-7 softmax).  Synchronises the device and clears the word.

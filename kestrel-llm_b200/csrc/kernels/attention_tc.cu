@@ -182,8 +182,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     // late tiles, which see the most keys, come first - across all kv heads
     const int kvh = blockIdx.x % p.nkv, tile = (int)(gridDim.x / p.nkv) - 1 - (int)(blockIdx.x / p.nkv), slice = blockIdx.z;
     const int slice_len = attn_slice_len(p);
-    const int seq = p.tile_seq[tile], row0 = p.tile_row0[tile];
     const int G = p.nq / p.nkv;
+    int seq, row0;
+    if (KIND != AT_KEPT || p.tile_seq) seq = p.tile_seq[tile], row0 = p.tile_row0[tile];
+    else attn_find_tile(p.cu_seqlens, p.nseq, G, rows_per_tile, tile, seq, row0);
     const int tok_begin = p.cu_seqlens[seq], n_tok = p.cu_seqlens[seq + 1] - tok_begin;
     const int kv_len = p.kv_lens[seq];
     const int pos_begin = kv_len - n_tok;
@@ -827,11 +829,13 @@ KESTREL_API int kestrel_attention_tc_biased(const void *q, const void *k_cache, 
 
 // Softmax attention over a window that keeps a request's first `keep_first` tokens visible, each head's output times gate[token, head]
 // (float32 [T, nq], or null), in one slice of keys.  A window is needed for kept tokens; window 0 sees everything.
+// tile_seq and tile_row0 null: all of the nseq requests' tiles.
 KESTREL_API int kestrel_attention_tc_kept(const void *q, const void *k_cache, const void *v_cache, void *out, const int *tile_seq,
-                                          const int *tile_row0, int tiles, int rows_per_tile, const int *cu_seqlens, const int *kv_lens,
+                                          const int *tile_row0, int tiles, int rows_per_tile, const int *cu_seqlens, int nseq, const int *kv_lens,
                                           const int *block_table, int table_width, int table_stride, int page_size, int cache_pages, int T, int nq,
                                           int nkv, int hd, int window, int keep_first, const float *gate, float scale, cudaStream_t stream) {
     if (T == 0 || tiles == 0) return 0;
+    KESTREL_REQUIRE((tile_seq == nullptr) == (tile_row0 == nullptr) && (tile_seq || nseq > 0), "attention_tc_kept: no tiles, and %d requests to cut into some", nseq);
     KESTREL_REQUIRE(window >= 0 && keep_first >= 0, "attention_tc_kept: window %d, %d kept tokens", window, keep_first);
     AttnParams p;
     CUtensorMap map_k, map_v;
@@ -840,6 +844,7 @@ KESTREL_API int kestrel_attention_tc_kept(const void *q, const void *k_cache, co
     if (rc) return rc;
     p.keep_first = window > 0 ? keep_first : 0;
     p.gate = gate;
+    p.nseq = nseq;
     const dim3 grid((unsigned)((long long)tiles * nkv));
     rc = rows_per_tile <= AT_BM ? at_launch<false, AT_KEPT, true>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile)
                                  : at_launch<false, AT_KEPT>(grid, stream, map_k, map_v, p, cache_pages, rows_per_tile);

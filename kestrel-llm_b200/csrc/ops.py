@@ -624,12 +624,14 @@ def attention_mma(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
 
 
 def attention_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, out: torch.Tensor,
-                 tile_seq: torch.Tensor, tile_row0: torch.Tensor, cu_seqlens: torch.Tensor, kv_lens: torch.Tensor,
+                 tile_seq: Optional[torch.Tensor], tile_row0: Optional[torch.Tensor], cu_seqlens: torch.Tensor, kv_lens: torch.Tensor,
                  block_table: torch.Tensor, page_size: int, nq: int, nkv: int, hd: int, window: int, scale: float,
                  slices: int = 1, slice_len: int = 1 << 30, max_kv_dev: Optional[torch.Tensor] = None,
-                 rows_per_tile: int = 128, score: Optional["ScoreOptions"] = None, keep_first: int = 0, gate: Optional[torch.Tensor] = None) -> None:
+                 rows_per_tile: int = 128, score: Optional["ScoreOptions"] = None, keep_first: int = 0, gate: Optional[torch.Tensor] = None,
+                 tiles: int = 0) -> None:
     """tcgen05 attention of the listed tiles, head size 128 (with a layer's `ScoreOptions`; sigmoid weights in one slice; or, plain softmax
-    in one slice, with ``keep_first`` tokens that stay visible to a windowed layer and a ``gate`` float32 [T, nq] on the heads' outputs): tiles of ``rows_per_tile`` rows, up
+    in one slice, with ``keep_first`` tokens that stay visible to a windowed layer and a ``gate`` float32 [T, nq] on the heads' outputs, where
+    the kernel finds its tiles itself if their lists are None: all ``tiles`` of the step, `count_row_tiles`): tiles of ``rows_per_tile`` rows, up
     to 256 (prompt portions; 16 for decode tokens); the key range may be cut into
     ``slices`` slices of ``slice_len`` keys (a multiple of 128) that are merged in ascending
     order; ``slices * slice_len`` must reach the longest request.  The cache tensors are
@@ -640,10 +642,16 @@ def attention_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
     _need(k_cache, "attention_tc.k_cache", torch.bfloat16)
     _need(v_cache, "attention_tc.v_cache", torch.bfloat16)
     _need(block_table, "attention_tc.block_table", torch.int32, 2)
-    _need(tile_seq, "attention_tc.tile_seq", torch.int32, 1)
-    _need(tile_row0, "attention_tc.tile_row0", torch.int32, 1)
-    T, tiles = q.shape[0], tile_seq.shape[0]
-    if q.shape[1] != nq * hd or out.shape != q.shape or tile_row0.shape[0] != tiles:
+    T, found = q.shape[0], tile_seq is None and tile_row0 is None
+    if found:
+        if gate is None and not keep_first or tiles <= 0:
+            raise KernelError("attention_tc: only the form with kept tokens or a gate finds its tiles, and it is told how many")
+        _need(cu_seqlens, "attention_tc.cu_seqlens", torch.int32, 1)
+    else:
+        _need(tile_seq, "attention_tc.tile_seq", torch.int32, 1)
+        _need(tile_row0, "attention_tc.tile_row0", torch.int32, 1)
+        tiles = tile_seq.shape[0]
+    if q.shape[1] != nq * hd or out.shape != q.shape or (not found and tile_row0.shape[0] != tiles):
         raise KernelError("attention_tc: shapes differ")
     if tuple(k_cache.shape[1:]) != (nkv, page_size, hd) or v_cache.shape != k_cache.shape:
         raise KernelError(f"attention_tc: cache of shape {tuple(k_cache.shape)}, expected [pages, {nkv}, {page_size}, {hd}]")
@@ -655,9 +663,9 @@ def attention_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
             if tuple(gate.shape) != (T, nq):
                 raise KernelError(f"attention_tc: gate of shape {tuple(gate.shape)}, expected [{T}, {nq}]")
         _check(library().kestrel_attention_tc_kept(
-            q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), tile_seq.data_ptr(), tile_row0.data_ptr(), tiles,
-            int(rows_per_tile), cu_seqlens.data_ptr(), kv_lens.data_ptr(), block_table.data_ptr(), block_table.shape[1], block_table.stride(0),
-            int(page_size), int(k_cache.shape[0]), T, nq, nkv, hd, int(window), int(keep_first), _p(gate), float(scale), _stream()))
+            q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), _p(tile_seq), _p(tile_row0), tiles,
+            int(rows_per_tile), cu_seqlens.data_ptr(), cu_seqlens.shape[0] - 1, kv_lens.data_ptr(), block_table.data_ptr(), block_table.shape[1],
+            block_table.stride(0), int(page_size), int(k_cache.shape[0]), T, nq, nkv, hd, int(window), int(keep_first), _p(gate), float(scale), _stream()))
         return
     part_o = part_ml = None
     if slices > 1:
@@ -696,8 +704,7 @@ def attention_rows_tc(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, b
         _need(gate, "attention_rows_tc.gate", torch.float32, 2)
         if tuple(gate.shape) != (T, nq):
             raise KernelError(f"attention_rows_tc: gate of shape {tuple(gate.shape)}, expected [{T}, {nq}]")
-    tile_seq, tile_row0 = row_tiles(batch, nq // nkv, 128)
-    tiles = tile_seq.shape[0]
+    tiles = count_row_tiles(batch, nq // nkv, 128)
     # A CTA walks its keys at some 1.5 us per 64.  Half of the SMs idle or more, and keys enough for two slices of 512: as many
     # slices as fill the SMs once.
     slices, slice_len = 1, (1 << 30) // 128 * 128
@@ -711,8 +718,8 @@ def attention_rows_tc(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, b
         part_o = torch.empty((T * nq, slices, vd), dtype=torch.float32, device=q.device)
         part_ml = torch.empty((T * nq, slices, 2), dtype=torch.float32, device=q.device)
     _check(library().kestrel_attention_rows_tc(
-        q.data_ptr(), cache.data_ptr(), out.data_ptr(), _p(part_o), _p(part_ml), tile_seq.data_ptr(), tile_row0.data_ptr(), tiles, 128,
-        batch.cu_seqlens.data_ptr(), batch.kv_lens.data_ptr(), block_table.data_ptr(), block_table.shape[1], block_table.stride(0), int(page_size),
+        q.data_ptr(), cache.data_ptr(), out.data_ptr(), _p(part_o), _p(part_ml), None, None, tiles, 128,
+        batch.cu_seqlens.data_ptr(), batch.num_seqs, batch.kv_lens.data_ptr(), block_table.data_ptr(), block_table.shape[1], block_table.stride(0), int(page_size),
         int(cache.shape[0]), T, nq, nkv, hd, vd, int(window), slices, slice_len, _p(gate), float(scale), _stream()))
     if slices > 1:
         global launches
@@ -1350,8 +1357,13 @@ def row_tiles(batch, rows_per_token: int, rows_per_tile: int = 256):
     return kept[key]
 
 
-def attention_tc_tiles(batch, group: int, nkv: int, window: int, keep_first: int = 0):
-    """`row_tiles` for `attention_tc` and the rows of a tile: 128 where such tiles fit the SMs at once (a CTA's two streams then share its key
+def count_row_tiles(batch, rows_per_token: int, rows_per_tile: int) -> int:
+    """How many tiles `row_tiles` lists, for kernels that find theirs on the device."""
+    return sum(-(-n * rows_per_token // rows_per_tile) for n in batch.counts)
+
+
+def attention_tc_rows(batch, group: int, nkv: int, window: int, keep_first: int = 0) -> int:
+    """Rows of a tile of `attention_tc`: 128 where such tiles fit the SMs at once (a CTA's two streams then share its key
     tiles out), or come in up to two rounds of them and the longest walk of a tile of 256 - one request's last tokens - would set the time: at
     half a step a key tile, spread over the SMs, plus three steps for a second round's start, at most three quarters of that walk
     (2,048 tokens of 16 / 4 heads 44 -> 35 us; four portions of 500, whose walks are short, 24 -> 27 and stay).  256 otherwise."""
@@ -1372,8 +1384,13 @@ def attention_tc_tiles(batch, group: int, nkv: int, window: int, keep_first: int
             if walk * nkv / (2.0 * sms) + 3.0 <= 0.75 * longest:
                 rows = 128
         kept[key] = rows
-    tile_seq, tile_row0 = row_tiles(batch, group, kept[key])
-    return tile_seq, tile_row0, kept[key]
+    return kept[key]
+
+
+def attention_tc_tiles(batch, group: int, nkv: int, window: int, keep_first: int = 0):
+    """`row_tiles` for `attention_tc`, and the rows of a tile."""
+    rows = attention_tc_rows(batch, group, nkv, window, keep_first)
+    return (*row_tiles(batch, group, rows), rows)
 
 
 # ---- differential attention: two maps a head over the same values --------------------------------

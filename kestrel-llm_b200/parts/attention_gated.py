@@ -234,24 +234,30 @@ class GatedWindowAttention(Mixer):
                 batch.max_count * G > self.TC_MIN_ROWS and \
                 ops.attention_tc_supported(128, cache.page_size):
             # prompt portions of head size 128: the tcgen05 kernel, rows in tiles of 256 or (softmax weights) 128 per request
+            if gate is not None or self.keep_first:         # in one slice; the kernel finds its tiles
+                rows = ops.attention_tc_rows(batch, G, self.kv_heads, self.window, self.keep_first)
+                ops.attention_tc(q, cache.k, cache.v, a, None, None, batch.cu_seqlens, batch.kv_lens, table, cache.page_size, self.heads,
+                                 self.kv_heads, 128, self.window, self.scale, rows_per_tile=rows, keep_first=self.keep_first, gate=gate,
+                                 tiles=ops.count_row_tiles(batch, G, rows))
+                return a
             if self.score.weighting == "sigmoid":
                 (tile_seq, tile_row0), rows = ops.row_tiles(batch, G, 256), 256
             else:
-                tile_seq, tile_row0, rows = ops.attention_tc_tiles(batch, G, self.kv_heads, self.window, self.keep_first)
+                tile_seq, tile_row0, rows = ops.attention_tc_tiles(batch, G, self.kv_heads, self.window)
             # Few tiles far into a long context (a later portion of a long prompt) leave most SMs idle: softmax weights
             # without a window then take the key range in slices, as many as fill the chip, merged in ascending order.
             # A whole prompt has tiles enough and stays in one slice (cut at 512 keys, 2,048 tokens of 16 heads took 188
             # instead of 171 us: the slices' float32 outputs and their merge cost more than the even load gains).
             slices, slice_len = 1, 1 << 30
             fill = self.TC_SLICE_FILL // max(1, int(tile_seq.shape[0]) * self.kv_heads)
-            if self.window == 0 and gate is None and self.score.weighting != "sigmoid" and fill >= 2 and batch.max_kv_len > 2 * self.TC_SLICE and \
+            if self.window == 0 and self.score.weighting != "sigmoid" and fill >= 2 and batch.max_kv_len > 2 * self.TC_SLICE and \
                     (self.score.weighting != "softmax_sink" or self.score.sink is not None):
                 per = -(-batch.max_kv_len // min(32, fill))          # keys a slice if the chip is to be filled, in whole key tiles
                 slice_len = max(self.TC_SLICE, (per + 127) // 128 * 128)
                 slices = -(-batch.max_kv_len // slice_len)
             ops.attention_tc(q, cache.k, cache.v, a, tile_seq, tile_row0, batch.cu_seqlens, batch.kv_lens, table, cache.page_size, self.heads,
                              self.kv_heads, 128, self.window, self.scale, slices=slices,
-                             slice_len=slice_len, rows_per_tile=rows, score=score, keep_first=self.keep_first, gate=gate)
+                             slice_len=slice_len, rows_per_tile=rows, score=score)
         elif self.dtype == torch.bfloat16 and not self.force_plain and self.decode and self._capped_only and gate is None and \
                 self.head_dim == self.v_head_dim and self.keep_first == 0 and \
                 ops.attention_decode_capped(q, cache.k, cache.v, batch, table, cache.page_size, a, self.heads, self.kv_heads, self.head_dim, self.window,
