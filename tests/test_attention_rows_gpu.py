@@ -51,3 +51,42 @@ def test_a_gate_on_outputs_from_slices_is_rounded_with_them(heads, portions, row
     want = (want[:, None, :] * gate.double()[:, :, None]).reshape(T, -1)
     half = torch.exp2(torch.floor(torch.log2(want.abs())) - 8)
     assert ((out.double() - want).abs() / half).max().item() <= 1 + 1 / 16
+
+
+@pytest.mark.parametrize("heads,portions", [(4, [(33, 100), (70, 0)]), (16, [(20, 1500), (9, 40)]), (1, [(300, 5), (1, 900)])])
+@pytest.mark.parametrize("rows,vd", [(72, 64), (256, 192), (40, 24)])
+@pytest.mark.parametrize("window", [0, 70])
+def test_rows_against_float64_among_stale_pages(heads, portions, rows, vd, window):
+    """Every number of the cache that no row may see is NaN, and one query row is infinite.  P is rounded to bfloat16, and so is the output:
+    2^-8 of the weights' mean of |value| and 2^-8 of the output, beside 2^-12 of the largest for exp2 and float32 sums."""
+    import torch
+    from kestrel_llm_b200.csrc import ops
+    torch.manual_seed(heads)
+    cache, batch = _step(portions, rows)
+    plane, dev, T = cache.k[0], "cuda", batch.num_tokens
+    plane.fill_(float("nan"))
+    kv = []
+    for i, (n, c) in enumerate(portions):
+        at = torch.arange(n + c, device=dev)
+        seen = at[(at > c - window) | (window == 0)]
+        x = torch.zeros(n + c, rows, dtype=torch.bfloat16, device=dev)
+        x[seen] = torch.randn(len(seen), rows, device=dev).to(torch.bfloat16)
+        plane[torch.tensor(cache.block_table(i, 0), device=dev)[seen // 16], 0, seen % 16] = x[seen]
+        kv.append(x.double())
+    q, gate = torch.randn(T, heads * rows, device=dev).to(torch.bfloat16), torch.rand(T, heads, device=dev)
+    q[12, 7] = float("inf")                     # head 0 of one token
+    out = torch.full((T, heads * vd), float("nan"), dtype=torch.bfloat16, device=dev)
+    ops.attention_rows_tc(q, plane, out, batch, batch.block_table(0), 16, heads, 1, rows, vd, window, rows ** -0.5, gate)
+    assert ops.library().kestrel_attention_rows_tc_error() == 0
+    for i, (n, c) in enumerate(portions):
+        t = slice(int(batch.cu_seqlens[i]), int(batch.cu_seqlens[i + 1]))
+        s = torch.einsum("nhd,ld->hnl", q[t].view(n, heads, rows).double(), kv[i]) * rows ** -0.5
+        dist = torch.arange(c, c + n, device=dev)[:, None] - torch.arange(n + c, device=dev)
+        s = s.masked_fill((dist < 0) | ((dist >= window) & (window > 0)), -float("inf"))
+        p = (s - s.amax(-1, keepdim=True)).exp()
+        p = p / p.sum(-1, keepdim=True) * gate[t].double().t()[:, :, None]
+        want, size = torch.einsum("hnl,ld->nhd", p, kv[i][:, :vd]), torch.einsum("hnl,ld->nhd", p, kv[i][:, :vd].abs())
+        got = out[t].view(n, heads, vd).double()
+        assert torch.equal(torch.isnan(want), torch.isnan(got))
+        limit = 2.0 ** -8 * (size + want.abs()) + 2.0 ** -12 * want.nan_to_num().abs().max()
+        assert ((got - want).abs() <= limit)[~torch.isnan(want)].all()
