@@ -21,8 +21,11 @@
 // The scan is the kernel of delta_rule.cu in another order of operations: a CTA of four warps
 // takes 16 value columns of one (request, head); the eight lanes of a column hold interleaved
 // parts of its key channels; per token a thread makes its part of b^T S, the lanes add in a
-// fixed shuffle tree, then each channel is updated and read out.  The order of every sum is
-// fixed, so a token's result does not depend on how the request was cut into steps or batched.
+// fixed shuffle tree, then each channel is updated and read out.  The order of every sum of the
+// scan is fixed, so its results do not depend on how the request was cut into steps or batched.
+// Layers in float32 always take it; in bfloat16 a step with portions of many tokens takes the
+// blocks of recurrence_blocks.cu instead, the same sums in another order, and which of the two
+// runs depends on the step's requests.
 #include "common.cuh"
 #include "head_norm.cuh"
 #include <math.h>

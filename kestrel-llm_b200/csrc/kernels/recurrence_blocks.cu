@@ -1,5 +1,5 @@
 // The sequential recurrences of linear_recurrence.cu and delta_rule.cu for portions of many tokens, in blocks of 16: the same sums in
-// another order, all of them float32.
+// another order, the products and the sums of pairs in float64, what lies between them in float32.
 //
 // A token's step, S <- diag(w_t) S + a_t (b_t^T S) + k_t v_t^T, is a chain of two reductions over the key channels, some 600 cycles
 // however many threads share it.  Over a block of 16 tokens the state S_0 at its start is all that has to be read in order:
@@ -17,20 +17,25 @@
 // (the warps' parts meet in shared memory), the 16 x 16 matrices, S^T update; two barriers.  A prepared block (38 KB at 128 channels) comes
 // by one bulk copy into a ring, values by cp.async four blocks ahead.
 //
-// Every product is float32: operands as two terms of 11 bits, three products (rb_split, rb_mma3).  From float64 the read-outs are as far as the
-// sequential scan's within the tests' limit.  With plain multiply-adds the same blocks are bound by the shared-memory reads of
-// operands that 16 columns cannot reuse: 3,300 cycles a block against 1,500 here (DELTA).
+// The products are the float64 ones of the tensor cores, and a portion's state is float64 from its first block to its last.  Read-outs and states
+// are then closer to a float64 evaluation than the sequential scan's: 0.7 to 0.97 of its distance in a model of the roundings, at memories of 5
+// to 300 tokens.  Operands as two terms of 11 bits on the tf32 products were not: those accumulators cut off instead of rounding, and with the
+// state among them the read-outs were 1.8 (memory 20) to 4.3 times (300) as far as the scan's; summed afresh each block still 1.3 times.
+// An SM makes 64 multiply-adds of float64 a cycle, 64 cycles a product and warp: 1,150 (GATE) to 2,300 (REMOVAL) cycles a block and
+// CTA, which is what bounds the scan where CTAs share an SM.  Prepared and scanned without their gates, tf32 -> float64: DELTA 213 -> 245 us, GATE
+// 137 -> 165, REMOVAL 106 -> 123 (sizes below).  With plain float32 multiply-adds the same blocks are bound by the shared-memory reads of
+// operands that 16 columns cannot reuse: 322 us for DELTA's scan alone.
 //
 // What is not finite stays so, and reaches the tokens and channels that it reaches in the scan: a block whose read-outs or corrections are
-// not finite sums them again token by token (an infinity may come out as NaN, whose terms have both signs).
+// not finite sums them again token by token (an infinity may come out as NaN, where terms of both signs meet).
 //
 // Three forms: GATE (no correction), REMOVAL (a, b given) and DELTA (a gated delta rule: with u = beta (v - (diag(w) S)^T k),
 // S <- diag(w) S + k u^T, so that b = w k and the writes u = X beta (v - b^T S_0) take the place of v).
 //
-// Measured, 16 heads, gates and blocks prepared + scan against gates kernel + sequential scan: DELTA (128 channels, requests of 592 and 1,185
-// tokens) 67 + 131 us against 37 + 523; GATE (64 channels, 2,048 tokens) 22 + 101 against 27 + 291; REMOVAL (128 channels, 700 tokens in
-// three requests, 350 the longest) 50 + 63 against 55 + 205.  (With the gates still a kernel of its own: 36 + 53 + 132, 27 + 23 + 101 and
-// 56 + 34 + 69.)  The scan's blocks are the chain of three products and their barriers; the preparation is bound by its instructions.
+// Measured, 16 heads, prepared + scanned against the sequential scan, the gates in either case made before: DELTA (128 channels, requests of 592
+// and 1,185 tokens) 245 us against 517; GATE (64 channels, 2,048 tokens) 165 against 287; REMOVAL (128 channels, 700 tokens in three
+// requests, 350 the longest) 123 against 213.  The layers, which make their gates in the preparation, take 413, 403 and 238 us
+// where they took 713, 838 and 371.
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include <initializer_list>
@@ -46,6 +51,7 @@
 enum { RB_GATE = 0, RB_REMOVAL = 1, RB_DELTA = 2 };
 
 __device__ int g_rb_error = 0;
+
 
 // a prepared block of a head: [b decayed | r decayed | k to the block's end | a to the block's end | P(0, 16) | matrices]
 template <int D, int FORM> struct RbLayout {
@@ -104,11 +110,11 @@ __device__ __forceinline__ float rb_sigmoid(float z) { return 1.0f / (1.0f + exp
 
 // One exchange of a sum of N values over the lanes: a lane keeps the half of the values that its bit of MASK names and adds the other
 // lane's share of them.  Five of them, from 32 values, leave lane l with the sum of value l.
-template <int N, int MASK> __device__ __forceinline__ void rb_exchange(float *x, int lane) {
+template <int N, int MASK> __device__ __forceinline__ void rb_exchange(double *x, int lane) {
     const bool up = (lane & MASK) != 0;
 #pragma unroll
     for (int i = 0; i < N / 2; ++i) {
-        const float keep = up ? x[i + N / 2] : x[i], give = up ? x[i] : x[i + N / 2];
+        const double keep = up ? x[i + N / 2] : x[i], give = up ? x[i] : x[i + N / 2];
         x[i] = keep + __shfl_xor_sync(0xffffffffu, give, MASK);
     }
 }
@@ -298,7 +304,7 @@ blocks_prepare_kernel(const RbParams p, const RbSource src) {
 #pragma unroll 1
     for (int i = 0; i < 4; ++i) {
         const int s = i == 0 ? warp : i == 1 ? 7 - warp : i == 2 ? 8 + warp : 15 - warp;
-        float xk[V], xa[V];
+        double xk[V], xa[V];
 #pragma unroll
         for (int j = 0; j < V; ++j) {           // neighbouring channels: they come in one load
             xk[j] = sk[s * D + lane * V + j];
@@ -306,27 +312,28 @@ blocks_prepare_kernel(const RbParams p, const RbSource src) {
         }
 #pragma unroll 1
         for (int part = s / TG; part < RB_B / TG; ++part) {
-            float x[32];                        // [t][the form's matrices]
+            double x[32];                       // [t][the form's matrices]
 #pragma unroll
             for (int u = 0; u < TG; ++u) {
                 const int t = part * TG + u;
-                float fA = 0.f, fK = 0.f, fQa = 0.f, fQk = 0.f;
+                double fA = 0.0, fK = 0.0, fQa = 0.0, fQk = 0.0;
                 if (t >= s) {
 #pragma unroll
                     for (int j = 0; j < V; ++j) {
                         const int o = t * D + lane * V + j;
                         if (t > s) {
                             if (FORM != RB_GATE) {
-                                const float bb = sb[o];
-                                fK = fmaf(bb, xk[j], fK);
-                                if (FORM == RB_REMOVAL) fA = fmaf(bb, xa[j], fA);
+                                const double bb = sb[o];
+                                fK = fma(bb, xk[j], fK);
+                                if (FORM == RB_REMOVAL) fA = fma(bb, xa[j], fA);
                             }
-                            xk[j] *= sw[o];
-                            if (FORM == RB_REMOVAL) xa[j] *= sw[o];
+                            const double ww = sw[o];
+                            xk[j] *= ww;
+                            if (FORM == RB_REMOVAL) xa[j] *= ww;
                         }
-                        const float rr = sr[o];
-                        fQk = fmaf(rr, xk[j], fQk);
-                        if (FORM == RB_REMOVAL) fQa = fmaf(rr, xa[j], fQa);
+                        const double rr = sr[o];
+                        fQk = fma(rr, xk[j], fQk);
+                        if (FORM == RB_REMOVAL) fQa = fma(rr, xa[j], fQa);
                     }
                 }
                 if (FORM == RB_REMOVAL) x[4 * u] = fA, x[4 * u + 1] = fK, x[4 * u + 2] = fQa, x[4 * u + 3] = fQk;
@@ -340,15 +347,15 @@ blocks_prepare_kernel(const RbParams p, const RbSource src) {
                 rb_exchange<4, 4>(x, lane);
                 rb_exchange<2, 2>(x, lane);
                 x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
-                mQk[(lane >> 1) * RB_LD + s] = x[0];
+                mQk[(lane >> 1) * RB_LD + s] = (float)x[0];
             } else {
                 rb_exchange<32, 16>(x, lane);
                 rb_exchange<16, 8>(x, lane);
                 rb_exchange<8, 4>(x, lane);
                 rb_exchange<4, 2>(x, lane);
                 rb_exchange<2, 1>(x, lane);
-                if (FORM == RB_REMOVAL) mat[(lane & 3) * RB_MAT + (part * TG + (lane >> 2)) * RB_LD + s] = x[0];
-                else (lane & 1 ? mQk : mK)[(lane >> 1) * RB_LD + s] = x[0];
+                if (FORM == RB_REMOVAL) mat[(lane & 3) * RB_MAT + (part * TG + (lane >> 2)) * RB_LD + s] = (float)x[0];
+                else (lane & 1 ? mQk : mK)[(lane >> 1) * RB_LD + s] = (float)x[0];
             }
         }
     }
@@ -359,16 +366,16 @@ blocks_prepare_kernel(const RbParams p, const RbSource src) {
     }
     // X, a column a thread, by substitution: REMOVAL (I - A)^-1; DELTA (I + beta A)^-1 beta with A in mK
     if (tid < RB_B) {
-        float x[RB_B];
+        double x[RB_B];
 #pragma unroll
         for (int t = 0; t < RB_B; ++t) {
             const float beta = FORM == RB_DELTA ? sbeta[t] : 0.f;
-            float sum = 0.f;
+            double sum = 0;
 #pragma unroll
-            for (int s = 0; s < t; ++s) sum = fmaf((FORM == RB_DELTA ? mK : mA)[t * RB_LD + s], x[s], sum);
+            for (int s = 0; s < t; ++s) sum = fma((double)(FORM == RB_DELTA ? mK : mA)[t * RB_LD + s], x[s], sum);
             const float one = t == tid ? 1.f : 0.f;
             x[t] = FORM == RB_DELTA ? beta * (one - sum) : one + sum;
-            mX[t * RB_LD + tid] = x[t];
+            mX[t * RB_LD + tid] = (float)x[t];
         }
     }
     __syncthreads();
@@ -409,40 +416,16 @@ blocks_prepare_kernel(const RbParams p, const RbSource src) {
     }
 }
 
-// One step of 8 along the sum, m16n8k8 with float32 results; operands are float32 numbers whose low 13 bits the unit ignores
-__device__ __forceinline__ void rb_mma(float *c, const uint32_t *a, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+// c += a * b, one step of 8 along the sum, m16n8k8 in float64
+__device__ __forceinline__ void rb_mma(double *c, const double *a, double b0, double b1) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+                 : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
 }
-// x as two terms of 11 bits, both rounded to the nearest: the first leaves 2^-12 of x (exactly what the subtraction gives), the second
-// 2^-24.  (Cut off instead of rounded the two terms leave 2^-21 and the products of the second ones, which are dropped, 2^-20: read-outs
-// were 5e-7 of the largest off where the scan is 8e-8 off.)  The unit ignores the low 13 bits of the second.  What is not finite is its
-// own first term: rounded as a number, the sum would carry out of the exponent and a NaN of all ones become a zero.
-__device__ __forceinline__ void rb_split(float x, uint32_t &hi, uint32_t &lo) {
-    const uint32_t u = __float_as_uint(x);
-    const bool number = (u & 0x7f800000u) != 0x7f800000u;
-    hi = number ? (u + 0x1000u) & 0xffffe000u : u;
-    lo = number ? __float_as_uint(x - __uint_as_float(hi)) + 0x1000u : 0u;
-}
-struct RbA { uint32_t hi[4], lo[4]; };
 // Operand A from a row-major pair of numbers per row: (row l / 4: x0 at 2 (l % 4), x1 behind it; row l / 4 + 8: x2, x3).  The unit's k index
 // l % 4 is taken for the even, l % 4 + 4 for the odd of the two; operand B pairs its numbers the same way.
-__device__ __forceinline__ void rb_a(RbA &a, float x0, float x1, float x2, float x3) {
-    rb_split(x0, a.hi[0], a.lo[0]);
-    rb_split(x2, a.hi[1], a.lo[1]);
-    rb_split(x1, a.hi[2], a.lo[2]);
-    rb_split(x3, a.hi[3], a.lo[3]);
-}
-// c += a * b in three products of the terms (the fourth is 2^-24 of the first); the small ones in a sum of their own, for shorter chains
-__device__ __forceinline__ void rb_mma3(float *c, float *small, const RbA &a, float y0, float y1) {
-    uint32_t h0, l0, h1, l1;
-    rb_split(y0, h0, l0);
-    rb_split(y1, h1, l1);
-    rb_mma(small, a.lo, h0, h1);
-    rb_mma(c, a.hi, h0, h1);
-    rb_mma(small, a.hi, l0, l1);
-}
+struct RbA { double x[4]; };
+__device__ __forceinline__ RbA rb_a(double x0, double x1, double x2, double x3) { return {{x0, x2, x1, x3}}; }
 
 template <int D, int FORM>
 __global__ void __launch_bounds__(128)
@@ -482,7 +465,7 @@ blocks_scan_kernel(const RbParams p, int stages) {
         for (int i = 0; i < min(stages, n_blocks); ++i) fetch(i);
     float *Sg = p.state + (size_t)p.slots[seq] * p.state_stride + (size_t)h * p.d * p.dv;     // [d][dv]
     // S^T of the warp's channels: S[ct] = columns lr, lr + 8 of the CTA by channels lc, lc + 1 of the tile
-    float S[CT][4];
+    double S[CT][4];
 #pragma unroll
     for (int ct = 0; ct < CT; ++ct)
 #pragma unroll
@@ -514,26 +497,25 @@ blocks_scan_kernel(const RbParams p, int stages) {
         asm volatile("cp.async.wait_group 2;" ::: "memory");       // this block's values; the barrier below shows them to all
         if (ok && !mbar_wait(bar0 + 8u * stage, (uint32_t)(i / stages) & 1u)) { atomicExch(&g_rb_error, 1); ok = false; }
         {   // what the warp's channels of the state give to the block's rows
-            float acc[NT][4], small[NT][4];
+            double acc[NT][4];
 #pragma unroll
             for (int n = 0; n < NT; ++n)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) acc[n][e] = small[n][e] = 0.f;
+                for (int e = 0; e < 4; ++e) acc[n][e] = 0.0;
 #pragma unroll
             for (int ct = 0; ct < CT; ++ct) {
-                RbA a;
-                rb_a(a, S[ct][0], S[ct][1], S[ct][2], S[ct][3]);
+                const RbA a = rb_a(S[ct][0], S[ct][1], S[ct][2], S[ct][3]);
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {                   // rows: BD, then RD (GATE: RD)
                     const float2 b = *reinterpret_cast<const float2 *>(st + (n * 8 + lr) * L::ROW_LD + ch0 + ct * 8 + lc);
-                    rb_mma3(acc[n], small[n], a, b.x, b.y);
+                    rb_mma(acc[n], a.x, b.x, b.y);
                 }
             }
 #pragma unroll
             for (int n = 0; n < NT; ++n)
 #pragma unroll
                 for (int e = 0; e < 2; ++e)
-                    *reinterpret_cast<float2 *>(&red[warp][lr + 8 * e][n * 8 + lc]) = make_float2(acc[n][2 * e] + small[n][2 * e], acc[n][2 * e + 1] + small[n][2 * e + 1]);
+                    *reinterpret_cast<float2 *>(&red[warp][lr + 8 * e][n * 8 + lc]) = make_float2((float)acc[n][2 * e], (float)acc[n][2 * e + 1]);
         }
         __syncthreads();                        // and every warp is done with the block before
         if (tid == 0 && i > 0 && i - 1 + stages < n_blocks) fetch(i - 1 + stages);
@@ -558,7 +540,8 @@ blocks_scan_kernel(const RbParams p, int stages) {
         const bool reads = warp >= 2;
         const int half = warp & 1;
         if (reads || FORM != RB_GATE) {
-            float acc[4] = {0.f, 0.f, 0.f, 0.f}, small[4] = {0.f, 0.f, 0.f, 0.f};
+            double sum[4] = {0.0, 0.0, 0.0, 0.0};
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
             const float *m0 = st + L::M, *m1 = m0 + RB_MAT;
             const int row = (half * 8 + lr) * RB_LD + lc;
             if (reads) total((FORM == RB_GATE ? 0 : 2) + half, acc);
@@ -569,26 +552,25 @@ blocks_scan_kernel(const RbParams p, int stages) {
                 if (FORM == RB_DELTA) {         // v - b^T S_0 takes the values' place
                     float x[4];
                     total(ks, x);
-                    rb_a(av, u0[0] - x[0], u1[0] - x[1], u0[8] - x[2], u1[8] - x[3]);
+                    av = rb_a((double)u0[0] - x[0], (double)u1[0] - x[1], (double)u0[8] - x[2], (double)u1[8] - x[3]);
                 } else {
-                    rb_a(av, u0[0], u1[0], u0[8], u1[8]);
+                    av = rb_a(u0[0], u1[0], u0[8], u1[8]);
                 }
                 const float *mv = FORM == RB_GATE ? m0 : FORM == RB_DELTA ? (reads ? m1 : m0) : (reads ? m0 + 3 * RB_MAT : m1);
                 float2 b = *reinterpret_cast<const float2 *>(mv + row + ks * 8);
-                rb_mma3(acc, small, av, b.x, b.y);
+                rb_mma(sum, av.x, b.x, b.y);
                 if (FORM == RB_REMOVAL) {
                     float x[4];
-                    RbA ah;
                     total(ks, x);
-                    rb_a(ah, x[0], x[1], x[2], x[3]);
+                    const RbA ah = rb_a(x[0], x[1], x[2], x[3]);
                     b = *reinterpret_cast<const float2 *>((reads ? m0 + 2 * RB_MAT : m0) + row + ks * 8);
-                    rb_mma3(acc, small, ah, b.x, b.y);
+                    rb_mma(sum, ah.x, b.x, b.y);
                 }
             }
             bool number = true;
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                acc[e] += small[e];
+                acc[e] = (float)(sum[e] + acc[e]);
                 number = number && fabsf(acc[e]) < INFINITY;
             }
             if (!__all_sync(0xffffffffu, number)) {
@@ -629,7 +611,6 @@ blocks_scan_kernel(const RbParams p, int stages) {
         }
         if (FORM != RB_GATE) __syncthreads();
         // the state at the block's end
-        float small[CT][4];
 #pragma unroll
         for (int ct = 0; ct < CT; ++ct) {
             const float2 d2 = *reinterpret_cast<const float2 *>(st + L::DT + ch0 + ct * 8 + lc);
@@ -637,8 +618,6 @@ blocks_scan_kernel(const RbParams p, int stages) {
             S[ct][1] *= d2.y;
             S[ct][2] *= d2.x;
             S[ct][3] *= d2.y;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) small[ct][e] = 0.f;
         }
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
@@ -646,32 +625,25 @@ blocks_scan_kernel(const RbParams p, int stages) {
 #pragma unroll
                 for (int ct = 0; ct < CT; ++ct) {
                     const float *b = rows + (ks * 8 + lc) * L::END_LD + ch0 + ct * 8 + lr;
-                    rb_mma3(S[ct], small[ct], a, b[0], b[L::END_LD]);
+                    rb_mma(S[ct], a.x, b[0], b[L::END_LD]);
                 }
             };
-            RbA a;
             if (FORM != RB_DELTA) {
                 const float *u0 = &vr[ks * 8 + lc][lr], *u1 = &vr[ks * 8 + lc + 1][lr];
-                rb_a(a, u0[0], u1[0], u0[8], u1[8]);
-                write(a, st + L::KW);
+                write(rb_a(u0[0], u1[0], u0[8], u1[8]), st + L::KW);
             }
             if (FORM != RB_GATE) {
                 const float2 x0 = *reinterpret_cast<const float2 *>(&corr[lr][ks * 8 + lc]), x1 = *reinterpret_cast<const float2 *>(&corr[lr + 8][ks * 8 + lc]);
-                rb_a(a, x0.x, x0.y, x1.x, x1.y);
-                write(a, st + (FORM == RB_DELTA ? L::KW : L::AW));
+                write(rb_a(x0.x, x0.y, x1.x, x1.y), st + (FORM == RB_DELTA ? L::KW : L::AW));
             }
         }
-#pragma unroll
-        for (int ct = 0; ct < CT; ++ct)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) S[ct][e] += small[ct][e];
     }
 #pragma unroll
     for (int ct = 0; ct < CT; ++ct)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int c = ch0 + ct * 8 + lc + (e & 1), j = col0 + lr + (e >> 1) * 8;
-            if (c < p.d && j < p.dv) Sg[(size_t)c * p.dv + j] = S[ct][e];
+            if (c < p.d && j < p.dv) Sg[(size_t)c * p.dv + j] = (float)S[ct][e];
         }
 }
 

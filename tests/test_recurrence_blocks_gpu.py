@@ -243,3 +243,43 @@ def test_what_is_not_finite_reaches_later_tokens_alone(form, what, at, value):
         assert (np.isfinite(a) == np.isfinite(b)).all(), name
         a, b = a[np.isfinite(a)].astype(np.float64), b[np.isfinite(a)]
         assert np.abs(a - b).max(initial=0) <= 2.0 ** -20 * np.abs(a).max(initial=1), name
+
+
+@pytest.mark.parametrize("form", ["gate", "removal", "delta"])
+@pytest.mark.parametrize("H,d,dv", [(3, 128, 128), (4, 64, 96), (2, 32, 40)])
+@pytest.mark.parametrize("memory", [5.0, 20.0, 300.0])
+def test_blocks_are_as_close_to_float64_as_the_scan(form, H, d, dv, memory):
+    """Over several hundred tokens, with memories as long: the distance of read-outs and states from float64 (2-norms, in which the rounding of
+    some 10,000 numbers averages out) is at most the scan's and a tenth."""
+    import torch
+    from kestrel_llm_b200.csrc import ops
+    rng = np.random.default_rng(int(memory) + d)
+    batch, cu, slots = _step((400, 133), d)
+    T = batch.num_tokens
+
+    def f32(x):
+        return torch.from_numpy(np.ascontiguousarray(x.reshape(x.shape[0], -1), dtype=np.float32)).cuda()
+
+    def f64(t, m):
+        return t.cpu().numpy().astype(np.float64).reshape(T, H, m)
+    r, k, v, w = rng.standard_normal((T, H, d)), rng.standard_normal((T, H, d)), rng.standard_normal((T, H, dv)), np.exp(-rng.exponential(1 / memory, (T, H, d)))
+    k = 1 - w if form == "gate" else k / np.sqrt((k * k).sum(-1, keepdims=True))
+    r, w, k, v, rate, beta = f32(r), f32(w), f32(k), f32(v), f32(-rng.random((T, H, d)) * k), f32(rng.random((T, H)))
+    state0 = f32(0.3 * rng.standard_normal((3, H, d, dv)))
+    pair = (rate, k) if form == "removal" else (None, None)
+    far = []
+    for blocks in (False, True):
+        state = state0.clone()
+        if form == "delta":
+            out = torch.empty((T, H * dv), device="cuda")
+            (ops.delta_blocks if blocks else ops.delta_scan)(r, k, w, v, 0, beta, state, batch, out, H, H, d, dv)
+        else:
+            out = (ops.recurrence_blocks if blocks else ops.recurrence_scan)(r, w, k, v, *pair, state, 0, batch, H, d, dv)
+        far.append((out.cpu().numpy().astype(np.float64), state.cpu().numpy().astype(np.float64)))
+    ops.raise_on_kernel_error()
+    v, w, k, bt = f64(v, dv), f64(w, d), f64(k, d), f64(beta, 1)
+    a, b = (-bt * k, w * k) if form == "delta" else (f64(rate, d), k) if form == "removal" else (None, None)
+    want = _evaluate(f64(r, d), w, k, bt * v if form == "delta" else v, a, b, state0.cpu().numpy().astype(np.float64), cu, slots)
+    for name, scan, blocks, exact in zip(("read-outs", "states"), *far, want):
+        ref, err = (np.linalg.norm(x - exact) / np.linalg.norm(exact) for x in (scan, blocks))
+        assert err <= 1.1 * ref, f"{name}: {err:.2e} from float64, the scan {ref:.2e}"
