@@ -1774,15 +1774,19 @@ def recurrence_scan(r: torch.Tensor, w: torch.Tensor, k: torch.Tensor, v: torch.
     return out
 
 
-BLOCK_TOKENS, BLOCK_TOKENS_ALL = 112, 256       # in blocks: as many tokens of one request, or a quarter of them where the step has as many in all
+# in blocks: as many tokens of one request, or a quarter of them where the step has as many in all, and tokens times heads
+BLOCK_TOKENS, BLOCK_TOKENS_ALL, BLOCK_HEADS_ALL = 112, 256, 4096
 
 
-def recurrence_in_blocks(batch, dtype: torch.dtype, d: int) -> bool:
+def recurrence_in_blocks(batch, dtype: torch.dtype, d: int, heads: int) -> bool:
     """Whether a step runs its recurrences in blocks of 16 tokens.  Not in float32, whose logits are the same bits however a request was
-    cut, and not in a recorded step.  One request's scan of few tokens ends before two launches do (16 heads, scan against blocks: 64
-    tokens 10 / 12 us without a correction, 21 / 26 with one, 23 / 27 the delta rule; 128 tokens 19 / 21, 41 / 32, 45 / 32); several
-    requests' scans share the SMs and lose earlier (eight of 32 tokens: 20 / 16, 56 / 42, 43 / 38)."""
-    enough = batch.max_count >= BLOCK_TOKENS or (4 * batch.max_count >= BLOCK_TOKENS and batch.num_tokens >= BLOCK_TOKENS_ALL)
+    cut, and not in a recorded step.  One request's scan of few tokens ends before two launches do: scan / blocks in us, beside which the
+    scan has its gates kernel (some 4 us), 112 tokens of 2, 8, 16 and 64 heads without a correction 17 / 15, 17 / 15, 17 / 22, 39 / 28, with one
+    36 / 30, 36 / 30, 36 / 40, 104 / 70, the delta rule 40 / 25, 40 / 25, 40 / 38, 75 / 68; 256 tokens of 16 heads 37 / 33, 79 / 61, 88 / 54.
+    Scans of several requests and many heads share the SMs and lose earlier: eight requests of 32 tokens, 2 heads 6 / 10, 12 / 21 and 13 / 18,
+    8 heads 13 / 13, 34 / 33, 25 / 31, 16 heads 20 / 20, 56 / 54, 43 / 45, 32 heads 37 / 30, 103 / 82, 86 / 65."""
+    enough = batch.max_count >= BLOCK_TOKENS or (4 * batch.max_count >= BLOCK_TOKENS and batch.num_tokens >= BLOCK_TOKENS_ALL and
+                                                 batch.num_tokens * heads >= BLOCK_HEADS_ALL)
     return dtype == torch.bfloat16 and not batch.captured and enough and d <= 128
 
 
@@ -1795,7 +1799,7 @@ def _block_scratch(T: int, batch, H: int, d: int, form: int, device) -> torch.Te
 
 def recurrence_blocks(r: torch.Tensor, w: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: Optional[torch.Tensor], b: Optional[torch.Tensor],
                       state: torch.Tensor, state_off: int, batch, H: int, d: int, dv: int) -> torch.Tensor:
-    """`recurrence_scan` in blocks of 16 tokens (two launches): other order of sums, all of them float32."""
+    """`recurrence_scan` in blocks of 16 tokens (two launches): other order of sums, products in float64."""
     _need(state, "recurrence_blocks.state", torch.float32, 2)
     T = r.shape[0]
     for t, name, n in ((r, "r", H * d), (w, "w", H * d), (k, "k", H * d), (v, "v", H * dv), (a, "a", H * d), (b, "b", H * d)):
@@ -1820,7 +1824,7 @@ def recurrence_blocks(r: torch.Tensor, w: torch.Tensor, k: torch.Tensor, v: torc
 
 def delta_blocks(qn: torch.Tensor, kn: torch.Tensor, decay: torch.Tensor, act: torch.Tensor, col_v: int, beta: torch.Tensor,
                  state: torch.Tensor, batch, out: torch.Tensor, H: int, G: int, d: int, dv: int) -> None:
-    """`delta_scan` in blocks of 16 tokens (two launches): other order of sums, all of them float32."""
+    """`delta_scan` in blocks of 16 tokens (two launches): other order of sums, products in float64."""
     _need(out, "delta_blocks.out", torch.float32, 2)
     _need(state, "delta_blocks.state", torch.float32, 2)
     _need(act, "delta_blocks.act", torch.float32, 2)

@@ -84,7 +84,7 @@ class ChannelDeltaMixer(Mixer):
         a = self.a2.forward(ops.partial_columns(fused, self.col_a1, self.ra, self.dtype))
         g = self.g2.forward(ops.partial_columns(fused, self.col_g1, self.rg, self.dtype))
         o = torch.empty((T, H * dv), dtype=f32, device=dev)
-        in_blocks = self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d)
+        in_blocks = self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d, H)
         if not (in_blocks and ops.gated_delta_blocks(act, self.col_v, fused, self.col_beta, a, self.A_log, self.dt_bias, cache.state, batch, o,
                                                      H, G, d, dv)):
             qn = torch.empty((T, G * d), dtype=f32, device=dev)

@@ -5,7 +5,7 @@ request's state slot (float32, zero at admission).  Both run on one scan,
 
 with everything that enters it in float32; what differs is how a layer makes w, a, b, k, v, r
 from its input h.  In bfloat16, portions of many tokens take the scan in blocks of 16 tokens
-(`ops.recurrence_blocks`), float32 sums in another order.
+(`ops.recurrence_blocks`): another order of sums, products in float64.
 
 `ForgetGateRecurrence` (the HGRN2 form of linear attention): H heads, d key and dv value channels,
 
@@ -69,7 +69,7 @@ class ForgetGateRecurrence(Mixer):
     def forward(self, x: torch.Tensor, batch, cache) -> ops.Partials:
         H, d, dv = self.H, self.d, self.dv
         fused = self.in_proj.forward(x)
-        o, in_blocks = None, self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d)
+        o, in_blocks = None, self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d, H)
         if in_blocks:
             o = ops.gated_blocks(fused, self.col_q, 0, self.col_v, self.col_f, self.f_bias, self.lower, None, 0.0, cache.state, batch, H, d, dv)
         if o is None:
@@ -119,7 +119,7 @@ class RemovalDeltaMixer(Mixer):
         H, d = self.H, self.d
         fused = self.in_proj.forward(x)
         wz = self.w2.forward(ops.partial_columns_act(fused, self.col_w1, self.rank, self.dtype, "tanh"))
-        o, in_blocks = None, self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d)
+        o, in_blocks = None, self.blocks and ops.recurrence_in_blocks(batch, self.dtype, d, H)
         if in_blocks:
             o = ops.gated_blocks(fused, self.col_r, self.col_k, self.col_v, self.col_a, self.a_bias, self.w0, wz, self.decay_rate, cache.state,
                                  batch, H, d, d)
