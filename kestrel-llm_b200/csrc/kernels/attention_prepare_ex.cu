@@ -474,7 +474,7 @@ KESTREL_API int kestrel_attn_prepare_maps(const float *partial, int S, long long
     KESTREL_REQUIRE(hd <= 32 * APX_PER_LANE && vd <= 32 * APX_PER_LANE, "attn_prepare_ex: head size %d / %d exceeds %d", hd, vd, 32 * APX_PER_LANE);
     const int need = nq * maps * hd + (has_kv ? nkv * (maps * hd + vd) : 0) + (gate_out ? nq : 0);
     KESTREL_REQUIRE(ld >= need, "attn_prepare_ex: the product has %d columns, the heads need %d", ld, need);
-    // the fast form for heads of several maps (those of one keep the kernel, and the bits, they have)
+    // the fast form for heads of several maps (those of one have theirs below, in bfloat16; in float32 they take the general kernel)
     if (maps > 1 && inv_freq && rot == hd && rot_mode == 0 && qk_norm == 1 && !bias && !v_norm && q_temp_every == 0 && !gate_out && nq > 0 && vd % hd == 0 &&
         (hd == 32 || hd == 64 || hd == 128) && ld % 4 == 0 && slice_stride % 4 == 0 && ((uintptr_t)partial & 15) == 0 && (dtype == KESTREL_F32 || dtype == KESTREL_BF16)) {
 #define APR_CASE(TT, H_) return apr_launch<TT, H_>(partial, S, slice_stride, ld, q_norm_w, k_norm_w, norm_eps, positions, seq_of_token, block_table, table_stride, page_size, \

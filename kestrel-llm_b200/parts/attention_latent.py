@@ -47,7 +47,9 @@ from .linear import Linear
 class LatentAttention(Mixer):
     force_plain = False        # tests: bfloat16 through the plain attention kernel too
     tcgen05 = True             # tests: off, portions stay on the mma.sync kernel
-    TC_MIN_ROWS = 64           # a step whose longest portion has more rows (tokens x heads) takes the tcgen05 kernel
+    # a step whose longest portion has more rows (tokens x heads) takes the tcgen05 kernel: a layer of 16 heads over 5 tokens 157 us on the mma.sync
+    # kernel and 155 on this one, 17 behind 500 159 and 155, 20 behind 2,900 428 and 182 (with a step built for each pass 233 / 230, 236 / 232, 436 / 241)
+    TC_MIN_ROWS = 64
     expand_prompts = True      # tests: off, starting portions too run over the cached latents
     EXPAND_MIN_TOKENS = 64     # a step whose longest portion has more tokens may take the expanded form
     graph_safe = True          # forward launches kernels over device tensors of the batch only (the expanded form reads the
