@@ -21,10 +21,10 @@
 // are then closer to a float64 evaluation than the sequential scan's: 0.7 to 0.97 of its distance in a model of the roundings, at memories of 5
 // to 300 tokens.  Operands as two terms of 11 bits on the tf32 products were not: those accumulators cut off instead of rounding, and with the
 // state among them the read-outs were 1.8 (memory 20) to 4.3 times (300) as far as the scan's; summed afresh each block still 1.3 times.
-// An SM makes 64 multiply-adds of float64 a cycle, 64 cycles a product and warp: 1,150 (GATE) to 2,300 (REMOVAL) cycles a block and
-// CTA, which is what bounds the scan where CTAs share an SM.  Prepared and scanned without their gates, tf32 -> float64: DELTA 213 -> 245 us, GATE
-// 137 -> 165, REMOVAL 106 -> 123 (sizes below).  With plain float32 multiply-adds the same blocks are bound by the shared-memory reads of
-// operands that 16 columns cannot reuse: 322 us for DELTA's scan alone.
+// An SM makes 64 multiply-adds of float64 a cycle, 64 cycles a product and warp: 1,150 (GATE), 1,660 (DELTA) and 2,300 (REMOVAL) cycles a
+// block and CTA, beside which come the conversions and the barriers: 2,250 cycles a block with one CTA an SM (GATE), 4,960 with two (DELTA).
+// Prepared and scanned without their gates, tf32 -> float64: DELTA 213 -> 245 us, GATE 137 -> 165, REMOVAL 106 -> 123 (sizes below).  With plain
+// float32 multiply-adds the same blocks are bound by the shared-memory reads of operands that 16 columns cannot reuse: 322 us for DELTA's scan.
 //
 // What is not finite stays so, and reaches the tokens and channels that it reaches in the scan: a block whose read-outs or corrections are
 // not finite sums them again token by token (an infinity may come out as NaN, where terms of both signs meet).
@@ -34,8 +34,8 @@
 //
 // Measured, 16 heads, prepared + scanned against the sequential scan, the gates in either case made before: DELTA (128 channels, requests of 592
 // and 1,185 tokens) 245 us against 517; GATE (64 channels, 2,048 tokens) 165 against 287; REMOVAL (128 channels, 700 tokens in three
-// requests, 350 the longest) 123 against 213.  The layers, which make their gates in the preparation, take 413, 403 and 238 us
-// where they took 713, 838 and 371.
+// requests, 350 the longest) 123 against 213.  The layers, which make their gates in the preparation, take 81 + 190, 26 + 147 and
+// 55 + 93 us for the two launches, where gates kernel and scan took 37 + 523, 27 + 291 and 55 + 205.
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include <initializer_list>
