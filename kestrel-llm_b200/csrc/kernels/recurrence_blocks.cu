@@ -9,33 +9,41 @@
 //     o_t = r_t^T S_t     = (r_t P(0, t))^T S_0     + sum_(s<=t) [r_t P(s, t) a_s] h_s    + [r_t P(s, t) k_s] v_s
 //     S_16                = P(0, 16) S_0            + sum_s (P(s, 16) a_s) h_s            + (P(s, 16) k_s) v_s
 //
-// The brackets are numbers per pair of tokens and head.  `blocks_prepare` makes them for all blocks at once, with the decayed vectors,
-// and solves the triangular system: h = X (b^T S_0) + XK v with X = (I - A)^-1, and what o takes from b^T S_0 and v.  `blocks_scan` then
-// walks a request's blocks: a CTA takes 16 value columns of a head, transposed, its four warps a quarter of the channels each, S^T in the
+// The brackets are numbers per pair of tokens and head.  `blocks_prepare` makes them for all blocks at once, with the decayed vectors, and
+// solves the triangular system, so that all that depends on S_0 is one product with rows made beforehand (X = (I - A)^-1):
+//
+//     h = F1^T S_0 + M1 v,   F1 = X b,        M1 = X K          S_16 = P(0, 16) S_0 + (a to the end)^T h + (k to the end)^T v
+//     o = F2^T S_0 + M2 v,   F2 = r + Qa F1,  M2 = Qa M1 + Qk
+//
+// `blocks_scan` walks a request's blocks: a CTA takes 16 value columns of a head, transposed, its warps a share of the channels each, S^T in the
 // accumulators of m16n8k8 products: the accumulators are the next product's operand A as they stand (the sum over channels may run in any
-// order, so the unit's k index takes the channels in the order in which the accumulators hold them).  Per block: S^T times the decayed b and r
-// (the warps' parts meet in shared memory), the 16 x 16 matrices, S^T update; two barriers.  A prepared block (38 KB at 128 channels) comes
-// by one bulk copy into a ring, values by cp.async four blocks ahead.
+// order, so the unit's k index takes the channels in the order in which the accumulators hold them).  Per block: S^T times F1 and F2, to which a
+// warp adds a share of M1 v and M2 v; one exchange of the warps' sums through shared memory; the writes.  GATE's writes need no sum: a block
+// has one barrier, off the state's path; the others have two.  A prepared block (29 KB for DELTA at 128 channels) comes by two bulk copies into a
+// ring, what meets the state and what is written to it, the first free again as soon as the products are done; values by cp.async three blocks ahead.
 //
-// The products are the float64 ones of the tensor cores, and a portion's state is float64 from its first block to its last.  Read-outs and states
-// are then closer to a float64 evaluation than the sequential scan's: 0.7 to 0.97 of its distance in a model of the roundings, at memories of 5
-// to 300 tokens.  Operands as two terms of 11 bits on the tf32 products were not: those accumulators cut off instead of rounding, and with the
-// state among them the read-outs were 1.8 (memory 20) to 4.3 times (300) as far as the scan's; summed afresh each block still 1.3 times.
-// An SM makes 64 multiply-adds of float64 a cycle, 64 cycles a product and warp: 1,150 (GATE), 1,660 (DELTA) and 2,300 (REMOVAL) cycles a
-// block and CTA, beside which come the conversions and the barriers: 2,250 cycles a block with one CTA an SM (GATE), 4,960 with two (DELTA).
-// Prepared and scanned without their gates, tf32 -> float64: DELTA 213 -> 245 us, GATE 137 -> 165, REMOVAL 106 -> 123 (sizes below).  With plain
-// float32 multiply-adds the same blocks are bound by the shared-memory reads of operands that 16 columns cannot reuse: 322 us for DELTA's scan.
+// The products are the float64 ones of the tensor cores; a portion's state and what the warps exchange are float64 from its first block to its
+// last.  Distance of read-outs and states from a float64 evaluation, at memories of 5 to 300 tokens: 0.44 to 0.9 of the sequential scan's.
+// Operands as two terms of 11 bits on the tf32 products were further off than the scan (those accumulators cut off instead of rounding);
+// float32 sums exchanged by the warps took read-outs at a memory of 5 from 0.44 to 0.6, states from 0.64 to 0.93.
 //
-// What is not finite stays so, and reaches the tokens and channels that it reaches in the scan: a block whose read-outs or corrections are
-// not finite sums them again token by token (an infinity may come out as NaN, where terms of both signs meet).
+// What bounds it.  An SM makes 64 multiply-adds of float64 a cycle, 64 cycles a product and quarter SM: 640 (GATE, 64 channels), 1,700 (DELTA) and
+// 2,200 (REMOVAL) cycles a block and CTA.  Conversions from float32 (8 cycles a warp) run beside them.  A lone CTA takes 1,600 (GATE) to 3,600
+// cycles a block, the chain of products, exchange and writes; two share an SM at 58 to 65 % of the products' rate.  GATE gains from eight warps
+// (118 us against 142 for the launches below), the others lose more by eight sums to add than they gain (DELTA 216 against 210).  With plain float32 multiply-adds the
+// blocks are bound by the shared-memory reads of operands that 16 columns cannot reuse: 322 us for DELTA's scan.
+// The preparation reads and converts a token's vectors once for four pairs, and exchanges each sum over the lanes (a third of its instructions).
+//
+// What is not finite stays so, and reaches the tokens and channels that it reaches in the scan: where a value or a prepared row is not
+// finite, its sums are made again from the tokens that count (an infinity may come out as NaN, where terms of both signs meet).
 //
 // Three forms: GATE (no correction), REMOVAL (a, b given) and DELTA (a gated delta rule: with u = beta (v - (diag(w) S)^T k),
-// S <- diag(w) S + k u^T, so that b = w k and the writes u = X beta (v - b^T S_0) take the place of v).
+// S <- diag(w) S + k u^T, so that b = w k, the writes u take the place of v, F1 = - X b with X = (I + beta K)^-1 beta, F2 = r + Qk F1,
+// M1 = X and M2 = Qk X).
 //
-// Measured, 16 heads, prepared + scanned against the sequential scan, the gates in either case made before: DELTA (128 channels, requests of 592
-// and 1,185 tokens) 245 us against 517; GATE (64 channels, 2,048 tokens) 165 against 287; REMOVAL (128 channels, 700 tokens in three
-// requests, 350 the longest) 123 against 213.  The layers, which make their gates in the preparation, take 81 + 190, 26 + 147 and
-// 55 + 93 us for the two launches, where gates kernel and scan took 37 + 523, 27 + 291 and 55 + 205.
+// Measured, 16 heads, prepared + scanned in us, beside the blocks that exchanged h and o in turn (four pairs' sums by a warp each) and the
+// sequential scan: DELTA (128 channels, requests of 592 and 1,185 tokens) 202 (244; 517); GATE (64 channels, 2,048 tokens) 113 (165; 287);
+// REMOVAL (128 channels, 700 tokens in three requests, 350 the longest) 100 (124; 213).
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include <initializer_list>
@@ -53,26 +61,32 @@ enum { RB_GATE = 0, RB_REMOVAL = 1, RB_DELTA = 2 };
 __device__ int g_rb_error = 0;
 
 
-// a prepared block of a head: [b decayed | r decayed | k to the block's end | a to the block's end | P(0, 16) | matrices]
+// A prepared block of a head: what meets the state, [rows that give h | rows that give o | what values add to h | to o], then what is
+// written to it, [k to the block's end | a to the block's end | P(0, 16)]; each comes by one bulk copy.
 template <int D, int FORM> struct RbLayout {
     static constexpr int ROW_LD = D + 8, END_LD = D + 4;        // rows read as pairs along the channels, and as pairs of rows
-    static constexpr int BD = 0;
-    static constexpr int RD = FORM == RB_GATE ? 0 : RB_B * ROW_LD;
-    static constexpr int KW = RD + RB_B * ROW_LD;
+    static constexpr bool H = FORM != RB_GATE;
+    static constexpr int F1 = 0;
+    static constexpr int F2 = H ? RB_B * ROW_LD : 0;
+    static constexpr int M1 = F2 + RB_B * ROW_LD;
+    static constexpr int M2 = H ? M1 + RB_MAT : M1;
+    static constexpr int KW = M2 + RB_MAT;
     static constexpr int AW = KW + RB_B * END_LD;
     static constexpr int DT = FORM == RB_REMOVAL ? AW + RB_B * END_LD : AW;
-    static constexpr int M = DT + D;            // GATE: Qk; DELTA: X beta, Qk X beta; REMOVAL: X, X K, Qa X, Qa X K + Qk
-    static constexpr int FLOATS = M + (FORM == RB_GATE ? 1 : FORM == RB_DELTA ? 2 : 4) * RB_MAT;
+    static constexpr int FLOATS = DT + D;
+    static constexpr int MATS = FORM == RB_GATE ? 1 : FORM == RB_DELTA ? 3 : 6;     // matrices of the preparation
 };
 
-// What a CTA of the scan holds beside its ring (a GATE block corrects nothing, and alternates between two buffers of sums)
-template <int FORM> struct RbScan {
-    static constexpr int ROWS = FORM == RB_GATE ? RB_B : 2 * RB_B;      // rows that meet the state: b and r
-    static constexpr int RED_LD = ROWS + 8;
-    unsigned long long bars[RB_STAGES];
-    float red[FORM == RB_GATE ? 2 : 1][4][RB_COLS][RED_LD];
+// What a CTA of the scan holds beside its ring (a GATE block waits for none of its sums: two buffers of them in turn)
+template <int D, int FORM> struct RbScan {
+    static constexpr int WARPS = FORM == RB_GATE && D >= 64 ? 8 : 4;   // a share of the channels each
+    static constexpr int NT = FORM == RB_GATE ? 2 : 4;                  // tiles of eight rows that meet the state
+    static constexpr int LD = RB_B + 8;                                 // (pairs of doubles of two neighbouring columns on all 32 banks)
+    unsigned long long bars[RB_STAGES][2];
+    double red_h[FORM == RB_GATE ? 1 : WARPS][FORM == RB_GATE ? 1 : RB_COLS][LD];             // the warps' sums by column and token
+    double red_o[FORM == RB_GATE ? 2 : 1][WARPS][RB_COLS][LD];
+    double corr[FORM == RB_GATE ? 1 : RB_COLS][LD];                     // h (DELTA: the writes), summed
     float vals[4][RB_B][RB_VLD];                // values [token][column] of four blocks in flight: loaded for the next block alone they set the pace (2,400 cycles a block)
-    float corr[FORM == RB_GATE ? 1 : RB_COLS][RB_LD];
 };
 
 struct RbParams {
@@ -119,21 +133,50 @@ template <int N, int MASK> __device__ __forceinline__ void rb_exchange(double *x
     }
 }
 
+// c += a * b, one step of 8 along the sum, m16n8k8 in float64
+__device__ __forceinline__ void rb_mma(double *c, const double *a, double b0, double b1) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+                 : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
+}
+// Operand A from a row-major pair of numbers per row: (row l / 4: x0 at 2 (l % 4), x1 behind it; row l / 4 + 8: x2, x3).  The unit's k index
+// l % 4 is taken for the even, l % 4 + 4 for the odd of the two; operand B pairs its numbers the same way.
+struct RbA { double x[4]; };
+__device__ __forceinline__ RbA rb_a(double x0, double x1, double x2, double x3) { return {{x0, x2, x1, x3}}; }
+
+__device__ __forceinline__ void rb_put2(double *to, double x, double y) { *reinterpret_cast<double2 *>(to) = make_double2(x, y); }
+template <int N> struct RbCount { static constexpr int value = N; };
+// V neighbouring numbers in one load
+template <int V> __device__ __forceinline__ void rb_load(float *x, const float *p) {
+    if constexpr (V == 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(p);
+        x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+    } else if constexpr (V == 2) {
+        const float2 v = *reinterpret_cast<const float2 *>(p);
+        x[0] = v.x, x[1] = v.y;
+    } else {
+        x[0] = p[0];
+    }
+}
+
 template <int D, int FORM, bool MADE>
 __global__ void __launch_bounds__(128)
 blocks_prepare_kernel(const RbParams p, const RbSource src) {
     using L = RbLayout<D, FORM>;
     constexpr int V = D / 32;                   // channels of a lane
-    pdl_launch_dependents();
     pdl_wait();
     const int blk = blockIdx.x, h = blockIdx.y, seq = blockIdx.z;
     const int t0 = p.cu_seqlens[seq] + blk * RB_B, t1 = p.cu_seqlens[seq + 1];
     if (t0 >= t1) return;
     extern __shared__ __align__(16) float rb_sm[];
     // [w | r | k | b | a] of the block's tokens, zero (w: one) beyond the head's channels and the request's tokens
-    float *sw = rb_sm, *sr = sw + RB_B * D, *sk = sr + RB_B * D, *sb = sk + RB_B * D, *sa = sb + (FORM == RB_GATE ? 0 : RB_B * D);
-    float *mat = sa + (FORM == RB_REMOVAL ? RB_B * D : 0);                     // A, K, Qa, Qk and two more, rows of RB_LD
-    float *mA = mat, *mK = mA + RB_MAT, *mQa = mK + RB_MAT, *mQk = mQa + RB_MAT, *mX = mQk + RB_MAT, *mY = mX + RB_MAT;
+    constexpr int LD = L::END_LD;               // of a token's row
+    float *sw = rb_sm, *sr = sw + RB_B * LD, *sk = sr + RB_B * LD, *sb = sk + RB_B * LD, *sa = sb + (FORM == RB_GATE ? 0 : RB_B * LD);
+    // per pair of tokens, rows of RB_LD: GATE Qk; DELTA K, Qk, X; REMOVAL K, Qk, A, Qa, X, X K
+    constexpr int MATS = L::MATS;
+    double *mat = reinterpret_cast<double *>(sa + (FORM == RB_REMOVAL ? RB_B * LD : 0));
+    double *mK = mat, *mQk = mat + (MATS > 1 ? RB_MAT : 0), *mA = mat + 2 * RB_MAT, *mQa = mat + 3 * RB_MAT, *mX = mat + (MATS - 2 + (FORM == RB_DELTA)) * RB_MAT,
+           *mY = mat + 5 * RB_MAT;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kh = FORM == RB_DELTA ? h / (p.H / p.G) : h, KH = FORM == RB_DELTA ? p.G : p.H;
     __shared__ float sbeta[RB_B], sinv[2][RB_B];
@@ -180,10 +223,11 @@ blocks_prepare_kernel(const RbParams p, const RbSource src) {
                     }
                 }
             }
-            *reinterpret_cast<float4 *>(sw + idx) = w4;
-            *reinterpret_cast<float4 *>(sr + idx) = r4;
-            *reinterpret_cast<float4 *>(sk + idx) = k4;
-            if (FORM == RB_REMOVAL) *reinterpret_cast<float4 *>(sa + idx) = a4;
+            const int at = t * LD + c;
+            *reinterpret_cast<float4 *>(sw + at) = w4;
+            *reinterpret_cast<float4 *>(sr + at) = r4;
+            *reinterpret_cast<float4 *>(sk + at) = k4;
+            if (FORM == RB_REMOVAL) *reinterpret_cast<float4 *>(sa + at) = a4;
         }
         if (FORM == RB_DELTA && tid < RB_B) {
             float z = 0.f;
@@ -203,7 +247,7 @@ blocks_prepare_kernel(const RbParams p, const RbSource src) {
                 float sk2 = 0.f, sr2 = 0.f;
 #pragma unroll
                 for (int j = 0; j < V; ++j) {
-                    const float k = sk[t * D + lane * V + j], r = sr[t * D + lane * V + j];
+                    const float k = sk[t * LD + lane * V + j], r = sr[t * LD + lane * V + j];
                     sk2 = fmaf(k, k, sk2);
                     sr2 = fmaf(r, r, sr2);
                 }
@@ -217,15 +261,15 @@ blocks_prepare_kernel(const RbParams p, const RbSource src) {
             __syncthreads();
 #pragma unroll
             for (int i = 0; i < RB_B * D / 128; ++i) {
-                const int idx = tid + 128 * i, t = idx / D;
-                const float u = sk[idx] * sinv[0][t];
+                const int t = (tid + 128 * i) / D, at = t * LD + (tid + 128 * i) % D;
+                const float u = sk[at] * sinv[0][t];
                 if (FORM == RB_REMOVAL) {
-                    sb[idx] = u;
-                    sa[idx] = -(sa[idx] * u);
+                    sb[at] = u;
+                    sa[at] = -(sa[at] * u);
                 } else {
-                    sk[idx] = u;
-                    sr[idx] *= sinv[1][t];
-                    sb[idx] = sw[idx] * u;
+                    sk[at] = u;
+                    sr[at] *= sinv[1][t];
+                    sb[at] = sw[at] * u;
                 }
             }
         }
@@ -249,16 +293,16 @@ blocks_prepare_kernel(const RbParams p, const RbSource src) {
         }
 #pragma unroll
         for (int i = 0; i < N; ++i) {
-            const int idx = (tid + 128 * i) * 4;
-            *reinterpret_cast<float4 *>(sw + idx) = w4[i];
-            *reinterpret_cast<float4 *>(sr + idx) = r4[i];
-            *reinterpret_cast<float4 *>(sk + idx) = k4[i];
+            const int at = (tid + 128 * i) * 4 / D * LD + (tid + 128 * i) * 4 % D;
+            *reinterpret_cast<float4 *>(sw + at) = w4[i];
+            *reinterpret_cast<float4 *>(sr + at) = r4[i];
+            *reinterpret_cast<float4 *>(sk + at) = k4[i];
             if (FORM == RB_REMOVAL) {
-                *reinterpret_cast<float4 *>(sb + idx) = b4[i];
-                *reinterpret_cast<float4 *>(sa + idx) = a4[i];
+                *reinterpret_cast<float4 *>(sb + at) = b4[i];
+                *reinterpret_cast<float4 *>(sa + at) = a4[i];
             }
             if (FORM == RB_DELTA)
-                *reinterpret_cast<float4 *>(sb + idx) = make_float4(w4[i].x * k4[i].x, w4[i].y * k4[i].y, w4[i].z * k4[i].z, w4[i].w * k4[i].w);
+                *reinterpret_cast<float4 *>(sb + at) = make_float4(w4[i].x * k4[i].x, w4[i].y * k4[i].y, w4[i].z * k4[i].z, w4[i].w * k4[i].w);
         }
     } else {
 #pragma unroll 4
@@ -267,202 +311,300 @@ blocks_prepare_kernel(const RbParams p, const RbSource src) {
             const bool in = t0 + t < t1 && c < p.d;
             const size_t oh = ((size_t)(t0 + t) * p.H + h) * p.d + c, ok = ((size_t)(t0 + t) * KH + kh) * p.d + c;
             const float w = in ? p.w[oh] : 1.f, k = in ? p.k[ok] : 0.f;
-            sw[idx] = w;
-            sr[idx] = in ? p.r[ok] : 0.f;
-            sk[idx] = k;
+            const int at = t * LD + c;
+            sw[at] = w;
+            sr[at] = in ? p.r[ok] : 0.f;
+            sk[at] = k;
             if (FORM == RB_REMOVAL) {
-                sb[idx] = in ? p.b[oh] : 0.f;
-                sa[idx] = in ? p.a[oh] : 0.f;
+                sb[at] = in ? p.b[oh] : 0.f;
+                sa[at] = in ? p.a[oh] : 0.f;
             }
-            if (FORM == RB_DELTA) sb[idx] = w * k;
+            if (FORM == RB_DELTA) sb[at] = w * k;
         }
     }
-    for (int idx = tid; idx < 6 * RB_MAT; idx += 128) mat[idx] = 0.f;
+    for (int idx = tid; idx < MATS * RB_MAT; idx += 128) mat[idx] = 0.0;
     __syncthreads();
 
     float *blkp = p.blocks + ((size_t)(p.cu_seqlens[seq] / RB_B + seq + blk) * p.H + h) * L::FLOATS;
-    // vectors decayed from the block's start and to its end, a channel a thread
-    for (int c = tid; c < D; c += 128) {
-        float run = 1.f;
+    // The pairs: a warp takes four neighbouring tokens s and walks t = s .. 15, so that a token's b, r and w are read and converted once
+    // for four pairs (16 a cycle and SM, a quarter of the multiply-adds' rate); blocks give the longest walk to another quarter of the SM each.
+    // The sums of TG tokens t go through the lanes together.
+    constexpr int SUMS = FORM == RB_GATE ? 1 : FORM == RB_DELTA ? 2 : 4, TG = FORM == RB_REMOVAL ? 2 : 4, VALUES = 4 * TG * SUMS;
+    {
+        const int s0 = ((warp + blk + h) & 3) * 4;
+        double xk[4][V], xa[FORM == RB_REMOVAL ? 4 : 1][V];
 #pragma unroll
-        for (int t = 0; t < RB_B; ++t) {
-            if (FORM != RB_GATE) blkp[L::BD + t * L::ROW_LD + c] = sb[t * D + c] * run;
-            run *= sw[t * D + c];
-            blkp[L::RD + t * L::ROW_LD + c] = sr[t * D + c] * run;
-        }
-        blkp[L::DT + c] = run;
-        run = 1.f;
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int t = RB_B - 1; t >= 0; --t) {
-            blkp[L::KW + t * L::END_LD + c] = sk[t * D + c] * run;
-            if (FORM == RB_REMOVAL) blkp[L::AW + t * L::END_LD + c] = sa[t * D + c] * run;
-            run *= sw[t * D + c];
-        }
-    }
-    // the pairs: a warp takes four tokens s, evenly long walks t = s .. 15 among them; the sums of TG t's go through the lanes together
-    constexpr int TG = FORM == RB_REMOVAL ? 8 : RB_B;
-#pragma unroll 1
-    for (int i = 0; i < 4; ++i) {
-        const int s = i == 0 ? warp : i == 1 ? 7 - warp : i == 2 ? 8 + warp : 15 - warp;
-        double xk[V], xa[V];
-#pragma unroll
-        for (int j = 0; j < V; ++j) {           // neighbouring channels: they come in one load
-            xk[j] = sk[s * D + lane * V + j];
-            xa[j] = FORM == RB_REMOVAL ? sa[s * D + lane * V + j] : 0.f;
-        }
-#pragma unroll 1
-        for (int part = s / TG; part < RB_B / TG; ++part) {
-            double x[32];                       // [t][the form's matrices]
+            for (int j = 0; j < V; ++j) {       // neighbouring channels: they come in one load
+                xk[i][j] = sk[(s0 + i) * LD + lane * V + j];
+                if (FORM == RB_REMOVAL) xa[i][j] = sa[(s0 + i) * LD + lane * V + j];
+            }
+        // tokens t .. t + TG - 1, OFF or (4) more behind s0
+        auto walk = [&](auto off, int t0_) {
+            constexpr int OFF = decltype(off)::value;
+            double x[VALUES];                   // [t][s][sum]
 #pragma unroll
             for (int u = 0; u < TG; ++u) {
-                const int t = part * TG + u;
-                double fA = 0.0, fK = 0.0, fQa = 0.0, fQk = 0.0;
-                if (t >= s) {
+                const int o = (t0_ + u) * LD + lane * V;
+                float b[V], w[V], r[V];
+                if (FORM != RB_GATE) rb_load<V>(b, sb + o);
+                rb_load<V>(w, sw + o);
+                rb_load<V>(r, sr + o);
+                double f[4][SUMS];
 #pragma unroll
-                    for (int j = 0; j < V; ++j) {
-                        const int o = t * D + lane * V + j;
-                        if (t > s) {
-                            if (FORM != RB_GATE) {
-                                const double bb = sb[o];
-                                fK = fma(bb, xk[j], fK);
-                                if (FORM == RB_REMOVAL) fA = fma(bb, xa[j], fA);
-                            }
-                            const double ww = sw[o];
-                            xk[j] *= ww;
-                            if (FORM == RB_REMOVAL) xa[j] *= ww;
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int m = 0; m < SUMS; ++m) f[i][m] = 0.0;
+#pragma unroll
+                for (int j = 0; j < V; ++j) {
+                    const double bb = FORM == RB_GATE ? 0.0 : (double)b[j], ww = w[j], rr = r[j];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        if (OFF + u > i) {
+                            if (FORM != RB_GATE) f[i][0] = fma(bb, xk[i][j], f[i][0]);
+                            if (FORM == RB_REMOVAL) f[i][2] = fma(bb, xa[i][j], f[i][2]);
+                            xk[i][j] *= ww;
+                            if (FORM == RB_REMOVAL) xa[i][j] *= ww;
                         }
-                        const double rr = sr[o];
-                        fQk = fma(rr, xk[j], fQk);
-                        if (FORM == RB_REMOVAL) fQa = fma(rr, xa[j], fQa);
+                        if (OFF + u >= i) {
+                            f[i][SUMS > 1 ? 1 : 0] = fma(rr, xk[i][j], f[i][SUMS > 1 ? 1 : 0]);
+                            if (FORM == RB_REMOVAL) f[i][3] = fma(rr, xa[i][j], f[i][3]);
+                        }
                     }
                 }
-                if (FORM == RB_REMOVAL) x[4 * u] = fA, x[4 * u + 1] = fK, x[4 * u + 2] = fQa, x[4 * u + 3] = fQk;
-                else if (FORM == RB_DELTA) x[2 * u] = fK, x[2 * u + 1] = fQk;
-                else x[u] = fQk;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int m = 0; m < SUMS; ++m) x[(u * 4 + i) * SUMS + m] = f[i][m];
             }
             // lane l ends with value l (GATE: l / 2)
-            if (FORM == RB_GATE) {
+            if constexpr (VALUES == 16) {
                 rb_exchange<16, 16>(x, lane);
                 rb_exchange<8, 8>(x, lane);
                 rb_exchange<4, 4>(x, lane);
                 rb_exchange<2, 2>(x, lane);
                 x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
-                mQk[(lane >> 1) * RB_LD + s] = (float)x[0];
+                mQk[(t0_ + (lane >> 3)) * RB_LD + s0 + ((lane >> 1) & 3)] = x[0];
             } else {
                 rb_exchange<32, 16>(x, lane);
                 rb_exchange<16, 8>(x, lane);
                 rb_exchange<8, 4>(x, lane);
                 rb_exchange<4, 2>(x, lane);
                 rb_exchange<2, 1>(x, lane);
-                if (FORM == RB_REMOVAL) mat[(lane & 3) * RB_MAT + (part * TG + (lane >> 2)) * RB_LD + s] = (float)x[0];
-                else (lane & 1 ? mQk : mK)[(lane >> 1) * RB_LD + s] = (float)x[0];
+                mat[(lane % SUMS) * RB_MAT + (t0_ + lane / (4 * SUMS)) * RB_LD + s0 + (lane / SUMS) % 4] = x[0];
+            }
+        };
+        walk(RbCount<0>(), s0);
+        if (TG == 2) walk(RbCount<2>(), s0 + 2);
+#pragma unroll 1
+        for (int t = s0 + 4; t < RB_B; t += TG) walk(RbCount<4>(), t);
+    }
+    __syncthreads();
+    // vectors decayed from the block's start (here, where b and r were, for what follows; GATE: done) and to its end, a channel a thread
+    for (int idx = tid; idx < 2 * D; idx += 128) {
+        const int c = idx % D;
+        float run = 1.f;
+        if (idx < D) {
+#pragma unroll
+            for (int t = 0; t < RB_B; ++t) {
+                const float w = sw[t * LD + c];
+                if (FORM != RB_GATE) sb[t * LD + c] *= run;
+                run *= w;
+                if (FORM != RB_GATE) sr[t * LD + c] *= run;
+                else blkp[L::F2 + t * L::ROW_LD + c] = sr[t * LD + c] * run;
+            }
+            blkp[L::DT + c] = run;
+        } else {
+#pragma unroll
+            for (int t = RB_B - 1; t >= 0; --t) {
+                blkp[L::KW + t * L::END_LD + c] = sk[t * LD + c] * run;
+                if (FORM == RB_REMOVAL) blkp[L::AW + t * L::END_LD + c] = sa[t * LD + c] * run;
+                run *= sw[t * LD + c];
             }
         }
     }
-    __syncthreads();
     if (FORM == RB_GATE) {
-        for (int idx = tid; idx < RB_MAT; idx += 128) blkp[L::M + idx] = mQk[idx];
+        pdl_launch_dependents();
+        for (int idx = tid; idx < RB_B * RB_B; idx += 128) blkp[L::M2 + idx / RB_B * RB_LD + idx % RB_B] = (float)mQk[idx / RB_B * RB_LD + idx % RB_B];
         return;
     }
-    // X, a column a thread, by substitution: REMOVAL (I - A)^-1; DELTA (I + beta A)^-1 beta with A in mK
-    if (tid < RB_B) {
+    // X, a column a thread, by substitution: REMOVAL (I - A)^-1; DELTA (I + beta A)^-1 beta with A in mK.  (Zero above the diagonal whatever A holds.)
+    if (warp == ((blk + h) & 3) && lane < RB_B) {
+        const double *A = FORM == RB_DELTA ? mK : mA;
         double x[RB_B];
 #pragma unroll
-        for (int t = 0; t < RB_B; ++t) {
-            const float beta = FORM == RB_DELTA ? sbeta[t] : 0.f;
-            double sum = 0;
+        for (int t = 0; t < RB_B; ++t) x[t] = 0.0;
 #pragma unroll
-            for (int s = 0; s < t; ++s) sum = fma((double)(FORM == RB_DELTA ? mK : mA)[t * RB_LD + s], x[s], sum);
-            const float one = t == tid ? 1.f : 0.f;
-            x[t] = FORM == RB_DELTA ? beta * (one - sum) : one + sum;
-            mX[t * RB_LD + tid] = (float)x[t];
+        for (int t = 0; t < RB_B; ++t) {
+            const double one = t == lane ? 1.0 : 0.0, beta = FORM == RB_DELTA ? (double)sbeta[t] : 0.0;
+            const double y = FORM == RB_DELTA ? beta * (one - x[t]) : one + x[t];      // x[t]: the sum over the tokens before
+            mX[t * RB_LD + lane] = t >= lane ? y : 0.0;
+#pragma unroll
+            for (int s = t + 1; s < RB_B; ++s) x[s] = fma(A[s * RB_LD + t], y, x[s]);
         }
     }
     __syncthreads();
-    // (sums over the tokens up to t alone: a later token's numbers may not be finite, and 0 x inf would not be 0)
+    // What values add: to h, and through h and directly to o.  (Sums over the tokens up to t alone: a later token's numbers may not be
+    // finite, and 0 x inf would not be 0.)
     for (int idx = tid; idx < RB_B * RB_B; idx += 128) {
         const int t = idx / RB_B, j = idx % RB_B;
+        double m = 0.0;
+#pragma unroll
+        for (int s = 0; s < RB_B; ++s)
+            if (s <= t) m = FORM == RB_DELTA ? fma(mQk[t * RB_LD + s], mX[s * RB_LD + j], m) : fma(mX[t * RB_LD + s], mK[s * RB_LD + j], m);
         if (FORM == RB_DELTA) {
-            float m = 0.f;
-#pragma unroll
-            for (int s = 0; s < RB_B; ++s)
-                if (s <= t) m = fmaf(mQk[t * RB_LD + s], mX[s * RB_LD + j], m);
-            blkp[L::M + t * RB_LD + j] = mX[t * RB_LD + j];
-            blkp[L::M + RB_MAT + t * RB_LD + j] = m;
+            blkp[L::M1 + t * RB_LD + j] = (float)mX[t * RB_LD + j];
+            blkp[L::M2 + t * RB_LD + j] = (float)m;
         } else {
-            float xk = 0.f, m1 = 0.f;
-#pragma unroll
-            for (int s = 0; s < RB_B; ++s)
-                if (s <= t) {
-                    xk = fmaf(mX[t * RB_LD + s], mK[s * RB_LD + j], xk);
-                    m1 = fmaf(mQa[t * RB_LD + s], mX[s * RB_LD + j], m1);
-                }
-            mY[t * RB_LD + j] = xk;
-            blkp[L::M + t * RB_LD + j] = mX[t * RB_LD + j];
-            blkp[L::M + RB_MAT + t * RB_LD + j] = xk;
-            blkp[L::M + 2 * RB_MAT + t * RB_LD + j] = m1;
+            blkp[L::M1 + t * RB_LD + j] = (float)m;
+            mY[t * RB_LD + j] = m;
         }
+    }
+    pdl_launch_dependents();                    // (late: the scan's CTAs are then spread over SMs that are free, longest first)
+    // What meets the state: F1 = X b (DELTA: - X b) gives h, F2 = r + Q F1 (Q = Qa; DELTA: Qk) gives o.  Transposed, 16 channels a tile of a
+    // warp, so that F1's accumulators are the operand of the product with Q.
+    const double *mQ = FORM == RB_DELTA ? mQk : mQa;
+    const int lr = lane >> 2, lc = (lane & 3) * 2;
+    for (int c0 = 16 * warp; c0 < D; c0 += 64) {
+        double f1[2][4], f2[2][4];
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                f1[n][e] = 0.0;
+                f2[n][e] = sr[(n * 8 + lc + (e & 1)) * LD + c0 + lr + (e >> 1) * 8];
+            }
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+            const float *b0 = sb + (ks * 8 + lc) * LD + c0 + lr, *b1 = b0 + LD;
+            const RbA a = rb_a(b0[0], b1[0], b0[8], b1[8]);
+#pragma unroll
+            for (int n = ks; n < 2; ++n) {
+                const double2 x = *reinterpret_cast<const double2 *>(mX + (n * 8 + lr) * RB_LD + ks * 8 + lc);
+                rb_mma(f1[n], a.x, x.x, x.y);
+            }
+        }
+        if (FORM == RB_DELTA)
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) f1[n][e] = -f1[n][e];
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+            const RbA a = rb_a(f1[ks][0], f1[ks][1], f1[ks][2], f1[ks][3]);
+#pragma unroll
+            for (int n = ks; n < 2; ++n) {
+                const double2 q = *reinterpret_cast<const double2 *>(mQ + (n * 8 + lr) * RB_LD + ks * 8 + lc);
+                rb_mma(f2[n], a.x, q.x, q.y);
+            }
+        }
+        bool number = true;
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) number = number && fabs(f1[n][e]) < INFINITY && fabs(f2[n][e]) < INFINITY;
+        if (!__all_sync(0xffffffffu, number)) {     // from the tokens up to t alone, as above
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int t = n * 8 + lc + (e & 1), c = c0 + lr + (e >> 1) * 8;
+                    double y = 0.0, z = sr[t * LD + c];
+#pragma unroll 1
+                    for (int s = 0; s <= t; ++s) {
+                        y = 0.0;
+#pragma unroll 1
+                        for (int q = 0; q <= s; ++q) y = fma(mX[s * RB_LD + q], (double)sb[q * LD + c], y);
+                        if (FORM == RB_DELTA) y = -y;
+                        z = fma(mQ[t * RB_LD + s], y, z);
+                    }
+                    f1[n][e] = y;
+                    f2[n][e] = z;
+                }
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int at = (n * 8 + lc + (e & 1)) * L::ROW_LD + c0 + lr + (e >> 1) * 8;
+                blkp[L::F1 + at] = (float)f1[n][e];
+                blkp[L::F2 + at] = (float)f2[n][e];
+            }
     }
     if (FORM == RB_REMOVAL) {
         __syncthreads();
         for (int idx = tid; idx < RB_B * RB_B; idx += 128) {
             const int t = idx / RB_B, j = idx % RB_B;
-            float m2 = mQk[t * RB_LD + j];
+            double m = mQk[t * RB_LD + j];
 #pragma unroll
             for (int s = 0; s < RB_B; ++s)
-                if (s <= t) m2 = fmaf(mQa[t * RB_LD + s], mY[s * RB_LD + j], m2);
-            blkp[L::M + 3 * RB_MAT + t * RB_LD + j] = m2;
+                if (s <= t) m = fma(mQa[t * RB_LD + s], mY[s * RB_LD + j], m);
+            blkp[L::M2 + t * RB_LD + j] = (float)m;
         }
     }
 }
 
-// c += a * b, one step of 8 along the sum, m16n8k8 in float64
-__device__ __forceinline__ void rb_mma(double *c, const double *a, double b0, double b1) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-                 : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
+// The request whose portion is the k-th longest (of equal ones the first; more than RB_ORDERED are taken as they come).  CTAs are placed in the
+// order of their index, so the longest get SMs of their own and the shorter ones share: prepared + scanned in us, in the requests' order and
+// by length, DELTA's 592 and 1,185 tokens 217 and 202, REMOVAL's 117, 233 and 350 119 and 100; four equal requests 261 and 268.
+#define RB_ORDERED 64
+__device__ __forceinline__ int rb_longest(const int *cu, int n, int k) {
+    if (n == 1 || n > RB_ORDERED) return k;
+    int found = 0;
+    for (int i = threadIdx.x & 31; i < n; i += 32) {
+        const int mine = cu[i + 1] - cu[i];
+        int longer = 0;
+        for (int j = 0; j < n; ++j) {
+            const int other = cu[j + 1] - cu[j];
+            longer += other > mine || (other == mine && j < i);
+        }
+        if (longer == k) found = i;
+    }
+    return __reduce_add_sync(0xffffffffu, found);
 }
-// Operand A from a row-major pair of numbers per row: (row l / 4: x0 at 2 (l % 4), x1 behind it; row l / 4 + 8: x2, x3).  The unit's k index
-// l % 4 is taken for the even, l % 4 + 4 for the odd of the two; operand B pairs its numbers the same way.
-struct RbA { double x[4]; };
-__device__ __forceinline__ RbA rb_a(double x0, double x1, double x2, double x3) { return {{x0, x2, x1, x3}}; }
 
 template <int D, int FORM>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(32 * RbScan<D, FORM>::WARPS)
 blocks_scan_kernel(const RbParams p, int stages) {
     using L = RbLayout<D, FORM>;
-    constexpr int NT = RbScan<FORM>::ROWS / 8;                   // tiles of eight rows that meet the state
-    constexpr int CT = D / 32;                                   // tiles of eight channels of a warp
-    constexpr int STAGE = L::FLOATS, RED_LD = RbScan<FORM>::RED_LD;
+    constexpr int WARPS = RbScan<D, FORM>::WARPS;
+    constexpr int NT = RbScan<D, FORM>::NT;
+    constexpr int CT = D / 8 / WARPS;                            // tiles of eight channels of a warp
+    constexpr int STAGE = L::FLOATS;
+    constexpr bool EARLY = FORM == RB_GATE;                      // a block's writes need none of its sums: its last operands are free a block earlier
     pdl_launch_dependents();
-    extern __shared__ float4 rb_smem4[];
-    float *ring = reinterpret_cast<float *>(rb_smem4);
-    __shared__ __align__(16) RbScan<FORM> sm;
-    auto &vals = sm.vals;
-    auto &corr = sm.corr;
+    extern __shared__ __align__(16) unsigned char rb_dyn[];
+    RbScan<D, FORM> &sm = *reinterpret_cast<RbScan<D, FORM> *>(rb_dyn);
+    float *ring = reinterpret_cast<float *>(rb_dyn + (sizeof(sm) + 127) / 128 * 128);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int lr = lane >> 2, lc = (lane & 3) * 2;               // a fragment's row (and row + 8) and its pair of columns
-    const int h = blockIdx.y, seq = blockIdx.z, col0 = blockIdx.x * RB_COLS;
-    const int ch0 = warp * (D / 4);
-    const uint32_t bar0 = smem_u32(&sm.bars[0]);
+    const int h = blockIdx.y, col0 = blockIdx.x * RB_COLS;
+    const int ch0 = warp * (D / WARPS);
+    const uint32_t bar0 = smem_u32(&sm.bars[0][0]);
     if (tid == 0) {
-        for (int b = 0; b < stages; ++b) mbar_init(bar0 + 8 * b, 1);
+        for (int b = 0; b < 2 * stages; ++b) mbar_init(bar0 + 8 * b, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     pdl_wait();
-    const int t0 = p.cu_seqlens[seq], t1 = p.cu_seqlens[seq + 1];
-    const int n_blocks = (t1 - t0 + RB_B - 1) / RB_B;
+    const int seq = rb_longest(p.cu_seqlens, gridDim.z, blockIdx.z);
+    const int t0 = p.cu_seqlens[seq], T = p.cu_seqlens[seq + 1] - t0;
+    const int n_blocks = (T + RB_B - 1) / RB_B;
+    const size_t src_step = (size_t)p.H * STAGE;
     const float *src = p.blocks + ((size_t)(t0 / RB_B + seq) * p.H + h) * STAGE;
-    auto fetch = [&](int i) {           // one thread: block i into stage i % stages
-        const uint32_t bar = bar0 + 8u * (uint32_t)(i % stages);
-        mbar_expect_tx(bar, STAGE * 4);
+    // one thread: of the block at `from`, what meets the state, or (part 1) what is written to it, into a stage; each has a barrier
+    auto fetch = [&](int stage, const float *from, int part) {
+        const uint32_t bar = bar0 + 16u * (uint32_t)stage + 8u * part;
+        const int off = part ? L::KW : 0, bytes = (part ? STAGE - L::KW : L::KW) * 4;
+        mbar_expect_tx(bar, bytes);
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     ::"r"(smem_u32(ring + (i % stages) * STAGE)), "l"(src + (size_t)i * p.H * STAGE), "r"(STAGE * 4), "r"(bar)
+                     ::"r"(smem_u32(ring + stage * STAGE + off)), "l"(from + off), "r"(bytes), "r"(bar)
                      : "memory");
     };
     if (tid == 0)
-        for (int i = 0; i < min(stages, n_blocks); ++i) fetch(i);
+        for (int i = 0; i < min(stages, n_blocks); ++i) fetch(i, src + i * src_step, 0), fetch(i, src + i * src_step, 1);
+    const float *ahead = src + stages * src_step;                // block i + stages
     float *Sg = p.state + (size_t)p.slots[seq] * p.state_stride + (size_t)h * p.d * p.dv;     // [d][dv]
     // S^T of the warp's channels: S[ct] = columns lr, lr + 8 of the CTA by channels lc, lc + 1 of the tile
     double S[CT][4];
@@ -473,170 +615,186 @@ blocks_scan_kernel(const RbParams p, int stages) {
             const int c = ch0 + ct * 8 + lc + (e & 1), j = col0 + lr + (e >> 1) * 8;
             S[ct][e] = (c < p.d && j < p.dv) ? Sg[(size_t)c * p.dv + j] : 0.f;
         }
-    // thread moves columns vj, vj + 1 of token vt; zeros beyond the request and the head
-    const int vt = tid >> 3, vj = (tid & 7) * 2;
-    auto load_v = [&](int i) {
-        const int t = t0 + i * RB_B + vt;
+    // a thread moves VN columns of a token's values; zeros beyond the request and the head
+    constexpr int VN = 8 / WARPS;
+    const int vt = tid / (RB_COLS / VN), vj = tid % (RB_COLS / VN) * VN;
+    const uint32_t v_to = smem_u32(&sm.vals[0][vt][vj]);
+    const float *v_from = p.v + (size_t)(t0 + vt) * p.ldv + (size_t)h * p.dv + col0 + vj;     // of block i + 3
+    int v_left = T - vt;                                         // its tokens from this one on
+    auto load_v = [&](int slot) {
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const bool in = i < n_blocks && t < t1 && col0 + vj + e < p.dv;
-            const float *from = in ? p.v + (size_t)t * p.ldv + (size_t)h * p.dv + col0 + vj + e : p.v;
-            const int bytes = in ? 4 : 0;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(&vals[i & 3][vt][vj + e])), "l"(from), "r"(bytes) : "memory");
+        for (int e = 0; e < VN; ++e) {
+            const bool in = v_left > 0 && col0 + vj + e < p.dv;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(v_to + (uint32_t)(slot * RB_B * RB_VLD + e) * 4), "l"(in ? v_from + e : p.v), "r"(in ? 4 : 0)
+                         : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
+        v_from += RB_B * p.ldv;
+        v_left -= RB_B;
     };
     load_v(0);
     load_v(1);
     load_v(2);
+    asm volatile("cp.async.wait_group 2;" ::: "memory");
+    __syncthreads();
     bool ok = true;
-    for (int i = 0; i < n_blocks; ++i) {
-        const int stage = i % stages;
+    int stage = 0, before = 0, left = T;                         // tokens from the block's first on
+    uint32_t phase = 0;
+    auto await = [&](int part) {
+        if (ok && !mbar_wait(bar0 + 16u * (uint32_t)stage + 8u * part, phase)) { atomicExch(&g_rb_error, 1); ok = false; }
+    };
+    // the sums and read-outs of a quarter of a block: tokens 8 n + lc, + 1 of columns lr + 8 e
+    const int qn = warp & 1, qe = (warp >> 1) & 1, out_j = col0 + lr + 8 * qe;
+    float *out = p.out + ((size_t)(t0 + qn * 8 + lc) * p.H + h) * p.dv + out_j;
+    const size_t out_row = (size_t)p.H * p.dv;
+    for (int i = 0; i < n_blocks; ++i, left -= RB_B, ahead += src_step, out += RB_B * out_row) {
         const float *st = ring + stage * STAGE;
-        float(*red)[RB_COLS][RED_LD] = sm.red[FORM == RB_GATE ? i & 1 : 0];       // GATE has one barrier a block: two buffers in turn
-        asm volatile("cp.async.wait_group 2;" ::: "memory");       // this block's values; the barrier below shows them to all
-        if (ok && !mbar_wait(bar0 + 8u * stage, (uint32_t)(i / stages) & 1u)) { atomicExch(&g_rb_error, 1); ok = false; }
-        {   // what the warp's channels of the state give to the block's rows
+        auto &red_o = sm.red_o[FORM == RB_GATE ? i & 1 : 0];
+        const float(*vr)[RB_VLD] = sm.vals[i & 3];
+        // operand A of tokens 8 ks .. of the values
+        auto values = [&](int ks, float *x) {
+            const float *u0 = &vr[ks * 8 + lc][lr], *u1 = &vr[ks * 8 + lc + 1][lr];
+            x[0] = u0[0], x[1] = u1[0], x[2] = u0[8], x[3] = u1[8];
+        };
+        auto decay = [&] {
+#pragma unroll
+            for (int ct = 0; ct < CT; ++ct) {
+                const float2 d2 = *reinterpret_cast<const float2 *>(st + L::DT + ch0 + ct * 8 + lc);
+                S[ct][0] *= d2.x;
+                S[ct][1] *= d2.y;
+                S[ct][2] *= d2.x;
+                S[ct][3] *= d2.y;
+            }
+        };
+        auto write = [&](int ks, const RbA &a, int rows) {
+#pragma unroll
+            for (int ct = 0; ct < CT; ++ct) {
+                const float *b = st + rows + (ks * 8 + lc) * L::END_LD + ch0 + ct * 8 + lr;
+                rb_mma(S[ct], a.x, b[0], b[L::END_LD]);
+            }
+        };
+        await(0);
+        {   // what the warp's channels of the state, and its share of the values, give to the block's h and o
             double acc[NT][4];
 #pragma unroll
             for (int n = 0; n < NT; ++n)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) acc[n][e] = 0.0;
+            // The share: the values of tokens 8 ks .. in the sums of tokens 8 half .. of h (eight warps: of h or o)
+            const int ks = (warp >> 1) & 1, half = warp & 1;
+            constexpr int SHARES = NT / 2;
+            if (ks <= half && (WARPS == 4 || SHARES == 2 || warp < 4)) {
+                float x[4];
+                values(ks, x);
+                const bool number = fabsf(x[0]) < INFINITY && fabsf(x[1]) < INFINITY && fabsf(x[2]) < INFINITY && fabsf(x[3]) < INFINITY;
+                const bool numbers = __all_sync(0xffffffffu, number);
+                const RbA a = rb_a(x[0], x[1], x[2], x[3]);
+                auto share = [&](bool of_h, double *y) {
+                    const float *mat = st + (of_h ? L::M1 : L::M2);
+                    if (numbers) {
+                        const float2 b = *reinterpret_cast<const float2 *>(mat + (half * 8 + lr) * RB_LD + ks * 8 + lc);
+                        rb_mma(y, a.x, b.x, b.y);
+                        return;
+                    }
+                    // The product meets the zeros of the matrix with the numbers of later tokens, and 0 x inf is not 0: from the tokens that count alone, as
+                    // the scan has it
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int t = half * 8 + lc + (e & 1), j = lr + (e >> 1) * 8;
+#pragma unroll 1
+                        for (int s = ks * 8; s < ks * 8 + 8 && s <= t; ++s)
+                            if (!(FORM == RB_REMOVAL && of_h && s == t)) y[e] = fma((double)mat[t * RB_LD + s], (double)vr[s][j], y[e]);
+                    }
+                };
+                double y[4] = {0.0, 0.0, 0.0, 0.0}, z[4] = {0.0, 0.0, 0.0, 0.0};
+                constexpr bool BOTH = WARPS == 4 && SHARES == 2;
+                const bool of_h = SHARES == 2 && (BOTH || warp < 4);
+                share(of_h, y);
+                if (BOTH) share(false, z);
+#pragma unroll
+                for (int n = 0; n < NT; ++n)                     // (neither the share nor its half is a constant)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const bool h_row = SHARES == 2 && n < 2;
+                        const double mine = BOTH && !h_row ? z[e] : y[e];
+                        acc[n][e] = (n & 1) == half && (BOTH || h_row == of_h) ? mine : 0.0;
+                    }
+            }
 #pragma unroll
             for (int ct = 0; ct < CT; ++ct) {
                 const RbA a = rb_a(S[ct][0], S[ct][1], S[ct][2], S[ct][3]);
 #pragma unroll
-                for (int n = 0; n < NT; ++n) {                   // rows: BD, then RD (GATE: RD)
-                    const float2 b = *reinterpret_cast<const float2 *>(st + (n * 8 + lr) * L::ROW_LD + ch0 + ct * 8 + lc);
+                for (int n = 0; n < NT; ++n) {
+                    const float2 b = *reinterpret_cast<const float2 *>(st + L::F1 + (n * 8 + lr) * L::ROW_LD + ch0 + ct * 8 + lc);
                     rb_mma(acc[n], a.x, b.x, b.y);
                 }
             }
 #pragma unroll
-            for (int n = 0; n < NT; ++n)
+            for (int n = 0; n < 2; ++n)
 #pragma unroll
-                for (int e = 0; e < 2; ++e)
-                    *reinterpret_cast<float2 *>(&red[warp][lr + 8 * e][n * 8 + lc]) = make_float2((float)acc[n][2 * e], (float)acc[n][2 * e + 1]);
-        }
-        __syncthreads();                        // and every warp is done with the block before
-        if (tid == 0 && i > 0 && i - 1 + stages < n_blocks) fetch(i - 1 + stages);
-        load_v(i + 3);
-        const float(*vr)[RB_VLD] = vals[i & 3];
-        // sum over the warps' channels of rows 8 n + lc, + 1 for columns lr, lr + 8
-        auto total = [&](int n, float *x) {
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                float2 s = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    const float2 y = *reinterpret_cast<const float2 *>(&red[w][lr + 8 * e][n * 8 + lc]);
-                    s.x += y.x;
-                    s.y += y.y;
+                for (int e = 0; e < 2; ++e) {
+                    if (FORM != RB_GATE) rb_put2(&sm.red_h[FORM == RB_GATE ? 0 : warp][FORM == RB_GATE ? 0 : lr + 8 * e][n * 8 + lc], acc[n][2 * e], acc[n][2 * e + 1]);
+                    rb_put2(&red_o[warp][lr + 8 * e][n * 8 + lc], acc[NT - 2 + n][2 * e], acc[NT - 2 + n][2 * e + 1]);
                 }
-                x[2 * e] = s.x;
-                x[2 * e + 1] = s.y;
-            }
-        };
-        // columns by tokens: warps 0, 1 the corrections (DELTA: the writes) of tokens 0-7, 8-15, warps 2, 3 the read-outs
-        const bool reads = warp >= 2;
-        const int half = warp & 1;
-        if (reads || FORM != RB_GATE) {
-            double sum[4] = {0.0, 0.0, 0.0, 0.0};
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            const float *m0 = st + L::M, *m1 = m0 + RB_MAT;
-            const int row = (half * 8 + lr) * RB_LD + lc;
-            if (reads) total((FORM == RB_GATE ? 0 : 2) + half, acc);
+        }
+        if (FORM != RB_DELTA) {                 // what needs none of the sums
+            await(1);
+            decay();
 #pragma unroll
             for (int ks = 0; ks < 2; ++ks) {
-                const float *u0 = &vr[ks * 8 + lc][lr], *u1 = &vr[ks * 8 + lc + 1][lr];
-                RbA av;
-                if (FORM == RB_DELTA) {         // v - b^T S_0 takes the values' place
-                    float x[4];
-                    total(ks, x);
-                    av = rb_a((double)u0[0] - x[0], (double)u1[0] - x[1], (double)u0[8] - x[2], (double)u1[8] - x[3]);
-                } else {
-                    av = rb_a(u0[0], u1[0], u0[8], u1[8]);
-                }
-                const float *mv = FORM == RB_GATE ? m0 : FORM == RB_DELTA ? (reads ? m1 : m0) : (reads ? m0 + 3 * RB_MAT : m1);
-                float2 b = *reinterpret_cast<const float2 *>(mv + row + ks * 8);
-                rb_mma(sum, av.x, b.x, b.y);
-                if (FORM == RB_REMOVAL) {
-                    float x[4];
-                    total(ks, x);
-                    const RbA ah = rb_a(x[0], x[1], x[2], x[3]);
-                    b = *reinterpret_cast<const float2 *>((reads ? m0 + 2 * RB_MAT : m0) + row + ks * 8);
-                    rb_mma(sum, ah.x, b.x, b.y);
-                }
-            }
-            bool number = true;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                acc[e] = (float)(sum[e] + acc[e]);
-                number = number && fabsf(acc[e]) < INFINITY;
-            }
-            if (!__all_sync(0xffffffffu, number)) {
-                // The products above meet the zeros of the matrices with the numbers of later tokens, and 0 x inf is not 0: a token's
-                // result from itself and the tokens before it alone, as the scan has it.
-                auto total_of = [&](int n, int j) { return red[0][j][n] + red[1][j][n] + red[2][j][n] + red[3][j][n]; };
-#pragma unroll 1
-                for (int e = 0; e < 4; ++e) {
-                    const int t = half * 8 + lc + (e & 1), j = lr + (e >> 1) * 8;
-                    float x = reads ? total_of((FORM == RB_GATE ? 0 : RB_B) + t, j) : 0.f;
-#pragma unroll 1
-                    for (int s = 0; s <= t; ++s) {
-                        const float *m = m0 + t * RB_LD + s;        // matrix i at i * RB_MAT
-                        const float v = vr[s][j], h = FORM == RB_GATE ? 0.f : total_of(s, j);
-                        if (FORM == RB_GATE) x = fmaf(m[0], v, x);
-                        if (FORM == RB_DELTA) x = fmaf(m[reads ? RB_MAT : 0], v - h, x);
-                        if (FORM == RB_REMOVAL) {
-                            x = fmaf(m[reads ? 2 * RB_MAT : 0], h, x);
-                            if (reads || s < t) x = fmaf(m[(reads ? 3 : 1) * RB_MAT], v, x);
-                        }
-                    }
-                    acc[0] = e == 0 ? x : acc[0], acc[1] = e == 1 ? x : acc[1], acc[2] = e == 2 ? x : acc[2], acc[3] = e == 3 ? x : acc[3];
-                }
-            }
-            if (reads) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int t = t0 + i * RB_B + half * 8 + lc + (e & 1), j = col0 + lr + (e >> 1) * 8;
-                    if (t < t1 && j < p.dv) p.out[((size_t)t * p.H + h) * p.dv + j] = acc[e];
-                }
-            } else {
-                // (none of the tokens beyond the request's end: what is not finite before them reaches their rows too)
-                const int left = t1 - t0 - i * RB_B - half * 8 - lc;
-#pragma unroll
-                for (int e = 0; e < 2; ++e)
-                    *reinterpret_cast<float2 *>(&corr[lr + 8 * e][half * 8 + lc]) = make_float2(left > 0 ? acc[2 * e] : 0.f, left > 1 ? acc[2 * e + 1] : 0.f);
+                float x[4];
+                values(ks, x);
+                write(ks, rb_a(x[0], x[1], x[2], x[3]), L::KW);
             }
         }
-        if (FORM != RB_GATE) __syncthreads();
-        // the state at the block's end
-#pragma unroll
-        for (int ct = 0; ct < CT; ++ct) {
-            const float2 d2 = *reinterpret_cast<const float2 *>(st + L::DT + ch0 + ct * 8 + lc);
-            S[ct][0] *= d2.x;
-            S[ct][1] *= d2.y;
-            S[ct][2] *= d2.x;
-            S[ct][3] *= d2.y;
-        }
-#pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-            auto write = [&](const RbA &a, const float *rows) {
-#pragma unroll
-                for (int ct = 0; ct < CT; ++ct) {
-                    const float *b = rows + (ks * 8 + lc) * L::END_LD + ch0 + ct * 8 + lr;
-                    rb_mma(S[ct], a.x, b[0], b[L::END_LD]);
-                }
-            };
-            if (FORM != RB_DELTA) {
-                const float *u0 = &vr[ks * 8 + lc][lr], *u1 = &vr[ks * 8 + lc + 1][lr];
-                write(rb_a(u0[0], u1[0], u0[8], u1[8]), st + L::KW);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");       // the next block's values; the barrier shows them to all
+        __syncthreads();                        // and every warp is done with what the block before needed, and with this block's rows
+        if (tid == 32 * (WARPS - 1)) {
+            if (i + stages < n_blocks) {
+                fetch(stage, ahead, 0);
+                if (EARLY) fetch(stage, ahead, 1);
             }
-            if (FORM != RB_GATE) {
-                const float2 x0 = *reinterpret_cast<const float2 *>(&corr[lr][ks * 8 + lc]), x1 = *reinterpret_cast<const float2 *>(&corr[lr + 8][ks * 8 + lc]);
-                write(rb_a(x0.x, x0.y, x1.x, x1.y), st + (FORM == RB_DELTA ? L::KW : L::AW));
+            if (!EARLY && i > 0 && i - 1 + stages < n_blocks) fetch(before, ahead - src_step, 1);
+        }
+        load_v((i + 3) & 3);
+        // the sums over the warps' channels, in their order
+        if (FORM != RB_GATE && warp < 4) {      // (none of the tokens beyond the request's end: what is not finite before them reaches their rows too)
+            double2 y = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) {
+                const double2 z = *reinterpret_cast<const double2 *>(&sm.red_h[FORM == RB_GATE ? 0 : w][FORM == RB_GATE ? 0 : lr + 8 * qe][qn * 8 + lc]);
+                y.x += z.x;
+                y.y += z.y;
+            }
+            rb_put2(&sm.corr[FORM == RB_GATE ? 0 : lr + 8 * qe][qn * 8 + lc], left > qn * 8 + lc ? y.x : 0.0, left > qn * 8 + lc + 1 ? y.y : 0.0);
+        }
+        if (WARPS == 4 || warp >= 4) {
+            double2 y = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) {
+                const double2 z = *reinterpret_cast<const double2 *>(&red_o[w][lr + 8 * qe][qn * 8 + lc]);
+                y.x += z.x;
+                y.y += z.y;
+            }
+            if (out_j < p.dv) {
+                if (left > qn * 8 + lc) out[0] = (float)y.x;
+                if (left > qn * 8 + lc + 1) out[out_row] = (float)y.y;
             }
         }
+        if (FORM != RB_GATE) {
+            if (FORM == RB_DELTA) {
+                await(1);
+                decay();
+            }
+            __syncthreads();
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) {
+                const double *y0 = &sm.corr[FORM == RB_GATE ? 0 : lr][ks * 8 + lc], *y1 = &sm.corr[FORM == RB_GATE ? 0 : lr + 8][ks * 8 + lc];
+                write(ks, rb_a(y0[0], y0[1], y1[0], y1[1]), FORM == RB_DELTA ? L::KW : L::AW);
+            }
+        }
+        before = stage;
+        if (++stage == stages) stage = 0, phase ^= 1u;
     }
 #pragma unroll
     for (int ct = 0; ct < CT; ++ct)
@@ -649,20 +807,20 @@ blocks_scan_kernel(const RbParams p, int stages) {
 
 static int rb_padded(int d) { return d <= 32 ? 32 : d <= 64 ? 64 : 128; }
 static long long rb_floats(int D, int form) {
-    const int rows = form == RB_GATE ? 1 : 2, ends = form == RB_REMOVAL ? 2 : 1, mats = form == RB_GATE ? 1 : form == RB_DELTA ? 2 : 4;
-    return (long long)RB_B * (rows * (D + 8) + ends * (D + 4)) + D + (long long)mats * RB_MAT;
+    const int rows = form == RB_GATE ? 1 : 2, ends = form == RB_REMOVAL ? 2 : 1;
+    return (long long)RB_B * (rows * (D + 8) + ends * (D + 4)) + D + (long long)rows * RB_MAT;
 }
 
 template <int D, int FORM>
 static int rb_launch(const RbParams &p, const RbSource *src, int nseq, int max_count, cudaStream_t stream) {
-    static_assert(RbLayout<D, FORM>::FLOATS % 4 == 0, "bulk copies move 16 bytes");
-    const size_t prep = (size_t)((FORM == RB_GATE ? 3 : FORM == RB_DELTA ? 4 : 5) * RB_B * D + 6 * RB_MAT) * sizeof(float);
-    constexpr size_t stage = (size_t)RbLayout<D, FORM>::FLOATS * sizeof(float), fixed = (sizeof(RbScan<FORM>) + 1023) / 1024 * 1024;
+    static_assert(RbLayout<D, FORM>::FLOATS % 4 == 0 && RbLayout<D, FORM>::KW % 4 == 0, "bulk copies move 16 bytes");
+    const size_t prep = (size_t)(FORM == RB_GATE ? 3 : FORM == RB_DELTA ? 4 : 5) * RB_B * RbLayout<D, FORM>::END_LD * sizeof(float) + RbLayout<D, FORM>::MATS * RB_MAT * sizeof(double);
+    constexpr size_t stage = (size_t)RbLayout<D, FORM>::FLOATS * sizeof(float), fixed = (sizeof(RbScan<D, FORM>) + 127) / 128 * 128;
     static bool attr_set = false;
     if (!attr_set) {
         if (cudaFuncSetAttribute(blocks_prepare_kernel<D, FORM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep) != cudaSuccess ||
             cudaFuncSetAttribute(blocks_prepare_kernel<D, FORM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep) != cudaSuccess ||
-            cudaFuncSetAttribute(blocks_scan_kernel<D, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(KESTREL_SMEM_MAX_DYNAMIC - fixed)) != cudaSuccess)
+            cudaFuncSetAttribute(blocks_scan_kernel<D, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, KESTREL_SMEM_MAX_DYNAMIC) != cudaSuccess)
             return kestrel_fail(-3, "recurrence_blocks: cannot set the shared memory size");
         attr_set = true;
     }
@@ -672,9 +830,9 @@ static int rb_launch(const RbParams &p, const RbSource *src, int nseq, int max_c
     static_assert(2 * stage + fixed <= KESTREL_SMEM_MAX_DYNAMIC, "two stages fit an SM");
     const dim3 grid((p.dv + RB_COLS - 1) / RB_COLS, p.H, nseq);
     // as many stages as the CTAs that share an SM leave room for, two at least
-    const size_t room = kestrel_spread_smem((long)grid.x * grid.y * grid.z, 2 * stage + fixed) - fixed;
+    const size_t smem = kestrel_spread_smem((long)grid.x * grid.y * grid.z, 2 * stage + fixed), room = smem - fixed;
     const int stages = (int)(room / stage) < RB_STAGES ? (int)(room / stage) : RB_STAGES;
-    kestrel_launch(blocks_scan_kernel<D, FORM>, grid, dim3(128), room, stream, p, stages);
+    kestrel_launch(blocks_scan_kernel<D, FORM>, grid, dim3(32 * RbScan<D, FORM>::WARPS), smem, stream, p, stages);
     return kestrel_check_launch("recurrence_blocks");
 }
 

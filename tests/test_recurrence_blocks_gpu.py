@@ -111,6 +111,32 @@ def test_delta_rule_in_blocks(counts, H, G, d, dv):
     _check("states", got["blocks"][1], got["scan"][1], want_s)
 
 
+@pytest.mark.parametrize("counts", [(20, 90, 33, 90, 47), tuple(16 + 7 * i % 40 for i in range(64)), tuple(17 + 5 * i % 30 for i in range(70))])
+@pytest.mark.parametrize("form", ["gate", "removal"])
+def test_requests_of_many_lengths(counts, form):
+    """Requests are walked longest first up to 64 of them, and as they come beyond: everyone's numbers are its own, the scan's up to rounding."""
+    import torch
+    from kestrel_llm_b200.csrc import ops
+    rng = np.random.default_rng(len(counts))
+    batch, cu, slots = _step(counts, 3)
+    T, H, d, dv = batch.num_tokens, 2, 32, 20
+
+    def f32(x):
+        return torch.from_numpy(np.ascontiguousarray(x.reshape(x.shape[0], -1), dtype=np.float32)).cuda()
+    k = rng.standard_normal((T, H, d))
+    k /= np.sqrt((k * k).sum(-1, keepdims=True))
+    pair = (f32(-rng.random((T, H, d)) * k), f32(k)) if form == "removal" else (None, None)
+    args = f32(rng.standard_normal((T, H, d))), f32(_decays(rng, (T, H, d))), f32(k), f32(rng.standard_normal((T, H, dv))), *pair
+    state0 = f32(rng.standard_normal((len(counts) + 1, H * d * dv)))
+    got = []
+    for fn in (ops.recurrence_scan, ops.recurrence_blocks):
+        state = state0.clone()
+        got.append((fn(*args, state, 0, batch, H, d, dv), state))
+    ops.raise_on_kernel_error()
+    for name, scan, blocks in zip(("read-outs", "states"), *got):
+        assert (scan - blocks).abs().max() <= 2.0 ** -20 * scan.abs().max(), name        # sums of 32 numbers in float32 on one side
+
+
 def _evaluate(r, w, k, v, a, b, state, cu, slots):
     """Read-outs and states in float64 from float32 operands [T, H, .]."""
     out, state = np.zeros(v.shape), state.copy()
