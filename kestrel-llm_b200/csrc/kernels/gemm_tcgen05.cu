@@ -72,6 +72,7 @@ struct QkvPrepParams {
     int nq, nkv, write_kv;
     const float *act_p;              // ACT: the numbers of an activation that has any
     float act_limit;                 // the gated forms: the bound of gated_act.cuh (0: none, SiLU)
+    int early_w;                     // the weights were complete before the kernel before this one began
     int group_rows;                  // PARTIAL: every group_rows features (whole tiles) have T token rows of their own in x; 0: all the same
 };
 
@@ -407,6 +408,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
 //   * the epilogue warps of both ranks arrive on the leader's accumulator-empty barrier.
 // No TMA load uses cluster multicast.  Persistent over tiles as the one-CTA kernel, two
 // accumulators in TMEM.
+// Launched with programmatic dependent launch as every kernel: barriers, TMEM and, where the
+// weights are a model's, the ring's first fill of them are there when the kernel before ends
+// (layers of two to four such products 7 to 11 us faster, a step of 512 tokens 1,312 -> 1,280).
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -517,13 +521,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     cluster_sync();                   // both ranks' barriers exist before anything arrives on them from afar
     tc_fence_after();
     const uint32_t tmem = *tmem_slot_ptr;
-    pdl_wait();
+    if (warp != 0) pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {
             int stage = 0;
             uint32_t phase = 0;
-            bool ok = true;
+            bool ok = true, first = true;
             for (int tile = pair; tile < tiles_total && ok; tile += n_pairs) {
                 const int split = tile / tiles_nt, tw = tile % tiles_nt;       // a tile of the output and its slice of K
                 int n0 = tile_n(tw) * 256 + (int)rank * TC_BM;
@@ -531,21 +535,28 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 if (MODE == TC_PARTIAL && prep.group_rows) t0 += tile_n(tw) * 256 / prep.group_rows * T;
                 if (MODE == TC_SWIGLU_T) n0 = tile_n(tw) * TC_BM + (rank ? up_row_offset : 0);     // this rank's half of the N operand: gate rows, or up rows
                 if (MODE == TC_QKV_PREP) n0 = (2 * tile_n(tw) + (int)rank) * TC_BM;                  // one head's rows from each rank
-                const int kb_end = min(num_kb, (split + 1) * kb_per_split);
-                for (int kb = split * kb_per_split; kb < kb_end; ++kb) {
-                    if (!mbar_wait(empty_bar(stage), phase ^ 1)) { atomicExch(&g_tc_error, 1); ok = false; break; }
-                    uint32_t leader_full = map_to_rank(full_bar(stage), 0);
-                    if (rank == 0) mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);
-                    uint32_t sa = base + (uint32_t)stage * STAGE_BYTES;
-                    int kc = kb * TC_BK;
-                    if (SWAP) {              // tokens are the M operand (this rank's 128), weights the N operand (this rank's half)
-                        tma_load_2d_pair(sa, &map_x, leader_full, kc, t0);
-                        tma_load_2d_pair(sa + A_BYTES, &map_w, leader_full, kc, n0);
-                    } else {
-                        tma_load_2d_pair(sa, &map_w, leader_full, kc, n0);
-                        if (MODE == TC_SWIGLU) tma_load_2d_pair(sa + A_BYTES, &map_w, leader_full, kc, up_row_offset + n0);
-                        tma_load_2d_pair(sa + A_TILES * A_BYTES, &map_x, leader_full, kc, t0);
+                const int kb_begin = split * kb_per_split, kb_end = min(num_kb, (split + 1) * kb_per_split);
+                auto load_w = [&](int st, int kb) {
+                    const uint32_t leader_full = map_to_rank(full_bar(st), 0), sa = base + (uint32_t)st * STAGE_BYTES;
+                    if (rank == 0) mbar_expect_tx(full_bar(st), 2 * STAGE_BYTES);
+                    // (SWAP: tokens are the M operand, this rank's 128; weights the N operand, this rank's half)
+                    tma_load_2d_pair(SWAP ? sa + A_BYTES : sa, &map_w, leader_full, kb * TC_BK, n0);
+                    if (MODE == TC_SWIGLU) tma_load_2d_pair(sa + A_BYTES, &map_w, leader_full, kb * TC_BK, up_row_offset + n0);
+                };
+                int early = kb_begin;               // k-blocks whose weights are on their way
+                if (first) {
+                    // weights that were complete before the kernel before this one began: the ring's first fill of them comes while that kernel ends
+                    if (prep.early_w)
+                        for (; early < kb_end && early - kb_begin < stages; ++early) load_w(early - kb_begin, early);
+                    pdl_wait();
+                    first = false;
+                }
+                for (int kb = kb_begin; kb < kb_end; ++kb) {
+                    if (kb >= early) {
+                        if (!mbar_wait(empty_bar(stage), phase ^ 1)) { atomicExch(&g_tc_error, 1); ok = false; break; }
+                        load_w(stage, kb);
                     }
+                    tma_load_2d_pair(base + (uint32_t)stage * STAGE_BYTES + (SWAP ? 0 : A_TILES * A_BYTES), &map_x, map_to_rank(full_bar(stage), 0), kb * TC_BK, t0);
                     if (++stage == stages) { stage = 0; phase ^= 1; }
                 }
             }
@@ -1020,11 +1031,13 @@ static int launch_tc_pair(const CUtensorMap &mw, const CUtensorMap &mx, void *ou
     size_t smem = (size_t)stages * STAGE_BYTES + 16 * stages + 48 + 1024;
     static int max_clusters = -1;
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.blockDim = dim3(TCP_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -1054,6 +1067,7 @@ static int launch_tc_pair(const CUtensorMap &mw, const CUtensorMap &mx, void *ou
     int per = (total_kb + splits - 1) / splits;
     int pairs = total < max_clusters ? (int)total : max_clusters;
     cfg.gridDim = dim3(2 * pairs);
+    cfg.numAttrs = g_kestrel_pdl ? 2 : 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<MODE>, mw, mx, out, T, N, K, ldo, stages, tiles_n, (int)total, up_off, accumulate,
                                        (int)tiles_nt, per, slice_stride, prep);
     if (e != cudaSuccess) return kestrel_fail(-3, "gemm_tc_pair: %s", cudaGetErrorString(e));
@@ -1089,6 +1103,7 @@ static int dispatch_tc(const void *x, const void *w, void *out, int T, int N, in
     if (persistent && g_pairs) {
         QkvPrepParams prep = {};
         prep.act_limit = act_limit;
+        prep.early_w = early_w;
         rc = kestrel_tensor_map_bf16(&mx, x, T, K, ldx, TCP_BN / 2);
         if (rc) return rc;
         if (MODE == TC_SWIGLU && swiglu_swapped_wins(T, N) && ((uintptr_t)out & 15) == 0 && ldo % 8 == 0)
@@ -1255,7 +1270,7 @@ KESTREL_API int kestrel_gemm_tc_qkv_prepare(const void *x, const void *w, int T,
     if (rc) return rc;
     rc = kestrel_tensor_map_bf16(&mx, x, T, K, ldx, TCP_BN / 2);
     if (rc) return rc;
-    QkvPrepParams prep;
+    QkvPrepParams prep = {};
     prep.bias = bias; prep.q_norm_w = q_norm_w; prep.k_norm_w = k_norm_w; prep.inv_freq = inv_freq;
     prep.norm_eps = norm_eps; prep.rot_scale = rot_scale; prep.positions = positions; prep.seq_of_token = seq_of_token;
     prep.block_table = block_table; prep.table_stride = table_stride; prep.page_size = page_size;
