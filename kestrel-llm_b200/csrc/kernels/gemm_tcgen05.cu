@@ -447,7 +447,7 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t desc_a, ui
         : "memory");
 }
 
-#define TCP_BN 256          // tokens of a pair's tile (128 loaded by each rank)
+#define TCP_BN 256          // most columns of a pair's tile: its N operand, half of which each rank loads
 #ifndef TCP_EPI_GROUPS
 #define TCP_EPI_GROUPS 4    // epilogue warps per TMEM lane quarter; each takes 256 / TCP_EPI_GROUPS token columns
 #endif
@@ -459,25 +459,27 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t desc_a, ui
 //               tokens give fewer output tiles than there are CTA pairs.
 // MODE SWIGLU : gate rows n and up rows up_row_offset + n, two accumulators that fill TMEM (no
 //               overlap), bfloat16 silu(gate) * up out; 48 KB a stage for twice the MMAs.
-// The epilogue is spread over 16 warps a CTA (four per TMEM lane quarter, 64 token columns
+// The N operand of a tile has bn columns, a multiple of 16 up to 256 (QKV_PREP: 256): the host takes the number with which
+// the tiles fill their rounds over the pairs best (pair_tile).
+// The epilogue is spread over 16 warps a CTA (four per TMEM lane quarter, every fourth 16 columns
 // each): where it does not overlap the next tile it is on the critical path, and four warps
 // alone, one per scheduler, run it at the pace of their own dependent instructions.
 template <int MODE>
 __global__ void __launch_bounds__(TCP_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                     void *__restrict__ out, int T, int N, int K, long long ldo, int stages, int tiles_n, int tiles_total,
-                    int up_row_offset, int accumulate, int tiles_nt, int kb_per_split, long long slice_stride,
+                    int up_row_offset, int accumulate, int tiles_nt, int kb_per_split, long long slice_stride, int tile_cols,
                     const QkvPrepParams prep) {
     pdl_launch_dependents();
+    const int bn = MODE == TC_QKV_PREP ? TCP_BN : tile_cols;
     constexpr bool SWAP = MODE == TC_SWIGLU_T || MODE == TC_QKV_PREP;      // tokens are the M operand
     constexpr int A_TILES = MODE == TC_SWIGLU ? 2 : 1;
     constexpr uint32_t A_BYTES = TC_BM * TC_BK * 2;
-    constexpr uint32_t B_BYTES = (TCP_BN / 2) * TC_BK * 2;
-    constexpr uint32_t STAGE_BYTES = A_TILES * A_BYTES + B_BYTES;     // per CTA; a stage of the pair is twice that
+    const uint32_t STAGE_BYTES = A_TILES * A_BYTES + (uint32_t)bn * TC_BK;     // per CTA: bn / 2 rows of the N operand; a stage of the pair is twice that
     constexpr uint32_t ACC_COLS = A_TILES * TCP_BN, TMEM_COLS = 512;
     constexpr int NBUF = TMEM_COLS / ACC_COLS;
-    // M = 256 (two CTAs), N = 256, bf16 x bf16 -> f32, both operands K-major
-    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TCP_BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+    // M = 256 (two CTAs), N = bn, bf16 x bf16 -> f32, both operands K-major
+    const uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 
     extern __shared__ uint8_t smem_raw[];
     uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -531,9 +533,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             for (int tile = pair; tile < tiles_total && ok; tile += n_pairs) {
                 const int split = tile / tiles_nt, tw = tile % tiles_nt;       // a tile of the output and its slice of K
                 int n0 = tile_n(tw) * 256 + (int)rank * TC_BM;
-                int t0 = tile_t(tw) * TCP_BN + (int)rank * (TCP_BN / 2);
+                int t0 = SWAP ? tile_t(tw) * 256 + (int)rank * TC_BM : tile_t(tw) * bn + (int)rank * (bn / 2);
                 if (MODE == TC_PARTIAL && prep.group_rows) t0 += tile_n(tw) * 256 / prep.group_rows * T;
-                if (MODE == TC_SWIGLU_T) n0 = tile_n(tw) * TC_BM + (rank ? up_row_offset : 0);     // this rank's half of the N operand: gate rows, or up rows
+                if (MODE == TC_SWIGLU_T) n0 = tile_n(tw) * (bn / 2) + (rank ? up_row_offset : 0);     // this rank's half of the N operand: gate rows, or up rows
                 if (MODE == TC_QKV_PREP) n0 = (2 * tile_n(tw) + (int)rank) * TC_BM;                  // one head's rows from each rank
                 const int kb_begin = split * kb_per_split, kb_end = min(num_kb, (split + 1) * kb_per_split);
                 auto load_w = [&](int st, int kb) {
@@ -600,7 +602,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             uint32_t acc_phase = (uint32_t)(j / NBUF) & 1u;
             const int split = tile / tiles_nt, tw = tile % tiles_nt;
             int n = tile_n(tw) * 256 + (int)rank * TC_BM + 32 * q + lane;
-            int t0 = tile_t(tw) * TCP_BN;
+            int t0 = tile_t(tw) * (SWAP ? 256 : bn);
             if (!mbar_wait(acc_full(b), acc_phase)) { if (lane == 0) atomicExch(&g_tc_error, 3); break; }
             tc_fence_after();
             uint32_t d = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)b * ACC_COLS;
@@ -610,7 +612,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 // of both heads; they exchange their parts of the sums of squares through shared memory.
                 __shared__ float ss_x[2][2][4][128];                     // [tile parity][head of the tile][group][token]
                 const int grp = (warp - 2) >> 2, tl = 32 * q + lane;
-                const int t = t0 + (int)rank * (TCP_BN / 2) + tl;
+                const int t = t0 + (int)rank * TC_BM + tl;
                 const bool t_ok = t < T;
                 const int heads = prep.nq + 2 * prep.nkv, head0 = 2 * tile_n(tw);
                 const int pos = t_ok ? prep.positions[t] : 0;
@@ -702,18 +704,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 continue;
             }
             if (SWAP) {
-                // lane = token, columns 0..127 = gate of 128 features, 128..255 = up of the same features;
-                // each group of four warps takes a quarter of the features
-                const int t = t0 + (int)rank * (TCP_BN / 2) + 32 * q + lane;
-                const int f0 = tile_n(tw) * TC_BM;
-                const int cf = ((warp - 2) >> 2) * (TC_BM / TCP_EPI_GROUPS);
+                // lane = token, the first half of the columns = gate of bn / 2 features, the other up of the same features;
+                // each group of four warps takes every fourth 16 of the features
+                const int t = t0 + (int)rank * TC_BM + 32 * q + lane;
+                const int feats = bn / 2, f0 = tile_n(tw) * feats;
                 __nv_bfloat16 *o = (__nv_bfloat16 *)out + (size_t)t * ldo + f0;
 #pragma unroll 1
-                for (int c = cf; c < cf + TC_BM / TCP_EPI_GROUPS; c += 16) {
+                for (int c = ((warp - 2) >> 2) * 16; c < feats; c += 16 * TCP_EPI_GROUPS) {
                     if (f0 + c >= N) break;
                     float g[16], u[16];
                     tc_ld16(d + c, g);
-                    tc_ld16(d + TC_BM + c, u);
+                    tc_ld16(d + feats + c, u);
                     if (t < T) {
                         if (f0 + c + 16 <= N && (ldo & 7) == 0) {          // 16 features of one token: two 16-byte stores
                             uint32_t pk[8];
@@ -740,15 +741,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 if (lane == 0) mbar_arrive_cluster(map_to_rank(acc_empty(b), 0));
                 continue;
             }
-            int valid = min(TCP_BN, T - t0);
-            const int c_begin = ((warp - 2) >> 2) * (TCP_BN / TCP_EPI_GROUPS);      // each group of four warps its columns
+            int valid = min(bn, T - t0);
             Xielu xielu;
             float act_bias = 0.f;
             if (MODE == TC_ACT && up_row_offset == 6) xielu = Xielu(prep.act_p);
             if (MODE == TC_ACT && prep.bias && n < N) act_bias = prep.bias[n];
 #pragma unroll 1
-            for (int c = c_begin; c < c_begin + TCP_BN / TCP_EPI_GROUPS; c += 16) {
-                if (c >= valid) break;
+            for (int c = ((warp - 2) >> 2) * 16; c < valid; c += 16 * TCP_EPI_GROUPS) {       // each group of four warps its columns
                 float g[16];
                 tc_ld16(d + c, g);
                 if (MODE == TC_SWIGLU) {
@@ -907,15 +906,23 @@ static int g_wide = 1, g_wide_min = 32;
 KESTREL_API void kestrel_gemm_tc_set_wide(int on, int more_than_tokens) { g_wide = on ? 1 : 0; if (more_than_tokens >= 0) g_wide_min = more_than_tokens; }
 static bool tc_wide(int T, int N) { return g_wide && T > g_wide_min && T <= 128 && T <= g_pair_min_tokens && N % (2 * TC_BM) == 0; }
 
-// Cost of a many-token product on CTA pairs cut into s slices along K, in k-blocks of one
+// Cost of a many-token product on CTA pairs with tiles of bn tokens, cut into s slices along K, in 1/256 k-blocks of one
 // pair's time (about 0.42 us at these sizes); -1 where s does not divide the k-blocks into slices
 // of at least sixteen.  A slice costs about g_pair_overhead_kb k-blocks beyond its own (pipeline
 // fill, the last tile's epilogue); the slices' float32 planes cost their write and their read
 // by the consumer as far as they no longer fit L2 (measured at 3,072 tokens: the down product in
 // three slices 227 + 89 us with its norm, whole 251 + 47).
 static int tc_splits(int T, int N, int K, bool wide);
-static long long pair_cost(int T, int N, int K, int s, long long *waves_out = nullptr) {
-    const long long tiles = (long long)((N + 255) / 256) * ((T + TCP_BN - 1) / TCP_BN);
+static int g_pair_tile = 0;         // columns of a pair's tile; 0: by cost
+KESTREL_API void kestrel_gemm_tc_set_pair_tile(int columns) { if (columns >= 0 && columns <= TCP_BN && columns % 16 == 0) g_pair_tile = columns; }
+// A k-block of a tile of bn columns.  Products of 512 tokens, 4,096 features, K = 12,288 on 32 pairs, us: 63.3 with 256 columns, 60.5 with 240, 58.9 with 224,
+// 59 to 60 below: from 224 columns down the operands that come in, not the products, set the pace, so fewer columns pay where a round of tiles
+// goes, or the last tile is less empty.  us, tiles of 256 -> of the columns chosen: 1,024 x 3,072 x 2,048 18.9 -> 17.6, 1,777 x 3,216 x 2,048 28.7 -> 27.4,
+// 700 x 10,304 x 2,048 30.5 -> 29.7, 300 x 4,096 x 4,096 18.9 -> 17.4, 200 x 2,048 x 2,048 11.5 -> 10.1; 2,048 x 4,096 x 4,096 stays at 256 (53).
+#define PAIR_TILE_MIN 128
+static long long pair_kb_cost(int bn) { return bn > 236 ? bn : 236; }
+static long long pair_cost(int T, int N, int K, int s, int bn, long long *waves_out = nullptr) {
+    const long long tiles = (long long)((N + 255) / 256) * ((T + bn - 1) / bn);
     const int total_kb = (K + TC_BK - 1) / TC_BK;
     const int pairs = kestrel_sms() / 2;
     const int per = (total_kb + s - 1) / s;
@@ -924,7 +931,20 @@ static long long pair_cost(int T, int N, int K, int s, long long *waves_out = nu
     if (waves_out) *waves_out = waves;
     long long planes = 8ll * T * N * (s - 1) - (64ll << 20);
     if (planes < 0) planes = 0;
-    return waves * (g_pair_overhead_kb + per) + planes / 2100000;
+    return waves * ((128ll + bn / 2) * g_pair_overhead_kb + per * pair_kb_cost(bn)) + 256 * (planes / 2100000);
+}
+// The tile's columns that cost least, of equal ones the most
+static int pair_tile(int T, int N, int K, int s, long long *cost_out = nullptr) {
+    int best = TCP_BN;
+    long long best_cost = -1;
+    for (int bn = TCP_BN; bn >= PAIR_TILE_MIN; bn -= 16) {
+        if (g_pair_tile) bn = g_pair_tile;
+        const long long cost = pair_cost(T, N, K, s, bn);
+        if (cost >= 0 && (best_cost < 0 || cost < best_cost)) best_cost = cost, best = bn;
+        if (g_pair_tile) break;
+    }
+    if (cost_out) *cost_out = best_cost;
+    return best;
 }
 
 KESTREL_API int kestrel_gemm_tc_splits(int T, int N, int K) { return tc_splits(T, N, K, tc_wide(T, N)); }
@@ -937,9 +957,10 @@ static int tc_splits(int T, int N, int K, bool wide) {
         int best = 1;
         long long best_cost = -1;
         for (int s = 1; s <= 8; ++s) {
-            long long cost = pair_cost(T, N, K, s);
+            long long cost;
+            pair_tile(T, N, K, s, &cost);
             if (cost < 0) continue;
-            if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
+            if (best_cost < 0 || cost * 16 < best_cost * 15) { best_cost = cost; best = s; }       // (a slice more is read by the consumer)
         }
         return best;
     }
@@ -1023,12 +1044,13 @@ static int launch_tc_persistent(const CUtensorMap &mw, const CUtensorMap &mx, vo
 
 template <int MODE>
 static int launch_tc_pair(const CUtensorMap &mw, const CUtensorMap &mx, void *out, int T, int N, int K, long long ldo,
-                          int up_off, int accumulate, int splits, long long slice_stride, cudaStream_t stream,
+                          int up_off, int accumulate, int splits, long long slice_stride, int bn, cudaStream_t stream,
                           const QkvPrepParams &prep = QkvPrepParams()) {
-    const int STAGE_BYTES = (MODE == TC_SWIGLU ? 2 : 1) * TC_BM * TC_BK * 2 + (TCP_BN / 2) * TC_BK * 2;
+    const int STAGE_BYTES = (MODE == TC_SWIGLU ? 2 : 1) * TC_BM * TC_BK * 2 + bn * TC_BK;
     int stages = (200 * 1024) / STAGE_BYTES;
     if (stages > 8) stages = 8;
-    size_t smem = (size_t)stages * STAGE_BYTES + 16 * stages + 48 + 1024;
+    // as much for every tile: a pair has its two SMs' shared memory alone
+    size_t smem = (size_t)200 * 1024 + 16 * 8 + 48 + 1024;
     static int max_clusters = -1;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
@@ -1059,7 +1081,7 @@ static int launch_tc_pair(const CUtensorMap &mw, const CUtensorMap &mx, void *ou
     if (max_clusters == 0) return 1;       // not an error: tells the caller to fall back
     // output tiles: 256 features x 256 tokens; with the operands swapped 128 features x 256 tokens
     // (QKV_PREP: 256 features = two heads of 128 x 256 tokens, N = all heads' rows)
-    int tiles_n = MODE == TC_SWIGLU_T ? (N + TC_BM - 1) / TC_BM : (N + 255) / 256, tiles_t = (T + TCP_BN - 1) / TCP_BN;
+    int tiles_n = MODE == TC_SWIGLU_T ? (N + bn / 2 - 1) / (bn / 2) : (N + 255) / 256, tiles_t = MODE == TC_SWIGLU_T ? (T + 255) / 256 : (T + bn - 1) / bn;
     long long tiles_nt = (long long)tiles_n * tiles_t, total = tiles_nt * splits;
     if (total > 0x7fffffff) return kestrel_fail(-2, "gemm_tc: too many tiles");
     if (splits > 1 && (MODE != TC_PARTIAL || accumulate)) return kestrel_fail(-2, "gemm_tc_pair: only plain float32 slices can be cut along K");
@@ -1069,7 +1091,7 @@ static int launch_tc_pair(const CUtensorMap &mw, const CUtensorMap &mx, void *ou
     cfg.gridDim = dim3(2 * pairs);
     cfg.numAttrs = g_kestrel_pdl ? 2 : 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<MODE>, mw, mx, out, T, N, K, ldo, stages, tiles_n, (int)total, up_off, accumulate,
-                                       (int)tiles_nt, per, slice_stride, prep);
+                                       (int)tiles_nt, per, slice_stride, bn, prep);
     if (e != cudaSuccess) return kestrel_fail(-3, "gemm_tc_pair: %s", cudaGetErrorString(e));
     return kestrel_check_launch("gemm_tc_pair");
 }
@@ -1091,6 +1113,20 @@ static bool swiglu_swapped_wins(int T, int ff) {
     return work_t < work_m || (work_t == work_m && tt > 1);
 }
 
+// Columns of its tiles, gate and up of half as many features (whole 16s): those with which ff features cost least
+static int swapped_tile(int T, int ff, int K) {
+    if (g_pair_tile && g_pair_tile % 32 == 0) return g_pair_tile;
+    const long long pairs = kestrel_sms() / 2, tt = (T + 255) / 256, kb = (K + TC_BK - 1) / TC_BK;
+    int best = TCP_BN;
+    long long best_cost = -1;
+    for (int bn = TCP_BN; bn >= PAIR_TILE_MIN; bn -= 32) {
+        const long long waves = (((ff + bn / 2 - 1) / (bn / 2)) * tt + pairs - 1) / pairs;
+        const long long cost = waves * kb * pair_kb_cost(bn) + 256 * g_pair_overhead_kb;      // (only the last epilogue is not overlapped)
+        if (best_cost < 0 || cost < best_cost) best_cost = cost, best = bn;
+    }
+    return best;
+}
+
 template <int MODE>
 static int dispatch_tc(const void *x, const void *w, void *out, int T, int N, int w_rows, int K, long long ldx, long long ldw,
                        long long ldo, int splits, long long slice_stride, int up_off, int early_w, cudaStream_t stream, float act_limit = 0.f) {
@@ -1104,12 +1140,19 @@ static int dispatch_tc(const void *x, const void *w, void *out, int T, int N, in
         QkvPrepParams prep = {};
         prep.act_limit = act_limit;
         prep.early_w = early_w;
-        rc = kestrel_tensor_map_bf16(&mx, x, T, K, ldx, TCP_BN / 2);
-        if (rc) return rc;
-        if (MODE == TC_SWIGLU && swiglu_swapped_wins(T, N) && ((uintptr_t)out & 15) == 0 && ldo % 8 == 0)
-            rc = launch_tc_pair<TC_SWIGLU_T>(mw, mx, out, T, N, K, ldo, up_off, 0, 1, 0, stream, prep);
-        else
-            rc = launch_tc_pair<MODE>(mw, mx, out, T, N, K, ldo, up_off, 0, splits, slice_stride, stream, prep);
+        if (MODE == TC_SWIGLU && swiglu_swapped_wins(T, N) && ((uintptr_t)out & 15) == 0 && ldo % 8 == 0) {
+            const int cols = swapped_tile(T, N, K);
+            CUtensorMap mw_t;
+            rc = kestrel_tensor_map_bf16(&mx, x, T, K, ldx, TC_BM);
+            if (rc == 0) rc = kestrel_tensor_map_bf16(&mw_t, w, w_rows, K, ldw, cols / 2);
+            if (rc) return rc;
+            rc = launch_tc_pair<TC_SWIGLU_T>(mw_t, mx, out, T, N, K, ldo, up_off, 0, 1, 0, cols, stream, prep);
+        } else {
+            const int cols = MODE == TC_PARTIAL ? pair_tile(T, N, K, splits) : TCP_BN;
+            rc = kestrel_tensor_map_bf16(&mx, x, T, K, ldx, cols / 2);
+            if (rc) return rc;
+            rc = launch_tc_pair<MODE>(mw, mx, out, T, N, K, ldo, up_off, 0, splits, slice_stride, cols, stream, prep);
+        }
         if (rc <= 0) return rc;            // 1 = pairs cannot be scheduled: go on with one CTA per tile
     }
     if (splits > 1) persistent = false;    // the one-CTA persistent kernel does not cut K
@@ -1168,11 +1211,13 @@ KESTREL_API int kestrel_gemm_tc_grouped(const void *x, const void *w, float *out
     int rc = kestrel_tensor_map_bf16(&mw, w, N, K, ldw, TC_BM);
     if (rc) return rc;
     if (T > g_pair_min_tokens) {
-        rc = kestrel_tensor_map_bf16(&mx, x, groups * T, K, ldx, TCP_BN / 2);
+        const int cols = pair_tile(T, N, K, splits);
+        rc = kestrel_tensor_map_bf16(&mx, x, groups * T, K, ldx, cols / 2);
         if (rc) return rc;
         QkvPrepParams prep = {};
         prep.group_rows = group_rows;
-        rc = launch_tc_pair<TC_PARTIAL>(mw, mx, out, T, N, K, ldo, 0, 0, splits, slice_stride, stream, prep);
+        prep.early_w = weights_static ? 1 : 0;
+        rc = launch_tc_pair<TC_PARTIAL>(mw, mx, out, T, N, K, ldo, 0, 0, splits, slice_stride, cols, stream, prep);
         return rc > 0 ? kestrel_fail(-3, "gemm_tc_grouped: CTA pairs cannot be scheduled here") : rc;
     }
     const int bn = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256;
@@ -1207,9 +1252,10 @@ KESTREL_API int kestrel_gemm_tc_add(const void *x, const void *w, float *residua
     CUtensorMap mw, mx;
     int rc = kestrel_tensor_map_bf16(&mw, w, N, K, ldw, TC_BM);
     if (rc) return rc;
-    rc = kestrel_tensor_map_bf16(&mx, x, T, K, ldx, TCP_BN / 2);
+    const int cols = pair_tile(T, N, K, 1);
+    rc = kestrel_tensor_map_bf16(&mx, x, T, K, ldx, cols / 2);
     if (rc) return rc;
-    return launch_tc_pair<TC_PARTIAL>(mw, mx, residual, T, N, K, ldo, 0, 1, 1, 0, stream);
+    return launch_tc_pair<TC_PARTIAL>(mw, mx, residual, T, N, K, ldo, 0, 1, 1, 0, cols, stream);
 }
 
 // out bf16 [T, N] = act(x w^T) in the product's epilogue (ACT above; many tokens on CTA pairs only).
@@ -1231,12 +1277,13 @@ KESTREL_API int kestrel_gemm_tc_act_with(const void *x, const void *w, const flo
     CUtensorMap mw, mx;
     int rc = kestrel_tensor_map_bf16(&mw, w, N, K, ldw, TC_BM);
     if (rc) return rc;
-    rc = kestrel_tensor_map_bf16(&mx, x, T, K, ldx, TCP_BN / 2);
+    const int cols = pair_tile(T, N, K, 1);
+    rc = kestrel_tensor_map_bf16(&mx, x, T, K, ldx, cols / 2);
     if (rc) return rc;
     QkvPrepParams prep = {};
     prep.bias = bias;
     prep.act_p = act_p;
-    return launch_tc_pair<TC_ACT>(mw, mx, out, T, N, K, ldo, act, 0, 1, 0, stream, prep);
+    return launch_tc_pair<TC_ACT>(mw, mx, out, T, N, K, ldo, act, 0, 1, 0, cols, stream, prep);
 }
 
 // The q, k, v product of a prompt portion and everything between it and attention in one kernel
@@ -1261,14 +1308,16 @@ KESTREL_API int kestrel_gemm_tc_qkv_prepare(const void *x, const void *w, int T,
         // 512 tokens, one round, 44 against 36)
         const int S = kestrel_gemm_tc_splits(T, N, K);
         long long waves = 0;
-        const long long whole = pair_cost(T, N, K, 1, &waves);
-        if (S > 1 && !(waves >= 3 && whole * 10 <= pair_cost(T, N, K, S) * 11)) return 1;
+        const long long whole = pair_cost(T, N, K, 1, TCP_BN, &waves);
+        long long cut = 0;
+        pair_tile(T, N, K, S, &cut);
+        if (S > 1 && !(waves >= 3 && whole * 10 <= cut * 11)) return 1;
     }
     if ((((uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) != 0) return 1;
     CUtensorMap mw, mx;
     int rc = kestrel_tensor_map_bf16(&mw, w, N, K, ldw, TC_BM);
     if (rc) return rc;
-    rc = kestrel_tensor_map_bf16(&mx, x, T, K, ldx, TCP_BN / 2);
+    rc = kestrel_tensor_map_bf16(&mx, x, T, K, ldx, TC_BM);
     if (rc) return rc;
     QkvPrepParams prep = {};
     prep.bias = bias; prep.q_norm_w = q_norm_w; prep.k_norm_w = k_norm_w; prep.inv_freq = inv_freq;
@@ -1276,7 +1325,7 @@ KESTREL_API int kestrel_gemm_tc_qkv_prepare(const void *x, const void *w, int T,
     prep.block_table = block_table; prep.table_stride = table_stride; prep.page_size = page_size;
     prep.k_cache = (__nv_bfloat16 *)k_cache; prep.v_cache = (__nv_bfloat16 *)v_cache; prep.q_out = (__nv_bfloat16 *)q_out;
     prep.nq = nq; prep.nkv = nkv; prep.write_kv = write_kv ? 1 : 0;
-    return launch_tc_pair<TC_QKV_PREP>(mw, mx, nullptr, T, N, K, 0, 0, 0, 1, 0, stream, prep);
+    return launch_tc_pair<TC_QKV_PREP>(mw, mx, nullptr, T, N, K, 0, 0, 0, 1, 0, TCP_BN, stream, prep);
 }
 
 KESTREL_API void kestrel_gemm_tc_set_qkv_fused(int mode) { g_qkv_fused = mode < 0 ? 0 : (mode > 2 ? 2 : mode); }

@@ -443,6 +443,12 @@ def gemm_tc_set_wide(on: bool = True, more_than_tokens: int = -1) -> None:
     fn(1 if on else 0, int(more_than_tokens))
 
 
+def gemm_tc_set_pair_tile(columns: int = 0) -> None:
+    """Columns of the tiles of products on CTA pairs, a multiple of 16 up to 256 (0: those that cost least).  For tests and measurements."""
+    fn = library().kestrel_gemm_tc_set_pair_tile
+    fn(int(columns))
+
+
 def gemm_tc_set_pair_tuning(min_tokens: int = -1, overhead_kb: int = -1) -> None:
     """Tuning of many-token products on CTA pairs: products of more than ``min_tokens`` tokens
     take them; a K slice is priced at ``overhead_kb`` k-blocks beyond its own (see gemm_tcgen05.cu)."""
