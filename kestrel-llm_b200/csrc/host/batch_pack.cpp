@@ -122,6 +122,18 @@ KESTREL_API int kbatch_pack(void *cache, int n, const long long *ids, const int 
     return (int)total;
 }
 
+// Uniform numbers in (0, 1] of n draws: out[i] follows from (seeds[i], indices[i]) alone, by two rounds of the splitmix64 finaliser
+// (24 bits, exact in float32).
+KESTREL_API void kbatch_uniforms(int n, const long long *seeds, const long long *indices, float *out) {
+    auto mix = [](uint64_t z) {
+        z += 0x9E3779B97F4A7C15ull;
+        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+        return z ^ (z >> 31);
+    };
+    for (int i = 0; i < n; ++i) out[i] = (float)((mix(mix((uint64_t)seeds[i]) ^ (uint64_t)indices[i]) >> 40) + 1) * (1.0f / 16777216.0f);
+}
+
 // The predicate of the runner's debug guards, on the host: walks every token of a packed
 // description and returns 0 if the kernels can place it, else (rule << 16) | (token & 0xffff)
 // for the first token that breaks a rule (STEP_CHECK_* in csrc/kernels/step_checks.cuh: 1 token

@@ -355,6 +355,19 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
                                     uniform.data_ptr(), out.data_ptr(), _stream()))
 
 
+def sample_options(logits: torch.Tensor, options: torch.Tensor, out: torch.Tensor) -> None:
+    """`sample` with the rows' options in one tensor: float32 [5, R] of temperature, top-p, min-p, uniform number and top-k (int32 bits)."""
+    _need(logits, "sample.logits", torch.float32, 2)
+    _need(options, "sample.options", torch.float32, 2)
+    _need(out, "sample.out", torch.int32, 1)
+    R, V = logits.shape
+    if tuple(options.shape) != (5, R) or out.shape[0] != R:
+        raise KernelError(f"sample: options {tuple(options.shape)} and {out.shape[0]} results for {R} rows")
+    at, row = options.data_ptr(), 4 * R
+    _check(library().kestrel_sample(logits.data_ptr(), logits.stride(0), R, V, at, at + 4 * row, at + row, at + 2 * row, at + 3 * row,
+                                    out.data_ptr(), _stream()))
+
+
 def repetition_penalty(logits: torch.Tensor, history: torch.Tensor, counts: torch.Tensor, penalty: torch.Tensor) -> None:
     """In place: for each of the first counts[r] tokens of history[r] (int32 [R, width], a request's
     last generated tokens), logits[r, token] becomes l / penalty[r] if l >= 0, else l * penalty[r] -

@@ -131,6 +131,8 @@ KESTREL_API int kbatch_pack(void *cache, int n, const long long *ids, const int 
 /* the check of the runner's debug guards, on the host: 0 if every token of the packed description can be placed by the kernels,
  * else (rule << 16) | (token & 0xffff) for the first that cannot (rules: 1 token id, 2 request index, 3 position,
  * 4 block-table column, 5 page id, 6 token outside its request's rows); pages[g] = pages of group g's tensors */
+/* uniform numbers in (0, 1] of n draws, functions of (seed, index) as 64-bit patterns */
+KESTREL_API void kbatch_uniforms(int n, const long long *seeds, const long long *indices, float *out);
 KESTREL_API int kbatch_check(const int *batch, const int *layout, int vocab, int page_size, const int *pages);
 
 /* ============================================================================================

@@ -9,11 +9,13 @@ and can be repeated.
 """
 from __future__ import annotations
 
+from array import array
 from typing import List, Optional, Sequence
 
 import numpy as np
 import torch
 
+from ..cache.manager import host_library
 from ..csrc import ops
 from .params import SamplingParams
 
@@ -34,30 +36,39 @@ def uniform_for(seed: int, index: int) -> float:
     return ((z >> 40) + 1) / float(1 << 24)
 
 
+class _Slot:
+    """A pinned buffer for the options of a call's rows, and the event behind its last copy to the device."""
+
+    __slots__ = ("floats", "ints", "pinned", "done", "pending")
+
+    def __init__(self, cap: int):
+        self.pinned = torch.empty((5 * cap,), dtype=torch.float32).pin_memory()
+        self.floats = self.pinned.numpy()
+        self.ints = self.floats.view(np.int32)
+        self.done, self.pending = torch.cuda.Event(), False
+
+
 class Sampler:
     RING = 4        # pinned buffers for the rows' options; a buffer is reused only after its copy has run
 
     def __init__(self, device):
         self.device = torch.device(device)
-        self._ring: List[torch.Tensor] = []
-        self._ring_done: List[object] = []
+        self._ring: List[_Slot] = []
         self._turn = 0
+        self._uniforms = host_library().kbatch_uniforms
 
-    def _pinned(self, rows: int) -> np.ndarray:
-        """A pinned float32 [5, rows] view whose last copy to the device has completed."""
-        if not self._ring or self._ring[0].shape[1] < rows:
-            cap = max(64, 1 << (rows - 1).bit_length())
-            for ev in self._ring_done:
-                if ev is not None:
-                    ev.synchronize()
-            self._ring = [torch.empty((5, cap), dtype=torch.float32).pin_memory() for _ in range(self.RING)]
-            self._ring_done = [None] * self.RING
-        t = self._turn
-        self._turn = (t + 1) % self.RING
-        if self._ring_done[t] is not None:
-            self._ring_done[t].synchronize()
-        self._current = t
-        return self._ring[t].numpy()[:, :rows]
+    def _slot(self, rows: int) -> _Slot:
+        """A buffer with room for the rows' options whose last copy to the device has completed."""
+        if not self._ring or self._ring[0].floats.size < 5 * rows:
+            for s in self._ring:
+                if s.pending:
+                    s.done.synchronize()
+            self._ring = [_Slot(max(64, 1 << (rows - 1).bit_length())) for _ in range(self.RING)]
+        self._turn = (self._turn + 1) % self.RING
+        slot = self._ring[self._turn]
+        if slot.pending:
+            slot.done.synchronize()
+        return slot
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], seeds: Sequence[int],
                indices: Sequence[int], generated: Optional[Sequence[Sequence[int]]] = None) -> torch.Tensor:
@@ -86,22 +97,21 @@ class Sampler:
         if all(p.greedy for p in params):
             ops.argmax(logits, out)
             return out
-        host = self._pinned(R) if self.device.type == "cuda" else np.empty((5, R), dtype=np.float32)
-        ks = np.empty((R,), dtype=np.int32)
-        for r, (p, s, i) in enumerate(zip(params, seeds, indices)):
-            host[0, r] = p.temperature if not p.greedy else 0.0
-            host[1, r] = p.top_p
-            host[2, r] = p.min_p
-            host[3, r] = uniform_for(s, i)
-            ks[r] = p.top_k
-        host[4] = ks.view(np.float32)
-        if self.device.type == "cuda":
-            dev = torch.empty((5, R), dtype=torch.float32, device=self.device)
-            dev.copy_(self._ring[self._current][:, :R], non_blocking=True)
-            ev = torch.cuda.Event()
-            ev.record()
-            self._ring_done[self._current] = ev
-        else:
-            dev = torch.from_numpy(host).to(self.device)
-        ops.sample(logits, dev[0], dev[4].view(torch.int32), dev[1], dev[2], dev[3], out)
+        # rows of temperature, top-p, min-p, uniform number and top-k (int32 bits), one behind the other: a copy of what is contiguous
+        # goes out of the pinned buffer itself
+        if not len(params) == len(seeds) == len(indices) == R:
+            raise ValueError(f"sample: {R} rows of logits, {len(params)} of options, {len(seeds)} seeds, {len(indices)} indices")
+        slot = self._slot(R)
+        host = slot.floats
+        host[:R] = [0.0 if p.greedy else p.temperature for p in params]
+        host[R:2 * R] = [p.top_p for p in params]
+        host[2 * R:3 * R] = [p.min_p for p in params]
+        slot.ints[4 * R:5 * R] = np.array([p.top_k for p in params], dtype=np.int32)
+        s, i = array("Q", [x & _MASK for x in seeds]), array("Q", [x & _MASK for x in indices])
+        self._uniforms(R, s.buffer_info()[0], i.buffer_info()[0], slot.pinned.data_ptr() + 12 * R)
+        dev = torch.empty((5, R), dtype=torch.float32, device=self.device)
+        dev.copy_(slot.pinned[:5 * R].view(5, R), non_blocking=True)
+        slot.done.record()
+        slot.pending = True
+        ops.sample_options(logits, dev, out)
         return out
