@@ -63,6 +63,26 @@ def test_gated_products_of_every_tile(tile, T, ff):
         ops.library().kestrel_gemm_tc_set_swiglu_swapped(1)
 
 
+@pytest.mark.parametrize("T,N,K", [(2048, 2048, 136), (1800, 2056, 72), (2500, 1032, 264)])     # uncut: as many tiles as fill the pairs; ragged ends
+def test_added_to_the_stream_by_every_tile(tile, T, N, K):
+    """The product added in place: float32 sums of exact products and one more addition, whatever the tile."""
+    from kestrel_llm_b200.csrc import ops
+    x, w = _operands(T, N, K, 3)
+    held = torch.randn((T, N), device=DEV, generator=torch.Generator(DEV).manual_seed(4)) * 8
+    want = held.double() + x.double() @ w.double().T
+    bound = 2.0 ** -24 * (K + 2) * (x.double().abs() @ w.double().abs().T + held.double().abs())
+    taken = 0
+    for columns in (256, 240, 208, 176, 128, 16, 0):
+        tile(columns)
+        out = held.clone()
+        rc = ops.library().kestrel_gemm_tc_add(x.data_ptr(), w.data_ptr(), out.data_ptr(), T, N, K, K, K, N, ops._stream())
+        ops.raise_on_kernel_error()
+        taken += rc == 0
+        assert rc == 1 or ((out.double() - want).abs() <= bound).all(), f"tiles of {columns}"
+        assert rc == 0 or torch.equal(out, held)
+    assert taken
+
+
 def test_a_tile_is_chosen_by_its_rounds():
     """1,024 tokens of 3,072 features: 48 tiles of 256 leave a third of 74 pairs idle; the tile taken fills them better, and sums are
     cut along K no more than before."""
