@@ -936,7 +936,7 @@ static bool tc_wide(int T, int N) { return g_wide && T > g_wide_min && T <= 128 
 
 // Cost of a many-token product on CTA pairs with tiles of bn tokens, cut into s slices along K, in 1/256 k-blocks of one
 // pair's time (about 0.42 us at these sizes); -1 where s does not divide the k-blocks into slices
-// of at least sixteen.  A slice costs about g_pair_overhead_kb k-blocks beyond its own (pipeline
+// of at least sixteen (four where the planes are small: a router's 1,000 x 32 x 2,048 14.0 -> 8.9 us).  A slice costs about g_pair_overhead_kb k-blocks beyond its own (pipeline
 // fill, the last tile's epilogue); the slices' float32 planes cost their write and their read
 // by the consumer as far as they no longer fit L2 (measured at 3,072 tokens: the down product in
 // three slices 227 + 89 us with its norm, whole 251 + 47).
@@ -954,7 +954,8 @@ static long long pair_cost(int T, int N, int K, int s, int bn, long long *waves_
     const int total_kb = (K + TC_BK - 1) / TC_BK;
     const int pairs = kestrel_sms() / 2;
     const int per = (total_kb + s - 1) / s;
-    if (s > 1 && (per < 16 || (total_kb + per - 1) / per != s)) return -1;
+    const int least = 4ll * T * N * s <= (2ll << 20) ? 4 : 16;      // (a narrow product's planes, as a router's, cost next to nothing)
+    if (s > 1 && (per < least || (total_kb + per - 1) / per != s)) return -1;
     const long long waves = (tiles * s + pairs - 1) / pairs;
     if (waves_out) *waves_out = waves;
     long long planes = 8ll * T * N * (s - 1) - (64ll << 20);
