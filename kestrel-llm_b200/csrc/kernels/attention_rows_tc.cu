@@ -8,12 +8,13 @@
 //   softmax  (warps 0-3)  a thread owns a row (TMEM lane): its 64 scores come out of TMEM once, maximum, exp2 and sum in float32, P goes
 //            back as packed bfloat16 over the first 32 columns of its score buffer;
 //   loader   (warp 4)     pages by TMA (boxes of a page, or of 64 rows of a larger page, by 64 columns; 128-byte swizzle) into a ring of
-//            four stages: a stage is freed by the tile's second product, three tiles before its next content is needed;
+//            six stages: a stage is freed by the tile's second product, five tiles before its next content is needed;
 //   issuer   (warp 5)     S(0) | S(t + 1), O += P(t) V(t): the scores of the next tile are made while this tile is softmaxed, for which
 //            there are two score buffers of 64 columns.
-// TMEM: S 2 x 64, O up to 256 columns.  What bounds it is the chain of a tile - scores out, softmax, P in, hand-overs - beside
-// 950 cycles of products a tile at 256 / 192, 2,900 cycles in all.  1,024 tokens of 16 heads behind 2,000, rows of 256, values of 192:
-// 77 us, where the mma.sync kernel (attention_window.cu) took 389.
+// TMEM: S 2 x 64, Q 128 (two numbers to a column), O up to 256 columns.  Q is operand A of S from TMEM: from shared memory each product of
+// 128 x 64 x 16 read 4 KB of Q beside 2 KB of keys.  What bounds the kernel is the chain of a tile: scores out, softmax, P in, hand-overs.
+// 1,024 tokens of 16 heads behind 2,000, rows of 256, values of 192: 72.0 us (78.6 with Q in shared memory and a ring of four), where the
+// mma.sync kernel (attention_window.cu) took 389.
 // As in attention_tc.cu the output is rescaled only when a row's maximum has outgrown its reference by more than 2^8, keys a row may
 // not see are masked in S, rows outside the CTA's key range are zeroed in shared memory before they are read as values (a page may hold
 // another request's stale numbers), key ranges may be cut into slices that attention_merge combines, tiles with most keys go first, and
@@ -25,10 +26,9 @@
 #define AR_THREADS 192
 #define AR_BM 128
 #define AR_BN 64
-#define AR_STAGES 4
+#define AR_STAGES 6
 #define AR_MAX_HD 256
-#define AR_Q_PANEL (AR_BM * 128)            // bytes of a panel of 64 columns: 128 query rows
-#define AR_K_PANEL (AR_BN * 128)            // 64 cache rows
+#define AR_K_PANEL (AR_BN * 128)            // bytes of a panel of 64 columns: 64 cache rows
 #define AR_RESCALE_STEP 8.0f
 
 __device__ int g_ar_error = 0;
@@ -88,11 +88,11 @@ attention_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const ArPara
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *aligned = smem_raw + (base - smem_u32(smem_raw));
-    const uint32_t q_s = base, k_s = base + (uint32_t)panels * AR_Q_PANEL;
-    const uint32_t bar_off = (uint32_t)panels * (AR_Q_PANEL + AR_STAGES * AR_K_PANEL);
+    const uint32_t k_s = base;
+    const uint32_t bar_off = (uint32_t)panels * AR_STAGES * AR_K_PANEL;
     const uint32_t bars = base + bar_off, tmem_slot = bars + 8 * R_COUNT;
     volatile uint32_t *tmem_slot_ptr = (volatile uint32_t *)(aligned + bar_off + 8 * R_COUNT);
-    uint8_t *k_ptr = aligned + (uint32_t)panels * AR_Q_PANEL;
+    uint8_t *k_ptr = aligned;
     auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -109,7 +109,7 @@ attention_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const ArPara
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot_ptr, tmem_o = tmem + 256;
+    const uint32_t tmem = *tmem_slot_ptr, tmem_q = tmem + 2 * AR_BN, tmem_o = tmem + 256;
     pdl_launch_dependents();            // after the allocation: a dependent's CTA that holds TMEM waits for this grid
     pdl_wait();
 
@@ -154,13 +154,14 @@ attention_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const ArPara
         if (lane == 0 && n_tiles > 0) {
             bool ok = mbar_wait(bar(R_Q_FULL), 0);
             if (!ok) atomicExch(&g_ar_error, 2);
+            tc_fence_after();
             auto issue_s = [&](int t) {
                 const int b = t % AR_STAGES;
                 if (!mbar_wait(bar(R_K_FULL + b), (uint32_t)(t / AR_STAGES) & 1u)) { atomicExch(&g_ar_error, 3); return false; }
                 tc_fence_after();
                 for (int ks = 0; ks < k_steps; ++ks)
-                    tc_mma(tmem + (t & 1) * AR_BN, smem_desc(q_s + (ks >> 2) * AR_Q_PANEL + (ks & 3) * 32),
-                           smem_desc(k_s + b * stage_bytes + (ks >> 2) * AR_K_PANEL + (ks & 3) * 32), idesc_s, ks > 0 ? 1u : 0u);
+                    ar_mma_ts(tmem + (t & 1) * AR_BN, tmem_q + ks * 8, smem_desc(k_s + b * stage_bytes + (ks >> 2) * AR_K_PANEL + (ks & 3) * 32), idesc_s,
+                              ks > 0 ? 1u : 0u);
                 tc_commit(bar(R_S_FULL + (t & 1)));
                 return true;
             };
@@ -182,22 +183,23 @@ attention_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const ArPara
     } else {
         // ------------------------------------------------------------------ softmax: thread r owns row r (TMEM lane r)
         const int r = tid;
-        const int chunks = panels * 8;                       // 16-byte chunks of a query row, zeros beyond hd
-        for (int idx = r; idx < AR_BM * chunks; idx += 128) {
-            const int rr = idx / chunks, c = idx % chunks;
-            const bool valid = rr < rows_here && c * 8 < hd;
-            size_t off = 0;
-            if (valid) {
-                const int row = row0 + rr;
-                off = ((size_t)(tok_begin + row / G) * p.nq + kvh * G + row % G) * hd + c * 8;
+        const int chunks = panels * 8;                       // 16-byte chunks of a cache row in shared memory
+        // the row's query, two numbers to a column as P's, zeros beyond hd and for rows that are not there
+        const uint32_t q_addr = tmem_q + (((uint32_t)(32 * warp)) << 16);
+        const int q_row = row0 + min(r, rows_here - 1);
+        const uint4 *q = reinterpret_cast<const uint4 *>(p.q + ((size_t)(tok_begin + q_row / G) * p.nq + kvh * G + q_row % G) * hd);
+        for (int c = 0; c < k_steps * 8; c += 16) {
+            uint32_t w[16];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const bool in = r < rows_here && (c / 4 + k) * 8 < hd;
+                const uint4 x = in ? q[c / 4 + k] : make_uint4(0, 0, 0, 0);
+                w[4 * k] = x.x, w[4 * k + 1] = x.y, w[4 * k + 2] = x.z, w[4 * k + 3] = x.w;
             }
-            const uint32_t dst = q_s + (c >> 3) * AR_Q_PANEL + swizzle128(rr, c & 7);
-            const int sz = valid ? 16 : 0;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(p.q + off), "r"(sz) : "memory");
+            ar_st16(q_addr + c, w);
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // cp.async writes -> tensor-core reads
+        ar_st_wait();
+        tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(R_Q_FULL));
 
@@ -378,7 +380,7 @@ KESTREL_API int kestrel_attention_rows_tc(const void *q, const void *cache, void
     p.gate = slices > 1 ? nullptr : gate;
     ap.vd = vd;
     // as much for every size: a CTA has all of an SM's TMEM and shares the SM with no other kernel that takes some
-    const size_t smem = (size_t)(AR_MAX_HD / 64) * (AR_Q_PANEL + AR_STAGES * AR_K_PANEL) + 8 * R_COUNT + 16 + 1024;
+    const size_t smem = (size_t)(AR_MAX_HD / 64) * AR_STAGES * AR_K_PANEL + 8 * R_COUNT + 16 + 1024;
     static bool attr_set = false;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(attention_rows_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
