@@ -949,27 +949,29 @@ KESTREL_API void kestrel_gemm_tc_set_pair_tile(int columns) { if (columns >= 0 &
 // 700 x 10,304 x 2,048 30.5 -> 29.7, 300 x 4,096 x 4,096 18.9 -> 17.4, 200 x 2,048 x 2,048 11.5 -> 10.1; 2,048 x 4,096 x 4,096 stays at 256 (53).
 #define PAIR_TILE_MIN 128
 static long long pair_kb_cost(int bn) { return bn > 236 ? bn : 236; }
-static long long pair_cost(int T, int N, int K, int s, int bn, long long *waves_out = nullptr) {
-    const long long tiles = (long long)((N + 255) / 256) * ((T + bn - 1) / bn);
+static long long pair_cost(int T, int N, int K, int s, int bn, int pairs, long long *waves_out = nullptr) {
     const int total_kb = (K + TC_BK - 1) / TC_BK;
-    const int pairs = kestrel_sms() / 2;
     const int per = (total_kb + s - 1) / s;
     const int least = 4ll * T * N * s <= (2ll << 20) ? 4 : 16;      // (a narrow product's planes, as a router's, cost next to nothing)
     if (s > 1 && (per < least || (total_kb + per - 1) / per != s)) return -1;
-    const long long waves = (tiles * s + pairs - 1) / pairs;
+    const long long tiles = (long long)((N + 255) / 256) * ((T + bn - 1) / bn) * s;
+    // (32-bit divisions where they do, and the device asked once: a launch waits for nine of these or more.  A plan took 5.8 us on the host, of
+    // layers whose every launch is a few; now 1.2)
+    const long long waves = tiles < (1ll << 30) ? (int)(tiles + pairs - 1) / pairs : (tiles + pairs - 1) / pairs;
     if (waves_out) *waves_out = waves;
     long long planes = 8ll * T * N * (s - 1) - (64ll << 20);
     if (planes < 0) planes = 0;
     return waves * ((128ll + bn / 2) * g_pair_overhead_kb + per * pair_kb_cost(bn)) + 256 * (planes / 2100000);
 }
 // The tile's columns that cost least, of equal ones the most
-static int pair_tile(int T, int N, int K, int s, long long *cost_out = nullptr) {
+static int pair_tile(int T, int N, int K, int s, long long *cost_out = nullptr, int pairs = kestrel_sms() / 2) {
     int best = TCP_BN;
     long long best_cost = -1;
     for (int bn = TCP_BN; bn >= PAIR_TILE_MIN; bn -= 16) {
         if (g_pair_tile) bn = g_pair_tile;
-        const long long cost = pair_cost(T, N, K, s, bn);
-        if (cost >= 0 && (best_cost < 0 || cost < best_cost)) best_cost = cost, best = bn;
+        const long long cost = pair_cost(T, N, K, s, bn, pairs);
+        if (cost < 0) break;            // no whole slices, whatever the columns
+        if (best_cost < 0 || cost < best_cost) best_cost = cost, best = bn;
         if (g_pair_tile) break;
     }
     if (cost_out) *cost_out = best_cost;
@@ -985,9 +987,10 @@ static int tc_splits(int T, int N, int K, bool wide) {
         if (!g_pairs || !g_persistent) return 1;
         int best = 1;
         long long best_cost = -1;
+        const int pairs = kestrel_sms() / 2;
         for (int s = 1; s <= 8; ++s) {
             long long cost;
-            pair_tile(T, N, K, s, &cost);
+            pair_tile(T, N, K, s, &cost, pairs);
             if (cost < 0) continue;
             if (best_cost < 0 || cost * 16 < best_cost * 15) { best_cost = cost; best = s; }       // (a slice more is read by the consumer)
         }
@@ -1337,7 +1340,7 @@ KESTREL_API int kestrel_gemm_tc_qkv_prepare(const void *x, const void *w, int T,
         // 512 tokens, one round, 44 against 36)
         const int S = kestrel_gemm_tc_splits(T, N, K);
         long long waves = 0;
-        const long long whole = pair_cost(T, N, K, 1, TCP_BN, &waves);
+        const long long whole = pair_cost(T, N, K, 1, TCP_BN, kestrel_sms() / 2, &waves);
         long long cut = 0;
         pair_tile(T, N, K, S, &cut);
         if (S > 1 && !(waves >= 3 && whole * 10 <= cut * 11)) return 1;
