@@ -418,6 +418,38 @@ KESTREL_API int kestrel_attention_decode_slots(int hd) {
     return kestrel_sms() * (per_sm < 1 ? 1 : per_sm);
 }
 
+template <int HD>
+static int decode_clusters(int slices) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, slices);
+    cfg.blockDim = dim3(AD_THREADS);
+    cfg.dynamicSmemBytes = decode_smem<HD>();
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = slices;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(attention_decode_kernel<HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, attention_decode_kernel<HD, true>, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        return kestrel_attention_decode_slots(HD) / slices;         // no answer: as if any CTAs made a cluster
+    }
+    return n;
+}
+
+// Clusters of `slices` CTAs, 2 to kestrel_attention_decode_cluster_slices(), that the GPU holds at once.  A cluster lies within one GPC, so they
+// are fewer than the CTAs' slots divided by their size.  Asked of the runtime once a head size and number.
+KESTREL_API int kestrel_attention_decode_clusters(int hd, int slices) {
+    if (slices < 2 || slices > AD_MAX_CLUSTER || (hd != 64 && hd != 128)) return 0;
+    static int known[2][AD_MAX_CLUSTER + 1];
+    int &n = known[hd == 128][slices];
+    if (n == 0) n = hd == 64 ? decode_clusters<64>(slices) : decode_clusters<128>(slices);
+    return n;
+}
+
 // Tiles of at most 16 rows (tile_seq / tile_row0): decode tokens.  The key range is cut into
 // `slices` slices of slice_len keys, a multiple of 64 - or a length that follows the longest
 // request at max_kv_ptr on the device - which are merged in ascending order; part_o / part_ml

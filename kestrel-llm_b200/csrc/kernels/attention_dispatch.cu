@@ -329,7 +329,11 @@ KESTREL_API int kestrel_attention(void *planner, long long step_serial, const in
             const int slots = use_decode ? kestrel_attention_decode_slots(hd) : kestrel_attention_mma_slots(hd);
             const int ctas = std::max(1, plan->ns * nkv);
             const int max_kv = std::max(1, plan->small_kv);
-            const int cand = std::max(1, std::min(std::min(slots / ctas, ceil_div(max_kv, use_decode ? 128 : 256)), 32));
+            int cand = std::max(1, std::min(std::min(slots / ctas, ceil_div(max_kv, use_decode ? 128 : 256)), 32));
+            // slices merged by a cluster: as many as let every cluster be resident, which lies within one GPC.  By CTAs alone the last
+            // clusters came in a second wave (8 kv heads, us): 9 requests at 1,500 keys 33.8 in four slices, 23.6 in three; 12 37.9 in
+            // three, 27.6 in two; 12 at 4,000 68.7 and 52.2.
+            while (use_decode && cand > 1 && cand <= kestrel_attention_decode_cluster_slices() && ctas > kestrel_attention_decode_clusters(hd, cand)) --cand;
             slice_len = round_up(ceil_div(max_kv, cand), 128);
             slices = ceil_div(max_kv, slice_len);
             if (slices <= 1) { slices = 1; slice_len = NO_SPLIT; }

@@ -1532,6 +1532,8 @@ def attention_decode_capped(q: torch.Tensor, k_cache: torch.Tensor, v_cache: tor
     in_cluster = lib.kestrel_attention_decode_cluster_slices()
     if cand > in_cluster and keys <= 384 * in_cluster:
         cand = in_cluster                      # few keys: what a slice saves is less than a second kernel that merges them costs
+    while 1 < cand <= in_cluster and n * nkv > lib.kestrel_attention_decode_clusters(hd, cand):
+        cand -= 1                              # a cluster lies within one GPC: the last ones would come in a second wave
     slice_len = (-(-keys // cand) + 63) // 64 * 64
     slices = -(-keys // slice_len)
     # a recorded step fixes the number of slices; without a window their length follows the longest request on the device

@@ -445,6 +445,7 @@ KESTREL_API int kestrel_attention_decode_capped(const void *q, const void *k_cac
 KESTREL_API int kestrel_attention_decode_supported(int hd, int page_size);
 KESTREL_API int kestrel_attention_decode_slots(int hd);
 KESTREL_API int kestrel_attention_decode_cluster_slices(void);
+KESTREL_API int kestrel_attention_decode_clusters(int hd, int slices); /* clusters of so many slices that the GPU holds at once */
 KESTREL_API int kestrel_attention_decode_error(void);
 
 /* ---- attention of a whole step: picks kernels, tiles the step's rows, cuts key ranges ----

@@ -1,0 +1,49 @@
+"""Decode attention whose slices are merged by clusters: as many slices as let every cluster be resident."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("requests", [1, 8, 9, 12, 18, 19])
+@pytest.mark.parametrize("capped", [False, True])
+def test_slices_by_clusters_against_float64(hd, requests, capped):
+    """Sums are float32 of bfloat16 products and P is rounded to bfloat16, and so is the output: 2^-8 of the weights' mean of |value| and 2^-8
+    of the output, beside 2^-12 of the largest for exp2 and float32 sums (a cap of scores by 50 in float32 moves them by less)."""
+    import torch
+    from kestrel_llm_b200.cache.manager import CacheManager
+    from kestrel_llm_b200.csrc import ops
+    from kestrel_llm_b200.engine import Entry, StepBatch
+    from kestrel_llm_b200.parts.base import PagedKVSpec
+    torch.manual_seed(requests)
+    dev, page, nq, nkv = torch.device("cuda:0"), 16, 16, 8
+    contexts = [1100 - 37 * i for i in range(requests)]
+    cache = CacheManager([PagedKVSpec(nkv, hd)], torch.bfloat16, dev, page, sum(c // page + 2 for c in contexts), requests, 2048)
+    cache.shuffle_free(3)
+    entries = []
+    for i, c in enumerate(contexts):
+        cache.admit(i)
+        cache.reserve(i, c)
+        cache.commit(i, c)
+        cache.reserve(i, 1)
+        entries.append(Entry(i, [1]))
+    batch = StepBatch(entries, cache, dev)
+    k, v = cache.k[0].normal_(), cache.v[0].normal_()
+    q = torch.randn(requests, nq * hd, device=dev).to(torch.bfloat16)
+    out = torch.full_like(q, float("nan"))
+    if capped:
+        assert ops.attention_decode_capped(q, k, v, batch, batch.block_table(0), page, out, nq, nkv, hd, 0, hd ** -0.5, 50.0)
+    else:
+        ops.attention(ops.AttentionPlanner(requests, requests), q, k, v, batch, 0, page, out, nq, nkv, hd, 0, hd ** -0.5)
+    assert ops.attention_decode_error() == 0
+    lib = ops.library()
+    for s in range(2, lib.kestrel_attention_decode_cluster_slices() + 1):
+        assert 1 <= lib.kestrel_attention_decode_clusters(hd, s) * s <= lib.kestrel_attention_decode_slots(hd)
+    for i, c in enumerate(contexts):
+        at = torch.tensor(cache.block_table(i, 0), device=dev)
+        rows = [x[at].transpose(0, 1).reshape(nkv, -1, hd)[:, :c + 1].double().repeat_interleave(nq // nkv, 0) for x in (k, v)]
+        s = torch.einsum("hd,hld->hl", q[i].view(nq, hd).double(), rows[0]) * hd ** -0.5
+        p = (50 * torch.tanh(s / 50) if capped else s).softmax(-1)
+        want, size = torch.einsum("hl,hld->hd", p, rows[1]), torch.einsum("hl,hld->hd", p, rows[1].abs())
+        limit = 2.0 ** -8 * (size + want.abs()) + 2.0 ** -12 * want.abs().max()
+        assert ((out[i].view(nq, hd).double() - want).abs() <= limit).all()
