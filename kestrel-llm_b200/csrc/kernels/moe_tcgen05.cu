@@ -7,7 +7,8 @@
 // gathered into one matrix xs [P, K], so that a tile of 128 rows of one expert is a TMA box of
 // xs; the experts' stacked weights [E, rows, K] are ONE 2-D tensor [E * rows, K] whose box starts
 // at row e * rows + n0.  A tile may reach into the next expert's rows of xs and a feature block
-// into the next expert's weight rows: what they compute is never stored.
+// into the next expert's weight rows: what they compute is never stored.  What bounds the products is the operands' way from L2 to the SMs
+// (about 6 TB/s), so a tile fetches the boxes that its own rows are in (moe_tc_box_rows), and its MMA's N are its rows in whole 16s.
 //   GATE_UP  two weight tiles a CTA (gate rows n0.. and up rows ff + n0..) into two accumulators;
 //            epilogue y = min(g, L) sigmoid(1.702 min(g, L)) (clamp(u, -L, L) + 1) as bfloat16
 //   DOWN     one weight tile; epilogue times the pair's routing weight, float32
@@ -29,17 +30,22 @@ __global__ void __launch_bounds__(MT_THREADS)
 moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, void *__restrict__ out,
               const int *__restrict__ offsets, const int *__restrict__ row_pair, const int *__restrict__ tile_expert,
               const int *__restrict__ tile_row0, const int *__restrict__ n_tiles, const float *__restrict__ pair_weight, float limit,
-              int w_rows_per_expert, int up_row_offset, int N, int K, long long ldo, int stages) {
+              int w_rows_per_expert, int up_row_offset, int N, int K, long long ldo, int box_rows, int stages) {
     pdl_launch_dependents();
     pdl_wait();                                       // the tile list is the predecessors' work
-    if ((int)blockIdx.y >= *n_tiles) return;
+    // the three loads together (the lists have an entry for every CTA; surplus ones are read, not used): the first copy needs the tile's
+    // rows, and one load after the other was a third latency in front of it, 1 % of a layer
+    int count, e, t0;
+    asm volatile("ld.global.b32 %0, [%3];\n\tld.global.b32 %1, [%4];\n\tld.global.b32 %2, [%5];"
+                 : "=&r"(count), "=&r"(e), "=&r"(t0) : "l"(n_tiles), "l"(tile_expert + blockIdx.y), "l"(tile_row0 + blockIdx.y) : "memory");
+    if ((int)blockIdx.y >= count) return;
+    const int valid = min(MT_BN, offsets[e + 1] - t0);
+    if (valid <= 0) return;                            // (a list of tiles without rows: N = 0 is no product)
     constexpr int A_TILES = GATE_UP ? 2 : 1;
     constexpr uint32_t A_BYTES = MT_BM * MT_BK * 2;
     constexpr uint32_t B_BYTES = MT_BN * MT_BK * 2;
     constexpr uint32_t STAGE_BYTES = A_TILES * A_BYTES + B_BYTES;
     constexpr uint32_t TMEM_COLS = A_TILES * MT_BN;
-    // M = 128, N = 128, bf16 x bf16 -> f32, both operands K-major
-    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MT_BN >> 3) << 17) | ((uint32_t)(MT_BM >> 4) << 24);
 
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -51,8 +57,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     volatile uint32_t *tmem_slot_ptr = (volatile uint32_t *)(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int e = tile_expert[blockIdx.y], t0 = tile_row0[blockIdx.y];
-    const int valid = min(MT_BN, offsets[e + 1] - t0);
+    // M = 128, N = the tile's rows in whole 16s, bf16 x bf16 -> f32, both operands K-major
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)((valid + 15) / 16 * 2) << 17) | ((uint32_t)(MT_BM >> 4) << 24);
     const int n0 = blockIdx.x * MT_BM;
     const int w_row = e * w_rows_per_expert + n0;
     const int num_kb = (K + MT_BK - 1) / MT_BK;
@@ -82,14 +88,16 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         if (lane == 0) {
             int stage = 0;
             uint32_t phase = 0;
+            const int boxes = (valid + box_rows - 1) / box_rows;
+            const uint32_t box_bytes = (uint32_t)box_rows * MT_BK * 2, bytes = A_TILES * A_BYTES + boxes * box_bytes;
             for (int kb = 0; kb < num_kb; ++kb) {
                 if (kb >= stages && !mbar_wait(empty_bar(stage), phase ^ 1)) { atomicExch(&g_moe_tc_error, 1); break; }
-                mbar_expect_tx(full_bar(stage), STAGE_BYTES);
+                mbar_expect_tx(full_bar(stage), bytes);
                 const uint32_t sa = base + (uint32_t)stage * STAGE_BYTES;
                 const int kc = kb * MT_BK;
                 tma_load_2d(sa, &map_w, full_bar(stage), kc, w_row);
                 if (GATE_UP) tma_load_2d(sa + A_BYTES, &map_w, full_bar(stage), kc, w_row + up_row_offset);
-                tma_load_2d(sa + A_TILES * A_BYTES, &map_x, full_bar(stage), kc, t0);
+                for (int b = 0; b < boxes; ++b) tma_load_2d(sa + A_TILES * A_BYTES + b * box_bytes, &map_x, full_bar(stage), kc, t0 + box_rows * b);
                 if (++stage == stages) { stage = 0; phase ^= 1; }
             }
         }
@@ -105,8 +113,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
 #pragma unroll
                 for (int k4 = 0; k4 < MT_BK / 16; ++k4) {
                     const uint32_t acc = (kb > 0 || k4 > 0) ? 1u : 0u;
-                    tc_mma(tmem, da + 2 * k4, db + 2 * k4, IDESC, acc);
-                    if (GATE_UP) tc_mma(tmem + MT_BN, smem_desc(sa + A_BYTES) + 2 * k4, db + 2 * k4, IDESC, acc);
+                    tc_mma(tmem, da + 2 * k4, db + 2 * k4, idesc, acc);
+                    if (GATE_UP) tc_mma(tmem + MT_BN, smem_desc(sa + A_BYTES) + 2 * k4, db + 2 * k4, idesc, acc);
                 }
                 tc_commit(empty_bar(stage));
                 if (++stage == stages) { stage = 0; phase ^= 1; }
@@ -176,6 +184,12 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     }
 }
 
+// Rows of a box of xs.  Boxes of 32 leave out most rows that are not a tile's own; a full tile is then four copies instead of one, so tiles
+// that are mostly full - more than 160 rows an expert on average, several tiles each - take one of 128.  A layer, us, with 128 -> with 32:
+// 64 experts of 1,024 over rows of 4,096, four a token: 300 tokens (19 rows an expert) 360 -> 325, 1,000 (62) 428 -> 412, 2,048 (128)
+// 600 -> 575; 32 experts of 768 over rows of 2,048, 2,000 tokens (250) 251.5 -> 253.5.
+static int moe_tc_box_rows(int P, int E) { return (long long)P <= 160ll * E ? 32 : MT_BN; }
+
 static int g_moe_tc_smem_kb = 104;
 // shared memory of a CTA's ring of stages in KB (104: two CTAs an SM; 200: one); for measurements
 KESTREL_API void kestrel_moe_tc_set_ring_kb(int kb) { g_moe_tc_smem_kb = kb < 64 ? 64 : (kb > 200 ? 200 : kb); }
@@ -183,7 +197,7 @@ KESTREL_API void kestrel_moe_tc_set_ring_kb(int kb) { g_moe_tc_smem_kb = kb < 64
 template <bool GATE_UP>
 static int moe_tc_launch(const CUtensorMap &mw, const CUtensorMap &mx, void *out, const int *offsets, const int *row_pair,
                          const int *tile_expert, const int *tile_row0, const int *n_tiles, int max_tiles, const float *pair_weight,
-                         float limit, int w_rows_per_expert, int up_off, int N, int K, long long ldo, cudaStream_t stream) {
+                         float limit, int w_rows_per_expert, int up_off, int N, int K, long long ldo, int box_rows, cudaStream_t stream) {
     constexpr int STAGE_BYTES = (GATE_UP ? 2 : 1) * MT_BM * MT_BK * 2 + MT_BN * MT_BK * 2;
     const int num_kb = (K + MT_BK - 1) / MT_BK;
     // two CTAs share an SM (half of its shared memory and at most half of TMEM each): the epilogue of
@@ -201,7 +215,7 @@ static int moe_tc_launch(const CUtensorMap &mw, const CUtensorMap &mx, void *out
     }
     dim3 grid((N + MT_BM - 1) / MT_BM, max_tiles);
     kestrel_launch(moe_tc_kernel<GATE_UP>, grid, dim3(MT_THREADS), smem, stream, mw, mx, out, offsets, row_pair, tile_expert, tile_row0, n_tiles,
-                   pair_weight, limit, w_rows_per_expert, up_off, N, K, ldo, stages);
+                   pair_weight, limit, w_rows_per_expert, up_off, N, K, ldo, box_rows, stages);
     return kestrel_check_launch("moe_tc");
 }
 
@@ -221,10 +235,11 @@ KESTREL_API int kestrel_moe_gate_up_tc(const void *xs, const void *w, const int 
     if (P == 0) return 0;
     KESTREL_REQUIRE(P > 0 && E > 0 && ff > 0 && K > 0 && max_tiles > 0 && max_tiles <= 65535, "moe_gate_up_tc: bad sizes");
     CUtensorMap mw, mx;
+    const int box = moe_tc_box_rows(P, E);
     int rc = kestrel_tensor_map_bf16(&mw, w, (long long)E * 2 * ff, K, K, MT_BM);
-    if (rc == 0) rc = kestrel_tensor_map_bf16(&mx, xs, P, K, K, MT_BN);
+    if (rc == 0) rc = kestrel_tensor_map_bf16(&mx, xs, P, K, K, box);
     if (rc != 0) return rc;
-    return moe_tc_launch<true>(mw, mx, act, offsets, nullptr, tile_expert, tile_row0, n_tiles, max_tiles, nullptr, limit, 2 * ff, ff, ff, K, ff, stream);
+    return moe_tc_launch<true>(mw, mx, act, offsets, nullptr, tile_expert, tile_row0, n_tiles, max_tiles, nullptr, limit, 2 * ff, ff, ff, K, ff, box, stream);
 }
 
 // act [P, ff]; w [E, N, ff]; y [P, N] float32 = (W_down[e] act) * weight of the pair
@@ -234,10 +249,11 @@ KESTREL_API int kestrel_moe_down_tc(const void *act, const void *w, const int *o
     if (P == 0) return 0;
     KESTREL_REQUIRE(P > 0 && E > 0 && ff > 0 && N > 0 && max_tiles > 0 && max_tiles <= 65535, "moe_down_tc: bad sizes");
     CUtensorMap mw, mx;
+    const int box = moe_tc_box_rows(P, E);
     int rc = kestrel_tensor_map_bf16(&mw, w, (long long)E * N, ff, ff, MT_BM);
-    if (rc == 0) rc = kestrel_tensor_map_bf16(&mx, act, P, ff, ff, MT_BN);
+    if (rc == 0) rc = kestrel_tensor_map_bf16(&mx, act, P, ff, ff, box);
     if (rc != 0) return rc;
-    return moe_tc_launch<false>(mw, mx, (void *)y, offsets, row_pair, tile_expert, tile_row0, n_tiles, max_tiles, pair_weight, 0.f, N, 0, N, ff, N, stream);
+    return moe_tc_launch<false>(mw, mx, (void *)y, offsets, row_pair, tile_expert, tile_row0, n_tiles, max_tiles, pair_weight, 0.f, N, 0, N, ff, N, box, stream);
 }
 
 // xs [P, K] rows sorted by expert; w [E, ff, K]; act [P, ff] bfloat16 = activation(W_up[e] xs) of experts without a gate
@@ -246,10 +262,11 @@ KESTREL_API int kestrel_moe_up_act_tc(const void *xs, const void *w, const int *
     if (P == 0) return 0;
     KESTREL_REQUIRE(P > 0 && E > 0 && ff > 0 && K > 0 && max_tiles > 0 && max_tiles <= 65535 && act_kind >= 1 && act_kind <= 4, "moe_up_act_tc: bad sizes");
     CUtensorMap mw, mx;
+    const int box = moe_tc_box_rows(P, E);
     int rc = kestrel_tensor_map_bf16(&mw, w, (long long)E * ff, K, K, MT_BM);
-    if (rc == 0) rc = kestrel_tensor_map_bf16(&mx, xs, P, K, K, MT_BN);
+    if (rc == 0) rc = kestrel_tensor_map_bf16(&mx, xs, P, K, K, box);
     if (rc != 0) return rc;
-    return moe_tc_launch<false>(mw, mx, act, offsets, nullptr, tile_expert, tile_row0, n_tiles, max_tiles, nullptr, (float)act_kind, ff, 0, ff, K, ff, stream);
+    return moe_tc_launch<false>(mw, mx, act, offsets, nullptr, tile_expert, tile_row0, n_tiles, max_tiles, nullptr, (float)act_kind, ff, 0, ff, K, ff, box, stream);
 }
 
 // xs[r, :] = x[row_pair[r] / top, :], 16 bytes a thread and step
