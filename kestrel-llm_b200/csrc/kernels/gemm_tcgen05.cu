@@ -949,10 +949,10 @@ KESTREL_API void kestrel_gemm_tc_set_pair_tile(int columns) { if (columns >= 0 &
 // 700 x 10,304 x 2,048 30.5 -> 29.7, 300 x 4,096 x 4,096 18.9 -> 17.4, 200 x 2,048 x 2,048 11.5 -> 10.1; 2,048 x 4,096 x 4,096 stays at 256 (53).
 #define PAIR_TILE_MIN 128
 static long long pair_kb_cost(int bn) { return bn > 236 ? bn : 236; }
-static long long pair_cost(int T, int N, int K, int s, int bn, int pairs, long long *waves_out = nullptr) {
+static long long pair_cost(int T, int N, int K, int s, int bn, int pairs, long long *waves_out = nullptr, bool narrow = true) {
     const int total_kb = (K + TC_BK - 1) / TC_BK;
     const int per = (total_kb + s - 1) / s;
-    const int least = 4ll * T * N * s <= (2ll << 20) ? 4 : 16;      // (a narrow product's planes, as a router's, cost next to nothing)
+    const int least = narrow && 4ll * T * N * s <= (2ll << 20) ? 4 : 16;      // (a narrow product's planes, as a router's, cost next to nothing)
     if (s > 1 && (per < least || (total_kb + per - 1) / per != s)) return -1;
     const long long tiles = (long long)((N + 255) / 256) * ((T + bn - 1) / bn) * s;
     // (32-bit divisions where they do, and the device asked once: a launch waits for nine of these or more.  A plan took 5.8 us on the host, of
@@ -964,12 +964,12 @@ static long long pair_cost(int T, int N, int K, int s, int bn, int pairs, long l
     return waves * ((128ll + bn / 2) * g_pair_overhead_kb + per * pair_kb_cost(bn)) + 256 * (planes / 2100000);
 }
 // The tile's columns that cost least, of equal ones the most
-static int pair_tile(int T, int N, int K, int s, long long *cost_out = nullptr, int pairs = kestrel_sms() / 2) {
+static int pair_tile(int T, int N, int K, int s, long long *cost_out = nullptr, int pairs = kestrel_sms() / 2, bool narrow = true) {
     int best = TCP_BN;
     long long best_cost = -1;
     for (int bn = TCP_BN; bn >= PAIR_TILE_MIN; bn -= 16) {
         if (g_pair_tile) bn = g_pair_tile;
-        const long long cost = pair_cost(T, N, K, s, bn, pairs);
+        const long long cost = pair_cost(T, N, K, s, bn, pairs, nullptr, narrow);
         if (cost < 0) break;            // no whole slices, whatever the columns
         if (best_cost < 0 || cost < best_cost) best_cost = cost, best = bn;
         if (g_pair_tile) break;
@@ -978,23 +978,27 @@ static int pair_tile(int T, int N, int K, int s, long long *cost_out = nullptr, 
     return best;
 }
 
+// Slices of a many-token product: K is cut only where that fills idle pairs.  `narrow`: small planes may be cut finer.  A product whose epilogue
+// has more to do (the residual's add, the prepare kernel's work) is asked without: it is taken whole wherever only finer slices would gain.
+static int pair_splits(int T, int N, int K, bool narrow) {
+    int best = 1;
+    long long best_cost = -1;
+    const int pairs = kestrel_sms() / 2;
+    for (int s = 1; s <= 8; ++s) {
+        long long cost;
+        pair_tile(T, N, K, s, &cost, pairs, narrow);
+        if (cost < 0) continue;
+        if (best_cost < 0 || cost * 16 < best_cost * 15) { best_cost = cost; best = s; }       // (a slice more is read by the consumer)
+    }
+    return best;
+}
+
 KESTREL_API int kestrel_gemm_tc_splits(int T, int N, int K) { return tc_splits(T, N, K, tc_wide(T, N)); }
 
 static int tc_splits(int T, int N, int K, bool wide) {
     if (T > g_pair_min_tokens) {
-        // many tokens on CTA pairs: tiles of 256 x 256 over the pairs of SMs; K is cut only where
-        // that fills idle pairs
         if (!g_pairs || !g_persistent) return 1;
-        int best = 1;
-        long long best_cost = -1;
-        const int pairs = kestrel_sms() / 2;
-        for (int s = 1; s <= 8; ++s) {
-            long long cost;
-            pair_tile(T, N, K, s, &cost, pairs);
-            if (cost < 0) continue;
-            if (best_cost < 0 || cost * 16 < best_cost * 15) { best_cost = cost; best = s; }       // (a slice more is read by the consumer)
-        }
-        return best;
+        return pair_splits(T, N, K, true);
     }
     int bn = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256;
     long long tiles = (long long)((N + TC_BM - 1) / TC_BM) * ((T + bn - 1) / bn) / (wide ? 2 : 1);
@@ -1280,7 +1284,7 @@ KESTREL_API int kestrel_gemm_tc_add(const void *x, const void *w, float *residua
                                     long long ldw, long long ldo, cudaStream_t stream) {
     if (T == 0) return 0;
     if (T <= g_pair_min_tokens || !g_persistent || !g_pairs || !kestrel_gemm_tc_supported(x, w, T, N, K, ldx, ldw)) return 1;
-    if (kestrel_gemm_tc_splits(T, N, K) > 1) return 1;      // too few output tiles for the CTA pairs: cut along K, as slices
+    if (pair_splits(T, N, K, false) > 1) return 1;      // too few output tiles for the CTA pairs: cut along K, as slices
     CUtensorMap mw, mx;
     int rc = kestrel_tensor_map_bf16(&mw, w, N, K, ldw, TC_BM);
     if (rc) return rc;
@@ -1305,7 +1309,7 @@ KESTREL_API int kestrel_gemm_tc_act_with(const void *x, const void *w, const flo
     if (T == 0) return 0;
     KESTREL_REQUIRE(act >= 1 && act <= 6 && (act == 6) == (act_p != nullptr), "gemm_tc_act: unknown activation %d, or its numbers are missing", act);
     if (T <= g_pair_min_tokens || !g_persistent || !g_pairs || !kestrel_gemm_tc_supported(x, w, T, N, K, ldx, ldw)) return 1;
-    if (kestrel_gemm_tc_splits(T, N, K) > 1) return 1;
+    if (pair_splits(T, N, K, false) > 1) return 1;
     CUtensorMap mw, mx;
     int rc = kestrel_tensor_map_bf16(&mw, w, N, K, ldw, TC_BM);
     if (rc) return rc;
@@ -1338,7 +1342,7 @@ KESTREL_API int kestrel_gemm_tc_qkv_prepare(const void *x, const void *w, int T,
         // or more, so that all but the last epilogue run under the next tile's products (measured:
         // 1,792 tokens 98 us uncut and fused against 117 us in two slices with the prepare kernel;
         // 512 tokens, one round, 44 against 36)
-        const int S = kestrel_gemm_tc_splits(T, N, K);
+        const int S = pair_splits(T, N, K, false);
         long long waves = 0;
         const long long whole = pair_cost(T, N, K, 1, TCP_BN, kestrel_sms() / 2, &waves);
         long long cut = 0;
