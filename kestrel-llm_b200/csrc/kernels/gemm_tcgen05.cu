@@ -1115,7 +1115,7 @@ static int launch_tc_pair(const CUtensorMap &mw, const CUtensorMap &mx, void *ou
         }
     }
     if (max_clusters == 0) return 1;       // not an error: tells the caller to fall back
-    // output tiles: 256 features x 256 tokens; with the operands swapped 128 features x 256 tokens
+    // output tiles: 256 features x bn tokens; with the operands swapped bn / 2 features x 256 tokens
     // (QKV_PREP: 256 features = two heads of 128 x 256 tokens, N = all heads' rows)
     int tiles_n = MODE == TC_SWIGLU_T ? (N + bn / 2 - 1) / (bn / 2) : (N + 255) / 256, tiles_t = MODE == TC_SWIGLU_T ? (T + 255) / 256 : (T + bn - 1) / bn;
     long long tiles_nt = (long long)tiles_n * tiles_t, total = tiles_nt * splits;

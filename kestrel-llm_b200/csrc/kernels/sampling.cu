@@ -14,8 +14,8 @@
 // request's draws do not depend on what else is in the batch.
 //
 // No sort: the k-th largest logit and the top-p cut are found by building the threshold's
-// bit pattern from the top bits down, one counting (or mass) pass per bit (sample_kernel) or
-// per four bits (sample_cluster_kernel).  Entries equal to a
+// bit pattern from the top bits down, one counting (or mass) pass per bit (sample_kernel), or in
+// the bin of values that holds it (sample_cluster_kernel).  Entries equal to a
 // threshold are all kept, where the reference's heap keeps the lower indices; the two differ
 // only on exact ties at a cut.
 #include "common.cuh"
