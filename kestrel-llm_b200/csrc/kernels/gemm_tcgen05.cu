@@ -936,7 +936,7 @@ static bool tc_wide(int T, int N) { return g_wide && T > g_wide_min && T <= 128 
 
 // Cost of a many-token product on CTA pairs with tiles of bn tokens, cut into s slices along K, in 1/256 k-blocks of one
 // pair's time (about 0.42 us at these sizes); -1 where s does not divide the k-blocks into slices
-// of at least sixteen (four where the planes are small: a router's 1,000 x 32 x 2,048 14.0 -> 8.9 us).  A slice costs about g_pair_overhead_kb k-blocks beyond its own (pipeline
+// of at least `least`.  A slice costs about g_pair_overhead_kb k-blocks beyond its own (pipeline
 // fill, the last tile's epilogue); the slices' float32 planes cost their write and their read
 // by the consumer as far as they no longer fit L2 (measured at 3,072 tokens: the down product in
 // three slices 227 + 89 us with its norm, whole 251 + 47).
@@ -945,50 +945,71 @@ static int g_pair_tile = 0;         // columns of a pair's tile; 0: by cost
 KESTREL_API void kestrel_gemm_tc_set_pair_tile(int columns) { if (columns >= 0 && columns <= TCP_BN && columns % 16 == 0) g_pair_tile = columns; }
 // A k-block of a tile of bn columns.  Products of 512 tokens, 4,096 features, K = 12,288 on 32 pairs, us: 63.3 with 256 columns, 60.5 with 240, 58.9 with 224,
 // 59 to 60 below: from 224 columns down the operands that come in, not the products, set the pace, so fewer columns pay where a round of tiles
-// goes, or the last tile is less empty.  us, tiles of 256 -> of the columns chosen: 1,024 x 3,072 x 2,048 18.9 -> 17.6, 1,777 x 3,216 x 2,048 28.7 -> 27.4,
-// 700 x 10,304 x 2,048 30.5 -> 29.7, 300 x 4,096 x 4,096 18.9 -> 17.4, 200 x 2,048 x 2,048 11.5 -> 10.1; 2,048 x 4,096 x 4,096 stays at 256 (53).
+// goes, or the last tile is less empty.  us, tiles of 256 -> of the columns chosen: 1,024 x 3,072 x 2,048 17.7 -> 16.1, 700 x 10,304 x 2,048 29.0 -> 28.0; in two
+// slices 300 x 4,096 x 4,096 17.8 -> 16.1, 200 x 2,048 x 2,048 10.7 -> 9.1; in three 257 x 6,144 x 4,096 24.2 -> 21.6; the same 1,777 x 3,216 x 2,048 (24.4)
+// and 2,048 x 4,096 x 4,096 (52.6); 117 more, drawn, are 0 to 16 % faster.
 #define PAIR_TILE_MIN 128
 static long long pair_kb_cost(int bn) { return bn > 236 ? bn : 236; }
-static long long pair_cost(int T, int N, int K, int s, int bn, int pairs, long long *waves_out = nullptr, bool narrow = true) {
+static long long pair_tiles(int T, int N, int bn) { return (long long)((N + 255) / 256) * ((T + bn - 1) / bn); }
+static long long pair_cost(int T, int N, int K, int s, int bn, int pairs, long long *waves_out = nullptr, int least = 16) {
     const int total_kb = (K + TC_BK - 1) / TC_BK;
     const int per = (total_kb + s - 1) / s;
-    const int least = narrow && 4ll * T * N * s <= (2ll << 20) ? 4 : 16;      // (a narrow product's planes, as a router's, cost next to nothing)
     if (s > 1 && (per < least || (total_kb + per - 1) / per != s)) return -1;
-    const long long tiles = (long long)((N + 255) / 256) * ((T + bn - 1) / bn) * s;
+    const long long tiles = pair_tiles(T, N, bn) * s;
     // (32-bit divisions where they do, and the device asked once: a launch waits for nine of these or more.  A plan took 5.8 us on the host, of
-    // layers whose every launch is a few; now 1.2)
+    // layers whose every launch is a few; now 0.6)
     const long long waves = tiles < (1ll << 30) ? (int)(tiles + pairs - 1) / pairs : (tiles + pairs - 1) / pairs;
     if (waves_out) *waves_out = waves;
     long long planes = 8ll * T * N * (s - 1) - (64ll << 20);
     if (planes < 0) planes = 0;
     return waves * ((128ll + bn / 2) * g_pair_overhead_kb + per * pair_kb_cost(bn)) + 256 * (planes / 2100000);
 }
-// The tile's columns that cost least, of equal ones the most
-static int pair_tile(int T, int N, int K, int s, long long *cost_out = nullptr, int pairs = kestrel_sms() / 2, bool narrow = true) {
+// The tile's columns with which s slices cost least, of equal ones the most
+static int pair_tile(int T, int N, int K, int s, long long *cost_out = nullptr, int pairs = kestrel_sms() / 2) {
+    if (g_pair_tile) {
+        if (cost_out) *cost_out = pair_cost(T, N, K, s, g_pair_tile, pairs, nullptr, 1);
+        return g_pair_tile;
+    }
     int best = TCP_BN;
     long long best_cost = -1;
     for (int bn = TCP_BN; bn >= PAIR_TILE_MIN; bn -= 16) {
-        if (g_pair_tile) bn = g_pair_tile;
-        const long long cost = pair_cost(T, N, K, s, bn, pairs, nullptr, narrow);
+        const long long cost = pair_cost(T, N, K, s, bn, pairs, nullptr, 1);
         if (cost < 0) break;            // no whole slices, whatever the columns
         if (best_cost < 0 || cost < best_cost) best_cost = cost, best = bn;
-        if (g_pair_tile) break;
     }
     if (cost_out) *cost_out = best_cost;
     return best;
 }
+KESTREL_API int kestrel_gemm_tc_pair_columns(int T, int N, int K, int slices) { return pair_tile(T, N, K, slices); }
 
-// Slices of a many-token product: K is cut only where that fills idle pairs.  `narrow`: small planes may be cut finer.  A product whose epilogue
-// has more to do (the residual's add, the prepare kernel's work) is asked without: it is taken whole wherever only finer slices would gain.
-static int pair_splits(int T, int N, int K, bool narrow) {
+// Slices of a many-token product whose planes its consumer adds: K is cut where that fills idle pairs, by the cost of whole tiles.  The slices are
+// not chosen by the cost of the narrower tiles: an accumulator in TMEM cuts its sums off instead of rounding them, so that a sum's
+// distance from float64 grows with the length of its slices (512 x 6,144 x 4,096, 2-norms: 4.4e-6 whole, 2.1e-6 in two, 1.4e-6 in
+// three, 1.0e-6 in four; float32 sums in order 0.6e-6), and what a narrower tile gains is not paid for with that.  512 x 6,144 x 4,096 with the kernel that
+// prepares attention, us: 35.7 in three slices, 32.5 whole.
+static int pair_slices(int T, int N, int K, int pairs) {
     int best = 1;
     long long best_cost = -1;
-    const int pairs = kestrel_sms() / 2;
     for (int s = 1; s <= 8; ++s) {
-        long long cost;
-        pair_tile(T, N, K, s, &cost, pairs, narrow);
+        const long long cost = pair_cost(T, N, K, s, TCP_BN, pairs);
         if (cost < 0) continue;
-        if (best_cost < 0 || cost * 16 < best_cost * 15) { best_cost = cost; best = s; }       // (a slice more is read by the consumer)
+        if (best_cost < 0 || cost < best_cost) best_cost = cost, best = s;
+    }
+    return best;
+}
+// More of them, as short as four k-blocks, where the planes are small (a router's 1,000 x 32 x 2,048 14.0 -> 8.9 us, in eight instead of two)
+#define PAIR_NARROW_BYTES (2ll << 20)
+static int pair_splits(int T, int N, int K) {
+    const int pairs = kestrel_sms() / 2;
+    int best = pair_slices(T, N, K, pairs);
+    if (4ll * T * N * (best + 1) > PAIR_NARROW_BYTES) return best;
+    long long best_cost;
+    pair_tile(T, N, K, best, &best_cost, pairs);
+    for (int s = best + 1; s <= 8 && 4ll * T * N * s <= PAIR_NARROW_BYTES; ++s) {
+        if (pair_cost(T, N, K, s, TCP_BN, pairs, nullptr, 4) < 0) continue;
+        long long cost;
+        pair_tile(T, N, K, s, &cost, pairs);
+        if (cost * 16 < best_cost * 15) best_cost = cost, best = s;       // (a slice more is read by the consumer)
     }
     return best;
 }
@@ -998,7 +1019,7 @@ KESTREL_API int kestrel_gemm_tc_splits(int T, int N, int K) { return tc_splits(T
 static int tc_splits(int T, int N, int K, bool wide) {
     if (T > g_pair_min_tokens) {
         if (!g_pairs || !g_persistent) return 1;
-        return pair_splits(T, N, K, true);
+        return pair_splits(T, N, K);
     }
     int bn = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256;
     long long tiles = (long long)((N + TC_BM - 1) / TC_BM) * ((T + bn - 1) / bn) / (wide ? 2 : 1);
@@ -1284,7 +1305,7 @@ KESTREL_API int kestrel_gemm_tc_add(const void *x, const void *w, float *residua
                                     long long ldw, long long ldo, cudaStream_t stream) {
     if (T == 0) return 0;
     if (T <= g_pair_min_tokens || !g_persistent || !g_pairs || !kestrel_gemm_tc_supported(x, w, T, N, K, ldx, ldw)) return 1;
-    if (pair_splits(T, N, K, false) > 1) return 1;      // too few output tiles for the CTA pairs: cut along K, as slices
+    if (pair_slices(T, N, K, kestrel_sms() / 2) > 1) return 1;      // too few output tiles for the CTA pairs: cut along K, as slices
     CUtensorMap mw, mx;
     int rc = kestrel_tensor_map_bf16(&mw, w, N, K, ldw, TC_BM);
     if (rc) return rc;
@@ -1309,7 +1330,7 @@ KESTREL_API int kestrel_gemm_tc_act_with(const void *x, const void *w, const flo
     if (T == 0) return 0;
     KESTREL_REQUIRE(act >= 1 && act <= 6 && (act == 6) == (act_p != nullptr), "gemm_tc_act: unknown activation %d, or its numbers are missing", act);
     if (T <= g_pair_min_tokens || !g_persistent || !g_pairs || !kestrel_gemm_tc_supported(x, w, T, N, K, ldx, ldw)) return 1;
-    if (pair_splits(T, N, K, false) > 1) return 1;
+    if (pair_slices(T, N, K, kestrel_sms() / 2) > 1) return 1;
     CUtensorMap mw, mx;
     int rc = kestrel_tensor_map_bf16(&mw, w, N, K, ldw, TC_BM);
     if (rc) return rc;
@@ -1320,6 +1341,19 @@ KESTREL_API int kestrel_gemm_tc_act_with(const void *x, const void *w, const flo
     prep.bias = bias;
     prep.act_p = act_p;
     return launch_tc_pair<TC_ACT>(mw, mx, out, T, N, K, ldo, act, 1, 0, cols, stream, prep);
+}
+
+// Whether the q, k, v product of so many tokens is taken whole, with the prepare kernel's work in its epilogue: where its planes would not be
+// cut along K, or cutting gains little while the tiles come in three rounds or more, so that all but the last epilogue run under the next tile's
+// products.  Fused | in slices with the prepare kernel, us, N = 6,144, K = 4,096: 1,792 tokens 74 | 108 in two; 1,000, two rounds, 51 | 60 in two; 512,
+// one round, 33 | 36 in three.  With fewer rounds the product keeps its slices although the fused form is the faster one: they are two and three times
+// closer to float64 (pair_slices).
+KESTREL_API int kestrel_gemm_tc_qkv_whole(int T, int N, int K) {
+    const int pairs = kestrel_sms() / 2, S = pair_slices(T, N, K, pairs);
+    if (S == 1) return 1;
+    long long waves = 0;
+    const long long whole = pair_cost(T, N, K, 1, TCP_BN, pairs, &waves);
+    return waves >= 3 && whole * 10 <= pair_cost(T, N, K, S, TCP_BN, pairs) * 11;
 }
 
 // The q, k, v product of a prompt portion and everything between it and attention in one kernel
@@ -1337,18 +1371,7 @@ KESTREL_API int kestrel_gemm_tc_qkv_prepare(const void *x, const void *w, int T,
     if (!g_qkv_fused || hd != TC_BM || rot != TC_BM || rot_mode != 0 || !inv_freq || nq <= 0 || nkv <= 0 || page_size <= 0) return 1;
     const int N = (nq + 2 * nkv) * TC_BM;
     if (T <= g_pair_min_tokens || !g_persistent || !g_pairs || !kestrel_gemm_tc_supported(x, w, T, N, K, ldx, ldw)) return 1;
-    if (g_qkv_fused < 2) {
-        // uncut where cutting along K gains nothing, or little while the tiles come in three rounds
-        // or more, so that all but the last epilogue run under the next tile's products (measured:
-        // 1,792 tokens 98 us uncut and fused against 117 us in two slices with the prepare kernel;
-        // 512 tokens, one round, 44 against 36)
-        const int S = pair_splits(T, N, K, false);
-        long long waves = 0;
-        const long long whole = pair_cost(T, N, K, 1, TCP_BN, kestrel_sms() / 2, &waves);
-        long long cut = 0;
-        pair_tile(T, N, K, S, &cut);
-        if (S > 1 && !(waves >= 3 && whole * 10 <= cut * 11)) return 1;
-    }
+    if (g_qkv_fused < 2 && !kestrel_gemm_tc_qkv_whole(T, N, K)) return 1;
     if ((((uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) != 0) return 1;
     CUtensorMap mw, mx;
     int rc = kestrel_tensor_map_bf16(&mw, w, N, K, ldw, TC_BM);
