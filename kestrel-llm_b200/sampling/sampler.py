@@ -97,10 +97,12 @@ class Sampler:
         if all(p.greedy for p in params):
             ops.argmax(logits, out)
             return out
+        if not len(params) == len(seeds) == len(indices) == R:          # longer ones are cut; with shorter ones rows would have no options
+            if min(len(params), len(seeds), len(indices)) != R:
+                raise ValueError(f"sample: {R} rows of logits, {len(params)} of options, {len(seeds)} seeds, {len(indices)} indices")
+            params, seeds, indices = params[:R], seeds[:R], indices[:R]
         # rows of temperature, top-p, min-p, uniform number and top-k (int32 bits), one behind the other: a copy of what is contiguous
         # goes out of the pinned buffer itself
-        if not len(params) == len(seeds) == len(indices) == R:
-            raise ValueError(f"sample: {R} rows of logits, {len(params)} of options, {len(seeds)} seeds, {len(indices)} indices")
         slot = self._slot(R)
         host = slot.floats
         host[:R] = [0.0 if p.greedy else p.temperature for p in params]
