@@ -545,12 +545,10 @@ blocks_prepare_kernel(const RbParams p, const RbSource src) {
     }
 }
 
-// The request whose portion is the k-th longest (of equal ones the first; more than RB_ORDERED are taken as they come).  CTAs are placed in the
-// order of their index, so the longest get SMs of their own and the shorter ones share: prepared + scanned in us, in the requests' order and
-// by length, DELTA's 592 and 1,185 tokens 217 and 202, REMOVAL's 117, 233 and 350 119 and 100; four equal requests 261 and 268.
-#define RB_ORDERED 64
+// The request whose portion is the k-th longest, of equal ones the first.  CTAs are placed in the order of their index, so the longest get
+// SMs of their own and the shorter ones share: prepared + scanned in us, in the requests' order and by length, DELTA's 592 and 1,185
+// tokens 218 and 202, REMOVAL's 117, 233 and 350 122 and 100.
 __device__ __forceinline__ int rb_longest(const int *cu, int n, int k) {
-    if (n == 1 || n > RB_ORDERED) return k;
     int found = 0;
     for (int i = threadIdx.x & 31; i < n; i += 32) {
         const int mine = cu[i + 1] - cu[i];
@@ -566,7 +564,7 @@ __device__ __forceinline__ int rb_longest(const int *cu, int n, int k) {
 
 template <int D, int FORM>
 __global__ void __launch_bounds__(32 * RbScan<D, FORM>::WARPS)
-blocks_scan_kernel(const RbParams p, int stages) {
+blocks_scan_kernel(const RbParams p, int stages, bool by_length) {
     using L = RbLayout<D, FORM>;
     constexpr int WARPS = RbScan<D, FORM>::WARPS;
     constexpr int NT = RbScan<D, FORM>::NT;
@@ -588,7 +586,7 @@ blocks_scan_kernel(const RbParams p, int stages) {
     }
     __syncthreads();
     pdl_wait();
-    const int seq = rb_longest(p.cu_seqlens, gridDim.z, blockIdx.z);
+    const int seq = by_length ? rb_longest(p.cu_seqlens, gridDim.z, blockIdx.z) : (int)blockIdx.z;
     const int t0 = p.cu_seqlens[seq], T = p.cu_seqlens[seq + 1] - t0;
     const int n_blocks = (T + RB_B - 1) / RB_B;
     const size_t src_step = (size_t)p.H * STAGE;
@@ -811,8 +809,14 @@ static long long rb_floats(int D, int form) {
     return (long long)RB_B * (rows * (D + 8) + ends * (D + 4)) + D + (long long)rows * RB_MAT;
 }
 
+// Whether the scan takes the requests by length: up to 64 of them, and not equal ones, which stay in their order and would
+// pay for the look (eight of 256 tokens, us: DELTA 203.4 with it, 202.5 without, GATE 74.4 and 73.5).
+KESTREL_API int kestrel_recurrence_blocks_by_length(int T, int nseq, int max_count) {
+    return nseq > 1 && nseq <= 64 && (long long)T < (long long)nseq * max_count ? 1 : 0;
+}
+
 template <int D, int FORM>
-static int rb_launch(const RbParams &p, const RbSource *src, int nseq, int max_count, cudaStream_t stream) {
+static int rb_launch(const RbParams &p, const RbSource *src, int T, int nseq, int max_count, cudaStream_t stream) {
     static_assert(RbLayout<D, FORM>::FLOATS % 4 == 0 && RbLayout<D, FORM>::KW % 4 == 0, "bulk copies move 16 bytes");
     const size_t prep = (size_t)(FORM == RB_GATE ? 3 : FORM == RB_DELTA ? 4 : 5) * RB_B * RbLayout<D, FORM>::END_LD * sizeof(float) + RbLayout<D, FORM>::MATS * RB_MAT * sizeof(double);
     constexpr size_t stage = (size_t)RbLayout<D, FORM>::FLOATS * sizeof(float), fixed = (sizeof(RbScan<D, FORM>) + 127) / 128 * 128;
@@ -832,16 +836,17 @@ static int rb_launch(const RbParams &p, const RbSource *src, int nseq, int max_c
     // as many stages as the CTAs that share an SM leave room for, two at least
     const size_t smem = kestrel_spread_smem((long)grid.x * grid.y * grid.z, 2 * stage + fixed), room = smem - fixed;
     const int stages = (int)(room / stage) < RB_STAGES ? (int)(room / stage) : RB_STAGES;
-    kestrel_launch(blocks_scan_kernel<D, FORM>, grid, dim3(32 * RbScan<D, FORM>::WARPS), smem, stream, p, stages);
+    kestrel_launch(blocks_scan_kernel<D, FORM>, grid, dim3(32 * RbScan<D, FORM>::WARPS), smem, stream, p, stages,
+                   kestrel_recurrence_blocks_by_length(T, nseq, max_count) != 0);
     return kestrel_check_launch("recurrence_blocks");
 }
 
 template <int FORM>
-static int rb_run(const RbParams &p, int nseq, int max_count, cudaStream_t stream, const RbSource *src = nullptr) {
+static int rb_run(const RbParams &p, int T, int nseq, int max_count, cudaStream_t stream, const RbSource *src = nullptr) {
     switch (rb_padded(p.d)) {
-        case 32: return rb_launch<32, FORM>(p, src, nseq, max_count, stream);
-        case 64: return rb_launch<64, FORM>(p, src, nseq, max_count, stream);
-        default: return rb_launch<128, FORM>(p, src, nseq, max_count, stream);
+        case 32: return rb_launch<32, FORM>(p, src, T, nseq, max_count, stream);
+        case 64: return rb_launch<64, FORM>(p, src, T, nseq, max_count, stream);
+        default: return rb_launch<128, FORM>(p, src, T, nseq, max_count, stream);
     }
 }
 
@@ -870,7 +875,7 @@ KESTREL_API int kestrel_recurrence_blocks(const float *r, const float *w, const 
     const RbParams p = {r, w, k, a, b, nullptr, v, (size_t)H * dv, state + state_off, (size_t)state_stride, cu_seqlens, slots, out, scratch, H, H, d, dv};
     const int rc = rb_check(p, T, nseq, max_count, scratch_floats, a ? RB_REMOVAL : RB_GATE);
     if (rc) return rc;
-    return a ? rb_run<RB_REMOVAL>(p, nseq, max_count, stream) : rb_run<RB_GATE>(p, nseq, max_count, stream);
+    return a ? rb_run<RB_REMOVAL>(p, T, nseq, max_count, stream) : rb_run<RB_GATE>(p, T, nseq, max_count, stream);
 }
 
 // kestrel_delta_scan for portions of many tokens
@@ -881,7 +886,7 @@ KESTREL_API int kestrel_delta_blocks(const float *qn, const float *kn, const flo
     const RbParams p = {qn, decay, kn, nullptr, nullptr, beta, v, (size_t)ldv, state, (size_t)state_stride, cu_seqlens, slots, out, scratch, H, G, d, dv};
     const int rc = rb_check(p, T, nseq, max_count, scratch_floats, RB_DELTA);
     if (rc) return rc;
-    return rb_run<RB_DELTA>(p, nseq, max_count, stream);
+    return rb_run<RB_DELTA>(p, T, nseq, max_count, stream);
 }
 
 // Whether vectors of four fetch everything that a kernel with gates reads
@@ -914,7 +919,7 @@ KESTREL_API int kestrel_gated_blocks(const float *x, int S, long long slice_stri
     p.H = H; p.G = H; p.d = d; p.dv = dv;
     const int rc = rb_check(p, T, nseq, max_count, scratch_floats, wz ? RB_REMOVAL : RB_GATE);
     if (rc) return rc;
-    return wz ? rb_run<RB_REMOVAL>(p, nseq, max_count, stream, &src) : rb_run<RB_GATE>(p, nseq, max_count, stream, &src);
+    return wz ? rb_run<RB_REMOVAL>(p, T, nseq, max_count, stream, &src) : rb_run<RB_GATE>(p, T, nseq, max_count, stream, &src);
 }
 
 // delta_gates (a decay per head and channel) and delta_scan in blocks.  act [T, C] = q | k | v after the convolution; beta logits at col_beta of
@@ -938,7 +943,7 @@ KESTREL_API int kestrel_gated_delta_blocks(const float *act, int C, int col_v, c
     p.H = H; p.G = G; p.d = d; p.dv = dv;
     const int rc = rb_check(p, T, nseq, max_count, scratch_floats, RB_DELTA);
     if (rc) return rc;
-    return rb_run<RB_DELTA>(p, nseq, max_count, stream, &src);
+    return rb_run<RB_DELTA>(p, T, nseq, max_count, stream, &src);
 }
 
 // Error word of the bounded waits (0: none, 1: a block's copy).  Synchronises the device and clears the word.

@@ -239,6 +239,7 @@ KESTREL_API int kestrel_delta_blocks(const float *qn, const float *kn, const flo
 KESTREL_API int kestrel_gated_blocks(const float *x, int S, long long slice_stride, int ld, int col_r, int col_k, int col_v, int col_a, const float *bias, const float *bias2, const float *wz, int Sw, long long w_stride, float rate, float *vsum, float *state, long long state_stride, const int *cu_seqlens, const int *slots, float *out, float *scratch, long long scratch_floats, int T, int nseq, int max_count, int H, int d, int dv, kestrel_stream_t stream);
 /* delta_gates with a decay per head and channel (a [T, H d]) and delta_scan the same way */
 KESTREL_API int kestrel_gated_delta_blocks(const float *act, int C, int col_v, const float *y, int Sy, long long y_stride, int ldy, int col_beta, const float *a, int Sa, long long a_stride, const float *A_log, const float *dt_bias, float *state, long long state_stride, const int *cu_seqlens, const int *slots, float *out, float *scratch, long long scratch_floats, int T, int nseq, int max_count, int H, int G, int d, int dv, kestrel_stream_t stream);
+KESTREL_API int kestrel_recurrence_blocks_by_length(int T, int nseq, int max_count);   /* whether a step's requests are scanned longest first */
 KESTREL_API int kestrel_recurrence_blocks_error(void);
 
 /* ---- attention over cached latents (attention_latent.cu) ---- */

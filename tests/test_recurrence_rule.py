@@ -17,3 +17,10 @@ def test_blocks_where_scans_share_the_sms(counts, heads, blocks):
     assert not ops.recurrence_in_blocks(step, torch.bfloat16, 129, heads)
     step.captured = True
     assert not ops.recurrence_in_blocks(step, torch.bfloat16, 128, heads)
+
+
+@pytest.mark.parametrize("counts,by_length", [([500], 0), ([500, 500], 0), ([256] * 8, 0), ([592, 1185], 1), ([1185, 592], 1), ([117, 233, 350], 1), ([16] * 63 + [17], 1),
+                                              ([16] * 64 + [17], 0)])
+def test_only_unequal_requests_are_scanned_by_length(counts, by_length):
+    from kestrel_llm_b200.csrc import ops
+    assert ops.library().kestrel_recurrence_blocks_by_length(sum(counts), len(counts), max(counts)) == by_length
