@@ -24,6 +24,7 @@
 // Every mbarrier wait is bounded; the error word is read by kestrel_attention_decode_error.
 // Formulas as in attention_plain.cu (reference: st.c:10779-10911, st.c:9762-9859).
 #include "attention_params.cuh"
+#include "device_table.h"
 #include "mma_sync.cuh"
 #include "tcgen05.cuh"
 #include <math.h>
@@ -435,19 +436,24 @@ static int decode_clusters(int slices) {
     if (cudaFuncSetAttribute(attention_decode_kernel<HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, attention_decode_kernel<HD, true>, &cfg) != cudaSuccess || n < 1) {
         cudaGetLastError();
-        return kestrel_attention_decode_slots(HD) / slices;         // no answer: as if any CTAs made a cluster
+        return 0;
     }
     return n;
 }
 
-// Clusters of `slices` CTAs, 2 to kestrel_attention_decode_cluster_slices(), that the GPU holds at once.  A cluster lies within one GPC, so they
-// are fewer than the CTAs' slots divided by their size.  Asked of the runtime once a head size and number.
+// Clusters of `slices` CTAs, 2 to kestrel_attention_decode_cluster_slices(), that the current device holds at once.  A cluster lies within one GPC,
+// so they are fewer than the CTAs' slots divided by their size.  Asked of the runtime once a device, head size and number; without an answer as if
+// any CTAs made a cluster.
 KESTREL_API int kestrel_attention_decode_clusters(int hd, int slices) {
     if (slices < 2 || slices > AD_MAX_CLUSTER || (hd != 64 && hd != 128)) return 0;
-    static int known[2][AD_MAX_CLUSTER + 1];
-    int &n = known[hd == 128][slices];
-    if (n == 0) n = hd == 64 ? decode_clusters<64>(slices) : decode_clusters<128>(slices);
-    return n;
+    static DeviceTable<2 * (AD_MAX_CLUSTER + 1)> known;
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        dev = -1;
+    }
+    const int n = known.get(dev, (hd == 128 ? AD_MAX_CLUSTER + 1 : 0) + slices, [&] { return hd == 64 ? decode_clusters<64>(slices) : decode_clusters<128>(slices); });
+    return n > 0 ? n : kestrel_attention_decode_slots(hd) / slices;
 }
 
 // Tiles of at most 16 rows (tile_seq / tile_row0): decode tokens.  The key range is cut into
