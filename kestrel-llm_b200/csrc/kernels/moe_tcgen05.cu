@@ -8,7 +8,7 @@
 // xs; the experts' stacked weights [E, rows, K] are ONE 2-D tensor [E * rows, K] whose box starts
 // at row e * rows + n0.  A tile may reach into the next expert's rows of xs and a feature block
 // into the next expert's weight rows: what they compute is never stored.  What bounds the products is the operands' way from L2 to the SMs
-// (about 6 TB/s), so a tile fetches the boxes that its own rows are in (moe_tc_box_rows), and its MMA's N are its rows in whole 16s.
+// (about 6 TB/s), so a tile fetches the boxes that its own rows are in (kestrel_moe_tc_box_rows), and its MMA's N are its rows in whole 16s.
 //   GATE_UP  two weight tiles a CTA (gate rows n0.. and up rows ff + n0..) into two accumulators;
 //            epilogue y = min(g, L) sigmoid(1.702 min(g, L)) (clamp(u, -L, L) + 1) as bfloat16
 //   DOWN     one weight tile; epilogue times the pair's routing weight, float32
@@ -184,11 +184,12 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     }
 }
 
-// Rows of a box of xs.  Boxes of 32 leave out most rows that are not a tile's own; a full tile is then four copies instead of one, so tiles
-// that are mostly full - more than 160 rows an expert on average, several tiles each - take one of 128.  A layer, us, with 128 -> with 32:
-// 64 experts of 1,024 over rows of 4,096, four a token: 300 tokens (19 rows an expert) 360 -> 325, 1,000 (62) 428 -> 412, 2,048 (128)
-// 600 -> 575; 32 experts of 768 over rows of 2,048, 2,000 tokens (250) 251.5 -> 253.5.
-static int moe_tc_box_rows(int P, int E) { return (long long)P <= 160ll * E ? 32 : MT_BN; }
+// Rows of a box of xs.  Boxes of 32 leave out most rows that are not a tile's own; a full tile is then four copies instead of one.  The two products and
+// what is around them, us, with boxes of 32 | 128, at rows an expert on average: 64 experts of 1,024 over rows of 4,096 294.4 | 295.0 at 19,
+// 321.0 | 322.1 at 38, 404.2 | 404.6 at 88, 439.2 | 436.6 at 112, 574.8 | 574.5 at 160; 128 of 768 over 2,048 306.5 | 307.4 at 62, 419.4 | 417.9 at 125;
+// 32 of 768 over 2,048 97.8 | 98.0 at 62, 111.0 | 110.8 at 88, 129.1 | 128.9 at 125, 210.1 | 208.6 at 250; 8 of 2,048 over 2,048 92.4 | 92.6 at 128,
+// 110.1 | 109.7 at 250.
+KESTREL_API int kestrel_moe_tc_box_rows(int P, int E) { return (long long)P <= 100ll * E ? 32 : MT_BN; }
 
 static int g_moe_tc_smem_kb = 104;
 // shared memory of a CTA's ring of stages in KB (104: two CTAs an SM; 200: one); for measurements
@@ -235,7 +236,7 @@ KESTREL_API int kestrel_moe_gate_up_tc(const void *xs, const void *w, const int 
     if (P == 0) return 0;
     KESTREL_REQUIRE(P > 0 && E > 0 && ff > 0 && K > 0 && max_tiles > 0 && max_tiles <= 65535, "moe_gate_up_tc: bad sizes");
     CUtensorMap mw, mx;
-    const int box = moe_tc_box_rows(P, E);
+    const int box = kestrel_moe_tc_box_rows(P, E);
     int rc = kestrel_tensor_map_bf16(&mw, w, (long long)E * 2 * ff, K, K, MT_BM);
     if (rc == 0) rc = kestrel_tensor_map_bf16(&mx, xs, P, K, K, box);
     if (rc != 0) return rc;
@@ -249,7 +250,7 @@ KESTREL_API int kestrel_moe_down_tc(const void *act, const void *w, const int *o
     if (P == 0) return 0;
     KESTREL_REQUIRE(P > 0 && E > 0 && ff > 0 && N > 0 && max_tiles > 0 && max_tiles <= 65535, "moe_down_tc: bad sizes");
     CUtensorMap mw, mx;
-    const int box = moe_tc_box_rows(P, E);
+    const int box = kestrel_moe_tc_box_rows(P, E);
     int rc = kestrel_tensor_map_bf16(&mw, w, (long long)E * N, ff, ff, MT_BM);
     if (rc == 0) rc = kestrel_tensor_map_bf16(&mx, act, P, ff, ff, box);
     if (rc != 0) return rc;
@@ -262,7 +263,7 @@ KESTREL_API int kestrel_moe_up_act_tc(const void *xs, const void *w, const int *
     if (P == 0) return 0;
     KESTREL_REQUIRE(P > 0 && E > 0 && ff > 0 && K > 0 && max_tiles > 0 && max_tiles <= 65535 && act_kind >= 1 && act_kind <= 4, "moe_up_act_tc: bad sizes");
     CUtensorMap mw, mx;
-    const int box = moe_tc_box_rows(P, E);
+    const int box = kestrel_moe_tc_box_rows(P, E);
     int rc = kestrel_tensor_map_bf16(&mw, w, (long long)E * ff, K, K, MT_BM);
     if (rc == 0) rc = kestrel_tensor_map_bf16(&mx, xs, P, K, K, box);
     if (rc != 0) return rc;
