@@ -57,6 +57,23 @@ def test_which_query_key_value_products_are_taken_whole(N, K, taken):
         assert lib.kestrel_gemm_tc_qkv_whole(T, N, K) == (S == 1 or (rounds >= 3 and whole * 10 <= _cost(T, N, K, S)[0] * 11)), T
 
 
+def test_the_tile_taken_costs_least_with_those_slices():
+    """Of tiles of 128 to 256 columns: a k-block costs as much as its columns, or as 236 where the operands' way in sets the pace."""
+    lib = _lib()
+    chosen = set()
+    for T, N, K in _sizes() + [(1024, 3072, 2048), (300, 4096, 4096), (2048, 4096, 4096)]:
+        S = lib.kestrel_gemm_tc_splits(T, N, K)
+        per, planes = -(-(-(-K // 64)) // S), 256 * (max(0, 8 * T * N * (S - 1) - (64 << 20)) // 2100000)
+
+        def cost(columns):
+            rounds = -(-(-(-N // 256) * -(-T // columns) * S) // (SMS // 2))
+            return rounds * ((128 + columns // 2) * OVERHEAD + per * max(columns, 236)) + planes
+        got = lib.kestrel_gemm_tc_pair_columns(T, N, K, S)
+        assert got == min(range(256, 127, -16), key=lambda c: (cost(c), -c)), (T, N, K, S)
+        chosen.add(got)
+    assert len(chosen) >= 6 and 256 in chosen
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("T,N,K", [(512, 6144, 4096), (2048, 3088, 2048), (1000, 6144, 4096), (300, 4096, 4096)])
 def test_sums_are_as_close_to_float64_as_in_those_slices(T, N, K):
