@@ -247,6 +247,21 @@ KESTREL_API void kestrel_attn_planner_destroy(void *planner) {
 
 KESTREL_API int kestrel_attn_planner_last_launches(void *planner) { return planner ? ((Planner *)planner)->last_launches : 0; }
 
+// Slices into which the key ranges of decode tokens are cut, `ctas` tiles and kv heads that are attended to at once, max_kv keys at most; decode: the
+// TMA decode kernel, else the mma.sync one.  As many as still let every CTA be resident at once (measured at batch 1 to 64, contexts
+// 2,048 to 65,536: a second wave of CTAs costs more than longer slices), at least 128 keys a slice (256 for the mma.sync kernel), at most 32.
+// The decode kernel merges up to 4 slices inside a cluster, more through scratch and a second kernel of a few microseconds (measured, one
+// request: 8,192 keys 21.7 us with 8 slices, 12.2 us with 32).  Slices merged by a cluster, which lies within one GPC: as many as let every
+// cluster be resident.  By CTAs alone the last clusters came in a second wave (8 kv heads, us): 9 requests at 1,500 keys 33.8 in four
+// slices, 23.6 in three; 12 37.9 in three, 27.6 in two; 12 at 4,000 68.7 and 52.2.
+KESTREL_API int kestrel_attention_slices(int decode, int hd, int ctas, int max_kv) {
+    if (ctas < 1 || max_kv < 1) return 1;
+    const int slots = decode ? kestrel_attention_decode_slots(hd) : kestrel_attention_mma_slots(hd);
+    int cand = std::max(1, std::min(std::min(slots / ctas, ceil_div(max_kv, decode ? 128 : 256)), 32));
+    while (decode && cand > 1 && cand <= kestrel_attention_decode_cluster_slices() && ctas > kestrel_attention_decode_clusters(hd, cand)) --cand;
+    return cand;
+}
+
 KESTREL_API int kestrel_attention(void *planner, long long step_serial, const int *batch_host, const int *batch_dev,
                                   const int *layout, int group, int captured, const void *q, const void *k_cache,
                                   const void *v_cache, void *out, int dtype, int cache_pages, int page_size, int nq, int nkv,
@@ -318,22 +333,10 @@ KESTREL_API int kestrel_attention(void *planner, long long step_serial, const in
     if (rc) return rc;
     int launches = 0;
     if (plan->ns > 0) {
-        // Decode tokens.  As many slices as still let every CTA be resident at once (measured at
-        // batch 1 to 64, contexts 2,048 to 65,536: a second wave of CTAs costs more than longer
-        // slices), at least 128 keys a slice (256 for the mma.sync kernel), at most 32.  A window
-        // is short; only full-length key ranges are cut.  The decode kernel merges up to 4 slices
-        // inside a cluster, more through scratch and a second kernel of a few microseconds
-        // (measured, one request: 8,192 keys 21.7 us with 8 slices, 12.2 us with 32).
+        // a window is short; only full-length key ranges are cut
         int slices = 1, slice_len = NO_SPLIT;
         if (window <= 0) {
-            const int slots = use_decode ? kestrel_attention_decode_slots(hd) : kestrel_attention_mma_slots(hd);
-            const int ctas = std::max(1, plan->ns * nkv);
-            const int max_kv = std::max(1, plan->small_kv);
-            int cand = std::max(1, std::min(std::min(slots / ctas, ceil_div(max_kv, use_decode ? 128 : 256)), 32));
-            // slices merged by a cluster: as many as let every cluster be resident, which lies within one GPC.  By CTAs alone the last
-            // clusters came in a second wave (8 kv heads, us): 9 requests at 1,500 keys 33.8 in four slices, 23.6 in three; 12 37.9 in
-            // three, 27.6 in two; 12 at 4,000 68.7 and 52.2.
-            while (use_decode && cand > 1 && cand <= kestrel_attention_decode_cluster_slices() && ctas > kestrel_attention_decode_clusters(hd, cand)) --cand;
+            const int max_kv = std::max(1, plan->small_kv), cand = kestrel_attention_slices(use_decode ? 1 : 0, hd, std::max(1, plan->ns * nkv), max_kv);
             slice_len = round_up(ceil_div(max_kv, cand), 128);
             slices = ceil_div(max_kv, slice_len);
             if (slices <= 1) { slices = 1; slice_len = NO_SPLIT; }

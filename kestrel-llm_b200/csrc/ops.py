@@ -1510,6 +1510,18 @@ def attention_decode_maps(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch
     return True
 
 
+def decode_capped_slices(hd: int, ctas: int, keys: int) -> int:
+    """Slices of `attention_decode_capped`, for ``ctas`` requests and kv heads with ``keys`` keys at most."""
+    lib = library()
+    cand = max(1, min(lib.kestrel_attention_decode_slots(hd) // max(1, ctas), -(-keys // 128), 32))
+    in_cluster = lib.kestrel_attention_decode_cluster_slices()
+    if cand > in_cluster and keys <= 384 * in_cluster:
+        cand = in_cluster                      # few keys: what a slice saves is less than a second kernel that merges them costs
+    while 1 < cand <= in_cluster and ctas > lib.kestrel_attention_decode_clusters(hd, cand):
+        cand -= 1                              # a cluster lies within one GPC: the last ones would come in a second wave
+    return cand
+
+
 def attention_decode_capped(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, batch, block_table: torch.Tensor, page_size: int,
                             out: torch.Tensor, nq: int, nkv: int, hd: int, window: int, scale: float, softcap: float = 0.0) -> bool:
     """A step of one token per request on the TMA decode kernel (head size 64 or 128, at most 16 heads a group), scores bounded by
@@ -1528,12 +1540,7 @@ def attention_decode_capped(q: torch.Tensor, k_cache: torch.Tensor, v_cache: tor
     n = int(batch.num_seqs)
     tile_seq, tile_row0 = _single_token_tiles(n, q.device)
     keys = min(window + 63, max(1, int(batch.max_kv_len))) if window and not batch.captured else window + 63 if window else max(1, int(batch.max_kv_len))
-    cand = max(1, min(lib.kestrel_attention_decode_slots(hd) // max(1, n * nkv), -(-keys // 128), 32))
-    in_cluster = lib.kestrel_attention_decode_cluster_slices()
-    if cand > in_cluster and keys <= 384 * in_cluster:
-        cand = in_cluster                      # few keys: what a slice saves is less than a second kernel that merges them costs
-    while 1 < cand <= in_cluster and n * nkv > lib.kestrel_attention_decode_clusters(hd, cand):
-        cand -= 1                              # a cluster lies within one GPC: the last ones would come in a second wave
+    cand, in_cluster = decode_capped_slices(hd, n * nkv, keys), lib.kestrel_attention_decode_cluster_slices()
     slice_len = (-(-keys // cand) + 63) // 64 * 64
     slices = -(-keys // slice_len)
     # a recorded step fixes the number of slices; without a window their length follows the longest request on the device

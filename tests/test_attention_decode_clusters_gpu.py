@@ -37,8 +37,17 @@ def test_slices_by_clusters_against_float64(hd, requests, capped):
         ops.attention(ops.AttentionPlanner(requests, requests), q, k, v, batch, 0, page, out, nq, nkv, hd, 0, hd ** -0.5)
     assert ops.attention_decode_error() == 0
     lib = ops.library()
-    for s in range(2, lib.kestrel_attention_decode_cluster_slices() + 1):
-        assert 1 <= lib.kestrel_attention_decode_clusters(hd, s) * s <= lib.kestrel_attention_decode_slots(hd)
+    most = lib.kestrel_attention_decode_cluster_slices()
+    held = [lib.kestrel_attention_decode_slots(hd)] * 2 + [lib.kestrel_attention_decode_clusters(hd, s) for s in range(2, most + 1)]
+    assert all(1 <= held[s] * s <= held[0] for s in range(2, most + 1))
+    # no more slices than let every cluster be resident, and one more would not be
+    keys = contexts[0] + 1
+    slices = ops.decode_capped_slices(hd, requests * nkv, keys) if capped else lib.kestrel_attention_slices(1, hd, requests * nkv, keys)
+    if slices <= most:
+        assert slices == 1 or requests * nkv <= held[slices]
+        assert slices == most or requests * nkv > held[slices + 1] or requests * nkv * (slices + 1) > held[0]
+    else:
+        assert not capped and requests * nkv * slices <= held[0]
     for i, c in enumerate(contexts):
         at = torch.tensor(cache.block_table(i, 0), device=dev)
         rows = [x[at].transpose(0, 1).reshape(nkv, -1, hd)[:, :c + 1].double().repeat_interleave(nq // nkv, 0) for x in (k, v)]
