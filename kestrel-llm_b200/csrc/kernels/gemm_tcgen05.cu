@@ -408,9 +408,11 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
 //   * the epilogue warps of both ranks arrive on the leader's accumulator-empty barrier.
 // No TMA load uses cluster multicast.  Persistent over tiles as the one-CTA kernel, two
 // accumulators in TMEM.
-// Launched with programmatic dependent launch as every kernel: barriers, TMEM and, where the
-// weights are a model's, the ring's first fill of them are there when the kernel before ends
-// (layers of two to four such products 7 to 11 us faster, a step of 512 tokens 1,312 -> 1,280).
+// Launched with programmatic dependent launch as every kernel: barriers and TMEM are there when the
+// kernel before ends, and so is the ring's first fill of weights where the caller says that they are
+// a model's (QkvPrepParams::early_w: plain, grouped and gated products; the forms that add to the
+// stream, apply an activation or prepare attention wait with their weights too).  Layers of two to
+// four such products are 7 to 11 us faster, a step of 512 tokens 1,312 -> 1,280.
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -1161,6 +1163,8 @@ static int launch_tc_pair(const CUtensorMap &mw, const CUtensorMap &mx, void *ou
 // at 32B sizes 256 tokens 153 -> 111 us.  It fetches a third more operand bytes per multiply-add,
 // so where both forms need the same rounds of work for ONE token tile (8B sizes up to 256 tokens:
 // 48 tiles in one round against 96 in two) the first form stays ahead, 51.6 against 55.0 us.
+// The rule counts the second form's tiles at 128 features; the launch then takes 64 to 128, those that cost least (swapped_tile), so it
+// costs no more than the rule assumes.
 // g_swiglu_swapped: 0 never, 1 by this rule, 2 always.
 static bool swiglu_swapped_wins(int T, int ff) {
     if (g_swiglu_swapped != 1) return g_swiglu_swapped == 2;
