@@ -6,8 +6,8 @@
 // share the rows, each takes 16 keys of every 64-key tile (mma.sync.m16n8k16, float32 softmax
 // statistics and accumulators in registers) and the four running (max, sum, out) states are
 // merged in warp order at the end; up to 4 slices of a key range are the CTAs of a cluster and
-// merge their results over distributed shared memory, more go through scratch and
-// attention_merge_kernel (clusters of 8 were measured to be placed badly among the kernels of a
+// merge their results over distributed shared memory, where the device holds all clusters at once;
+// others, and more slices, go through scratch and attention_merge_kernel (clusters of 8 were measured to be placed badly among the kernels of a
 // step: twice the time at 4 requests).  What differs further is how the tiles arrive: a fifth warp fetches
 // them with TMA (boxes of one page - or 64 keys of a larger page - by 64 dims, 128-byte swizzle)
 // into a ring of stages and runs ahead of the consumers as far as the ring allows; full/empty
@@ -505,8 +505,8 @@ KESTREL_API int kestrel_attention_decode_capped(const void *q, const void *k_cac
         p.cap_in = 2.0f / softcap;                    // on a score in base-2 units: 2^(v cap_in) = e^(2 s / cap)
         p.cap_out = softcap * 1.4426950408889634f;
     }
-    // up to AD_MAX_CLUSTER slices are merged inside the kernel by a cluster; more go through scratch
-    const bool cluster = slices > 1 && slices <= AD_MAX_CLUSTER;
+    // up to AD_MAX_CLUSTER slices are merged inside the kernel by a cluster, unless the caller gave scratch for them; more go through scratch
+    const bool cluster = slices > 1 && slices <= AD_MAX_CLUSTER && !(part_o && part_ml);
     if (cluster) rc = hd == 64 ? launch_decode<64, true>(mk, mv, p, tiles, cache_pages, stream) : launch_decode<128, true>(mk, mv, p, tiles, cache_pages, stream);
     else rc = hd == 64 ? launch_decode<64, false>(mk, mv, p, tiles, cache_pages, stream) : launch_decode<128, false>(mk, mv, p, tiles, cache_pages, stream);
     if (rc || slices == 1 || cluster) return rc;

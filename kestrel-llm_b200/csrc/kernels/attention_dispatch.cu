@@ -250,16 +250,19 @@ KESTREL_API int kestrel_attn_planner_last_launches(void *planner) { return plann
 // Slices into which the key ranges of decode tokens are cut, `ctas` tiles and kv heads that are attended to at once, max_kv keys at most; decode: the
 // TMA decode kernel, else the mma.sync one.  As many as still let every CTA be resident at once (measured at batch 1 to 64, contexts
 // 2,048 to 65,536: a second wave of CTAs costs more than longer slices), at least 128 keys a slice (256 for the mma.sync kernel), at most 32.
-// The decode kernel merges up to 4 slices inside a cluster, more through scratch and a second kernel of a few microseconds (measured, one
-// request: 8,192 keys 21.7 us with 8 slices, 12.2 us with 32).  Slices merged by a cluster, which lies within one GPC: as many as let every
-// cluster be resident.  By CTAs alone the last clusters came in a second wave (8 kv heads, us): 9 requests at 1,500 keys 33.8 in four
-// slices, 23.6 in three; 12 37.9 in three, 27.6 in two; 12 at 4,000 68.7 and 52.2.
 KESTREL_API int kestrel_attention_slices(int decode, int hd, int ctas, int max_kv) {
     if (ctas < 1 || max_kv < 1) return 1;
     const int slots = decode ? kestrel_attention_decode_slots(hd) : kestrel_attention_mma_slots(hd);
-    int cand = std::max(1, std::min(std::min(slots / ctas, ceil_div(max_kv, decode ? 128 : 256)), 32));
-    while (decode && cand > 1 && cand <= kestrel_attention_decode_cluster_slices() && ctas > kestrel_attention_decode_clusters(hd, cand)) --cand;
-    return cand;
+    return std::max(1, std::min(std::min(slots / ctas, ceil_div(max_kv, decode ? 128 : 256)), 32));
+}
+// Whether the decode kernel merges that many slices inside clusters, else through scratch and a second kernel of a few microseconds (measured,
+// one request: 8,192 keys 21.7 us with 8 slices, 12.2 us with 32): up to 4, where every cluster is resident, which lies within one GPC.
+// Attention of 9, 12 and 12 requests at up to 1,500, 1,500 and 4,000 keys (8 kv heads, us): 25.9, 29.5 and 58 in four, three and three slices by clusters, the
+// last of which come in a second wave; 17.4, 21.0 and 43 in as few slices as let every cluster be resident, by which the outputs are
+// 0.5 to 1.5 % further from float64 (a key that is its warp's new maximum has the probability 1, which needs no rounding, and there are
+// fewer of them); 16.2, 18.9 and 36 in four, three and three through scratch.
+KESTREL_API int kestrel_attention_slices_in_clusters(int hd, int ctas, int slices) {
+    return slices > 1 && slices <= kestrel_attention_decode_cluster_slices() && ctas <= kestrel_attention_decode_clusters(hd, slices) ? 1 : 0;
 }
 
 KESTREL_API int kestrel_attention(void *planner, long long step_serial, const int *batch_host, const int *batch_dev,
@@ -342,9 +345,14 @@ KESTREL_API int kestrel_attention(void *planner, long long step_serial, const in
             if (slices <= 1) { slices = 1; slice_len = NO_SPLIT; }
         }
         float *part_o = nullptr, *part_ml = nullptr;
-        const bool needs_scratch = slices > (use_decode ? kestrel_attention_decode_cluster_slices() : 1);
-        if (needs_scratch) {
+        bool scratch = slices > 1 && !(use_decode && kestrel_attention_slices_in_clusters(hd, std::max(1, plan->ns * nkv), slices));
+        if (scratch) {
             rc = slice_scratch(*pl, T, nq, hd, slices, stream, &part_o, &part_ml);
+            if (rc && use_decode && slices <= kestrel_attention_decode_cluster_slices()) {
+                cudaGetLastError();                 // no memory now: clusters, the last of them in a second wave
+                scratch = false;
+                rc = 0;
+            }
             if (rc) return rc;
         }
         const int *follow = (captured && slices > 1) ? max_kv_dev : nullptr;
@@ -357,7 +365,7 @@ KESTREL_API int kestrel_attention(void *planner, long long step_serial, const in
                                        cu_seqlens, kv_lens, table, W, page_size, T, nq, nkv, hd, window, slices, slice_len, follow,
                                        scale, stream);
         if (rc) return rc;
-        launches += needs_scratch ? 2 : 1;
+        launches += scratch ? 2 : 1;
     }
     if (plan->nl > 0) {
         if (use_tc) {

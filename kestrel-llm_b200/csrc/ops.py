@@ -1517,8 +1517,6 @@ def decode_capped_slices(hd: int, ctas: int, keys: int) -> int:
     in_cluster = lib.kestrel_attention_decode_cluster_slices()
     if cand > in_cluster and keys <= 384 * in_cluster:
         cand = in_cluster                      # few keys: what a slice saves is less than a second kernel that merges them costs
-    while 1 < cand <= in_cluster and ctas > lib.kestrel_attention_decode_clusters(hd, cand):
-        cand -= 1                              # a cluster lies within one GPC: the last ones would come in a second wave
     return cand
 
 
@@ -1540,12 +1538,13 @@ def attention_decode_capped(q: torch.Tensor, k_cache: torch.Tensor, v_cache: tor
     n = int(batch.num_seqs)
     tile_seq, tile_row0 = _single_token_tiles(n, q.device)
     keys = min(window + 63, max(1, int(batch.max_kv_len))) if window and not batch.captured else window + 63 if window else max(1, int(batch.max_kv_len))
-    cand, in_cluster = decode_capped_slices(hd, n * nkv, keys), lib.kestrel_attention_decode_cluster_slices()
-    slice_len = (-(-keys // cand) + 63) // 64 * 64
+    slice_len = (-(-keys // decode_capped_slices(hd, n * nkv, keys)) + 63) // 64 * 64
     slices = -(-keys // slice_len)
     # a recorded step fixes the number of slices; without a window their length follows the longest request on the device
     follow = batch.device_buffer.data_ptr() + 4 * int(batch.layout[_cdecl.constants()["KB_O_MAX_KV"]]) if batch.captured and not window else None
-    part = torch.empty((T * nq * slices * (hd + 2),), dtype=torch.float32, device=q.device) if slices > in_cluster else None
+    part = None
+    if slices > 1 and not lib.kestrel_attention_slices_in_clusters(hd, n * nkv, slices):
+        part = torch.empty((T * nq * slices * (hd + 2),), dtype=torch.float32, device=q.device)
     _check(lib.kestrel_attention_decode_capped(
         q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), _p(part), part.data_ptr() + 4 * T * nq * slices * hd if part is not None else None,
         tile_seq.data_ptr(), tile_row0.data_ptr(), n, batch.cu_seqlens.data_ptr(), batch.kv_lens.data_ptr(), block_table.data_ptr(), block_table.shape[1],

@@ -453,6 +453,7 @@ KESTREL_API int kestrel_attention_decode_cluster_slices(void);
 KESTREL_API int kestrel_attention_decode_clusters(int hd, int slices); /* clusters of so many slices that the GPU holds at once */
 KESTREL_API int kestrel_attention_decode_error(void);
 KESTREL_API int kestrel_attention_slices(int decode, int hd, int ctas, int max_kv); /* slices of the key ranges of decode tokens: ctas tiles and kv heads at once, on the decode kernel or the mma.sync one */
+KESTREL_API int kestrel_attention_slices_in_clusters(int hd, int ctas, int slices); /* whether the decode kernel merges that many inside clusters */
 
 /* ---- attention of a whole step: picks kernels, tiles the step's rows, cuts key ranges ----
  * A planner belongs to the mixers of one model.  It keeps the tile lists of the current step on

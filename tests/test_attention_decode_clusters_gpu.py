@@ -1,4 +1,4 @@
-"""Decode attention whose slices are merged by clusters: as many slices as let every cluster be resident."""
+"""Decode attention whose slices are merged by clusters where every one is resident, else through scratch."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -40,14 +40,12 @@ def test_slices_by_clusters_against_float64(hd, requests, capped):
     most = lib.kestrel_attention_decode_cluster_slices()
     held = [lib.kestrel_attention_decode_slots(hd)] * 2 + [lib.kestrel_attention_decode_clusters(hd, s) for s in range(2, most + 1)]
     assert all(1 <= held[s] * s <= held[0] for s in range(2, most + 1))
-    # no more slices than let every cluster be resident, and one more would not be
-    keys = contexts[0] + 1
-    slices = ops.decode_capped_slices(hd, requests * nkv, keys) if capped else lib.kestrel_attention_slices(1, hd, requests * nkv, keys)
-    if slices <= most:
-        assert slices == 1 or requests * nkv <= held[slices]
-        assert slices == most or requests * nkv > held[slices + 1] or requests * nkv * (slices + 1) > held[0]
-    else:
-        assert not capped and requests * nkv * slices <= held[0]
+    # as many slices as let every CTA be resident, and clusters of them only where every one is
+    ctas, keys = requests * nkv, contexts[0] + 1
+    slices = ops.decode_capped_slices(hd, ctas, keys) if capped else lib.kestrel_attention_slices(1, hd, ctas, keys)
+    assert slices == max(1, min(held[0] // ctas, -(-keys // 128), most if capped else 32))
+    for s in range(1, most + 2):
+        assert lib.kestrel_attention_slices_in_clusters(hd, ctas, s) == (1 < s <= most and ctas <= held[s])
     for i, c in enumerate(contexts):
         at = torch.tensor(cache.block_table(i, 0), device=dev)
         rows = [x[at].transpose(0, 1).reshape(nkv, -1, hd)[:, :c + 1].double().repeat_interleave(nq // nkv, 0) for x in (k, v)]
