@@ -353,9 +353,9 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                     float ms = ld_cluster_f32(finml_s + 8 * r, s);
                     if (ms == -INFINITY) continue;
                     float f = exp2f(ms - M);
-                    L += ld_cluster_f32(finml_s + 8 * r + 4, s) * f;
+                    L = fmaf(ld_cluster_f32(finml_s + 8 * r + 4, s), f, L);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[j] += ld_cluster_f32(fin_s + (r * HD + d0 + j) * 4, s) * f;
+                    for (int j = 0; j < 8; ++j) acc[j] = fmaf(ld_cluster_f32(fin_s + (r * HD + d0 + j) * 4, s), f, acc[j]);
                 }
                 int row = row0 + r;
                 size_t qrow = (size_t)(tok_begin + row / G) * p.nq + kvh * G + row % G;
@@ -510,7 +510,8 @@ KESTREL_API int kestrel_attention_decode_capped(const void *q, const void *k_cac
     if (cluster) rc = hd == 64 ? launch_decode<64, true>(mk, mv, p, tiles, cache_pages, stream) : launch_decode<128, true>(mk, mv, p, tiles, cache_pages, stream);
     else rc = hd == 64 ? launch_decode<64, false>(mk, mv, p, tiles, cache_pages, stream) : launch_decode<128, false>(mk, mv, p, tiles, cache_pages, stream);
     if (rc || slices == 1 || cluster) return rc;
-    return kestrel_attention_merge(part_o, part_ml, out, tile_seq, tile_row0, tiles, 16, cu_seqlens, slices, hd, nq, nkv, nullptr, stream);
+    // as many slices as clusters take give the same bits either way
+    return attention_merge_gated(part_o, part_ml, out, tile_seq, tile_row0, tiles, 16, cu_seqlens, 0, slices, hd, nq, nkv, nullptr, nullptr, stream, slices <= AD_MAX_CLUSTER);
 }
 
 // Differential attention of decode tokens on the same kernel: q [T, 2 nq, 2 dim] padded rows (attention_prepare_ex.cu, `maps`) over

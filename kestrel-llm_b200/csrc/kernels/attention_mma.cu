@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(AMG_THREADS)
 attention_merge_kernel(const float *__restrict__ part_o, const float *__restrict__ part_ml,
                        __nv_bfloat16 *__restrict__ out, const int *__restrict__ tile_seq,
                        const int *__restrict__ tile_row0, const int *__restrict__ cu_seqlens,
-                       int slices, int hd, int nq, int nkv, const float *__restrict__ sink, const float *__restrict__ gate, int nseq) {
+                       int slices, int hd, int nq, int nkv, const float *__restrict__ sink, const float *__restrict__ gate, int nseq, bool contracted) {
     pdl_launch_dependents();
     __shared__ float f_s[AMG_MAX_SLICES], lf_s[AMG_MAX_SLICES];
     __shared__ float red[AMG_THREADS / 32];
@@ -417,12 +417,12 @@ attention_merge_kernel(const float *__restrict__ part_o, const float *__restrict
         float2 v = *reinterpret_cast<const float2 *>(ml + 2 * s);
         float f = v.x == -INFINITY ? 0.f : exp2f(v.x - M);
         f_s[s] = f;
-        lf_s[s] = f != 0.f ? v.y * f : 0.f;
+        lf_s[s] = f == 0.f ? 0.f : contracted ? v.y : v.y * f;
     }
     __syncthreads();
-    if (tid == 0) {             // the sum of the weights in ascending order, as the rows' own sums
+    if (tid == 0) {             // the sum of the weights in ascending order, as the rows' own sums (contracted: as attention_decode.cu's clusters sum them)
         float L = 0.f;
-        for (int s = 0; s < slices; ++s) L += lf_s[s];
+        for (int s = 0; s < slices; ++s) L = contracted ? fmaf(lf_s[s], f_s[s], L) : L + lf_s[s];
         // a softmax with one more term exp(sink[head]) that carries no value: entered once, here, against the rows' maximum
         if (sink) L += exp2f(sink[qrow % nq] * 1.4426950408889634f - M);
         inv_l = L;
@@ -528,17 +528,17 @@ static int launch_attention(const AttnParams &p, int tiles, cudaStream_t stream)
 // (float32 [T, nq], or null) before its one rounding; also used by attention_decode.cu, attention_tc.cu and attention_rows_tc.cu
 int attention_merge_gated(const float *part_o, const float *part_ml, void *out, const int *tile_seq, const int *tile_row0, int tiles,
                           int rows_per_tile, const int *cu_seqlens, int nseq, int slices, int hd, int nq, int nkv, const float *sink, const float *gate,
-                          cudaStream_t stream) {
+                          cudaStream_t stream, bool contracted) {
     KESTREL_REQUIRE(rows_per_tile >= 1 && rows_per_tile <= 65535, "attention_merge: tiles of %d rows", rows_per_tile);
     KESTREL_REQUIRE(slices >= 1 && slices <= AMG_MAX_SLICES, "attention_merge: %d slices; the kernel merges up to %d", slices, AMG_MAX_SLICES);
     KESTREL_REQUIRE(tiles <= 0x7fffffff && nkv <= 65535, "attention_merge: grid too large");
-    if (rows_per_tile > 16 && slices <= AMW_MAX_SLICES && hd % 4 == 0 && hd <= 128 && (((uintptr_t)part_o | (uintptr_t)out) & 15) == 0) {
+    if (rows_per_tile > 16 && !contracted && slices <= AMW_MAX_SLICES && hd % 4 == 0 && hd <= 128 && (((uintptr_t)part_o | (uintptr_t)out) & 15) == 0) {
         kestrel_launch(attention_merge_rows_kernel, dim3(tiles, nkv, (rows_per_tile + 7) / 8), dim3(256), 0, stream, part_o, part_ml,
                        (__nv_bfloat16 *)out, tile_seq, tile_row0, cu_seqlens, slices, hd, nq, nkv, rows_per_tile, sink, gate, nseq);
         return kestrel_check_launch("attention_merge");
     }
     kestrel_launch(attention_merge_kernel, dim3(tiles, nkv, rows_per_tile), dim3(AMG_THREADS), 0, stream, part_o, part_ml, (__nv_bfloat16 *)out,
-                   tile_seq, tile_row0, cu_seqlens, slices, hd, nq, nkv, sink, gate, nseq);
+                   tile_seq, tile_row0, cu_seqlens, slices, hd, nq, nkv, sink, gate, nseq, contracted);
     return kestrel_check_launch("attention_merge");
 }
 

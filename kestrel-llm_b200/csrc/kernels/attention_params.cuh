@@ -78,4 +78,4 @@ __device__ __forceinline__ void attn_find_tile(const int *cu_seqlens, int nseq, 
 // a factor per (token, head) on the outputs; tile_seq null: the tiles of nseq requests, found from cu_seqlens
 int attention_merge_gated(const float *part_o, const float *part_ml, void *out, const int *tile_seq, const int *tile_row0, int tiles,
                           int rows_per_tile, const int *cu_seqlens, int nseq, int slices, int hd, int nq, int nkv, const float *sink, const float *gate,
-                          cudaStream_t stream);
+                          cudaStream_t stream, bool contracted = false);

@@ -54,3 +54,38 @@ def test_slices_by_clusters_against_float64(hd, requests, capped):
         want, size = torch.einsum("hl,hld->hd", p, rows[1]), torch.einsum("hl,hld->hd", p, rows[1].abs())
         limit = 2.0 ** -8 * (size + want.abs()) + 2.0 ** -12 * want.abs().max()
         assert ((out[i].view(nq, hd).double() - want).abs() <= limit).all()
+
+
+@pytest.mark.parametrize("hd,nq,nkv", [(64, 16, 8), (128, 24, 3), (128, 32, 2)])
+@pytest.mark.parametrize("slices", [2, 3, 4])
+def test_scratch_and_clusters_give_the_same_bits(hd, nq, nkv, slices):
+    """Requests of one to 1,100 keys, so that some have fewer keys than slices reach: the same parts merged in the same order."""
+    import torch
+    from kestrel_llm_b200.cache.manager import CacheManager
+    from kestrel_llm_b200.csrc import ops
+    from kestrel_llm_b200.engine import Entry, StepBatch
+    from kestrel_llm_b200.parts.base import PagedKVSpec
+    torch.manual_seed(slices)
+    dev, page, contexts = torch.device("cuda:0"), 16, [1099, 0, 63, 700, 256, 1000]
+    cache = CacheManager([PagedKVSpec(nkv, hd)], torch.bfloat16, dev, page, sum(c // page + 2 for c in contexts), len(contexts), 2048)
+    entries = []
+    for i, c in enumerate(contexts):
+        cache.admit(i)
+        cache.reserve(i, c)
+        cache.commit(i, c)
+        cache.reserve(i, 1)
+        entries.append(Entry(i, [1]))
+    batch, n = StepBatch(entries, cache, dev), len(contexts)
+    k, v = cache.k[0].normal_(), cache.v[0].normal_()
+    q = torch.randn(n, nq * hd, device=dev).to(torch.bfloat16)
+    table, rows, first = batch.block_table(0), torch.arange(n, dtype=torch.int32, device=dev), torch.zeros(n, dtype=torch.int32, device=dev)
+    got = []
+    for scratch in (False, True):
+        out = torch.full_like(q, float("nan"))
+        part = torch.full((n * nq * slices * (hd + 2),), float("nan"), device=dev) if scratch else None
+        ops._check(ops.library().kestrel_attention_decode(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), part.data_ptr() if scratch else None, part.data_ptr() + 4 * n * nq * slices * hd if scratch else None,
+            rows.data_ptr(), first.data_ptr(), n, batch.cu_seqlens.data_ptr(), batch.kv_lens.data_ptr(), table.data_ptr(), table.shape[1], table.stride(0), page,
+            int(k.shape[0]), n, nq, nkv, hd, 0, slices, -(-1100 // (64 * slices)) * 64, None, hd ** -0.5, ops._stream()))
+        got.append(out)
+    assert ops.attention_decode_error() == 0 and torch.isfinite(got[0].float()).all() and torch.equal(got[0], got[1])
